@@ -677,10 +677,7 @@ __device__ __noinline__ void me_run(Smem &, int g, int gt, const uint8_t *ref, i
 
 // v2 intra reference samples (reference src/predict.c:480-520): above-right
 // and below-left are replicated.  S.ra[0] / S.rl[0] hold the corner.
-// For leaves up to IPRED_MAX the predictions of the intra modes in `mode_mask`
-// (DC excepted: it is the constant S.dc) are also evaluated once into
-// S.ipred, so residual jobs read them instead of re-deriving every sample.
-__device__ __noinline__ void build_refs(Smem &, const Leaf L, uint32_t mode_mask) {
+__device__ __noinline__ void build_refs(const Leaf L) {
     Smem &S = smem_state();
     const int N = L.cu;
     const bool ha = L.py > 0, hl = L.px > 0;
@@ -704,237 +701,149 @@ __device__ __noinline__ void build_refs(Smem &, const Leaf L, uint32_t mode_mask
         S.rl[0] = (uint8_t)tl;
     }
     SYNC();
-    PROBE_T0();
-    const uint32_t fill = N <= IPRED_MAX ? (mode_mask & ~2u & ((1u << 18) - 1)) : 0u;
     if (threadIdx.x < 32) {
         // DC value (reference src/predict.c:140-161): samples 1..N of each run.
         int sum = 0;
         for (int i = threadIdx.x; i < N; i += 32) sum += S.ra[i + 2] + S.rl[i + 2];
         sum = __reduce_add_sync(0xffffffffu, sum);
-        if (threadIdx.x == 0) { S.dc = (sum + N) / (2 * N); S.dc_u8 = (uint8_t)S.dc; S.ipred_ok = fill; }
-    } else if (fill) {
-        // the nm modes of `fill`, N*N samples each: sample i belongs to the
-        // (i >> 2lg)-th set bit of fill
-        const int lg = __ffs(N) - 1, npx = N * N, nm = __popc(fill);
-        // every mode but DC (the medium and slow presets' set): the k-th
-        // mode is k, or k + 1 past DC, with no bit search
-        const bool all = fill == ((1u << 18) - 1) - 2u;
-        for (int i = threadIdx.x - 32; i < nm * npx; i += NT - 32) {
-            const int k = i >> (2 * lg);
-            const int m = all ? k + (k != 0) : __fns(fill, 0, k + 1), p = i & (npx - 1);
-            S.ipred[m][p] = (uint8_t)intra_at(S.ra + 1, S.rl + 1, N, m, 0, p & (N - 1), p >> lg);
-        }
+        if (threadIdx.x == 0) S.dc = (sum + N) / (2 * N);
     }
     SYNC();
-    PROBE(63);
 }
 
-// An intra sample the leaf's prediction cache does not hold (leaves above
-// IPRED_MAX): out of line, so the residual jobs' hot loops stay small.
-__device__ __noinline__ int intra_sample(int cu, int m, int dc, int x, int y) {
-    const Smem &S = smem_state();
-    return intra_at(S.ra + 1, S.rl + 1, cu, m, dc, x, y);
-}
-
-// Where a candidate's luma prediction comes from: sample (x, y) of a cu x cu
-// leaf is src[(y * cu + x) & mask] (an inter prediction slot or a cached
-// intra mode; the DC mode is a one-byte source under mask 0), or src is null
-// for an intra mode the leaf's cache does not hold (intra_sample).  Resolved
-// once per residual job, so the job's sample loops are plain loads.
-struct PredSrc {
-    const uint8_t *src;
-    int mask;
-};
-__device__ __forceinline__ PredSrc pred_src(const Smem &S, int slot) {
-    if (slot < NPRED) return {S.pred[slot], 0xFFFF};
-    const int m = slot - K_INTRA;
-    if (m == 1) return {&S.dc_u8, 0};
-    if (m < 18 && ((S.ipred_ok >> m) & 1u)) return {S.ipred[m], 0xFFFF};
-    return {nullptr, 0};
-}
-
-__device__ __forceinline__ int lpred(const Smem &S, int cu, int slot, int dc, int x, int y) {
-    if (slot < NPRED) return S.pred[slot][y * cu + x];
-    const int m = slot - K_INTRA;
-    if (m == 1) return dc;
-    if (m < 18 && ((S.ipred_ok >> m) & 1u)) return S.ipred[m][y * cu + x];
-    return intra_sample(cu, m, dc, x, y);
-}
-
-// Luma residual jobs, 8x8 TUs: one octet per (candidate, TU).
-__device__ __noinline__ void luma_jobs8(Smem &, const Leaf L, const int *cl, int ncl, const QuantParams &,
-                           bool accum, bool wrec, int16_t *emit, int woff = 0) {
-    Smem &S = smem_state();
-    const QuantParams &qp = S.qparam[0];
-    const int cu = L.cu, ntu = cu >> 3, ntu2 = ntu * ntu, J = ncl * ntu2;
-    const int lt = lg2i(ntu);   // TU counts are powers of two: shifts, not divisions
-    if (threadIdx.x == 0) OPCOUNT(2, J);
-    const int hw = threadIdx.x >> 5, lane = threadIdx.x & 31, oct = lane >> 3, l8 = lane & 7;
-    const int warp = (hw + NW - woff % NW) % NW;   // job rank of this warp
-    int *scr = S.scratch[hw] + oct * 72;
-    const int dc = S.dc;
-    for (int base = 0; base < J; base += NW * 4) {
-        PROBE_T0();
-        const int j = base + warp * 4 + oct;
-        const bool act = j < J;
-        const int jj = act ? j : 0;
-        const int k = jj >> (2 * lt), t = jj & (ntu2 - 1), ty = t >> lt, tx = t & (ntu - 1);
-        const int slot = cl[k];
-        const PredSrc ps = pred_src(S, slot);
-        int res[8], pr[8];
-        const int r = ty * 8 + l8;
-        if (ps.src) {
-#pragma unroll
-            for (int n = 0; n < 8; ++n) pr[n] = ps.src[(r * cu + tx * 8 + n) & ps.mask];
-        } else {
-#pragma unroll
-            for (int n = 0; n < 8; ++n) pr[n] = intra_sample(cu, slot - K_INTRA, dc, tx * 8 + n, r);
-        }
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-            res[n] = clampi((int)S.cur_y[(L.ly + r) * 64 + L.lx + tx * 8 + n] - pr[n], -512, 511);
-        int qc[8], rc[8];
-        PROBE(60);
-        const int bits = tu8_code(l8, res, scr, qp, qc, rc);
-        PROBE(61);
-        int sse = 0;
-        const int x = tx * 8 + l8;
-        if (ps.src) {
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) pr[kk] = ps.src[((ty * 8 + kk) * cu + x) & ps.mask];
-        } else {
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) pr[kk] = intra_sample(cu, slot - K_INTRA, dc, x, ty * 8 + kk);
-        }
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            const int y = ty * 8 + kk;
-            const int v = clampi(pr[kk] + rc[kk], 0, 255);
-            const int d = (int)S.cur_y[(L.ly + y) * 64 + L.lx + x] - v;
-            sse += d * d;
-            if (act && wrec) RY(S, L.lx + x, L.ly + y) = (uint8_t)v;
-            if (act && accum && cu <= 16) S.crec[slot][0][y * cu + x] = (uint8_t)v;
-            if (act && emit) emit[t * 64 + kk * 8 + l8] = (int16_t)qc[kk];
-        }
-        sse = oct_sum(sse);
-        if (act && accum && l8 == 0) {
-            atomicAdd(&S.acc_sse[slot][0], sse);
-            atomicAdd(&S.acc_bits[slot][0], bits);
-        }
-        PROBE(62);
+// Intra prediction samples (x, y) and (x + 1, y) of an N x N leaf in the low
+// two bytes (the per-sample form is intra_at; reference
+// src/predict.c:117-340).
+__device__ __forceinline__ uint32_t intra2(const Smem &S, int N, int mode, int x, int y) {
+    const uint8_t *ra = S.ra + 1, *rl = S.rl + 1;
+    if (mode == 0) {
+        const int sh = __ffs(N), l = rl[y + 1], c = ra[0];
+        const int v0 = (ra[x + 1] * (N - 1 - y) + l * (N - 1 - x) + c * (x + y) + N) >> sh;
+        const int v1 = (ra[x + 2] * (N - 1 - y) + l * (N - 2 - x) + c * (x + 1 + y) + N) >> sh;
+        return (uint32_t)mini(v0, 255) | (uint32_t)mini(v1, 255) << 8;
     }
+    if (mode == 1 || mode > 17) return (uint32_t)S.dc * 0x101u;
+    const bool vert = mode < 9;
+    const uint8_t *pri = vert ? ra : rl, *sec = vert ? rl : ra;
+    const int disp = c_ang_disp[mode];
+    const int pos0 = vert ? (x << 5) + y * disp : (y << 5) + x * disp;
+    uint32_t v = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int p = e ? pos0 + (vert ? 32 : disp) : pos0;
+        const uint8_t *src = p >= 0 ? pri : sec;    // a negative position only occurs for disp < 0
+        const int q = absi(p), i0 = (q >> 5) + 1, fr = q & 31;
+        const int a = src[mini(i0, 2 * N)], b = src[mini(i0 + 1, 2 * N)];
+        v |= (uint32_t)(a + (((b - a) * fr + 16) >> 5)) << (8 * e);
+    }
+    return v;
 }
 
-// Luma residual jobs, 4x4 TUs inside each 8x8 TU: one quad per
-// (candidate, TU, sub-block); the sub-block-0 quad adds the outer flag bit
-// (reference src/encoder.c:508-535).
-__device__ __noinline__ void luma_jobs4(Smem &, const Leaf L, const int *cl, int ncl, const QuantParams &,
-                           bool accum, bool wrec, int16_t *emit, int woff = 0) {
+// Prediction samples (x, y) and (x + 1, y), x even, of a candidate slot.
+__device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int slot, int x, int y) {
+    if (slot < NPRED) return *(const uint16_t *)(S.pred[slot] + y * cu + x);
+    return intra2(S, cu, slot - K_INTRA, x, y);
+}
+
+// Luma residual coding of the listed candidates: one warp per (candidate,
+// 8x8 area), with one 8x8 TU, four 4x4 TUs or both (reference
+// src/encoder.c:476-560; the four-TU form has an outer flag bit).  `accum`
+// adds distortion and bits to the slot's sums and keeps the reconstruction of
+// leaves up to 16x16; `wrec` writes the reconstruction, `emit` the levels in
+// syntax order.  `woff` rotates the warps the areas start on.
+//
+// Bound: issue slots (150 instructions per area and type, four warps a
+// scheduler); an area on a warp keeps the chain of a leaf with fewer areas
+// than warps short, and both types share one load of the samples and, for
+// intra modes, one evaluation of the prediction, so no prediction buffers of
+// the 18 modes exist.
+__device__ __noinline__ void luma_areas(const Leaf L, const int *cl, int ncl, bool accum, bool wrec, int16_t *emit,
+                                        int woff) {
     Smem &S = smem_state();
-    const QuantParams &qp = S.qparam[0];
-    const int cu = L.cu, ntu = cu >> 3, ntu2 = ntu * ntu, per = ntu2 * 4, J = ncl * per;
-    const int lt = lg2i(ntu);   // TU counts are powers of two: shifts, not divisions
-    if (threadIdx.x == 0) OPCOUNT(3, J);
-    const int hw = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, l4 = lane & 3;
-    const int warp = (hw + NW - woff % NW) % NW;   // job rank of this warp
-    int *scr = S.scratch[hw] + qd * 20;
-    const int dc = S.dc;
-    for (int base = 0; base < J; base += NW * 8) {
-        const int j = base + warp * 8 + qd;
-        const bool act = j < J;
-        const int jj = act ? j : 0;
-        const int k = jj >> (2 * lt + 2), rem = jj & (per - 1), t = rem >> 2, q = rem & 3;
-        const int ty = t >> lt, tx = t & (ntu - 1);
-        const int sx = tx * 8 + (q & 1) * 4, sy = ty * 8 + (q & 2) * 2;
-        const int slot = cl[k];
-        const PredSrc ps = pred_src(S, slot);
-        int res[4], pr[4];
-        if (ps.src) {
-#pragma unroll
-            for (int n = 0; n < 4; ++n) pr[n] = ps.src[((sy + l4) * cu + sx + n) & ps.mask];
-        } else {
-#pragma unroll
-            for (int n = 0; n < 4; ++n) pr[n] = intra_sample(cu, slot - K_INTRA, dc, sx + n, sy + l4);
+    const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
+    const uint4 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
+    const uint4 *bands = S.qparam[0].band;
+    const uint4 b80 = bands[band_rc(8, row, col)], b81 = bands[band_rc(8, row, col + 1)];
+    const uint4 b40 = bands[band_rc(4, row & 3, col & 3)], b41 = bands[band_rc(4, row & 3, (col & 3) + 1)];
+    for (int it = ((threadIdx.x >> 5) + NW - woff) & (NW - 1); it < J; it += NW) {
+        const int e = cl[it >> (2 * lt)], slot = e & CL_SLOT, t = it & ((1 << (2 * lt)) - 1);
+        const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
+        const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
+        const uint32_t pv = pred2(S, cu, slot, x, y);
+        if ((e & CL_EXACT) && __any_sync(0xffffffffu, pv != cv)) S.inexact = 1;
+        if (lane == 0) { OPCOUNT(2, (e & CL_8) ? 1 : 0); OPCOUNT(3, (e & CL_4) ? 4 : 0); }
+        if (e & CL_8) {
+            const AreaCode c = code_area(cv, pv, f8, i8, b80, b81);
+            if (accum) {
+                const uint32_t s = __reduce_add_sync(0xffffffffu, c.sums);
+                const int bits = base_bits8(c) + 2 * (int)(s & 1023u);
+                if (lane == 0) {
+                    atomicAdd(&S.acc_sse[slot][0], (int)(s >> 10));
+                    atomicAdd(&S.acc_bits[slot][0], bits);
+                }
+                if (cu <= 16) *(uint16_t *)(S.crec[slot][0] + y * cu + x) = (uint16_t)c.rec;
+            }
+            if (wrec) *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
+            if (emit) *(uint32_t *)(emit + t * 64 + 2 * lane) = __byte_perm((uint32_t)c.q0, (uint32_t)c.q1, 0x5410);
         }
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-            res[n] = clampi((int)S.cur_y[(L.ly + sy + l4) * 64 + L.lx + sx + n] - pr[n], -512, 511);
-        int qc[4], rc[4];
-        int bits = tu4_code(l4, res, scr, qp, qc, rc);
-        if (q == 0) bits += 1;
-        int sse = 0;
-        const int x = sx + l4;
-        if (ps.src) {
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) pr[kk] = ps.src[((sy + kk) * cu + x) & ps.mask];
-        } else {
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) pr[kk] = intra_sample(cu, slot - K_INTRA, dc, x, sy + kk);
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const int y = sy + kk;
-            const int v = clampi(pr[kk] + rc[kk], 0, 255);
-            const int d = (int)S.cur_y[(L.ly + y) * 64 + L.lx + x] - v;
-            sse += d * d;
-            if (act && wrec) RY(S, L.lx + x, L.ly + y) = (uint8_t)v;
-            if (act && accum && cu <= 16) S.crec[slot][1][y * cu + x] = (uint8_t)v;
-            if (act && emit) emit[t * 64 + q * 16 + kk * 4 + l4] = (int16_t)qc[kk];
-        }
-        sse = quad_sum(sse);
-        if (act && accum && l4 == 0) {
-            atomicAdd(&S.acc_sse[slot][1], sse);
-            atomicAdd(&S.acc_bits[slot][1], bits);
+        if (e & CL_4) {
+            const AreaCode c = code_area(cv, pv, f4, i4, b40, b41);
+            if (accum) {
+                const uint32_t s = __reduce_add_sync(0xffffffffu, c.sums);
+                int bits = base_bits4(c, lane);
+                bits += __shfl_xor_sync(0xffffffffu, bits, 2);
+                bits += __shfl_xor_sync(0xffffffffu, bits, 16);
+                if (lane == 0) {
+                    atomicAdd(&S.acc_sse[slot][1], (int)(s >> 10));
+                    atomicAdd(&S.acc_bits[slot][1], bits + 1 + 2 * (int)(s & 1023u));
+                }
+                if (cu <= 16) *(uint16_t *)(S.crec[slot][1] + y * cu + x) = (uint16_t)c.rec;
+            }
+            if (wrec) *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
+            if (emit)
+                *(uint32_t *)(emit + t * 64 + (row >> 2) * 32 + (col >> 2) * 16 + (row & 3) * 4 + (col & 3)) =
+                    __byte_perm((uint32_t)c.q0, (uint32_t)c.q1, 0x5410);
         }
     }
 }
 
-// Chroma residual jobs (reference src/encoder.c:429-475 qt_code_chroma):
-// 4x4 TUs, one quad per (option, component, TU).  Option o, component c
-// predicts from S.cpred[cbase + 2*o + c]; results accumulate in slot o.
-__device__ __noinline__ void chroma_jobs(Smem &, const Leaf L, int nopt, int cbase, const QuantParams &,
-                            bool accum, bool wrec, int16_t *emit, int woff = 0) {
+// Chroma residual coding (reference src/encoder.c:429-475 qt_code_chroma):
+// 4x4 TUs, four (option, component, TU) jobs per warp, one on each quarter of
+// the area's lanes.  Option o, component c predicts from
+// S.cpred[cbase + 2*o + c]; results accumulate in slot o.
+__device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, bool accum, bool wrec, int16_t *emit,
+                                          int woff) {
     Smem &S = smem_state();
-    const QuantParams &qp = S.qparam[1];
-    const int cs = L.cu >> 1, nt = cs >> 2, nt2 = nt * nt, per = 2 * nt2, J = nopt * per;
-    const int ln = lg2i(nt);    // TU counts are powers of two: shifts, not divisions
-    if (threadIdx.x == 0) OPCOUNT(3, J);
+    const int cs = L.cu >> 1, ln = lg2i(cs) - 2, J = nopt << (2 * ln + 1);
     const int lxc = L.lx >> 1, lyc = L.ly >> 1;
-    const int hw = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, l4 = lane & 3;
-    const int warp = (hw + NW - woff % NW) % NW;   // job rank of this warp
-    int *scr = S.scratch[hw] + qd * 20;
-    for (int base = 0; base < J; base += NW * 8) {
-        const int j = base + warp * 8 + qd;
-        const bool act = j < J;
-        const int jj = act ? j : 0;
-        const int o = jj >> (2 * ln + 1), rem = jj & (per - 1), c = rem >> (2 * ln), t = rem & (nt2 - 1);
-        const int ty = t >> ln, tx = t & (nt - 1);
-        const uint8_t *pr = S.cpred[cbase + 2 * o + c];
-        const uint8_t *org = S.cur_c[c];
-        int res[4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int x = tx * 4 + n, y = ty * 4 + l4;
-            res[n] = clampi((int)org[(lyc + y) * 32 + lxc + x] - (int)pr[y * cs + x], -512, 511);
+    const int lane = threadIdx.x & 31, r = (lane >> 2) & 3, cc = 2 * (lane & 1);
+    const int quarter = ((lane >> 3) & 2) | ((lane >> 1) & 1);
+    const uint4 f4 = S.frag[2][lane], i4 = S.frag[3][lane];
+    const uint4 b0 = S.qparam[1].band[band_rc(4, r, cc)], b1 = S.qparam[1].band[band_rc(4, r, cc + 1)];
+    if (threadIdx.x == 0) OPCOUNT(3, J);
+    for (int base = 4 * (((threadIdx.x >> 5) + NW - woff) & (NW - 1)); base < J; base += 4 * NW) {
+        const bool act = base + quarter < J;
+        const int j = act ? base + quarter : 0;
+        const int o = j >> (2 * ln + 1), c = (j >> (2 * ln)) & 1, t = j & ((1 << (2 * ln)) - 1);
+        const int x = (t & ((1 << ln) - 1)) * 4 + cc, y = (t >> ln) * 4 + r;
+        const uint32_t cv = *(const uint16_t *)(S.cur_c[c] + (lyc + y) * 32 + lxc + x);
+        const uint32_t pv = *(const uint16_t *)(S.cpred[cbase + 2 * o + c] + y * cs + x);
+        const AreaCode a = code_area(cv, pv, f4, i4, b0, b1);
+        if (accum) {
+            uint32_t s = a.sums;    // of the quarter's eight lanes: index bits 0, 2 and 3
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 4);
+            s += __shfl_xor_sync(0xffffffffu, s, 8);
+            const int bits = base_bits4(a, lane) + 2 * (int)(s & 1023u);
+            if (act && (lane & 13) == 0) {
+                atomicAdd(&S.acc_sse[o][0], (int)(s >> 10));
+                atomicAdd(&S.acc_bits[o][0], bits);
+            }
         }
-        int qc[4], rc[4];
-        const int bits = tu4_code(l4, res, scr, qp, qc, rc);
-        int sse = 0;
-        const int x = tx * 4 + l4;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const int y = ty * 4 + kk;
-            const int v = clampi((int)pr[y * cs + x] + rc[kk], 0, 255);
-            const int d = (int)org[(lyc + y) * 32 + lxc + x] - v;
-            sse += d * d;
-            if (act && wrec) RC(S, c, lxc + x, lyc + y) = (uint8_t)v;
-            if (act && emit) emit[c * cs * cs + t * 16 + kk * 4 + l4] = (int16_t)qc[kk];
-        }
-        sse = quad_sum(sse);
-        if (act && accum && l4 == 0) {
-            atomicAdd(&S.acc_sse[o][0], sse);
-            atomicAdd(&S.acc_bits[o][0], bits);
-        }
+        if (act && wrec) *(uint16_t *)&RC(S, c, lxc + x, lyc + y) = (uint16_t)a.rec;
+        if (act && emit)
+            *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = __byte_perm((uint32_t)a.q0, (uint32_t)a.q1, 0x5410);
     }
 }
 
@@ -1088,31 +997,21 @@ __device__ void zero_acc(Smem &S) {
         (&S.acc_sse[0][0])[i] = 0;
         (&S.acc_bits[0][0])[i] = 0;
     }
-    if (threadIdx.x < 4) S.acc64[threadIdx.x] = 0;
+    if (threadIdx.x == 0) { S.acc64 = 0; S.inexact = 0; }
 }
 
 // Sum over the CU of |orig - pred| per listed slot into acc_sse[slot][0]
-// (fast-preset SAD proxy).
-__device__ void sad_jobs(Smem &S, const Leaf &L, const int *cl, int ncl) {
-    const int cu = L.cu, n = cu * cu, dc = S.dc;
-    for (int k = 0; k < ncl; ++k) {
-        const int slot = cl[k];
-        int acc = 0;
-        for (int p = threadIdx.x; p < n; p += NT) {
-            const int y = p >> lg2i(cu), x = p & (cu - 1);
-            acc += absi((int)S.cur_y[(L.ly + y) * 64 + L.lx + x] - lpred(S, cu, slot, dc, x, y));
-        }
-        acc = __reduce_add_sync(0xffffffffu, acc);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&S.acc_sse[slot][0], acc);
+// (fast-preset SAD proxy): one warp per (candidate, 8x8 area).
+__device__ void sad_areas(Smem &S, const Leaf &L, const int *cl, int ncl) {
+    const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
+    const int lane = threadIdx.x & 31;
+    for (int it = threadIdx.x >> 5; it < J; it += NW) {
+        const int slot = cl[it >> (2 * lt)] & CL_SLOT, t = it & ((1 << (2 * lt)) - 1);
+        const int x = (t & ((1 << lt) - 1)) * 8 + 2 * (lane & 3), y = (t >> lt) * 8 + (lane >> 2);
+        const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
+        const unsigned s = __reduce_add_sync(0xffffffffu, __vsadu4(cv, pred2(S, cu, slot, x, y)));
+        if (lane == 0) atomicAdd(&S.acc_sse[slot][0], (int)s);
     }
-}
-
-// Thirteen nibbles a0..a12 packed low to high (kind k at bits 4k..4k+3).
-__host__ __device__ constexpr uint64_t nib13(int a0, int a1, int a2, int a3, int a4, int a5, int a6, int a7,
-                                             int a8, int a9, int a10, int a11, int a12) {
-    return (uint64_t)a0 | (uint64_t)a1 << 4 | (uint64_t)a2 << 8 | (uint64_t)a3 << 12 | (uint64_t)a4 << 16 |
-           (uint64_t)a5 << 20 | (uint64_t)a6 << 24 | (uint64_t)a7 << 28 | (uint64_t)a8 << 32 | (uint64_t)a9 << 36 |
-           (uint64_t)a10 << 40 | (uint64_t)a11 << 44 | (uint64_t)a12 << 48;
 }
 
 __device__ __forceinline__ long long best_of(const Smem &S, int slot, bool use4, long long lambda,
@@ -1218,29 +1117,34 @@ __device__ void luma_from_cache(Smem &S, const Leaf &L, int slot, bool dct8) {
     }
 }
 
-__device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L, const QuantParams &,
-                          const QuantParams &, bool emit, CtuOut *out, bool use_cache = false) {
+// `from`: 0 codes the node from its record alone; 1 replays the winner of the
+// decision just made (its references, inter predictions and, up to 16x16, its
+// reconstruction are still in shared memory); 2 as 1 with the luma
+// reconstruction already in the tile.
+__device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L, bool emit, CtuOut *out, int from) {
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
-    const QuantParams &ql = S.qparam[0], &qc = S.qparam[1];
     const Node nd = S.nodes[qt_index(L.depth, L.cx, L.cy)];
     int mvpx, mvpy;
     mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
     const int cu = L.cu;
     int16_t *el = emit ? out->coef + S.ncoef : nullptr;
     int16_t *ec = emit ? el + cu * cu : nullptr;
+    const bool use_cache = from && P.preset >= 2 && cu <= 16;
+    const int cl_size = nd.dct_size ? CL_8 : CL_4;
     bool coded = true;
     if (nd.intra) {
-        if (use_cache) {
-            luma_from_cache(S, L, K_INTRA + nd.intra_mode, nd.dct_size);
-        } else {
-            build_refs(S, L, nd.intra_mode < 18 ? 1u << nd.intra_mode : 0u);
-            if (threadIdx.x == 0) { S.cl2[0] = K_INTRA + nd.intra_mode; }
+        if (from < 2) {
+            if (use_cache) {
+                luma_from_cache(S, L, K_INTRA + nd.intra_mode, nd.dct_size);
+            } else {
+                if (threadIdx.x == 0) S.cl2[0] = (K_INTRA + nd.intra_mode) | cl_size;
+                if (!from) build_refs(L);
+                else SYNC();
+                luma_areas(L, S.cl2, 1, false, true, el, 0);
+            }
             SYNC();
-            if (nd.dct_size) luma_jobs8(S, L, S.cl2, 1, ql, false, true, el);
-            else luma_jobs4(S, L, S.cl2, 1, ql, false, true, el);
         }
-        SYNC();
         if (nd.ch_intra) {
             chroma_dc_pred(S, L, 0);
             cfl_blend(S, L, 0);
@@ -1249,7 +1153,7 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
         } else {
             chroma_dc_pred(S, L, 0);
         }
-        chroma_jobs(S, L, 1, 0, qc, false, true, ec);
+        chroma_areas(L, 1, 0, false, true, ec, 0);
     } else {
         int mvx, mvy;
         if (nd.merge || nd.skip) { mvx = mvpx + L.px * 4; mvy = mvpy + L.py * 4; }
@@ -1282,9 +1186,12 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
             cr1 = r1;
         }
         if (!nd.skip) {
+            const int src = from ? S.win_slot : 0;   // the decision's prediction is still in its slot
             if (threadIdx.x == 0) {
-                S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
-                S.cl2[0] = 0;
+                if (!from) {
+                    S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
+                }
+                S.cl2[0] = src | cl_size;
             }
             SYNC();
             // Chroma prediction does not depend on this leaf's luma, so both
@@ -1293,21 +1200,18 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
             if (nd.ch_intra || cflat) chroma_dc_pred(S, L, 0);
             else chroma_mc_bi(S, P, L, cr1, cr2, mvx, mvy);
             if (use_cache) {
-                luma_from_cache(S, L, S.win_slot, nd.dct_size);
-                chroma_jobs(S, L, 1, 0, qc, false, true, ec);
+                luma_from_cache(S, L, src, nd.dct_size);
+                chroma_areas(L, 1, 0, false, true, ec, 0);
             } else {
-                if (flat) {
+                if (!from && flat) {
                     for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
                     SYNC();
-                } else {
+                } else if (!from) {
                     const int slots[1] = {0};
                     luma_mc_slots(S, P, L, 1, slots, false);
                 }
-                const int ntu = cu >> 3;
-                const int wl = nd.dct_size ? mini(NW, (ntu * ntu + 3) / 4) : mini(NW, (ntu * ntu * 4 + 7) / 8);
-                if (nd.dct_size) luma_jobs8(S, L, S.cl2, 1, ql, false, true, el);
-                else luma_jobs4(S, L, S.cl2, 1, ql, false, true, el);
-                chroma_jobs(S, L, 1, 0, qc, false, true, ec, wl);
+                luma_areas(L, S.cl2, 1, false, true, el, 0);
+                chroma_areas(L, 1, 0, false, true, ec, mini(NW / 2, (cu * cu) >> 6));
             }
         } else {
             coded = false;
@@ -1336,12 +1240,10 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
 // ====================================================================
 // Leaf decision (reference src/encoder.c:784-1277).
 // ====================================================================
-__device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const Leaf L,
-                                 const QuantParams &, const QuantParams &) {
+__device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const Leaf L) {
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
-    const QuantParams &ql = S.qparam[0], &qc = S.qparam[1];
-    const int cu = L.cu, tid = threadIdx.x;
+    const int cu = L.cu, tid = threadIdx.x, lane = tid & 31;
     const bool fast = P.preset <= 1;
     const bool medium = P.preset >= 2;
     const bool key = P.frame_type == 0;
@@ -1351,21 +1253,15 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     COUNT_D(L.depth);
     int mvpx, mvpy;
     mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
-    {
-        // intra modes this leaf will score (the candidate list below)
-        const bool ti = key || cu <= 16 || medium;
-        const int st = P.preset == 0 ? 6 : (P.preset == 1 ? 3 : 1);
-        uint32_t mm = 0;
-        if (ti)
-            for (int m = 0; m < 18; m += st) mm |= 1u << m;
-        build_refs(S, L, mm);
-    }
     zero_acc(S);
+    build_refs(L);
     PHASE_D(0, L.depth);
 
     // ---- candidate set -------------------------------------------------
+    // Present slots, one bit each: inter candidates 0..4, intra modes from
+    // K_INTRA on.
+    uint32_t cand = 0;
     bool has_glb = false, has_tmp = false, has_me1 = false;
-    int n8only = 0;          // merges coded with 8x8 TUs only, in S.cl2
     int tdx = 0, tdy = 0;
     const int rf = is_b ? dpb_fwd(P) : -1, rb = is_b ? dpb_bwd(P) : -1;
     const int g = tid / GT, gt = tid - g * GT;
@@ -1397,12 +1293,11 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         PHASE_D(1, L.depth);
         if (has_glb && S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) has_glb = false;
         if (has_tmp && S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) has_tmp = false;
+        cand = 1u << K_ME0 | (uint32_t)has_me1 << K_ME1 | (uint32_t)has_glb << K_GLB | (uint32_t)has_tmp << K_TMP |
+               (uint32_t)medium << K_MRG;
         int slots[5], ns = 0;
-        slots[ns++] = K_ME0;
-        if (has_me1) slots[ns++] = K_ME1;
-        if (has_glb) slots[ns++] = K_GLB;
-        if (has_tmp) slots[ns++] = K_TMP;
-        if (medium) slots[ns++] = K_MRG;
+        for (int k = 0; k < NPRED; ++k)
+            if (cand >> k & 1u) slots[ns++] = k;
         if (tid == 0) {
             S.cand_mvx[K_ME0] = S.me[0].mvx; S.cand_mvy[K_ME0] = S.me[0].mvy; S.cand_ref[K_ME0] = 0;
             S.cand_mvx[K_ME1] = S.me[1].mvx; S.cand_mvy[K_ME1] = S.me[1].mvy; S.cand_ref[K_ME1] = 1;
@@ -1410,9 +1305,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
             S.cand_mvx[K_TMP] = S.me[3].mvx; S.cand_mvy[K_TMP] = S.me[3].mvy; S.cand_ref[K_TMP] = 0;
             S.cand_mvx[K_MRG] = mvpx + L.px * 4; S.cand_mvy[K_MRG] = mvpy + L.py * 4; S.cand_ref[K_MRG] = 0;
             for (int k = 0; k < NPRED; ++k) S.cand_ref2[k] = -1;
-            S.cl2[0] = K_MRG;
         }
-        if (medium) n8only = 1;
         SYNC();
         luma_mc_slots(S, P, L, ns, slots, false);
         PHASE_D(2, L.depth);
@@ -1425,13 +1318,11 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
             me_run(S, 1, gt, P.ref_y[rb], P.stride_y, P.W, P.H, L.lx, L.ly, cu, cx0, cy0, sr);
         SYNC();
         PHASE_D(1, L.depth);
+        const uint32_t hf = rf >= 0, hb = rb >= 0, mrg = medium;
+        cand = hf | hb << 1 | (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;
         int slots[5], ns = 0;
-        if (rf >= 0) slots[ns++] = K_B0 + 0;
-        if (rb >= 0) slots[ns++] = K_B0 + 1;
-        const bool mrg = medium && !fast;
-        if (mrg && rf >= 0 && rb >= 0) slots[ns++] = K_B0 + 2;
-        if (mrg && rf >= 0) slots[ns++] = K_B0 + 3;
-        if (mrg && rb >= 0) slots[ns++] = K_B0 + 4;
+        for (int k = 0; k < NPRED; ++k)
+            if (cand >> k & 1u) slots[ns++] = k;
         if (tid == 0) {
             const int mmx = mvpx + L.px * 4, mmy = mvpy + L.py * 4;
             for (int k = 0; k < NPRED; ++k) S.cand_ref2[k] = -1;
@@ -1441,12 +1332,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
             S.cand_ref2[K_B0 + 2] = rb;
             S.cand_mvx[K_B0 + 3] = mmx; S.cand_mvy[K_B0 + 3] = mmy; S.cand_ref[K_B0 + 3] = rf < 0 ? 0 : rf;
             S.cand_mvx[K_B0 + 4] = mmx; S.cand_mvy[K_B0 + 4] = mmy; S.cand_ref[K_B0 + 4] = rb < 0 ? 0 : rb;
-            int n = 0;
-            if (mrg && rf >= 0 && rb >= 0) S.cl2[n++] = K_B0 + 2;
-            if (mrg && rf >= 0) S.cl2[n++] = K_B0 + 3;
-            if (mrg && rb >= 0) S.cl2[n++] = K_B0 + 4;
         }
-        n8only = (mrg && rf >= 0 && rb >= 0) + (mrg && rf >= 0) + (mrg && rb >= 0);
         SYNC();
         luma_mc_slots(S, P, L, ns, slots, false);
         PHASE_D(2, L.depth);
@@ -1454,58 +1340,29 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
 
     // ---- residual coding / SAD proxies for every candidate --------------
     const bool try_intra = key || cu <= 16 || medium;
-    const int step = P.preset == 0 ? 6 : (P.preset == 1 ? 3 : 1);
     const bool use4 = medium && cu <= 32;
-    if (tid == 0) {
-        int n = 0;
-        if (is_p) {
-            S.cl[n++] = K_ME0;
-            if (has_me1) S.cl[n++] = K_ME1;
-            if (has_glb) S.cl[n++] = K_GLB;
-            if (has_tmp) S.cl[n++] = K_TMP;
-        } else if (is_b) {
-            if (rf >= 0) S.cl[n++] = K_B0 + 0;
-            if (rb >= 0) S.cl[n++] = K_B0 + 1;
-        }
-        const int ninter = n;
-        if (try_intra)
-            for (int mi = 0; mi < 18; ++mi) {
-                const int m = mi * step;
-                if (m >= 18) break;
-                S.cl[n++] = K_INTRA + m;
-            }
-        S.ncl = n;
-        S.flag = ninter;
+    if (try_intra) cand |= (P.preset == 0 ? 0x1041u : P.preset == 1 ? 0x9249u : 0x3FFFFu) << K_INTRA;
+    const int ncl = __popc(cand);
+    // slots 2..4 of a B leaf and the merge slot of a P leaf: 8x8 TUs only
+    const uint32_t merges = is_b ? 0x1Cu : 1u << K_MRG;
+    if (tid < 32) {
+        const bool m8 = merges >> lane & 1u;
+        if (cand >> lane & 1u)
+            S.cl[__popc(cand & ((1u << lane) - 1u))] =
+                lane | CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0);
     }
     SYNC();
-    const int ncl = S.ncl, ninter = S.flag;
     if (fast) {
-        sad_jobs(S, L, S.cl, ncl);
+        sad_areas(S, L, S.cl, ncl);
         SYNC();
     } else {
-        // The three job lists start on different warps so that small
-        // leaves spread them over the CTA instead of stacking them on the
-        // first warps (accumulation is by integer atomics: order-free).
-        const int ntu2 = (cu >> 3) * (cu >> 3);
-        const int w8 = mini(NW, (ncl * ntu2 + 3) / 4), w4 = use4 ? mini(NW, (ncl * ntu2 * 4 + 7) / 8) : 0;
-        luma_jobs8(S, L, S.cl, ncl, ql, true, false, nullptr);
-        if (use4) luma_jobs4(S, L, S.cl, ncl, ql, true, false, nullptr, w8);
-        if (n8only) luma_jobs8(S, L, S.cl2, n8only, ql, true, false, nullptr, w8 + w4);
+        luma_areas(L, S.cl, ncl, true, false, nullptr, 0);
         SYNC();
         PHASE_D(3, L.depth);
-        if (is_p && medium) {
-            // Skip pre-check (src/encoder.c:1064-1142): luma SSE of the merge
-            // prediction, then fresh chroma SSE when the luma is exact.
-            long long acc = 0;
-            for (int p = tid; p < cu * cu; p += NT) {
-                const int y = p >> lg2i(cu), x = p & (cu - 1);
-                const int d = (int)S.cur_y[(L.ly + y) * 64 + L.lx + x] - (int)S.pred[K_MRG][p];
-                acc += d * d;
-            }
-            acc = __reduce_add_sync(0xffffffffu, (unsigned)acc);
-            if ((tid & 31) == 0 && acc) atomicAdd((unsigned long long *)&S.acc64[0], (unsigned long long)acc);
-            SYNC();
-            if (S.acc64[0] == 0 && P.ref_valid[0]) {
+        if (is_p) {
+            // Skip pre-check (src/encoder.c:1064-1142): the merge prediction
+            // equals the source luma, then fresh chroma SSE.
+            if (!S.inexact && P.ref_valid[0]) {
                 chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
                 const int cs = cu >> 1;
                 long long ac = 0;
@@ -1516,127 +1373,75 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
                     ac += db * db + dr * dr;
                 }
                 ac = __reduce_add_sync(0xffffffffu, (unsigned)ac);
-                if ((tid & 31) == 0 && ac) atomicAdd((unsigned long long *)&S.acc64[1], (unsigned long long)ac);
+                if (lane == 0 && ac) atomicAdd((unsigned long long *)&S.acc64, (unsigned long long)ac);
                 SYNC();
-            } else if (tid == 0) {
-                S.acc64[1] = 1;   // no skip candidate
             }
-            SYNC();
         }
     }
 
     PHASE_D(4, L.depth);
     // ---- in-order candidate scan (strict <, first minimum wins) ---------
-    // Each lane of warp 0 scores one candidate of the scan order (inter
-    // candidates, then the intra modes), then a warp argmin on (cost,
-    // position) picks the first minimum exactly as a sequential scan with
-    // strict < does.  The node takes the winner's fields, the others keep
-    // their defaults (a sequential scan leaves the same result because every
+    // Lane k of warp 0 scores slot k (inter candidates, then the intra modes,
+    // the order of a sequential scan); lane 23 the skip candidate of a P
+    // leaf, which comes between them.  The smallest (cost, position) is the
+    // first minimum, as a sequential scan with strict < leaves it.  The node
+    // takes the winner's fields, the others keep their defaults (every
     // candidate sets all the fields later candidates could have changed).
     if (tid < 32) {
-        enum { C_NONE, C_P_ME0, C_P_ME1, C_P_GLB, C_P_TMP, C_P_MRG, C_P_SKIP,
-               C_B_DIR0, C_B_DIR1, C_B_M2, C_B_M3, C_B_M4, C_INTRA };
-        // Scan parameters of each kind, one nibble per kind (kind k in bits
-        // 4k..4k+3), so that every lane runs the same code whatever its kind:
-        //   SL1   slot + 1 of the candidate's sums (0: none; intra: its slot)
-        //   EXT   extra bits; MRX: added with multiref; PLB: level bits of
-        //         the SAD proxy
-        //   FA    1 MV bits, 2 SAD proxy on fast presets, 4 merge (8x8-only
-        //         sums), 8 second reference
-        //   FB    1 bi-predicted, 2 skip, 4 intra, 8 merge MV (the MVP)
-        //        NONE ME0 ME1 GLB TMP MRG SKIP DIR0 DIR1 M2  M3  M4  INTRA
-        constexpr uint64_t SL1 = nib13(0, 1, 2, 3, 4, 5, 0, 1, 2, 3, 4, 5, 0);
-        constexpr uint64_t EXT = nib13(0, 6, 8, 6, 6, 6, 2, 6, 6, 6, 6, 6, 8);
-        constexpr uint64_t MRX = nib13(0, 2, 0, 1, 2, 0, 0, 0, 0, 0, 0, 0, 0);
-        constexpr uint64_t PLB = nib13(0, 3, 0, 0, 0, 0, 0, 3, 3, 0, 0, 0, 8);
-        constexpr uint64_t FA = nib13(0, 3, 9, 1, 1, 4, 0, 3, 11, 4, 4, 12, 2);
-        constexpr uint64_t FB = nib13(0, 0, 0, 0, 0, 8, 2, 0, 0, 1, 0, 0, 4);
-        static_assert(K_ME0 == 0 && K_ME1 == 1 && K_GLB == 2 && K_TMP == 3 && K_MRG == 4 && K_B0 == 0,
-                      "SL1 holds the candidate slots + 1");
-        const int lane = tid;
+        constexpr int SKIP_LANE = NCAND;
         const long long lam = P.lambda;
-        const int base_x = mvpx + L.px * 4, base_y = mvpy + L.py * 4;
-        uint32_t klist = 0;   // the inter kinds of the scan order, a nibble each
-        int nk = 0;
-        auto push = [&](int k) { klist |= (uint32_t)k << (4 * nk); ++nk; };
-        if (is_b) {
-            if (rf >= 0) push(C_B_DIR0);
-            if (rb >= 0) push(C_B_DIR1);
-            if (medium && !fast) {
-                if (rf >= 0 && rb >= 0) push(C_B_M2);
-                if (rf >= 0) push(C_B_M3);
-                if (rb >= 0) push(C_B_M4);
+        const bool inter = lane < NPRED, intra = lane >= K_INTRA && lane < NCAND, skip = lane == SKIP_LANE;
+        const bool merge = merges >> lane & 1u;      // 8x8-only sums, the MVP's vector
+        const int pos = lane < NPRED ? lane : (skip ? NPRED : lane + 1);
+        const bool valid = (cand >> lane & 1u) ||
+                           (skip && is_p && medium && P.ref_valid[0] && !S.inexact && S.acc64 == 0);
+        // extra bits: 6 for inter, 8 for the second reference, 8 for intra,
+        // 2 for skip, and the multiref syntax of a P leaf's searches
+        int extra = intra ? 8 : skip ? 2 : 6;
+        if (is_p && lane == K_ME1) extra = 8;
+        if (P.multiref && is_p) extra += (lane == K_ME0 || lane == K_TMP) ? 2 : lane == K_GLB ? 1 : 0;
+        const int f_ref = is_b ? (lane == K_B0 + 1 || lane == K_B0 + 4) : lane == K_ME1;
+        int f_dct = 1, f_mx = 0, f_my = 0, bits = extra;
+        uint32_t kh = 0xFFFFFFFFu, kl = 0xFFFFFFFFu;
+        long long cost = (long long)1 << 58;         // no candidate
+        if (valid) {
+            if (inter && (!merge || is_p)) {
+                // (a P merge carries the first search's vector difference)
+                const int v = merge ? K_ME0 : lane;
+                f_mx = S.cand_mvx[v] - mvpx - L.px * 4;
+                f_my = S.cand_mvy[v] - mvpy - L.py * 4;
+                if (!merge) bits += se_bits(f_mx) + se_bits(f_my);
             }
-        } else if (is_p) {
-            push(C_P_ME0);
-            if (has_me1) push(C_P_ME1);
-            if (has_glb) push(C_P_GLB);
-            if (has_tmp) push(C_P_TMP);
-            if (medium) {
-                push(C_P_MRG);
-                if (P.ref_valid[0] && S.acc64[0] == 0 && S.acc64[1] == 0) push(C_P_SKIP);
-            }
-        }
-        const int n = nk + (try_intra ? ncl - ninter : 0);
-        int kind = C_NONE, slot = 0;
-        if (lane < nk) kind = (klist >> (4 * lane)) & 15;
-        else if (lane < n) { kind = C_INTRA; slot = S.cl[ninter + lane - nk]; }
-        const int sh = 4 * kind;
-        const int fa = (int)(FA >> sh) & 15, fb = (int)(FB >> sh) & 15;
-        const int sl = kind == C_INTRA ? slot : (int)((SL1 >> sh) & 15) - 1;
-        const bool mvbits = fa & 1, proxy = fast && (fa & 2), merge8 = fa & 4;
-        const int extra = (int)((EXT >> sh) & 15) + (P.multiref ? (int)((MRX >> sh) & 15) : 0);
-        const int plb = (int)((PLB >> sh) & 15);
-        const int mvsl = mvbits ? sl : ((fb & 8) ? K_ME0 : -1);
-        const int f_intra = (fb >> 2) & 1, f_skip = (fb >> 1) & 1, f_merge = merge8, f_bi = fb & 1;
-        const int f_ref = fa >> 3, f_mode = f_intra ? slot - K_INTRA : 1;
-        int f_dct = 1, f_mx = 0, f_my = 0;
-        // cost = distortion + lambda * (extra + MV bits + level bits), with
-        // distortion / level bits from best_of (explicit inter and intra),
-        // the 8x8-only sums (merges), the SAD proxy (fast presets) or
-        // nothing (skip)
-        long long cost = (long long)1 << 60;   // no candidate: defaults, as the sequential scan
-        if (kind != C_NONE) {
-            long long dl = 0;
-            int lb = 0;
-            if (sl >= 0) {
-                if (proxy) {
-                    const long long sad = S.acc_sse[sl][0];
-                    dl = (sad * sad) >> (2 * lg2i(cu));   // / (cu * cu), sad >= 0
-                    lb = plb;
-                } else if (merge8) {
-                    dl = S.acc_sse[sl][0];
-                    lb = S.acc_bits[sl][0];
+            long long d = 0;
+            if (!skip) {
+                if (fast) {
+                    const long long sad = S.acc_sse[lane][0];
+                    d = (sad * sad) >> (2 * lg2i(cu));   // / (cu * cu), sad >= 0
+                    bits += intra ? 8 : 3;
                 } else {
-                    dl = best_of(S, sl, use4, lam, lb, f_dct);
+                    int lb;
+                    d = best_of(S, lane, use4 && !merge, lam, lb, f_dct);
+                    bits += lb;
                 }
             }
-            int mb = 0;
-            if (mvsl >= 0) {
-                f_mx = S.cand_mvx[mvsl] - base_x; f_my = S.cand_mvy[mvsl] - base_y;
-                if (mvbits) mb = se_bits(f_mx) + se_bits(f_my);
-            }
-            cost = dl + lam * (extra + mb + lb);
+            cost = d + lam * bits;
         }
-        // first minimum: smallest cost, then smallest scan position
-        long long bc = cost;
-        int bl = lane;
-        for (int o = 16; o > 0; o >>= 1) {
-            const long long oc = __shfl_xor_sync(0xffffffffu, bc, o);
-            const int ol = __shfl_xor_sync(0xffffffffu, bl, o);
-            if (oc < bc || (oc == bc && ol < bl)) { bc = oc; bl = ol; }
-        }
-        if (lane == bl) {
-            const int ws = sl;   // every kind's winner slot is its sums' slot (-1: skip, none)
-            S.win_slot = ws;
+        // costs stay below 2^58: distortion < 2^28, lambda <= 2^30, bits < 2^18
+        const unsigned long long k = (unsigned long long)cost << 5 | (unsigned)pos;
+        kh = (uint32_t)(k >> 32);
+        kl = (uint32_t)k;
+        const uint32_t mh = __reduce_min_sync(0xffffffffu, kh);
+        const uint32_t ml = __reduce_min_sync(0xffffffffu, kh == mh ? kl : 0xFFFFFFFFu);
+        if (kh == mh && kl == ml) {
+            S.win_slot = skip ? -1 : lane;
             Node &nd = S.nodes[qt_index(L.depth, L.cx, L.cy)];
-            nd.intra = (uint8_t)f_intra; nd.skip = (uint8_t)f_skip; nd.merge = (uint8_t)f_merge;
-            nd.bi = (uint8_t)f_bi;
-            nd.intra_mode = (uint8_t)f_mode; nd.intra_cmode = 0; nd.ch_intra = 0;
+            nd.intra = intra; nd.skip = skip; nd.merge = inter && merge;
+            nd.bi = is_b && lane == K_B0 + 2;
+            nd.intra_mode = (uint8_t)(intra ? lane - K_INTRA : 1); nd.intra_cmode = 0; nd.ch_intra = 0;
             nd.ref_sel = (uint8_t)f_ref; nd.dct_size = (uint8_t)f_dct;
             nd.mvd_x = (int16_t)f_mx; nd.mvd_y = (int16_t)f_my;
             nd.split = 0;
-            S.best_cost = bc;
+            S.best_cost = cost;
         }
     }
     SYNC();
@@ -1644,14 +1449,14 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     PHASE_D(5, L.depth);
     // ---- intra chroma choice: MC vs CfL-blended DC (src/encoder.c:1194-1221)
     const Node nd0 = S.nodes[qt_index(L.depth, L.cx, L.cy)];
-    if (nd0.intra && !fast && medium) {
+    const bool luma_done = nd0.intra && medium;
+    if (luma_done) {
         if (cu <= 16) {
             luma_from_cache(S, L, K_INTRA + nd0.intra_mode, nd0.dct_size);
         } else {
-            if (tid == 0) S.cl2[0] = K_INTRA + nd0.intra_mode;
+            if (tid == 0) S.cl2[0] = (K_INTRA + nd0.intra_mode) | (nd0.dct_size ? CL_8 : CL_4);
             SYNC();
-            if (nd0.dct_size) luma_jobs8(S, L, S.cl2, 1, ql, false, true, nullptr);
-            else luma_jobs4(S, L, S.cl2, 1, ql, false, true, nullptr);
+            luma_areas(L, S.cl2, 1, false, true, nullptr, 0);
         }
         SYNC();
         if (P.ref_valid[0]) chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
@@ -1660,7 +1465,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         cfl_blend(S, L, 2);
         zero_acc(S);
         SYNC();
-        chroma_jobs(S, L, 2, 0, qc, true, false, nullptr);
+        chroma_areas(L, 2, 0, true, false, nullptr, 0);
         SYNC();
         if (tid == 0) {
             const long long lam = P.lambda;
@@ -1674,9 +1479,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     const long long best = S.best_cost;
     PHASE_D(6, L.depth);
     // ---- replay of the winner ------------------------------------------
-    // (luma from the scoring pass's cache where it holds the winner)
-    const Node ndw = S.nodes[qt_index(L.depth, L.cx, L.cy)];
-    leaf_code(S, P, L, ql, qc, false, nullptr, !fast && cu <= 16 && !ndw.skip && S.win_slot >= 0);
+    leaf_code(S, P, L, false, nullptr, luma_done ? 2 : 1);
     PHASE_D(7, L.depth);
     return best;
 }
@@ -1689,22 +1492,20 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
 // kept the leaf decision it had then — so its decision (still in
 // S.nodes) and cost (S.node_cost) are reused and only the replay runs.
 template <int D>
-__device__ long long leaf_eval(Smem &S, const FrameParams &P, const Leaf &L, const QuantParams &ql,
-                               const QuantParams &qc, bool cached) {
+__device__ long long leaf_eval(Smem &S, const FrameParams &P, const Leaf &L, bool cached) {
     const int idx = qt_index(L.depth, L.cx, L.cy);
     if (cached) {
         const long long c = S.node_cost[idx];
-        leaf_code(S, P, L, ql, qc, false, nullptr);
+        leaf_code(S, P, L, false, nullptr, 0);
         return c;
     }
-    const long long c = leaf_decide(S, P, L, ql, qc);
+    const long long c = leaf_decide(S, P, L);
     if (threadIdx.x == 0) S.node_cost[idx] = c;
     return c;
 }
 
 template <int D>
-__device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy,
-                          const QuantParams &ql, const QuantParams &qc, bool cached) {
+__device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy, bool cached) {
     constexpr int cu = 64 >> D;
     const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
     const bool in_frame = px + cu <= P.W && py + cu <= P.H;
@@ -1713,7 +1514,7 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
         constexpr int h = 4 >> D;   // child offset in cells
         if (!in_frame) {
             for (int q = 0; q < 4; ++q)
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, ql, qc, false);
+                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, false);
             return;
         }
         const int fast_leaf_depth = P.preset == 0 ? 3 : 2;
@@ -1721,18 +1522,18 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
             if (threadIdx.x == 0) nd.split = 1;
             SYNC();
             for (int q = 0; q < 4; ++q)
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, ql, qc, false);
+                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, false);
             return;
         }
         const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
         snap<D>(S, L, 0, true);
-        const long long parent = leaf_eval<D>(S, P, L, ql, qc, cached);
+        const long long parent = leaf_eval<D>(S, P, L, cached);
         snap<D>(S, L, 1, true);
         snap<D>(S, L, 0, false);
         long long child = 0;
         for (int q = 0; q < 4; ++q) {
             const Leaf C(P, ctu_x, ctu_y, D + 1, cx + (q & 1) * h, cy + (q >> 1) * h);
-            child += leaf_eval<D + 1>(S, P, C, ql, qc, false);
+            child += leaf_eval<D + 1>(S, P, C, false);
         }
         if (child <= parent) {
             if (threadIdx.x == 0) nd.split = 1;
@@ -1742,7 +1543,7 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
             bool same_state = true;
             for (int q = 0; q < 4; ++q) {
                 const int qx = cx + (q & 1) * h, qy = cy + (q >> 1) * h;
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, qx, qy, ql, qc, same_state);
+                qt_decide<D + 1>(S, P, ctu_x, ctu_y, qx, qy, same_state);
                 if (S.nodes[qt_index(D + 1, qx, qy)].split) same_state = false;
             }
         } else {
@@ -1752,31 +1553,29 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
     } else {
         if (!in_frame) return;
         const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-        leaf_eval<D>(S, P, L, ql, qc, cached);
+        leaf_eval<D>(S, P, L, cached);
         if (threadIdx.x == 0) nd.split = 0;
         SYNC();
     }
 }
 
 template <int D>
-__device__ void qt_write(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy,
-                         const QuantParams &ql, const QuantParams &qc, CtuOut *out) {
+__device__ void qt_write(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy, CtuOut *out) {
     constexpr int cu = 64 >> D;
     const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
     const bool in_frame = px + cu <= P.W && py + cu <= P.H;
     if constexpr (D < 3) {
         constexpr int h = 4 >> D;
         if (!in_frame || S.nodes[qt_index(D, cx, cy)].split) {
-            if (!in_frame && false) return;
             for (int q = 0; q < 4; ++q)
-                qt_write<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, ql, qc, out);
+                qt_write<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, out);
             return;
         }
     } else {
         if (!in_frame) return;
     }
     const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-    leaf_code(S, P, L, ql, qc, true, out);
+    leaf_code(S, P, L, true, out, 0);
 }
 
 // ====================================================================
@@ -1943,27 +1742,23 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
 
     // Quantiser parameters in shared memory: every residual job reads them
     // at fixed offsets.
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < 4; ++b) {
-            S.qparam[0].set_band(b, P.eff_l[b], P.rcp_l[b]);
-            S.qparam[1].set_band(b, P.eff_c[b], P.rcp_c[b]);
-        }
-        S.qparam[0].lambda = P.lambda;
-        S.qparam[1].lambda = P.lambda_c;
+    if (threadIdx.x < 8) {
+        const int b = threadIdx.x & 3;
+        if (threadIdx.x < 4) S.qparam[0].set_band(b, P.eff_l[b], P.rcp_l[b], P.lambda);
+        else S.qparam[1].set_band(b, P.eff_c[b], P.rcp_c[b], P.lambda_c);
     }
     SYNC();
-    const QuantParams &ql = S.qparam[0], &qc = S.qparam[1];
 
     // ---- decide, then write in syntax order ----------------------------
     PHASE_T0();
-    qt_decide<0>(S, P, ctu_x, ctu_y, 0, 0, ql, qc, false);
+    qt_decide<0>(S, P, ctu_x, ctu_y, 0, 0, false);
     PHASE(8);
     for (int i = threadIdx.x; i < 64; i += NT) {
         S.grid[i].dx = 0; S.grid[i].dy = 0; S.grid[i].intra = 1;
     }
     SYNC();
     CtuOut *out = P.out + row * P.ctu_cols + col;
-    qt_write<0>(S, P, ctu_x, ctu_y, 0, 0, ql, qc, out);
+    qt_write<0>(S, P, ctu_x, ctu_y, 0, 0, out);
     SYNC();
     PHASE(9);
     // ---- in-loop filters ------------------------------------------------
@@ -1995,6 +1790,14 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     }
 }
 
+// The transform fragments (forward and inverse, 8x8 and 4x4) of every lane,
+// once per CTA.
+__device__ void init_fragments(Smem &S) {
+    if (threadIdx.x < 128)
+        S.frag[threadIdx.x >> 5][threadIdx.x & 31] =
+            dct_fragment(threadIdx.x < 64 ? 8 : 4, (threadIdx.x >> 5) & 1, threadIdx.x & 31);
+}
+
 // One CTA per CTU of one anti-diagonal (items[blockIdx.x]).
 __global__ void __launch_bounds__(NT, CTAS_PER_SM)
 ctu_kernel(const FrameParams *__restrict__ params, const int *__restrict__ items) {
@@ -2003,6 +1806,7 @@ ctu_kernel(const FrameParams *__restrict__ params, const int *__restrict__ items
     FrameParams &P = g_fp;
     const int item = items[blockIdx.x];
     if (threadIdx.x == 0) P = params[item >> 20];
+    init_fragments(S);
     SYNC();
     encode_ctu(S, P, (item >> 10) & 1023, item & 1023);
 }
@@ -2035,6 +1839,7 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
     Smem &S = *reinterpret_cast<Smem *>(smem_raw);
     FrameParams &P = g_fp;
     __shared__ int s_item;
+    init_fragments(S);    // visible to all after the first item's barrier
 #ifdef TCB_PHASE_PROFILE
     const long long k0 = clock64();   // residency of the CTA (slot 14); neighbour waits in slot 13
 #endif
@@ -2312,11 +2117,10 @@ __device__ __forceinline__ int dq_eff(const QuantParams &qp, int pos, int n) {
 }
 
 // 8x8 TU from levels on an octet; writes pred + residual into the tile.
-__device__ void dec_luma8(Smem &S, const Leaf &L, int slot, const int16_t *lv, const QuantParams &qp) {
+__device__ void dec_luma8(Smem &S, const Leaf &L, const int16_t *lv, const QuantParams &qp) {
     const int cu = L.cu, ntu = cu >> 3, J = ntu * ntu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, oct = lane >> 3, l8 = lane & 7;
     int *scr = S.scratch[warp] + oct * 64;
-    const int dc = S.dc;
     for (int base = 0; base < J; base += NW * 4) {
         const int t = base + warp * 4 + oct;
         const int t0 = t < J ? t : 0, ty0 = t0 / ntu, tx0 = t0 - ty0 * ntu;
@@ -2348,19 +2152,18 @@ __device__ void dec_luma8(Smem &S, const Leaf &L, int slot, const int16_t *lv, c
             for (int n = 0; n < 8; ++n) acc += (long long)c_dct8[n][k] * col[n];
             const int r = (int16_t)(int)((acc + 8192) >> 14);
             const int y = ty * 8 + k;
-            if (act) RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(lpred(S, cu, slot, dc, x, y) + r, 0, 255);
+            if (act) RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(S.pred[0][y * cu + x] + r, 0, 255);
         }
     }
 }
 
 // 4x4 TUs from levels on quads.  Luma: per 8x8 TU four sub-blocks in
 // raster order; chroma (chroma_c >= 0): (cs/4)^2 TUs of that component.
-__device__ void dec_tu4(Smem &S, const Leaf &L, int slot, int chroma_c, const int16_t *lv,
+__device__ void dec_tu4(Smem &S, const Leaf &L, int chroma_c, const int16_t *lv,
                         const QuantParams &qp) {
     const int cu = L.cu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, l4 = lane & 3;
     int *scr = S.scratch[warp] + qd * 16;
-    const int dc = S.dc;
     const int cs = cu >> 1;
     const int J = chroma_c >= 0 ? (cs >> 2) * (cs >> 2) : (cu >> 3) * (cu >> 3) * 4;
     for (int base = 0; base < J; base += NW * 8) {
@@ -2410,7 +2213,7 @@ __device__ void dec_tu4(Smem &S, const Leaf &L, int slot, int chroma_c, const in
                 const int v = clampi((int)S.cpred[chroma_c][y * cs + x] + r, 0, 255);
                 RC(S, chroma_c, (L.lx >> 1) + x, (L.ly >> 1) + y) = (uint8_t)v;
             } else {
-                RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(lpred(S, cu, slot, dc, x, y) + r, 0, 255);
+                RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(S.pred[0][y * cu + x] + r, 0, 255);
             }
         }
     }
@@ -2429,10 +2232,13 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
     const int mvx = (int16_t)(mvpx + L.px * 4 + (use_mvd ? nd.mvd_x : 0));
     const int mvy = (int16_t)(mvpy + L.py * 4 + (use_mvd ? nd.mvd_y : 0));
     const bool bidir = P.frame_type == 2;
-    int slot = 0;
     if (nd.intra) {
-        build_refs(S, L, nd.intra_mode < 18 ? 1u << nd.intra_mode : 0u);
-        slot = K_INTRA + nd.intra_mode;
+        build_refs(L);
+        const int lg = lg2i(cu) - 1;
+        for (int i = threadIdx.x; i < cu * cu / 2; i += NT)
+            *(uint16_t *)(S.pred[0] + 2 * i) =
+                (uint16_t)intra2(S, cu, nd.intra_mode, 2 * (i & (cu / 2 - 1)), i >> lg);
+        SYNC();
     } else {
         int r1 = -1, r2 = -1;
         if (bidir) {
@@ -2457,7 +2263,6 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
             for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
             SYNC();
         }
-        slot = 0;
     }
     if (nd.skip) {
         for (int i = threadIdx.x; i < cu * cu; i += NT) {
@@ -2470,8 +2275,8 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
         return;
     }
     // Luma residual: each 8x8 region carries its own TU-size flag.
-    dec_luma8(S, L, slot, el, ql);
-    dec_tu4(S, L, slot, -1, el, ql);
+    dec_luma8(S, L, el, ql);
+    dec_tu4(S, L, -1, el, ql);
     SYNC();
     // Chroma prediction.
     if (nd.intra) {
@@ -2489,8 +2294,8 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
         if (r >= 0) chroma_mc_bi(S, P, L, r, -1, mvx, mvy);
         else chroma_dc_pred(S, L, 0);
     }
-    dec_tu4(S, L, 0, 0, ec, qc);
-    dec_tu4(S, L, 0, 1, ec + (cu >> 1) * (cu >> 1), qc);
+    dec_tu4(S, L, 0, ec, qc);
+    dec_tu4(S, L, 1, ec + (cu >> 1) * (cu >> 1), qc);
     SYNC();
     if (threadIdx.x == 0) S.ncoef += cu * cu + (cu * cu >> 1);
     grid_update(S, L, nd, mvpx, mvpy);
@@ -2550,12 +2355,10 @@ decode_kernel(const FrameParams *__restrict__ params, const int *__restrict__ it
     if (threadIdx.x == 0) { S.ncoef = 0; S.tu8mask = rec->tu8mask; }
     SYNC();
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 4; ++b) {
-            S.qparam[0].set_band(b, P.eff_l[b], P.rcp_l[b]);
-            S.qparam[1].set_band(b, P.eff_c[b], P.rcp_c[b]);
+        for (int b = 0; b < 4; ++b) {   // the decoder reads the quantiser steps only
+            S.qparam[0].eff[b] = P.eff_l[b];
+            S.qparam[1].eff[b] = P.eff_c[b];
         }
-        S.qparam[0].lambda = 0;
-        S.qparam[1].lambda = 0;
     }
     SYNC();
     const QuantParams &ql = S.qparam[0], &qc = S.qparam[1];

@@ -30,11 +30,15 @@ enum {
     K_INTRA = 5,    // intra modes 0..17 -> slots 5..22
     NCAND = 23
 };
-constexpr int NPRED = 5;
-#ifndef TCB_IPRED_MAX
-#define TCB_IPRED_MAX 32
-#endif
-constexpr int IPRED_MAX = TCB_IPRED_MAX;   // largest leaf whose intra predictions are kept            // inter prediction buffers (slots 0..4)
+constexpr int NPRED = 5;            // inter prediction buffers (slots 0..4)
+
+// Entry of a leaf's candidate list: the slot and which TU sizes are scored.
+enum {
+    CL_SLOT = 0xFF,
+    CL_8 = 0x100,       // one 8x8 TU per 8x8 area
+    CL_4 = 0x200,       // four 4x4 TUs per 8x8 area
+    CL_EXACT = 0x400    // note whether the prediction equals the source
+};
 
 struct MeGroup {
     int part[2][32];    // per-warp partial sums, double-buffered (see group_int_sads)
@@ -57,9 +61,8 @@ struct Smem {
     uint8_t pred[NPRED][64 * 64];
     uint8_t cpred[4][32 * 32];
     uint8_t ra[2 * 64 + 4], rl[2 * 64 + 4];     // index i+1 holds ref[i], i in -1..2N
-    uint8_t ipred[18][IPRED_MAX * IPRED_MAX];    // intra predictions of the current leaf (<= IPRED_MAX)
-    uint32_t ipred_ok;                           // modes held in ipred
-    int scratch[NW][288];     // per warp: 4 octets x 72 or 8 quads x 20 ints (padded rows)
+    int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
+    uint4 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
     // Luma reconstruction of every scored candidate of the current leaf
@@ -69,12 +72,12 @@ struct Smem {
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
     int acc_sse[NCAND][2];
     int acc_bits[NCAND][2];
-    long long acc64[4];
+    long long acc64;
     int cl[NCAND];             // candidate list for job loops
-    int cl2[8];                // 8x8-only candidates (merges)
+    int cl2[1];                // the one candidate a replay codes
     int cand_mvx[NPRED], cand_mvy[NPRED], cand_ref[NPRED], cand_ref2[NPRED];
-    int ncl, dc, flag;
-    uint8_t dc_u8;             // S.dc as a one-byte prediction source (PredSrc)
+    int dc;
+    int inexact;               // the merge prediction of the current leaf differs from the source
     long long best_cost;
     int sao[3];
     int band_sum[32], band_cnt[32], band_sq[32], band_new[32], band_cand[32];

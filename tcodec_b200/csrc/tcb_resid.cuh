@@ -1,28 +1,44 @@
-// tcb_resid.cuh — fused residual path of one transform unit on a group of
-// lanes of one warp: forward DCT-II (14-bit, two rounded passes) -> JND-band
-// dead-zone quantisation -> RDOQ-lite (keep-vs-zero of |level| == 1) ->
-// bit-model estimate -> centroid dequantisation -> inverse DCT.
+// tcb_resid.cuh — fused residual path of one 8x8 luma area (one 8x8 TU or
+// four 4x4 TUs) or of four 4x4 chroma TUs on one warp: forward DCT-II (14-bit,
+// two rounded passes) -> JND-band dead-zone quantisation -> RDOQ-lite
+// (keep-vs-zero of |level| == 1) -> bit-model estimate -> centroid
+// dequantisation -> inverse DCT -> reconstruction and SSE.
 //
-//   8x8 TU: an "octet" of 8 consecutive lanes, lane r owns row r on the
-//           row pass and column r afterwards.
-//   4x4 TU: a "quad" of 4 consecutive lanes, same ownership.
+// The four transform passes run on the tensor cores (mma.sync f16, f32
+// accumulators) and give the reference's integers exactly:
 //
-// The row<->column exchange goes through a shared-memory scratch private to
-// the lane group: 8 rows of 9 ints per octet (72), 4 rows of 5 ints per quad
-// (20).  The padded rows put the 32 lanes of a warp (four octets at 72-int
-// or eight quads at 20-int offsets) on 32 different banks for both the row
-// writes and the column reads.  All 32 lanes of the
-// warp must call these routines together (they use full-mask shuffles of
-// width 8 / 4); inactive groups pass dummy data and discard the results.
+//  * A matrix entry C (|C| <= 10703) is split as 128 Ch + Cl with
+//    |Ch| <= 84, |Cl| <= 64; the 16 rows of the A operand are the 8 rows of
+//    Ch and the 8 rows of Cl, so one MMA gives both partial sums.
+//  * The first pass multiplies the residuals (|r| <= 255, exact in f16).  The
+//    later passes multiply intermediates t, |t| < 8192, split as 64 th + tl
+//    with 0 <= tl < 64: k = 16 holds [64 C | C] against [th; tl].
+//  * Every product is an integer and every accumulator starts at 1.5 * 2^23,
+//    so its bits are 0x4B400000 + sum as long as |sum| < 2^22.  Residuals of
+//    8-bit pictures have norm <= 2040, a non-zero level dequantises to at
+//    most 1.75 |c| (q eff + eff / 6 with q eff <= |c| + eff / 3 and
+//    eff <= 1.5 |c|), so no intermediate exceeds 3571 and no partial sum
+//    182 * 3571 < 2^20.
+//
+// Data layout: lane l owns row l >> 2, columns 2 (l & 3) and 2 (l & 3) + 1 of
+// the 8x8 area.  That is the C fragment of an m16n8 MMA (rows 0..7: the Ch
+// sums, rows 8..15: the Cl sums of the same positions), and read as the next
+// pass's B fragment it is its transpose, so the row pass feeds the column
+// pass without a shuffle or shared memory.  Four 4x4 TUs are the same code
+// with block-diagonal matrices.
+//
+// Compared with eight (four) lanes per TU and rows exchanged through shared
+// memory: 150 instructions per area and type instead of about 250 per 8x8 TU
+// and 50 per 4x4 TU, in a serial chain of about 150 instead of 1000, and
+// 3 KB of code instead of 38 KB.
 //
 // Arithmetic follows reference src/transform.c:331-439 (dct4_point,
 // dct8_point2, tc_fdct*/tc_idct*_res), src/encoder.c:333-385 (rdoq_level1,
 // count_siglevel_bits, lastpos_cost) and tcodec_common.h:226-246
-// (quant/dequant).  Accumulators are 32-bit: encoder residuals are clipped
-// to [-512, 511], so |coef| <= 4096, |dequant| <= 4096 + eff/2 <= 8037, and
-// the largest inverse-pass sum is 8037 * 43284 / 2^14 * 43284 < 2^30.
+// (quant/dequant).
 #pragma once
 #include <math.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include "tcb_common.cuh"
 
@@ -57,238 +73,158 @@ static inline cudaError_t upload_dct_tables() {
 
 struct QuantParams {
     int eff[4];
-    uint32_t rcp[4];
-    int off[4];           // eff / 3: quantiser rounding offset
-    int bias[4];          // eff / 6: centroid dequantiser bias
-    long long lambda;     // RDOQ lambda
-    __host__ __device__ void set_band(int b, int e, uint32_t r) {
-        eff[b] = e; rcp[b] = r; off[b] = e / 3; bias[b] = e / 6;
+    // Per band: {quant step | dequantiser bias (eff / 6) << 16, reciprocal,
+    // quantiser offset (eff / 3) | (eff <= 1) << 16, RDOQ threshold}.  A level
+    // of magnitude 1 dequantises to dq = eff + eff / 6 and is dropped when
+    // c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference
+    // src/encoder.c:333-355), i.e. when dq (2 |c| - dq) < lambda: for the
+    // |c| below ceil((dq + ceil(lambda / dq)) / 2).
+    uint4 band[4];
+    __host__ __device__ void set_band(int b, int e, uint32_t r, long long lambda) {
+        const int dq = e + e / 6;
+        const long long thr = ((lambda + dq - 1) / dq + dq + 1) >> 1;
+        eff[b] = e;
+        band[b].x = (uint32_t)e | (uint32_t)(e / 6) << 16;
+        band[b].y = r;
+        band[b].z = (uint32_t)(e / 3) | (e <= 1 ? 1u << 16 : 0u);
+        band[b].w = (uint32_t)(thr < 0x7FFFFFFF ? thr : 0x7FFFFFFF);
     }
 };
 
-// Frequency band of coefficient (row k, column col) of an N x N TU in
-// raster order: DC, first quarter, second quarter, rest (the raster-index
-// bands of freq_band).  With k a compile-time constant only the DC case
-// depends on col.
-template <int N>
-__device__ __forceinline__ int band_rc(int k, int col) {
-    if (k == 0) return col == 0 ? 0 : 1;
-    if (N == 8) return k < 2 ? 1 : (k < 4 ? 2 : 3);
-    return k < 2 ? 2 : 3;
-}
+// Frequency band of coefficient (row r, column c) of an N x N TU in raster
+// order: DC, first quarter, second quarter, rest (the raster-index bands of
+// freq_band).
+__device__ __forceinline__ int band_rc(int N, int r, int c) { return freq_band(r * N + c, N * N); }
 
-__device__ __forceinline__ int oct_sum(int v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 4, 8);
-    v += __shfl_xor_sync(0xffffffffu, v, 2, 8);
-    v += __shfl_xor_sync(0xffffffffu, v, 1, 8);
-    return v;
-}
-__device__ __forceinline__ int oct_max(int v) {
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 4, 8));
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 2, 8));
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 1, 8));
-    return v;
-}
-__device__ __forceinline__ int quad_sum(int v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 2, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 1, 4);
-    return v;
-}
-__device__ __forceinline__ int quad_max(int v) {
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 2, 4));
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 1, 4));
-    return v;
-}
-
-// Quantise + RDOQ-lite one coefficient of band `band` (reference
-// src/encoder.c:333-355): dead-zone quantiser with offset eff / 3, then a
-// level of magnitude 1 is dropped when zero costs less.
-__device__ __forceinline__ int quant_rdoq(int c, int band, const QuantParams &qp) {
-    const int eff = qp.eff[band];
-    const uint32_t rcp = qp.rcp[band];
-    const int off = qp.off[band];
-    int q = 0;
-    if (c > 0) q = udiv_rcp((uint32_t)(c + off), eff, rcp);
-    else if (c < 0) q = -udiv_rcp((uint32_t)(-c + off), eff, rcp);
-    if (q == 1 || q == -1) {
-        // zero wins when c^2 + lambda < (c - dq)^2 + 2 lambda, i.e. when
-        // dq * (2c - dq) < lambda; |c| <= 2^15 and |dq| <= 9194 keep the
-        // product below 2^30
-        const int dq = q > 0 ? eff + qp.bias[band] : -eff - qp.bias[band];
-        if ((long long)(dq * (2 * c - dq)) < qp.lambda) q = 0;
+// A fragments of the forward (inv 0) or inverse (inv 1) transform for this
+// lane: {64 Ch, 64 Cl, Ch, Cl} of matrix row lane >> 2, columns
+// 2 (lane & 3) + {0, 1}; N = 4: two 4x4 matrices on the diagonal.
+__device__ inline uint4 dct_fragment(int N, int inv, int lane) {
+    const int m = lane >> 2;
+    float ch[2], cl[2];
+    for (int e = 0; e < 2; ++e) {
+        const int k = 2 * (lane & 3) + e;
+        int c = 0;
+        if (N == 8) c = inv ? c_dct8[k][m] : c_dct8[m][k];
+        else if ((k >> 2) == (m >> 2)) c = inv ? c_dct4[k & 3][m & 3] : c_dct4[m & 3][k & 3];
+        const int h = (c + 64) >> 7;
+        ch[e] = (float)h;
+        cl[e] = (float)(c - 128 * h);
     }
+    auto pack = [](float a, float b) {
+        const __half2 v = __floats2half2_rn(a, b);
+        return *reinterpret_cast<const uint32_t *>(&v);
+    };
+    return make_uint4(pack(64.f * ch[0], 64.f * ch[1]), pack(64.f * cl[0], 64.f * cl[1]), pack(ch[0], ch[1]),
+                      pack(cl[0], cl[1]));
+}
+
+constexpr float MMA_BIAS = 12582912.0f;                  // 1.5 * 2^23, bits 0x4B400000
+// -(0x4B400000 * 129) mod 2^32 plus the rounding term of the 14-bit shift
+constexpr uint32_t MMA_UNBIAS = 0u - 0x4B400000u * 129u + 8192u;
+
+__device__ __forceinline__ void mma_k8(float d[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    d[0] = d[1] = d[2] = d[3] = MMA_BIAS;
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+__device__ __forceinline__ void mma_k16(float d[4], const uint4 a, uint32_t b0, uint32_t b1) {
+    d[0] = d[1] = d[2] = d[3] = MMA_BIAS;
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+// Rounded 14-bit result of one position from its two partial sums (+ bias).
+template <int BIAS>
+__device__ __forceinline__ int mma_round(float hi, float lo) {
+    return (int)((__float_as_uint(hi) << 7) + __float_as_uint(lo) + (MMA_UNBIAS + (uint32_t)BIAS * 16384u)) >> 14;
+}
+__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
+    const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+// B fragment halves of two intermediates given as t + 8192 (0..16383):
+// hi = half2(t >> 6), lo = half2(t & 63).  0x6400 | v is the half 1024 + v.
+__device__ __forceinline__ void split_b(int t0, int t1, uint32_t &hi, uint32_t &lo) {
+    const uint32_t pk = __byte_perm((uint32_t)t0, (uint32_t)t1, 0x5410);
+    lo = h2_sub((pk & 0x003F003Fu) | 0x64006400u, 0x64006400u);            // - 1024
+    hi = h2_sub(((pk >> 6) & 0x03FF03FFu) | 0x64006400u, 0x64806480u);     // - (1024 + 8192 / 64)
+}
+// Two 8-bit samples (low 16 bits of v) as half2(1024 + v0, 1024 + v1).
+__device__ __forceinline__ uint32_t bytes_h2(uint32_t v) { return __byte_perm(v, 0x64u, 0x4140); }
+
+// One coefficient: dead-zone quantiser with RDOQ-lite.  Returns the level's
+// magnitude; dq is the signed dequantised value.
+__device__ __forceinline__ int quant_one(int c, const uint4 b, int &dq) {
+    const int a = absi(c);
+    const uint32_t n = (uint32_t)a + (b.z & 0xFFFFu);
+    int q = (int)(__umulhi(n, b.y) + n * (b.z >> 16));     // step <= 1: reciprocal 0, level n
+    if (q == 1 && a < (int)b.w) q = 0;
+    const int m = q ? q * (int)(b.x & 0xFFFFu) + (int)(b.x >> 16) : 0;
+    dq = c < 0 ? -m : m;
     return q;
 }
 
-__device__ __forceinline__ int dequant_band(int q, int band, const QuantParams &qp) {
-    const int eff = qp.eff[band], bias = qp.bias[band];
-    return q > 0 ? q * eff + bias : (q < 0 ? q * eff - bias : 0);
+// What the warp knows of one coded area.
+struct AreaCode {
+    int q0, q1;        // this lane's signed levels
+    uint32_t rec;      // this lane's two reconstructed samples (low 16 bits)
+    uint32_t sums;     // this lane's SSE << 10 | bit lengths of its levels
+};
+
+// Codes the area whose samples this lane holds two of: cv (source) and pv
+// (prediction), 16 bits each, with the transform fragments f / i and the
+// quantiser bands b0 / b1 of the lane's two positions.  All 32 lanes.
+__device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint4 f, const uint4 i, const uint4 b0,
+                                              const uint4 b1) {
+    AreaCode r;
+    float d[4];
+    uint32_t hi, lo;
+    mma_k8(d, f.z, f.w, h2_sub(bytes_h2(cv), bytes_h2(pv)));
+    split_b(mma_round<8192>(d[0], d[2]), mma_round<8192>(d[1], d[3]), hi, lo);
+    mma_k16(d, f, hi, lo);
+    const int c0 = mma_round<0>(d[0], d[2]), c1 = mma_round<0>(d[1], d[3]);
+    int dq0, dq1;
+    const int m0 = quant_one(c0, b0, dq0), m1 = quant_one(c1, b1, dq1);
+    r.q0 = c0 < 0 ? -m0 : m0;
+    r.q1 = c1 < 0 ? -m1 : m1;
+    split_b(dq0 + 8192, dq1 + 8192, hi, lo);
+    mma_k16(d, i, hi, lo);
+    split_b(mma_round<8192>(d[0], d[2]), mma_round<8192>(d[1], d[3]), hi, lo);
+    mma_k16(d, i, hi, lo);
+    const int v0 = clampi((int)(pv & 0xFF) + mma_round<0>(d[0], d[2]), 0, 255);
+    const int v1 = clampi((int)(pv >> 8) + mma_round<0>(d[1], d[3]), 0, 255);
+    const int e0 = (int)(cv & 0xFF) - v0, e1 = (int)(cv >> 8) - v1;
+    r.rec = (uint32_t)v0 | (uint32_t)v1 << 8;
+    r.sums = ((uint32_t)(e0 * e0 + e1 * e1) << 10) + (uint32_t)(bitlen((unsigned)m0) + bitlen((unsigned)m1));
+    return r;
 }
 
-// Bit-model term of one quantised level (reference src/encoder.c:360-370).
-__device__ __forceinline__ int level_bits(int v) {
-    return v == 0 ? 1 : 2 + 2 * bitlen((unsigned)absi(v));
+// Bit estimate of a TU without its levels' bit lengths.  The reference counts
+// 1 + 2 nz, a level term (1 for a zero, 2 + 2 bitlen otherwise) for every
+// position up to the last and the last position's cost
+// (src/encoder.c:360-385): with B the sum of the bit lengths that is
+// 2 B + 2 + 3 nz + last + lastpos_cost(last), last = -1 for an empty TU.
+__device__ __forceinline__ int tu_base_bits(int nz, int last) { return 2 + 3 * nz + last + lastpos_cost(last); }
+
+// The 8x8 TU of the area: raster position of (lane, e) is 2 lane + e.
+__device__ __forceinline__ int base_bits8(const AreaCode &c) {
+    const unsigned n0 = __ballot_sync(0xffffffffu, c.q0 != 0), n1 = __ballot_sync(0xffffffffu, c.q1 != 0);
+    const unsigned any = n0 | n1;
+    const int h = 31 - __clz((int)any);
+    const int last = any ? 2 * h + (int)((n1 >> h) & 1u) : -1;
+    return tu_base_bits(__popc(n0) + __popc(n1), last);
 }
 
-// Exact 8- and 4-point DCT sums by partial butterflies.  The 14-bit
-// matrices keep the cosine symmetries exactly (lround is odd-symmetric):
-// c8[k][7-n] = (-1)^k c8[k][n], c8[2m][3-n] = (-1)^m c8[2m][n] for n < 4,
-// c4[k][3-n] = (-1)^k c4[k][n].  So every sum the reference forms,
-// out[k] = sum_n c[k][n] x[n] (forward) or out[n] = sum_k c[k][n] y[k]
-// (inverse), is the same integer from even / odd halves: 24 products per
-// 8-point transform instead of 64, 8 per 4-point instead of 16.
-__device__ __forceinline__ void fdct8_sums(const int x[8], int out[8]) {
-    int E[4], O[4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) { E[n] = x[n] + x[7 - n]; O[n] = x[n] - x[7 - n]; }
-    const int EE0 = E[0] + E[3], EE1 = E[1] + E[2], EO0 = E[0] - E[3], EO1 = E[1] - E[2];
-    out[0] = c_dct8[0][0] * EE0 + c_dct8[0][1] * EE1;
-    out[4] = c_dct8[4][0] * EE0 + c_dct8[4][1] * EE1;
-    out[2] = c_dct8[2][0] * EO0 + c_dct8[2][1] * EO1;
-    out[6] = c_dct8[6][0] * EO0 + c_dct8[6][1] * EO1;
-#pragma unroll
-    for (int k = 1; k < 8; k += 2)
-        out[k] = c_dct8[k][0] * O[0] + c_dct8[k][1] * O[1] + c_dct8[k][2] * O[2] + c_dct8[k][3] * O[3];
-}
-__device__ __forceinline__ void idct8_sums(const int y[8], int out[8]) {
-    const int e0 = c_dct8[0][0] * y[0] + c_dct8[4][0] * y[4], e1 = c_dct8[0][1] * y[0] + c_dct8[4][1] * y[4];
-    const int o0 = c_dct8[2][0] * y[2] + c_dct8[6][0] * y[6], o1 = c_dct8[2][1] * y[2] + c_dct8[6][1] * y[6];
-    const int ev[4] = {e0 + o0, e1 + o1, e1 - o1, e0 - o0};
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        const int od = c_dct8[1][n] * y[1] + c_dct8[3][n] * y[3] + c_dct8[5][n] * y[5] + c_dct8[7][n] * y[7];
-        out[n] = ev[n] + od;
-        out[7 - n] = ev[n] - od;
-    }
-}
-__device__ __forceinline__ void fdct4_sums(const int x[4], int out[4]) {
-    const int E0 = x[0] + x[3], E1 = x[1] + x[2], O0 = x[0] - x[3], O1 = x[1] - x[2];
-    out[0] = c_dct4[0][0] * E0 + c_dct4[0][1] * E1;
-    out[2] = c_dct4[2][0] * E0 + c_dct4[2][1] * E1;
-    out[1] = c_dct4[1][0] * O0 + c_dct4[1][1] * O1;
-    out[3] = c_dct4[3][0] * O0 + c_dct4[3][1] * O1;
-}
-__device__ __forceinline__ void idct4_sums(const int y[4], int out[4]) {
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        const int ev = c_dct4[0][n] * y[0] + c_dct4[2][n] * y[2], od = c_dct4[1][n] * y[1] + c_dct4[3][n] * y[3];
-        out[n] = ev + od;
-        out[3 - n] = ev - od;
-    }
-}
-
-// 8x8 TU on an octet.  In: res_row = clipped residual row `l8`.
-// Out: q_col[k] = quantised level at (k, l8); r_col[k] = reconstructed
-// residual at (k, l8) (int16-wrapped like tc_coeff_t); returns the bit
-// estimate 1 + 2*nz + sig/level bits + last-position cost (uniform).
-__device__ __forceinline__ int tu8_code(int l8, const int res_row[8], int *scr,
-                                        const QuantParams &qp, int q_col[8], int r_col[8]) {
-    int t[8];
-    fdct8_sums(res_row, t);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) scr[l8 * 9 + k] = (t[k] + 8192) >> 14;
-    __syncwarp();
-    int col[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) col[i] = scr[i * 9 + l8];
-    __syncwarp();
-    int nz = 0, last = -1, lball = 0;
-    int cs8[8];
-    fdct8_sums(col, cs8);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int c = (int16_t)((cs8[k] + 8192) >> 14);
-        const int pos = k * 8 + l8;
-        const int q = (int16_t)quant_rdoq(c, band_rc<8>(k, l8), qp);
-        q_col[k] = q;
-        if (q) { ++nz; last = pos; }
-        lball += level_bits(q);
-    }
-    // The level bits of positions up to `last` are those of all 64 less one
-    // per zero past it (level_bits(0) == 1), so they need not wait for
-    // `last`: one packed sum (level bits << 8 | nonzero count, at most 2048
-    // and 64) and one max, side by side.
-    const int packed = oct_sum((lball << 8) | nz);
-    last = oct_max(last);
-    nz = packed & 0xFF;
-    const int lb = (packed >> 8) - (63 - last);
-    const int bits = 1 + 2 * nz + lb + lastpos_cost(last);
-    // Dequantise and hand columns back as rows for the inverse row pass.
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        scr[k * 9 + l8] = (int16_t)dequant_band(q_col[k], band_rc<8>(k, l8), qp);
-    }
-    __syncwarp();
-    int row[8];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) row[n] = scr[l8 * 9 + n];
-    __syncwarp();
-    int is8[8];
-    idct8_sums(row, is8);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) scr[l8 * 9 + k] = (is8[k] + 8192) >> 14;
-    __syncwarp();
-#pragma unroll
-    for (int n = 0; n < 8; ++n) col[n] = scr[n * 9 + l8];
-    __syncwarp();
-    idct8_sums(col, is8);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) r_col[k] = (int16_t)((is8[k] + 8192) >> 14);
-    return bits;
-}
-
-// 4x4 TU on a quad (lane l4 owns row / column l4).  Same contract as
-// tu8_code with n = 16 coefficients.
-__device__ __forceinline__ int tu4_code(int l4, const int res_row[4], int *scr,
-                                        const QuantParams &qp, int q_col[4], int r_col[4]) {
-    int t[4];
-    fdct4_sums(res_row, t);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) scr[l4 * 5 + k] = (t[k] + 8192) >> 14;
-    __syncwarp();
-    int col[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) col[i] = scr[i * 5 + l4];
-    __syncwarp();
-    int nz = 0, last = -1, lball = 0;
-    int cs4[4];
-    fdct4_sums(col, cs4);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int c = (int16_t)((cs4[k] + 8192) >> 14);
-        const int pos = k * 4 + l4;
-        const int q = (int16_t)quant_rdoq(c, band_rc<4>(k, l4), qp);
-        q_col[k] = q;
-        if (q) { ++nz; last = pos; }
-        lball += level_bits(q);
-    }
-    // as in tu8_code: all 16 level bits less one per zero past `last`
-    const int packed = quad_sum((lball << 8) | nz);
-    last = quad_max(last);
-    nz = packed & 0xFF;
-    const int lb = (packed >> 8) - (15 - last);
-    const int bits = 1 + 2 * nz + lb + lastpos_cost(last);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        scr[k * 5 + l4] = (int16_t)dequant_band(q_col[k], band_rc<4>(k, l4), qp);
-    }
-    __syncwarp();
-    int row[4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) row[n] = scr[l4 * 5 + n];
-    __syncwarp();
-    int is4[4];
-    idct4_sums(row, is4);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) scr[l4 * 5 + k] = (is4[k] + 8192) >> 14;
-    __syncwarp();
-#pragma unroll
-    for (int n = 0; n < 4; ++n) col[n] = scr[n * 5 + l4];
-    __syncwarp();
-    idct4_sums(col, is4);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r_col[k] = (int16_t)((is4[k] + 8192) >> 14);
-    return bits;
+// The lane's 4x4 TU (lanes of a quarter share bits 4 and 1 of their index,
+// and within it the raster position grows with the lane index).
+__device__ __forceinline__ int base_bits4(const AreaCode &c, int lane) {
+    const unsigned qm = ((lane & 2) ? 0xCCCCCCCCu : 0x33333333u) & ((lane & 16) ? 0xFFFF0000u : 0x0000FFFFu);
+    const unsigned n0 = __ballot_sync(0xffffffffu, c.q0 != 0) & qm, n1 = __ballot_sync(0xffffffffu, c.q1 != 0) & qm;
+    const unsigned any = n0 | n1;
+    const int h = 31 - __clz((int)any);
+    const int last = any ? ((h >> 2) & 3) * 4 + (h & 1) * 2 + (int)((n1 >> h) & 1u) : -1;
+    return tu_base_bits(__popc(n0) + __popc(n1), last);
 }
 
 }  // namespace tcb
