@@ -25,17 +25,12 @@
 #include <mutex>
 
 #include "tcb_engine.cuh"
+#include "tcb_pair16.cuh"
 #include "tcb_pixel.cuh"
 #include "tcb_launch.h"
 #include "tcb_encoder.h"
 
 namespace tcb {
-
-// Motion search patterns (reference src/motion.c:347-367).
-__constant__ int8_t c_hex_large[7][2] = {{0, 0}, {-2, -4}, {2, -4}, {-4, 0}, {4, 0}, {-2, 4}, {2, 4}};
-__constant__ int8_t c_hex_small[7][2] = {{0, 0}, {-1, -2}, {1, -2}, {-2, 0}, {2, 0}, {-1, 2}, {1, 2}};
-__constant__ int8_t c_diamond[5][2] = {{0, 0}, {0, -1}, {-1, 0}, {1, 0}, {0, 1}};
-__constant__ int8_t c_qpel[9][2] = {{0, 0}, {1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, 1}, {1, -1}, {-1, -1}};
 
 #define SYNC() __syncthreads()
 
@@ -85,8 +80,9 @@ __device__ unsigned long long tcb_op_counts[4];
 #define OPCOUNT(k, v) do {} while (0)
 #endif
 
-__device__ __forceinline__ void group_bar(int g) {
-    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(GT) : "memory");
+// Barrier of motion-search group g (named barrier g + 1) of n threads.
+__device__ __forceinline__ void group_bar(int g, int n) {
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(n) : "memory");
 }
 
 // Four bytes from any address.  Reads only the aligned words that hold
@@ -149,14 +145,25 @@ __device__ void mvp_at(const MvCell *grid, int cx, int cy, int &mx, int &my) {
 }
 
 // ====================================================================
-// Motion search on one warp group (reference src/motion.c:384-485).
+// Motion search on one warp group (reference src/motion.c:384-485): the
+// integer stages (me_integer), then, once every search of the leaf is done
+// with them, the quarter-sample refinement (me_qpel).  A group is 128
+// threads, or 256 when a leaf has at most two searches.
 // ====================================================================
 
+// Search patterns (reference src/motion.c:347-367), one nibble (value + 8)
+// per point: large hexagon, small hexagon, diamond.  Point 0 is the centre.
+__host__ __device__ constexpr uint32_t nib7(int a, int b, int c, int d, int e, int f, int g) {
+    return (uint32_t)(a + 8) | (uint32_t)(b + 8) << 4 | (uint32_t)(c + 8) << 8 | (uint32_t)(d + 8) << 12 |
+           (uint32_t)(e + 8) << 16 | (uint32_t)(f + 8) << 20 | (uint32_t)(g + 8) << 24;
+}
 __device__ __forceinline__ void pat_point(int pat, int p, int &dx, int &dy) {
-    if (pat == 0) { dx = c_hex_large[p][0]; dy = c_hex_large[p][1]; }
-    else if (pat == 1) { dx = c_hex_small[p][0]; dy = c_hex_small[p][1]; }
-    else if (pat == 2) { dx = c_diamond[p][0]; dy = c_diamond[p][1]; }
-    else { dx = 0; dy = 0; }
+    const uint32_t px = pat == 0 ? nib7(0, -2, 2, -4, 4, -2, 2) : pat == 1 ? nib7(0, -1, 1, -2, 2, -1, 1)
+                                                                          : nib7(0, 0, -1, 1, 0, 0, 0);
+    const uint32_t py = pat == 0 ? nib7(0, -4, -4, 0, 0, 4, 4) : pat == 1 ? nib7(0, -2, -2, 0, 0, 2, 2)
+                                                                         : nib7(0, -1, 0, 0, 1, 0, 0);
+    dx = (int)(px >> (4 * p) & 15u) - 8;
+    dy = (int)(py >> (4 * p) & 15u) - 8;
 }
 
 __device__ __forceinline__ int lg2i(int v) { return 31 - __clz(v); }
@@ -164,139 +171,75 @@ __device__ __forceinline__ int lg2i(int v) { return 31 - __clz(v); }
 // tiles: 64, 32), else by division (partial CTUs at the frame edge).
 __device__ __forceinline__ int div_p2(int i, int d) { return (d & (d - 1)) == 0 ? i >> lg2i(d) : i / d; }
 
-// SADs of the K <= 7 integer candidates base + pat[p0 + k] * scale, k < K,
-// on the 128 threads of group g; every thread ends with all K values in
-// sad[] (out-of-frame candidates: 0x7FFFFFFF, reference sad_at).  Each warp
-// reduces its lanes' partial sums into S.me[g].part[par]; after the one
-// group barrier every thread adds the partials up itself, and `par` flips so
-// the next call writes the other buffer (a thread can only get to that
-// call's barrier after all threads have read this one's).
-//
-// Work split (4-byte words of the block, blk = 8 << n):
-//   blk >= 32  every thread covers words gt, gt + 128, ... of all K candidates;
-//   blk == 16  64 words: warps 0-1 take candidates 0, 2, 4, 6 and warps 2-3
-//              candidates 1, 3, 5, one word of each per thread;
-//   blk == 8   16 words: each half warp takes one candidate (k = gt >> 4).
-// BIG: only blocks of 32x32 and up reach this copy (the small-block shapes
-// are left out of its code).
-template <bool BIG = false>
-__device__ __forceinline__ void group_int_sads(Smem &S, int g, int gt, int &par, const uint8_t *ref, int s, int W, int H,
-                               const uint8_t *cur, int blk, int pat, int p0, int K, int bx, int by, int scale,
-                               int sad[7]) {
-    const int lgb = lg2i(blk), lgwpr = lgb - 2, lgw = 2 * lgb - 2;   // words per row, words
-    const int wig = gt >> 5, lane = gt & 31;
-    if (gt == 0) OPCOUNT(0, K * blk * blk);
-    int *part = S.me[g].part[par];
-    if (BIG || blk >= 32) {
-        int cx[7], cy[7];
-        bool in[7];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) {
-            int dx = 0, dy = 0;
-            if (k < K) pat_point(pat, p0 + k, dx, dy);
-            cx[k] = bx + dx * scale; cy[k] = by + dy * scale;
-            in[k] = k < K && cx[k] >= 0 && cy[k] >= 0 && cx[k] + blk <= W && cy[k] + blk <= H;
-        }
-        int acc[7] = {0, 0, 0, 0, 0, 0, 0};
-        for (int w = gt; w < (1 << lgw); w += GT) {
-            const int r = w >> lgwpr, c4 = (w & ((1 << lgwpr) - 1)) << 2;
-            const uint32_t cv = *(const uint32_t *)(cur + r * 64 + c4);
-#pragma unroll
-            for (int k = 0; k < 7; ++k)
-                if (in[k]) acc[k] += (int)__vsadu4(ld4u(ref + (size_t)(cy[k] + r) * s + cx[k] + c4), cv);
-        }
-#pragma unroll
-        for (int k = 0; k < 7; ++k)
-            if (k < K) {
-                const int v = (int)__reduce_add_sync(0xffffffffu, (unsigned)acc[k]);
-                if (lane == 0) part[wig * 8 + k] = v;
-            }
-    } else if (blk == 16) {
-        const int kb = gt >> 6, w = gt & 63, r = w >> 2, c4 = (w & 3) << 2;
-        const uint32_t cv = *(const uint32_t *)(cur + r * 64 + c4);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int k = kb + 2 * m;
-            int v = 0;
-            if (k < K) {
-                int dx, dy;
-                pat_point(pat, p0 + k, dx, dy);
-                const int x = bx + dx * scale, y = by + dy * scale;
-                if (x >= 0 && y >= 0 && x + 16 <= W && y + 16 <= H)
-                    v = (int)__vsadu4(ld4u(ref + (size_t)(y + r) * s + x + c4), cv);
-            }
-            if (2 * m < K) {     // warp-uniform
-                v = (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
-                if (lane == 0) part[wig * 8 + m] = v;
-            }
-        }
-    } else {   // blk == 8
-        const int k = gt >> 4, w = gt & 15, r = w >> 1, c4 = (w & 1) << 2;
-        int v = 0;
-        if (k < K) {
-            int dx, dy;
-            pat_point(pat, p0 + k, dx, dy);
-            const int x = bx + dx * scale, y = by + dy * scale;
-            if (x >= 0 && y >= 0 && x + 8 <= W && y + 8 <= H)
-                v = (int)__vsadu4(ld4u(ref + (size_t)(y + r) * s + x + c4),
-                                  *(const uint32_t *)(cur + r * 64 + c4));
-        }
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if ((lane & 15) == 0) part[k] = v;
-    }
-    group_bar(g);
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        if (k < K) {
-            int sum;
-            if (BIG || blk >= 32) sum = part[k] + part[8 + k] + part[16 + k] + part[24 + k];
-            else if (blk == 16) sum = part[((k & 1) * 2) * 8 + (k >> 1)] + part[((k & 1) * 2 + 1) * 8 + (k >> 1)];
-            else sum = part[k];
-            int dx, dy;
-            pat_point(pat, p0 + k, dx, dy);
-            const int x = bx + dx * scale, y = by + dy * scale;
-            sad[k] = (x >= 0 && y >= 0 && x + blk <= W && y + blk <= H) ? sum : 0x7FFFFFFF;
-        }
-    }
-    par ^= 1;
+// SAD of 16 samples at any address against 16 aligned ones.  Reads only the
+// aligned words that hold p[0..15] (see ld4u).
+__device__ __forceinline__ unsigned sad16(const uint8_t *p, const uint4 c, unsigned acc) {
+    const uintptr_t a = (uintptr_t)p;
+    const uint32_t *w = (const uint32_t *)(a & ~(uintptr_t)3), sh = (uint32_t)(a & 3) * 8;
+    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+    const uint32_t w4 = sh ? __ldg(w + 4) : 0u;
+    acc += __vsadu4(__funnelshift_r(w0, w1, sh), c.x);
+    acc += __vsadu4(__funnelshift_r(w1, w2, sh), c.y);
+    acc += __vsadu4(__funnelshift_r(w2, w3, sh), c.z);
+    return acc + __vsadu4(__funnelshift_r(w3, w4, sh), c.w);
+}
+__device__ __forceinline__ unsigned sad8(const uint8_t *p, const uint2 c, unsigned acc) {
+    const uintptr_t a = (uintptr_t)p;
+    const uint32_t *w = (const uint32_t *)(a & ~(uintptr_t)3), sh = (uint32_t)(a & 3) * 8;
+    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = sh ? __ldg(w + 2) : 0u;
+    acc += __vsadu4(__funnelshift_r(w0, w1, sh), c.x);
+    return acc + __vsadu4(__funnelshift_r(w1, w2, sh), c.y);
 }
 
-// One integer stage: `iters` passes over pattern points 1..npts, each point
-// taken relative to the running best (sequential commit, first improvement
-// wins; reference src/motion.c:398-448).
-// with_center: the stage's first batch also takes pattern point 0 (the
-// centre itself, (0, 0) in every pattern), whose SAD becomes the starting
-// bsad, as the search's initial SAD at the centre would (one barrier round
-// fewer per search).
-template <bool BIG = false>
-__device__ void int_stage(Smem &S, int g, int gt, int &par, const uint8_t *ref, int s, int W, int H,
-                          const uint8_t *cur, int blk, int pat, int npts, int iters, int scale,
-                          int &bx, int &by, int &bsad, bool with_center = false) {
-    for (int it = 0; it < iters; ++it) {
-        bool improved = false;
-        int p0 = with_center ? 0 : 1;
-        while (p0 <= npts) {
-            const int K = npts - p0 + 1;
-            int sad[7];
-            group_int_sads<BIG>(S, g, gt, par, ref, s, W, H, cur, blk, pat, p0, K, bx, by, scale, sad);
-            int found = -1, fs = 0;
-            const int k0 = p0 == 0 ? 1 : 0;
-            if (p0 == 0) { bsad = sad[0]; with_center = false; }
-#pragma unroll
-            for (int k = 0; k < 7; ++k)
-                if (found < 0 && k >= k0 && k < K && sad[k] < bsad) { found = k; fs = sad[k]; }
-            if (found < 0) break;
-            int dx, dy;
-            pat_point(pat, p0 + found, dx, dy);
-            bx += dx * scale; by += dy * scale; bsad = fs;
-            improved = true;
-            p0 = p0 + found + 1;
-        }
-        if (!improved) break;
+// The frame plane and block a search works on.
+struct MeBlock {
+    const uint8_t *ref, *cur;   // reference plane, block in S.cur_y
+    int s, W, H, blk;
+    __device__ __forceinline__ bool inside(int x, int y) const {
+        return x >= 0 && y >= 0 && x + blk <= W && y + blk <= H;
     }
+};
+
+// SADs of pattern points p0 .. p0 + K - 1 (K <= 7) around (bx, by), each on
+// an eighth of the group (16 or 32 lanes); out-of-frame points get 0x7FFFFFFF
+// (reference sad_at).  Lane k of every warp returns point p0 + k's SAD.  The
+// results go through part[par], which flips per call: a thread only gets to
+// the next call's barrier after all have read this one's.
+__device__ __forceinline__ int batch_sads(Smem &S, int g, int gt, int nthr, int &par, const MeBlock &M, int pat, int p0,
+                                          int K, int bx, int by, int scale) {
+    const int lpc = nthr >> 3, k = gt / lpc, l = gt & (lpc - 1), lane = gt & 31;
+    unsigned v = 0;
+    bool in = false;
+    if (gt == 0) OPCOUNT(0, K * M.blk * M.blk);
+    if (k < K) {
+        int dx, dy;
+        pat_point(pat, p0 + k, dx, dy);
+        const int x = bx + dx * scale, y = by + dy * scale;
+        in = M.inside(x, y);
+        if (in) {
+            const uint8_t *r = M.ref + (size_t)y * M.s + x;
+            if (M.blk == 8) {
+                if (l < 8) v = sad8(r + (size_t)l * M.s, *(const uint2 *)(M.cur + l * 64), 0);
+            } else {
+                const int lc = lg2i(M.blk) - 4, n = M.blk << lc;
+#pragma unroll 2
+                for (int c = l; c < n; c += lpc) {
+                    const int row = c >> lc, xo = (c & ((1 << lc) - 1)) * 16;
+                    v = sad16(r + (size_t)row * M.s + xo, *(const uint4 *)(M.cur + row * 64 + xo), v);
+                }
+            }
+        }
+    }
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    if (lpc == 32) v += __shfl_xor_sync(0xffffffffu, v, 16);
+    int *part = S.me[g].part[par];
+    if (l == 0) part[k] = in ? (int)v : 0x7FFFFFFF;
+    group_bar(g, nthr);
+    par ^= 1;
+    return lane < K ? part[lane] : 0x7FFFFFFF;
 }
 
 // ---- small hexagon and diamond of blocks up to 16x16 from a SAD table ----
@@ -304,371 +247,285 @@ __device__ void int_stage(Smem &S, int g, int gt, int &par, const uint8_t *ref, 
 // their candidates are looked up in a table of the (2R+1)^2 integer
 // positions around a window centre (R = FrameParams::search_window, 2..5,
 // chosen per frame size by the engine tuning; 4 by default): one position
-// per thread, one barrier per table, instead of one barrier round per batch
-// of candidates.  The table is refilled around the running best when a
-// candidate falls outside it (R >= 2 keeps every pattern point of the new
-// centre inside); the walk (order of candidates, first-improvement commits)
-// is that of int_stage, on the same SAD values, so R changes the speed and
-// never the result.  Two tables alternate in the search's prediction slot
-// (past the quarter-sample anchors), so refilling one never races with a
+// per thread (two threads, half the rows each, in a group of 256), one
+// barrier per table, instead of one barrier round per batch of candidates.
+// The table is refilled around the running best when a candidate falls
+// outside it (R >= 2 keeps every pattern point of the new centre inside); the
+// walk (order of candidates, first-improvement commits) is that of the
+// batched stages, on the same SAD values, so R changes the speed and never
+// the result.  Two tables alternate, so refilling one never races with a
 // lagging thread still reading the other.
-constexpr int WIN_RMAX = 5, WIN_NMAX = 2 * WIN_RMAX + 1, WIN_OFF = 2560;
-static_assert(WIN_OFF + 2 * WIN_NMAX * WIN_NMAX * 4 <= 64 * 64, "SAD tables overflow the 4 KB slot");
-static_assert(WIN_NMAX * WIN_NMAX <= GT, "one table position per thread of the group");
+constexpr int WIN_RMAX = 5, WIN_NMAX = 2 * WIN_RMAX + 1, WIN_WORDS = WIN_NMAX * WIN_NMAX;
+static_assert(2 * WIN_WORDS <= plane_words(8), "SAD tables overflow the group's planes");
+static_assert(WIN_WORDS <= 128, "one table position per thread of the smallest group");
 
 __device__ __forceinline__ int window_radius(int r) { return r >= 2 && r <= WIN_RMAX ? r : 4; }
 
-template <int B>
-__device__ void fill_sad_window(Smem &S, int g, int gt, int buf, const uint8_t *ref, int s, int W, int H,
-                                const uint8_t *cur, int wx, int wy, int R) {
-    const int N = 2 * R + 1;
-    int *tab = (int *)(S.pred[g] + WIN_OFF) + buf * WIN_NMAX * WIN_NMAX;
-    if (gt == 0) OPCOUNT(0, N * N * B * B);
-    if (gt < N * N) {
-        const int x = wx + gt % N - R, y = wy + gt / N - R;
-        int v = 0x7FFFFFFF;
-        if (x >= 0 && y >= 0 && x + B <= W && y + B <= H) {
-            int acc = 0;
-#pragma unroll 2
-            for (int r = 0; r < B; ++r)
-#pragma unroll
-                for (int c = 0; c < B / 4; ++c)
-                    acc += (int)__vsadu4(ld4u(ref + (size_t)(y + r) * s + x + 4 * c),
-                                         *(const uint32_t *)(cur + r * 64 + 4 * c));
-            v = acc;
-        }
-        tab[gt] = v;
-    }
-    group_bar(g);
-}
-
-struct SadWindow {
-    int wx = 0, wy = 0, buf = 0, R = 4;
-    bool valid = false;
-};
-
-// The walk looks up a pass's remaining points all at once, lane p of every
-// warp taking point p, and a ballot finds the first one (in point order)
-// that improves on the running best or leaves the table: the sequential
-// walk's next event.  An improvement is committed and the points after it
-// are looked up around the new best; a point off the table refills the
-// table around the running best (as the sequential walk does on reaching
-// it) and the lookups start again from that point.  Every warp of the group
-// runs the same walk, so the refills stay group-uniform.
-__device__ void int_stage_windowed(Smem &S, int g, int gt, const uint8_t *ref, int s, int W, int H,
-                                   const uint8_t *cur, int blk, int pat, int npts, int iters, SadWindow &win,
-                                   int &bx, int &by, int &bsad) {
-    const int lane = gt & 31;
-    int ldx = 0, ldy = 0;   // this lane's pattern point (lanes 1..npts)
-    if (lane >= 1 && lane <= npts) pat_point(pat, lane, ldx, ldy);
-    for (int it = 0; it < iters; ++it) {
-        bool improved = false;
-        int p0 = 1;
-        while (p0 <= npts) {
-            const bool act = lane >= p0 && lane <= npts;
-            const int x = bx + ldx, y = by + ldy, R = win.R;
-            const bool off = !win.valid || x < win.wx - R || x > win.wx + R || y < win.wy - R || y > win.wy + R;
-            int v = 0x7FFFFFFF;
-            if (act && !off) {
-                const int *tab = (const int *)(S.pred[g] + WIN_OFF) + win.buf * WIN_NMAX * WIN_NMAX;
-                v = tab[(y - win.wy + R) * (2 * R + 1) + (x - win.wx + R)];
-            }
-            const unsigned ev = __ballot_sync(0xffffffffu, act && (off || v < bsad));
-            if (!ev) break;                       // no point of this pass improves
-            const int f = __ffs(ev) - 1;
-            if (__shfl_sync(0xffffffffu, (int)off, f)) {
-                win.buf ^= 1; win.wx = bx; win.wy = by; win.valid = true;
-                if (blk == 16) fill_sad_window<16>(S, g, gt, win.buf, ref, s, W, H, cur, win.wx, win.wy, R);
-                else fill_sad_window<8>(S, g, gt, win.buf, ref, s, W, H, cur, win.wx, win.wy, R);
-                p0 = f;                           // look point f up in the new table
-                continue;
-            }
-            bsad = __shfl_sync(0xffffffffu, v, f);
-            bx += __shfl_sync(0xffffffffu, ldx, f);
-            by += __shfl_sync(0xffffffffu, ldy, f);
-            improved = true;
-            p0 = f + 1;
-        }
-        if (!improved) break;
-    }
-}
-
-// Sum over group g of one int per thread (one barrier, double-buffered as in
-// group_int_sads).
-__device__ __forceinline__ int group_sum(Smem &S, int g, int gt, int &par, int v) {
-    v = (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
-    int *part = S.me[g].part[par];
-    if ((gt & 31) == 0) part[(gt >> 5) * 8] = v;
-    group_bar(g);
-    const int sum = part[0] + part[8] + part[16] + part[24];
-    par ^= 1;
-    return sum;
-}
-
-// Sub-pel SAD of one candidate straight from the reference frame: six-tap
-// diagonal interpolation where the margins allow, else the bilinear sub-pel
-// SAD (reference src/motion.c:308-341 and 450-481).
-__device__ int group_subpel_sad(Smem &S, int g, int gt, int &par, const uint8_t *ref, int s,
-                                const uint8_t *cur, int blk, int qx, int qy, bool six) {
-    const int fx = qx >> 2, fy = qy >> 2, dx = qx & 3, dy = qy & 3;
-    const int lgb = lg2i(blk);
-    int acc = 0;
-    const int total = blk * blk;
-    if (gt == 0) OPCOUNT(1, total);
-    for (int i = gt; i < total; i += GT) {
-        const int yy = i >> lgb, xx = i & (blk - 1);
-        int p;
-        if (six) {
-            p = luma_hv(ref, s, fx + xx, fy + yy, dx, dy);
+__device__ __forceinline__ void fill_sad_window(int g, int gt, int nthr, int *tab, const MeBlock &M, int wx, int wy,
+                                                int R) {
+    const int N = 2 * R + 1, two = nthr >> 8, pos = gt >> two;
+    if (gt == 0) OPCOUNT(0, N * N * M.blk * M.blk);
+    const int py = pos / N, x = wx + pos - py * N - R, y = wy + py - R;
+    const int rows = M.blk >> two, r0 = (gt & two) * rows;
+    const bool in = pos < N * N && M.inside(x, y);
+    unsigned v = 0;
+    if (in) {
+        const uint8_t *r = M.ref + (size_t)(y + r0) * M.s + x, *c = M.cur + r0 * 64;
+        if (M.blk == 16) {
+#pragma unroll 4
+            for (int i = 0; i < rows; ++i) v = sad16(r + (size_t)i * M.s, *(const uint4 *)(c + i * 64), v);
         } else {
-            const uint8_t *q = ref + (size_t)(fy + yy) * s + fx + xx;
-            const int top = interp_qpel(q[0], q[1], dx);
-            const int bot = interp_qpel(q[s], q[s + 1], dx);
-            p = interp_qpel(top, bot, dy);
+#pragma unroll 4
+            for (int i = 0; i < rows; ++i) v = sad8(r + (size_t)i * M.s, *(const uint2 *)(c + i * 64), v);
         }
-        acc += absi((int)cur[yy * 64 + xx] - p);
     }
-    return group_sum(S, g, gt, par, acc);
+    if (two) v += __shfl_xor_sync(0xffffffffu, v, 1);
+    if (pos < N * N) tab[pos] = in ? (int)v : 0x7FFFFFFF;
+    group_bar(g, nthr);
 }
 
-// Quarter-sample anchors of a search of a block up to 16x16 whose eight
-// refinement points all take the six-tap path.  Each point lies within 3
-// quarter samples of the integer best (bx, by) (the eight offsets of c_qpel
-// move the running best by at most one quarter sample each way per point),
-// so its integer part is bx-1..bx, by-1..by, and every sample luma_hv reads
-// for it is one of, relative to (bx-1, by-1):
-//   I   integer samples                  (B+2) x (B+2) bytes
-//   Hh  horizontal half samples f6h      rows by-3 .. by+B+2, columns bx-1 .. bx+B-1
-//   V   vertical half samples f6v        (B+1) rows x (B+2) columns
-//   D   centre half samples f6hv         (B+1) x (B+1)
-// (unclipped six-tap values, reference src/motion.c:70-107), computed once
-// per search by the group into the search's own 4 KB prediction slot, which
-// nothing reads while the searches run.
-template <int B>
-struct QpelAnchors {
-    static constexpr int GI = B + 2, GH = B + 1, GV = B + 2, GD = B + 1;
-    static constexpr int OFF_H = 336, OFF_V = OFF_H + 2 * (B + 6) * GH, OFF_D = OFF_V + 2 * (B + 1) * GV;
-    static constexpr int BYTES = OFF_D + 2 * GD * GD;
-    static_assert(GI * GI <= OFF_H && BYTES <= 64 * 64, "anchor grids overflow the 4 KB slot");
-    uint8_t *I;
-    int16_t *Hh, *V, *D;
-    __device__ explicit QpelAnchors(uint8_t *area)
-        : I(area), Hh((int16_t *)(area + OFF_H)), V((int16_t *)(area + OFF_V)), D((int16_t *)(area + OFF_D)) {}
-
-    __device__ void build(Smem &S, int g, int gt, const uint8_t *ref, int s, int bx, int by) const {
-        const int ox = bx - 1, oy = by - 1;
-        for (int i = gt; i < GI * GI; i += GT) {
-            const int r = i / GI, c = i - r * GI;
-            I[i] = ref[(size_t)(oy + r) * s + ox + c];
-        }
-        for (int i = gt; i < (B + 6) * GH; i += GT) {
-            const int r = i / GH, c = i - r * GH;
-            Hh[i] = (int16_t)f6h(ref + (size_t)(oy - 2 + r) * s, ox + c);
-        }
-        for (int i = gt; i < (B + 1) * GV; i += GT) {
-            const int r = i / GV, c = i - r * GV;
-            V[i] = (int16_t)f6v(ref, s, ox + c, oy + r);
-        }
-        group_bar(g);
-        for (int i = gt; i < GD * GD; i += GT) {
-            const int r = i / GD, c = i - r * GD;
-            const int16_t *h = Hh + r * GH + c;   // half samples of rows oy+r-2 .. oy+r+3
-            D[i] = (int16_t)((h[0] - 5 * h[GH] + 20 * h[2 * GH] + 20 * h[3 * GH] - 5 * h[4 * GH] + h[5 * GH] +
-                              16) >> 5);
-        }
-        group_bar(g);
-    }
-
-    // luma_hv's combination for sample (X, Y) of the grid at phase (dx, dy).
-    __device__ __forceinline__ int sample(int X, int Y, int dx, int dy) const {
-        const uint8_t *ip = I + Y * GI + X;
-        const int a00 = ip[0], a10 = ip[1], a01 = ip[GI], a11 = ip[GI + 1];
-        int b = 0, e = 0, c = 0, f = 0, d = 0;
-        if (dx != 0) { b = Hh[(Y + 2) * GH + X]; e = Hh[(Y + 3) * GH + X]; }
-        if (dy != 0) {
-            c = V[Y * GV + X];
-            if (dx != 0) { f = V[Y * GV + X + 1]; d = D[Y * GD + X]; }
-        }
-        int top, mid, bot;
-        switch (dx) {
-            case 0:  top = a00;               mid = c;               bot = a01; break;
-            case 1:  top = (a00 + b + 1) >> 1; mid = (c + d + 1) >> 1; bot = (a01 + e + 1) >> 1; break;
-            case 2:  top = b;                 mid = d;               bot = e; break;
-            default: top = (b + a10 + 1) >> 1; mid = (d + f + 1) >> 1; bot = (e + a11 + 1) >> 1; break;
-        }
-        int r;
-        switch (dy) {
-            case 0:  r = top; break;
-            case 1:  r = (top + mid + 1) >> 1; break;
-            case 2:  r = mid; break;
-            default: r = (mid + bot + 1) >> 1; break;
-        }
-        return clampi(r, 0, 255);
-    }
-};
-
-// Quarter-pel refinement of a B x B block (B <= 16) from anchors: the eight
-// points of reference src/motion.c:450-481 with their first-improvement
-// commits, one group barrier per point.
-// Quarter-pel refinement straight from the reference frame, for searches
-// whose points may leave the six-tap margins or for blocks above 16x16
-// (out of line: most small-block searches never run it).
-// Six-tap sub-pel SAD of a 32x32 or 64x64 block on column segments: thread
-// gt takes column gt & (blk-1) and blk*blk/128 consecutive rows, walking
-// down them with six-row windows of the integer samples at x, x+1 and of
-// the horizontal half samples at x.  Each new row costs six byte loads and
-// one horizontal six-tap; the vertical (c, f) and centre (d) half samples
-// come from the windows, and the phase combination is luma_hv's (reference
-// src/motion.c:190-260).  luma_hv per sample re-derives up to eleven six-tap
-// filters; this is the same arithmetic on the same samples.
-__device__ int group_subpel_sad_cols(Smem &S, int g, int gt, int &par, const uint8_t *ref, int s,
-                                     const uint8_t *cur, int blk, int qx, int qy) {
-    const int fx = qx >> 2, fy = qy >> 2, dx = qx & 3, dy = qy & 3;
-    const int lgb = lg2i(blk), L = blk * blk / GT;      // rows per thread: 8 or 32
-    const int xx = gt & (blk - 1), y0 = (gt >> lgb) * L, X = fx + xx;
-    if (gt == 0) OPCOUNT(1, blk * blk);
-    int i0[6], i1[6], hw[6];   // rows Y-2 .. Y+3 of the current output row Y
-    const uint8_t *row = ref + (size_t)(fy + y0 - 2) * s + X;
-    auto load_row = [&](const uint8_t *r, int &a, int &b, int &h) {
-        const int m2 = r[-2], m1 = r[-1], c0 = r[0], c1 = r[1], p2 = r[2], p3 = r[3];
-        a = c0; b = c1;
-        h = (m2 - 5 * m1 + 20 * c0 + 20 * c1 - 5 * p2 + p3 + 16) >> 5;
-    };
-#pragma unroll
-    for (int k = 0; k < 5; ++k) load_row(row + (size_t)k * s, i0[k], i1[k], hw[k]);
-    int acc = 0;
-#pragma unroll 1
-    for (int j = 0; j < L; ++j) {
-        load_row(row + (size_t)(j + 5) * s, i0[5], i1[5], hw[5]);
-        const int a00 = i0[2], a10 = i1[2], a01 = i0[3], a11 = i1[3];
-        const int b = hw[2], e = hw[3];
-        const int c = (i0[0] - 5 * i0[1] + 20 * i0[2] + 20 * i0[3] - 5 * i0[4] + i0[5] + 16) >> 5;
-        const int f = (i1[0] - 5 * i1[1] + 20 * i1[2] + 20 * i1[3] - 5 * i1[4] + i1[5] + 16) >> 5;
-        const int d = (hw[0] - 5 * hw[1] + 20 * hw[2] + 20 * hw[3] - 5 * hw[4] + hw[5] + 16) >> 5;
-        int top, mid, bot;
-        switch (dx) {
-            case 0:  top = a00;               mid = c;               bot = a01; break;
-            case 1:  top = (a00 + b + 1) >> 1; mid = (c + d + 1) >> 1; bot = (a01 + e + 1) >> 1; break;
-            case 2:  top = b;                 mid = d;               bot = e; break;
-            default: top = (b + a10 + 1) >> 1; mid = (d + f + 1) >> 1; bot = (e + a11 + 1) >> 1; break;
-        }
-        int r;
-        switch (dy) {
-            case 0:  r = top; break;
-            case 1:  r = (top + mid + 1) >> 1; break;
-            case 2:  r = mid; break;
-            default: r = (mid + bot + 1) >> 1; break;
-        }
-        acc += absi((int)cur[(y0 + j) * 64 + xx] - clampi(r, 0, 255));
-#pragma unroll
-        for (int k = 0; k < 5; ++k) { i0[k] = i0[k + 1]; i1[k] = i1[k + 1]; hw[k] = hw[k + 1]; }
-    }
-    return group_sum(S, g, gt, par, acc);
-}
-
-__device__ __noinline__ void qpel_refine_direct(int g, int gt, int &par, const uint8_t *ref, int s, int W, int H,
-                                                const uint8_t *cur, int blk, int &mx, int &my, int &bsad) {
-    Smem &S = smem_state();
-    for (int p = 1; p < 9; ++p) {
-        const int qx = mx + c_qpel[p][0], qy = my + c_qpel[p][1];
-        const int fx = qx >> 2, fy = qy >> 2;
-        if (fx < 0 || fy < 0 || fx + blk + 1 > W || fy + blk + 1 > H) continue;
-        const bool six = fx >= 2 && fy >= 2 && fx + blk + 2 < W && fy + blk + 2 < H;
-        const int sum = six && blk >= 32 ? group_subpel_sad_cols(S, g, gt, par, ref, s, cur, blk, qx, qy)
-                                         : group_subpel_sad(S, g, gt, par, ref, s, cur, blk, qx, qy, six);
-        if (sum < bsad) { bsad = sum; mx = qx; my = qy; }
-    }
-}
-
-// An 8x8 block's 64 samples leave half the group idle, so the idle half
-// scores the next point around the same best: a pair of points per group
-// barrier, the first improvement committed (the second point is scored
-// again around the new best when the first one wins).  16x16 blocks take
-// one point per barrier.  Either way the commits are the sequential walk's.
-template <int B>
-__device__ void qpel_refine_anchored(Smem &S, int g, int gt, int &par, const uint8_t *ref, int s,
-                                     const uint8_t *cur, int bx, int by, int &mx, int &my, int &bsad) {
-    const QpelAnchors<B> A(S.pred[g]);
-    A.build(S, g, gt, ref, s, bx, by);
-    constexpr int NS = B * B;                     // samples of a point: 64 or 256
-    constexpr int PPP = NS < GT ? GT / NS : 1;    // points per barrier: 2 (8x8) or 1 (16x16)
-    constexpr int SPT = NS > GT ? NS / GT : 1;    // samples per thread and point: 1 or 2
-    static_assert(PPP * NS == GT * SPT && PPP <= 2, "one pass covers the group");
-    const int wig = gt >> 5, lane = gt & 31;
-    const int kk = PPP == 2 ? gt / NS : 0;        // this thread's point of the pair
-    const int i0 = gt & (NS - 1);
-    int p = 1;
-    while (p < 9) {
-        const int K = mini(9 - p, PPP);
-        if (gt == 0) OPCOUNT(1, K * NS);
-        int *part = S.me[g].part[par];
-        int acc = 0;
-        if (kk < K) {
-            const int qx = mx + c_qpel[p + kk][0], qy = my + c_qpel[p + kk][1];
-            const int X0 = (qx >> 2) - (bx - 1), Y0 = (qy >> 2) - (by - 1), dx = qx & 3, dy = qy & 3;
-#pragma unroll
-            for (int j = 0; j < SPT; ++j) {
-                const int i = i0 + j * GT, x = i % B, y = i / B;
-                acc += absi((int)cur[y * 64 + x] - A.sample(X0 + x, Y0 + y, dx, dy));
-            }
-        }
-        acc = (int)__reduce_add_sync(0xffffffffu, (unsigned)acc);   // kk is warp-uniform
-        if (lane == 0) part[wig * 8] = acc;
-        group_bar(g);
-        const int s0 = PPP == 2 ? part[0] + part[8] : part[0] + part[8] + part[16] + part[24];
-        const int s1 = part[16] + part[24];           // the pair's second point (8x8)
-        par ^= 1;
-        int found = -1, fs = 0;
-        if (s0 < bsad) { found = 0; fs = s0; }
-        else if (K > 1 && s1 < bsad) { found = 1; fs = s1; }
-        if (found < 0) {
-            p += K;
-            continue;
-        }
-        mx += c_qpel[p + found][0];
-        my += c_qpel[p + found][1];
-        bsad = fs;
-        p += found + 1;
-    }
-}
-
-__device__ __noinline__ void me_run(Smem &, int g, int gt, const uint8_t *ref, int s, int W, int H,
-                       int lx, int ly, int blk, int center_x, int center_y, int sr) {
+// The integer stages of one search: large hexagon (6 points, 2 passes,
+// scaled), small hexagon (6, 3), diamond (4, 4); each pass takes its points
+// relative to the running best and commits the first improvement
+// (reference src/motion.c:398-448).  A pass scores all its remaining points
+// at once, one lane per point; the first one that improves is the sequential
+// walk's next commit, and the points after it are scored again around it.
+// The first batch also takes the centre, whose SAD the search starts from.
+__device__ __noinline__ void me_integer(int g, int gt, int nthr, int id, const uint8_t *ref, int lx, int ly, int blk,
+                                        int center_x, int center_y, int sr) {
     Smem &S = smem_state();
     ME_T0();
-    const uint8_t *cur = S.cur_y + ly * 64 + lx;
+    const MeBlock M = {ref, S.cur_y + ly * 64 + lx, g_fp.stride_y, g_fp.W, g_fp.H, blk};
+    const int lane = gt & 31;
     int par = 0;
-    int bx = clampi(center_x, 0, W - blk), by = clampi(center_y, 0, H - blk);
-    int bsad = 0;                       // set from the centre by the first batch below
-    const int scale = maxi(1, sr / 4);
-    // large hexagon (6 points, 2 passes, scaled), small hexagon (6, 3),
-    // diamond (4, 4); a loop rather than three inlined copies of the stage
-    // large hexagon (6 points, 2 passes, scaled), then small hexagon (6, 3)
-    // and diamond (4, 4), the last two from SAD tables for blocks up to 16x16
-    int_stage(S, g, gt, par, ref, s, W, H, cur, blk, 0, 6, 2, scale, bx, by, bsad, true);
-    if (blk <= 16) {
-        SadWindow win;
-        win.R = window_radius(g_fp.search_window);
-        int_stage_windowed(S, g, gt, ref, s, W, H, cur, blk, 1, 6, 3, win, bx, by, bsad);
-        int_stage_windowed(S, g, gt, ref, s, W, H, cur, blk, 2, 4, 4, win, bx, by, bsad);
-    } else {
-        int_stage<true>(S, g, gt, par, ref, s, W, H, cur, blk, 1, 6, 3, 1, bx, by, bsad);
-        int_stage<true>(S, g, gt, par, ref, s, W, H, cur, blk, 2, 4, 4, 1, bx, by, bsad);
+    int bx = clampi(center_x, 0, M.W - blk), by = clampi(center_y, 0, M.H - blk);
+    int bsad = 0x7FFFFFFF;
+    bool centre = true;
+    int *tab = (int *)S.plane + g * plane_words(8);
+    int wx = 0, wy = 0, R = -1;         // table around (wx, wy); R < 0: none yet
+    const int radius = window_radius(g_fp.search_window);
+#pragma unroll 1
+    for (int pat = 0; pat < 3; ++pat) {
+        const int npts = pat == 2 ? 4 : 6, scale = pat == 0 ? maxi(1, sr / 4) : 1;
+        const bool table = pat > 0 && blk <= 16;
+        int ldx = 0, ldy = 0;           // this lane's pattern point (lanes 1..npts)
+        if (lane <= npts) pat_point(pat, lane, ldx, ldy);
+#pragma unroll 1
+        for (int it = 0; it < pat + 2; ++it) {
+            bool improved = false;
+            int p0 = 1;
+            while (p0 <= npts) {
+                int v = 0x7FFFFFFF, base = 0;   // lane's SAD; lane of point 0
+                bool off = false;
+                if (table) {
+                    const bool act = lane >= p0 && lane <= npts;
+                    const int x = bx + ldx - wx + R, y = by + ldy - wy + R;
+                    off = act && (R < 0 || x < 0 || x > 2 * R || y < 0 || y > 2 * R);
+                    if (act && !off) v = tab[y * (2 * R + 1) + x];
+                } else {
+                    base = centre ? 0 : p0;
+                    v = batch_sads(S, g, gt, nthr, par, M, pat, base, npts + 1 - base, bx, by, scale);
+                    if (centre) bsad = __shfl_sync(0xffffffffu, v, 0);
+                    centre = false;
+                }
+                const unsigned ev = __ballot_sync(0xffffffffu, off || v < bsad);
+                if (!ev) break;                   // no point of this pass improves
+                const int f = __ffs(ev) - 1;
+                if (__shfl_sync(0xffffffffu, (int)off, f)) {
+                    // off the table: refill it around the running best, as
+                    // the sequential walk does on reaching this point
+                    tab = (int *)S.plane + g * plane_words(8) + (tab == (int *)S.plane + g * plane_words(8) ? WIN_WORDS : 0);
+                    wx = bx; wy = by; R = radius;
+                    fill_sad_window(g, gt, nthr, tab, M, wx, wy, R);
+                    p0 = f;
+                    continue;
+                }
+                bsad = __shfl_sync(0xffffffffu, v, f);
+                bx += scale * __shfl_sync(0xffffffffu, ldx, f + base);
+                by += scale * __shfl_sync(0xffffffffu, ldy, f + base);
+                improved = true;
+                p0 = f + base + 1;
+            }
+            if (!improved) break;
+        }
     }
     ME_MARK(11);
-    // Quarter-pel refinement around the running best, first improvement
-    // commits (reference src/motion.c:450-481).
-    int mx = bx * 4, my = by * 4;
-    const bool inner = bx - 1 >= 2 && by - 1 >= 2 && bx + blk + 2 < W && by + blk + 2 < H;
-    if (inner && blk == 16) {
-        qpel_refine_anchored<16>(S, g, gt, par, ref, s, cur, bx, by, mx, my, bsad);
-    } else if (inner && blk == 8) {
-        qpel_refine_anchored<8>(S, g, gt, par, ref, s, cur, bx, by, mx, my, bsad);
-    } else {
-        qpel_refine_direct(g, gt, par, ref, s, W, H, cur, blk, mx, my, bsad);
+    if (gt == 0) { S.me[id].bx = bx; S.me[id].by = by; S.me[id].best = bsad; }
+}
+
+// ---- quarter-sample refinement from half-sample planes -------------------
+// The eight points of reference src/motion.c:450-481, each taken around the
+// running best with first-improvement commits, stay within 3 quarter samples
+// of the integer best (bx, by).  The group forms once, in the planes of its
+// search, the integer samples and the horizontal, vertical and centre half
+// samples around the block (unclipped six-tap values biased by 208,
+// reference src/motion.c:70-107); a point's sample is then the average of two
+// columns of the half-sample grid averaged over two of its rows (a position
+// on the grid averages a value with itself, which returns it), clamped, as
+// the nine-anchor form of src/motion.c:190-260 has it.  Points whose six-tap
+// support leaves the frame take the bilinear form from the integer samples
+// (src/motion.c:308-341).
+//
+// A word holds the samples at x and x + B / 2, so every whole-sample shift is
+// an index and every operation works on two samples.  All points still to be
+// tried are scored together, a warp per point (per quarter of a point from
+// 32x32 on), and their SADs kept per position: after a commit most points
+// around the new best are already known.  Bound: shared-memory loads and
+// packed integer operations, 9 to 18 instructions per two samples and point
+// where one point at a time from bytes took about 70 per sample.
+__device__ __forceinline__ int plane_div(int i, int blk) {   // i / plane_stride(blk), i < 5000
+    const uint32_t m = blk == 64 ? 65536 / 38 + 1 : blk == 32 ? 65536 / 22 + 1 : blk == 16 ? 65536 / 14 + 1
+                                                                                      : 65536 / 10 + 1;
+    return (int)((uint32_t)i * m >> 16);
+}
+
+__device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *area, const uint8_t *ref, int blk) {
+    Smem &S = smem_state();
+    ME_T0();
+    MeGroup &E = S.me[id];
+    const int s = g_fp.stride_y, W = g_fp.W, H = g_fp.H, B = blk, half = B >> 1, ST = half + 6;
+    const int bx = E.bx, by = E.by, lane = gt & 31, warp = gt >> 5, gw = nthr >> 5;
+    uint32_t *pI = area, *pH = pI + (B + 6) * ST, *pV = pH + (B + 6) * ST, *pD = pV + (B + 1) * ST;
+    // integer samples of rows by - 3 .., columns bx - 3 .. (clamped: samples
+    // outside the frame are never part of a point that is scored)
+    for (int i = gt; i < (B + 6) * ST; i += nthr) {
+        const int r = plane_div(i, B), x = bx - 3 + i - r * ST;
+        const uint8_t *row = ref + (size_t)clampi(by - 3 + r, 0, H - 1) * s;
+        pI[i] = (uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16;
+    }
+    if (gt < QPOS * QPOS) E.tab[gt] = 0;
+    group_bar(g, nthr);
+    // horizontal halves at columns bx - 1 .. (word j reads columns j .. j + 5)
+    // of every row; vertical halves of rows by - 1 .. at columns bx - 1 ..
+    for (int i = gt; i < (B + 6) * ST - 5; i += nthr)
+        pH[i] = pair_six_tap(pI[i], pI[i + 1], pI[i + 2], pI[i + 3], pI[i + 4], pI[i + 5], PAIR_K_RAW);
+    for (int i = gt; i < (B + 1) * ST - 2; i += nthr) {
+        const uint32_t *q = pI + i + 2;
+        pV[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
+    }
+    group_bar(g, nthr);
+    for (int i = gt; i < (B + 1) * ST - 5; i += nthr) {
+        const uint32_t *q = pH + i;
+        pD[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
+    }
+    group_bar(g, nthr);
+
+    // Lane p (1..8) holds point p; the points' offsets as in pat_point.
+    int ox = 0, oy = 0;
+    if (lane >= 1 && lane <= 8) {
+        const uint32_t px = 0x79798879u, py = 0x77997988u;   // (+-1, 0), (0, +-1), then the corners
+        ox = (int)(px >> (4 * (lane - 1)) & 15u) - 8;
+        oy = (int)(py >> (4 * (lane - 1)) & 15u) - 8;
+    }
+    int ux = 3, uy = 3, bsad = E.best, p0 = 1;     // running best: quarter-sample offset + 3
+    unsigned long long known = 0;
+#pragma unroll 1
+    for (;;) {
+        const int cx = ux + ox, cy = uy + oy, fx = (4 * bx + cx - 3) >> 2, fy = (4 * by + cy - 3) >> 2;
+        const bool act = lane >= p0 && lane <= 8 && fx >= 0 && fy >= 0 && fx + B + 1 <= W && fy + B + 1 <= H;
+        const int idx = act ? cy * QPOS + cx : 0;
+        const unsigned need = __ballot_sync(0xffffffffu, act && !(known >> idx & 1ull));
+        if (need) {
+            const int K = __popc(need), lsp = B >= 32 ? 2 : 0, n = (B * half) >> lsp, lgh = lg2i(half);
+            if (gt == 0) OPCOUNT(1, K * B * B);
+            for (int it = warp; it < K << lsp; it += gw) {
+                unsigned m = need;
+                for (int j = it >> lsp; j > 0; --j) m &= m - 1;
+                const int f = __ffs(m) - 1;
+                const int X = __shfl_sync(0xffffffffu, cx, f) + 1, Y = __shfl_sync(0xffffffffu, cy, f) + 1;
+                // position in quarter samples from (bx - 1, by - 1): 1..7
+                const int qfx = bx - 1 + (X >> 2), qfy = by - 1 + (Y >> 2);
+                const uint32_t *cur = S.cur_pair + (it & ((1 << lsp) - 1)) * n;
+                const int y0 = ((it & ((1 << lsp) - 1)) * n) >> lgh;
+                unsigned acc = 0;
+                if (qfx >= 2 && qfy >= 2 && qfx + B + 2 < W && qfy + B + 2 < H) {
+                    // half-grid columns h0, h1 and rows v0, v1: even ones lie
+                    // on samples (planes I, V), odd ones between (H, D); rows
+                    // likewise (I, H / V, D)
+                    const int h0 = X >> 1, h1 = (X + 1) >> 1, v0 = Y >> 1, v1 = (Y + 1) >> 1;
+                    auto at = [&](int v, int h) {
+                        const uint32_t *q = (v & 1) ? ((h & 1) ? pD : pV) + (v >> 1) * ST
+                                                    : ((h & 1) ? pH + 2 * ST : pI + 2 * ST + 2) + (v >> 1) * ST;
+                        return q + (h >> 1) + y0 * ST;
+                    };
+                    // integer samples carry no bias in their plane
+                    const uint32_t *q00 = at(v0, h0), *q01 = at(v0, h1), *q10 = at(v1, h0), *q11 = at(v1, h1);
+                    const uint32_t b00 = (v0 | h0) & 1 ? 0 : PAIR_B, b01 = (v0 | h1) & 1 ? 0 : PAIR_B;
+                    const uint32_t b10 = (v1 | h0) & 1 ? 0 : PAIR_B, b11 = (v1 | h1) & 1 ? 0 : PAIR_B;
+#pragma unroll 4
+                    for (int i = lane; i < n; i += 32) {
+                        const int o = (i >> lgh) * ST + (i & (half - 1));
+                        const uint32_t t = pair_avg(q00[o] + b00, q01[o] + b01);
+                        const uint32_t b = pair_avg(q10[o] + b10, q11[o] + b11);
+                        const uint32_t v = pair_min(pair_max(pair_avg(t, b), PAIR_B), PAIR_B + 255u * 0x00010001u) - PAIR_B;
+                        acc += __vsadu4(v, cur[i]);
+                    }
+                } else {
+                    const uint32_t *q = pI + (2 + (Y >> 2) + y0) * ST + 2 + (X >> 2);
+                    const uint32_t dx = X & 3, dy = Y & 3, k2 = 0x00020002u;
+                    for (int i = lane; i < n; i += 32) {
+                        const int o = (i >> lgh) * ST + (i & (half - 1));
+                        const uint32_t t = ((q[o] * (4 - dx) + q[o + 1] * dx + k2) >> 2) & 0x00FF00FFu;
+                        const uint32_t b = ((q[o + ST] * (4 - dx) + q[o + ST + 1] * dx + k2) >> 2) & 0x00FF00FFu;
+                        acc += __vsadu4(((t * (4 - dy) + b * dy + k2) >> 2) & 0x00FF00FFu, cur[i]);
+                    }
+                }
+                acc = __reduce_add_sync(0xffffffffu, acc);
+                if (lane == 0) atomicAdd(&E.tab[(Y - 1) * QPOS + X - 1], (int)acc);
+            }
+            group_bar(g, nthr);
+            const unsigned long long mine = (need >> lane & 1u) ? 1ull << idx : 0ull;
+            known |= (unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) << 32 |
+                     __reduce_or_sync(0xffffffffu, (unsigned)mine);
+        }
+        const int v = act ? E.tab[idx] : 0x7FFFFFFF;
+        const unsigned ev = __ballot_sync(0xffffffffu, v < bsad);
+        if (!ev) break;
+        const int f = __ffs(ev) - 1;
+        bsad = __shfl_sync(0xffffffffu, v, f);
+        ux = __shfl_sync(0xffffffffu, cx, f);
+        uy = __shfl_sync(0xffffffffu, cy, f);
+        p0 = f + 1;
     }
     ME_MARK(12);
-    if (gt == 0) { S.me[g].mvx = mx; S.me[g].mvy = my; S.me[g].best = bsad; }
+    if (gt == 0) { E.mvx = 4 * bx + ux - 3; E.mvy = 4 * by + uy - 3; E.best = bsad; }
+}
+
+// One search of a leaf: slot id (S.me index), reference plane, start.
+struct MeJob {
+    const uint8_t *ref;
+    int cx, cy;
+};
+
+// The leaf's searches (bits of `mask`, jobs indexed by search id): integer
+// stages on one warp group each, then the refinement; a 64x64 leaf's planes
+// leave room for two refinements at a time.
+__device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, MeJob j0, MeJob j1, MeJob j2, MeJob j3, int sr) {
+    Smem &S = smem_state();
+    const int cu = L.cu, half = cu >> 1, lgh = lg2i(half), n = __popc(mask);
+    for (int i = threadIdx.x; i < cu * half; i += NT) {
+        const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
+        S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
+    }
+    auto nth = [&](int k) {
+        unsigned m = mask;
+        for (; k > 0; --k) m &= m - 1;
+        return m ? __ffs((int)m) - 1 : -1;
+    };
+    auto job = [&](int id) { return id == 0 ? j0 : id == 1 ? j1 : id == 2 ? j2 : j3; };
+    const int nthr = n <= 2 ? 256 : 128, g = threadIdx.x / nthr, gt = threadIdx.x & (nthr - 1);
+    if (g < n) {
+        const int id = nth(g);
+        const MeJob J = job(id);
+        me_integer(g, gt, nthr, id, J.ref, L.lx, L.ly, cu, J.cx, J.cy, sr);
+    }
+    SYNC();   // the SAD tables share the planes' memory
+    const int qthr = cu == 64 ? 256 : nthr, per = NT / qthr, q = threadIdx.x / qthr, qt = threadIdx.x & (qthr - 1);
+    for (int k = q; k < n; k += per) {
+        const int id = nth(k);
+        me_qpel(q, qt, qthr, id, S.plane + q * plane_words(cu), job(id).ref, cu);
+    }
+    SYNC();
 }
 
 // ====================================================================
@@ -1264,7 +1121,6 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     bool has_glb = false, has_tmp = false, has_me1 = false;
     int tdx = 0, tdy = 0;
     const int rf = is_b ? dpb_fwd(P) : -1, rb = is_b ? dpb_bwd(P) : -1;
-    const int g = tid / GT, gt = tid - g * GT;
     const int cx0 = (mvpx + L.px * 4) >> 2, cy0 = (mvpy + L.py * 4) >> 2;
     if (is_p) {
         const int sr = fast ? 16 : 24;
@@ -1278,18 +1134,10 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
                 if (!pg.intra) { has_tmp = true; tdx = pg.dx; tdy = pg.dy; }
             }
         }
-        // ---- motion searches on four warp groups ------------------------
-        if (g == 0)
-            me_run(S, 0, gt, P.ref_y[0], P.stride_y, P.W, P.H, L.lx, L.ly, cu, cx0, cy0, sr);
-        else if (g == 1 && has_me1)
-            me_run(S, 1, gt, P.ref_y[1], P.stride_y, P.W, P.H, L.lx, L.ly, cu, cx0, cy0, sr);
-        else if (g == 2 && has_glb)
-            me_run(S, 2, gt, P.ref_y[0], P.stride_y, P.W, P.H, L.lx, L.ly, cu,
-                   (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2, sr);
-        else if (g == 3 && has_tmp)
-            me_run(S, 3, gt, P.ref_y[0], P.stride_y, P.W, P.H, L.lx, L.ly, cu,
-                   (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2, sr);
-        SYNC();
+        const MeJob j0 = {P.ref_y[0], cx0, cy0}, j1 = {P.ref_y[1], cx0, cy0},
+                    j2 = {P.ref_y[0], (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2},
+                    j3 = {P.ref_y[0], (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2};
+        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, j0, j1, j2, j3, sr);
         PHASE_D(1, L.depth);
         if (has_glb && S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) has_glb = false;
         if (has_tmp && S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) has_tmp = false;
@@ -1312,11 +1160,8 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     } else if (is_b) {
         // Forward / backward searches (reference src/encoder.c:795-852).
         const int sr = fast ? 16 : 32;
-        if (g == 0 && rf >= 0)
-            me_run(S, 0, gt, P.ref_y[rf], P.stride_y, P.W, P.H, L.lx, L.ly, cu, cx0, cy0, sr);
-        else if (g == 1 && rb >= 0)
-            me_run(S, 1, gt, P.ref_y[rb], P.stride_y, P.W, P.H, L.lx, L.ly, cu, cx0, cy0, sr);
-        SYNC();
+        const MeJob j0 = {P.ref_y[maxi(rf, 0)], cx0, cy0}, j1 = {P.ref_y[maxi(rb, 0)], cx0, cy0};
+        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, j0, j1, j0, j1, sr);
         PHASE_D(1, L.depth);
         const uint32_t hf = rf >= 0, hb = rb >= 0, mrg = medium;
         cand = hf | hb << 1 | (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;

@@ -10,8 +10,6 @@ constexpr int NT = 512;             // threads per CTA (one CTU)
 constexpr int CTAS_PER_SM = 1;      // CTUs resident per SM
 constexpr int NW = NT / 32;         // warps per CTA
 constexpr int NGROUP = 4;           // motion-search warp groups
-constexpr int GT = NT / NGROUP;     // threads per motion-search group
-static_assert(GT == 128, "the motion-search work split assumes 4-warp groups");
 
 // Recon tile: luma rows -1..63 and columns -8..63 of the CTU, chroma rows
 // -1..31 and columns -4..31.  Column offsets keep the interior aligned.
@@ -40,13 +38,26 @@ enum {
     CL_EXACT = 0x400    // note whether the prediction equals the source
 };
 
+constexpr int QPOS = 7;               // quarter-sample positions per axis around an integer best: -3..3
 struct MeGroup {
-    int part[2][32];    // per-warp partial sums, double-buffered (see group_int_sads)
+    int part[2][8];         // SADs of a batch of candidates, double-buffered (see batch_sads)
+    int tab[QPOS * QPOS];   // SADs of the quarter-sample positions scored so far
+    int bx, by;             // integer best
     int mvx, mvy, best;
 };
 
+// Sample planes of a quarter-sample refinement (me_qpel) of a B x B block, in
+// 32-bit words that hold two columns B / 2 apart: integer samples and
+// horizontal halves (B + 6 rows), vertical and centre halves (B + 1 rows).
+__host__ __device__ constexpr int plane_stride(int B) { return B / 2 + 6; }
+__host__ __device__ constexpr int plane_words(int B) { return (4 * B + 14) * plane_stride(B); }
+constexpr int PLANES64 = 2;           // searches of a 64x64 leaf refined at a time
+constexpr int PLANE_WORDS = PLANES64 * plane_words(64);
+static_assert(NGROUP * plane_words(32) <= PLANE_WORDS && NGROUP * plane_words(16) <= PLANE_WORDS,
+              "every group's planes fit below 64x64");
+
 struct Smem {
-    uint8_t cur_y[64 * 64];
+    alignas(16) uint8_t cur_y[64 * 64];
     uint8_t cur_c[2][32 * 32];
     uint8_t rec_y[RY_H * RY_W];
     uint8_t rec_c[2][RC_H * RC_W];
@@ -58,17 +69,25 @@ struct Smem {
     MvCell grid[64];
     Node nodes[QT_NODES];
     long long node_cost[QT_NODES];
-    uint8_t pred[NPRED][64 * 64];
-    uint8_t cpred[4][32 * 32];
+    union {
+        // after the searches of a leaf
+        struct {
+            alignas(16) uint8_t pred[NPRED][64 * 64];
+            uint8_t cpred[4][32 * 32];
+            // Luma reconstruction of every scored candidate of the current
+            // leaf (leaves up to 16x16), [slot][8x8 TUs, 4x4 TUs]: the replay
+            // of the winner copies it instead of coding the winner again.
+            uint8_t crec[NCAND][2][16 * 16];
+        };
+        // during them: SAD tables of the integer stages, then sample planes
+        alignas(16) uint32_t plane[PLANE_WORDS];
+    };
+    uint32_t cur_pair[64 * 32];      // leaf's source samples (x, x + cu / 2) as 16-bit lanes, for the searches
     uint8_t ra[2 * 64 + 4], rl[2 * 64 + 4];     // index i+1 holds ref[i], i in -1..2N
     int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
     uint4 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
-    // Luma reconstruction of every scored candidate of the current leaf
-    // (leaves up to 16x16), [slot][8x8 TUs, 4x4 TUs]: the replay of the
-    // winner copies it instead of coding the winner again.
-    uint8_t crec[NCAND][2][16 * 16];
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
     int acc_sse[NCAND][2];
     int acc_bits[NCAND][2];
