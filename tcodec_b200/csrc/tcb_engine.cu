@@ -532,142 +532,180 @@ __device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, MeJob j0, 
 // Leaf helpers
 // ====================================================================
 
-// v2 intra reference samples (reference src/predict.c:480-520): above-right
-// and below-left are replicated.  S.ra[0] / S.rl[0] hold the corner.
+// v2 intra reference samples (reference src/predict.c:480-520): sample i of
+// the above (left) run, i >= 0, those past the block replicating the last.
+//
+// An angular mode interpolates at p = 32 (position along its primary run) +
+// displacement between samples p / 32 + 1 and p / 32 + 2 of that run, or, for
+// p < 0, at -p of the other run (intra_at).  Both cases read one array per
+// direction (0: vertical modes, primary run above; 1: horizontal modes):
+// entry j > 0 is primary sample j, entry j <= 0 is secondary sample 1 - j, and
+// with P = floor(p / 32), f = p mod 32 the prediction is
+// (32 E[k] + (E[k + 1] - E[k]) f + 16) >> 5 at k = P + 1 (p >= 0) or
+// k = P (p < 0), since -p = 32 (-P - 1) + (32 - f).
 __device__ __noinline__ void build_refs(const Leaf L) {
     Smem &S = smem_state();
-    const int N = L.cu;
+    const int N = L.cu, n = 4 * N + 3;
     const bool ha = L.py > 0, hl = L.px > 0;
-    for (int i = threadIdx.x; i <= 2 * N; i += NT) {
-        const int j = i < N ? i : N - 1;
-        int a, l;
-        if (ha) a = RY(S, L.lx + j, L.ly - 1);
-        else a = hl ? RY(S, L.lx - 1, L.ly) : 128;
-        if (hl) l = RY(S, L.lx - 1, L.ly + j);
-        else l = ha ? RY(S, L.lx, L.ly - 1) : 128;
-        S.ra[i + 1] = (uint8_t)a;
-        S.rl[i + 1] = (uint8_t)l;
+    auto sample = [&](bool left, int i) -> int {
+        const int j = mini(i, N - 1);
+        if (left) return hl ? RY(S, L.lx - 1, L.ly + j) : (ha ? RY(S, L.lx, L.ly - 1) : 128);
+        return ha ? RY(S, L.lx + j, L.ly - 1) : (hl ? RY(S, L.lx - 1, L.ly) : 128);
+    };
+    for (int i = threadIdx.x; i < 2 * n; i += NT) {
+        const bool horiz = i >= n;
+        const int j = (horiz ? i - n : i) - 3 * N / 2;
+        S.edge[horiz][EDGE_BASE + j] = (uint8_t)sample(horiz == (j > 0), j > 0 ? j : 1 - j);
     }
-    if (threadIdx.x == 0) {
-        int tl;
-        if (ha && hl) tl = RY(S, L.lx - 1, L.ly - 1);
-        else if (ha) tl = RY(S, L.lx, L.ly - 1);
-        else if (hl) tl = RY(S, L.lx - 1, L.ly);
-        else tl = 128;
-        S.ra[0] = (uint8_t)tl;
-        S.rl[0] = (uint8_t)tl;
-    }
+    if (threadIdx.x == 0) S.above0 = sample(false, 0);
     SYNC();
     if (threadIdx.x < 32) {
         // DC value (reference src/predict.c:140-161): samples 1..N of each run.
         int sum = 0;
-        for (int i = threadIdx.x; i < N; i += 32) sum += S.ra[i + 2] + S.rl[i + 2];
+        for (int i = threadIdx.x + 1; i <= N; i += 32) sum += S.edge[0][EDGE_BASE + i] + S.edge[1][EDGE_BASE + i];
         sum = __reduce_add_sync(0xffffffffu, sum);
-        if (threadIdx.x == 0) S.dc = (sum + N) / (2 * N);
+        if (threadIdx.x == 0) S.dc = (sum + N) >> __ffs(N);   // / (2 N)
     }
     SYNC();
 }
 
 // Intra prediction samples (x, y) and (x + 1, y) of an N x N leaf in the low
-// two bytes (the per-sample form is intra_at; reference
-// src/predict.c:117-340).
-__device__ __forceinline__ uint32_t intra2(const Smem &S, int N, int mode, int x, int y) {
-    const uint8_t *ra = S.ra + 1, *rl = S.rl + 1;
+// two bytes; disp is the mode's angular displacement (the per-sample form is
+// intra_at; reference src/predict.c:117-340).
+__device__ __forceinline__ uint32_t intra2(const Smem &S, int N, int mode, int disp, int x, int y) {
     if (mode == 0) {
-        const int sh = __ffs(N), l = rl[y + 1], c = ra[0];
+        const uint8_t *ra = S.edge[0] + EDGE_BASE;
+        const int sh = __ffs(N), l = S.edge[1][EDGE_BASE + y + 1], c = S.above0;
         const int v0 = (ra[x + 1] * (N - 1 - y) + l * (N - 1 - x) + c * (x + y) + N) >> sh;
         const int v1 = (ra[x + 2] * (N - 1 - y) + l * (N - 2 - x) + c * (x + 1 + y) + N) >> sh;
         return (uint32_t)mini(v0, 255) | (uint32_t)mini(v1, 255) << 8;
     }
     if (mode == 1 || mode > 17) return (uint32_t)S.dc * 0x101u;
     const bool vert = mode < 9;
-    const uint8_t *pri = vert ? ra : rl, *sec = vert ? rl : ra;
-    const int disp = c_ang_disp[mode];
-    const int pos0 = vert ? (x << 5) + y * disp : (y << 5) + x * disp;
-    uint32_t v = 0;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int p = e ? pos0 + (vert ? 32 : disp) : pos0;
-        const uint8_t *src = p >= 0 ? pri : sec;    // a negative position only occurs for disp < 0
-        const int q = absi(p), i0 = (q >> 5) + 1, fr = q & 31;
-        const int a = src[mini(i0, 2 * N)], b = src[mini(i0 + 1, 2 * N)];
-        v |= (uint32_t)(a + (((b - a) * fr + 16) >> 5)) << (8 * e);
-    }
-    return v;
+    const uint8_t *E = S.edge[vert ? 0 : 1] + EDGE_BASE + 1;
+    const int p0 = vert ? (x << 5) + y * disp : (y << 5) + x * disp, p1 = p0 + (vert ? 32 : disp);
+    const uint8_t *e0 = E + (p0 >> 5) + (p0 >> 31), *e1 = E + (p1 >> 5) + (p1 >> 31);
+    const int a0 = e0[0], b0 = e0[1], a1 = e1[0], b1 = e1[1];
+    const uint32_t v0 = (uint32_t)(32 * a0 + 16 + (b0 - a0) * (p0 & 31)) >> 5;
+    const uint32_t v1 = (uint32_t)(32 * a1 + 16 + (b1 - a1) * (p1 & 31)) >> 5;
+    return v0 | v1 << 8;
 }
 
-// Prediction samples (x, y) and (x + 1, y), x even, of a candidate slot.
-__device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int slot, int x, int y) {
+// Entry of a candidate list for slot `slot` with the TU sizes `sizes`.
+__device__ __forceinline__ int cl_entry(int slot, int sizes) {
+    const int m = slot - K_INTRA;
+    return slot | sizes | (m > 1 && m < 18 ? (int)c_ang_disp[m] * 65536 : 0);
+}
+// Prediction samples (x, y) and (x + 1, y), x even, of a candidate (list entry e).
+__device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, int y) {
+    const int slot = e & CL_SLOT;
     if (slot < NPRED) return *(const uint16_t *)(S.pred[slot] + y * cu + x);
-    return intra2(S, cu, slot - K_INTRA, x, y);
+    return intra2(S, cu, slot - K_INTRA, e >> 16, x, y);
 }
 
-// Luma residual coding of the listed candidates: one warp per (candidate,
-// 8x8 area), with one 8x8 TU, four 4x4 TUs or both (reference
-// src/encoder.c:476-560; the four-TU form has an outer flag bit).  `accum`
-// adds distortion and bits to the slot's sums and keeps the reconstruction of
-// leaves up to 16x16; `wrec` writes the reconstruction, `emit` the levels in
-// syntax order.  `woff` rotates the warps the areas start on.
+// Scores the listed candidates: distortion and bits of one 8x8 TU, of four
+// 4x4 TUs, or of both per 8x8 area, added to the slots' sums (reference
+// src/encoder.c:476-560; the four-TU form has an outer flag bit).  Keeps the
+// reconstructions of leaves up to 16x16.
 //
-// Bound: issue slots (150 instructions per area and type, four warps a
-// scheduler); an area on a warp keeps the chain of a leaf with fewer areas
-// than warps short, and both types share one load of the samples and, for
-// intra modes, one evaluation of the prediction, so no prediction buffers of
-// the 18 modes exist.
-__device__ __noinline__ void luma_areas(const Leaf L, const int *cl, int ncl, bool accum, bool wrec, int16_t *emit,
-                                        int woff) {
+// A warp codes a group of areas for every candidate of its stream.  Bound:
+// issue slots (four warps a scheduler).  Both TU sizes share one prediction
+// and run interleaved; what a lane adds up over its group's areas is reduced
+// once per candidate.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves:
+// larger ones would leave warps without a candidate in the last round (21
+// candidates: 11 rounds of 2 areas in 2 streams, 6 of 4 in 4).  An 8x8
+// leaf's single area is split by TU size instead, over 8 streams.
+__device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl) {
     Smem &S = smem_state();
-    const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
+    const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt, warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
     const uint4 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
     const uint4 *bands = S.qparam[0].band;
     const uint4 b80 = bands[band_rc(8, row, col)], b81 = bands[band_rc(8, row, col + 1)];
     const uint4 b40 = bands[band_rc(4, row & 3, col & 3)], b41 = bands[band_rc(4, row & 3, (col & 3) + 1)];
-    for (int it = ((threadIdx.x >> 5) + NW - woff) & (NW - 1); it < J; it += NW) {
-        const int e = cl[it >> (2 * lt)], slot = e & CL_SLOT, t = it & ((1 << (2 * lt)) - 1);
+#ifdef TCB_PHASE_PROFILE
+    if (threadIdx.x < ncl) { OPCOUNT(2, cl[threadIdx.x] & CL_8 ? 1 << la : 0); OPCOUNT(3, cl[threadIdx.x] & CL_4 ? 4 << la : 0); }
+#endif
+    const int lG = la == 6 ? 2 : la == 0 ? 0 : 1;            // log2 of a group's areas
+    const int lg = la == 0 ? 1 : la - lG;                    // log2 of the groups (8x8: TU sizes)
+    const int group = warp & ((1 << lg) - 1), step = NW >> lg;
+    const int sizes = la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4;
+    const int t0 = la == 0 ? 0 : group << lG;
+    for (int k = warp >> lg; k < ncl; k += step) {
+        const int e = cl[k], slot = e & CL_SLOT, do_sizes = e & sizes;
+        if (!do_sizes) continue;
+        int s8 = 0, n8 = 0, s4 = 0, n4 = 0;
+        bool differs = false;
+        for (int t = t0; t < t0 + (1 << lG); ++t) {
+            const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row, at = y * cu + x;
+            const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
+            const uint32_t pv = pred2(S, cu, e, x, y);
+            differs |= pv != cv;
+            auto add8 = [&](const AreaCode &c) {
+                s8 += c.sse;
+                n8 += c.bits;
+                const int b = S.last_bits[last8(c, lane)];
+                if (lane == 0) n8 += b;
+                if (la <= 2) *(uint16_t *)(S.crec[slot][0] + at) = (uint16_t)c.rec;
+            };
+            auto add4 = [&](const AreaCode &c) {
+                s4 += c.sse;
+                n4 += c.bits;
+                const int b = S.last_bits[last4(c, lane)];
+                if ((lane & 13) == 0) n4 += b;
+                if (la <= 2) *(uint16_t *)(S.crec[slot][1] + at) = (uint16_t)c.rec;
+            };
+            if (do_sizes == (CL_8 | CL_4)) {
+                const AreaCode c8 = code_area(cv, pv, f8, i8, b80, b81);
+                const AreaCode c4 = code_area(cv, pv, f4, i4, b40, b41);
+                add8(c8);
+                add4(c4);
+            } else if (do_sizes == CL_8) {
+                add8(code_area(cv, pv, f8, i8, b80, b81));
+            } else {
+                add4(code_area(cv, pv, f4, i4, b40, b41));
+            }
+        }
+        if ((e & CL_EXACT) && __any_sync(0xffffffffu, differs)) S.inexact = 1;
+        int v = 0;   // lanes 0..3: the four sums of the slot
+        if (do_sizes & CL_8) {
+            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s8), b = (int)__reduce_add_sync(0xffffffffu, (unsigned)n8);
+            v = lane == 0 ? a : lane == 1 ? b : 0;
+        }
+        if (do_sizes & CL_4) {
+            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s4), b = (int)__reduce_add_sync(0xffffffffu, (unsigned)n4);
+            v = lane == 2 ? a : lane == 3 ? b + (1 << lG) : v;
+        }
+        if (lane < 4) atomicAdd(&S.acc[slot][0][0] + lane, v);
+    }
+}
+
+// Codes the luma of a leaf with one candidate and TU size (list entry e) into
+// the reconstruction tile; `emit` takes the levels in syntax order.  A warp
+// per 8x8 area.
+__device__ __noinline__ void luma_replay(const Leaf L, int e, int16_t *emit) {
+    Smem &S = smem_state();
+    const int cu = L.cu, lt = lg2i(cu) - 3;
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
+    int t = threadIdx.x >> 5;
+    if (t >= 1 << (2 * lt)) return;
+    const bool d8 = e & CL_8;
+    const uint4 f = S.frag[d8 ? 0 : 2][lane], i = S.frag[d8 ? 1 : 3][lane];
+    const uint4 b0 = S.qparam[0].band[d8 ? band_rc(8, row, col) : band_rc(4, row & 3, col & 3)];
+    const uint4 b1 = S.qparam[0].band[d8 ? band_rc(8, row, col + 1) : band_rc(4, row & 3, (col & 3) + 1)];
+    const int pos = d8 ? 2 * lane : (row >> 2) * 32 + (col >> 2) * 16 + (row & 3) * 4 + (col & 3);
+    for (; t < 1 << (2 * lt); t += NW) {
         const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
         const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
-        const uint32_t pv = pred2(S, cu, slot, x, y);
-        if ((e & CL_EXACT) && __any_sync(0xffffffffu, pv != cv)) S.inexact = 1;
-        if (lane == 0) { OPCOUNT(2, (e & CL_8) ? 1 : 0); OPCOUNT(3, (e & CL_4) ? 4 : 0); }
-        if (e & CL_8) {
-            const AreaCode c = code_area(cv, pv, f8, i8, b80, b81);
-            if (accum) {
-                const uint32_t s = __reduce_add_sync(0xffffffffu, c.sums);
-                const int bits = base_bits8(c) + 2 * (int)(s & 1023u);
-                if (lane == 0) {
-                    atomicAdd(&S.acc_sse[slot][0], (int)(s >> 10));
-                    atomicAdd(&S.acc_bits[slot][0], bits);
-                }
-                if (cu <= 16) *(uint16_t *)(S.crec[slot][0] + y * cu + x) = (uint16_t)c.rec;
-            }
-            if (wrec) *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
-            if (emit) *(uint32_t *)(emit + t * 64 + 2 * lane) = __byte_perm((uint32_t)c.q0, (uint32_t)c.q1, 0x5410);
-        }
-        if (e & CL_4) {
-            const AreaCode c = code_area(cv, pv, f4, i4, b40, b41);
-            if (accum) {
-                const uint32_t s = __reduce_add_sync(0xffffffffu, c.sums);
-                int bits = base_bits4(c, lane);
-                bits += __shfl_xor_sync(0xffffffffu, bits, 2);
-                bits += __shfl_xor_sync(0xffffffffu, bits, 16);
-                if (lane == 0) {
-                    atomicAdd(&S.acc_sse[slot][1], (int)(s >> 10));
-                    atomicAdd(&S.acc_bits[slot][1], bits + 1 + 2 * (int)(s & 1023u));
-                }
-                if (cu <= 16) *(uint16_t *)(S.crec[slot][1] + y * cu + x) = (uint16_t)c.rec;
-            }
-            if (wrec) *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
-            if (emit)
-                *(uint32_t *)(emit + t * 64 + (row >> 2) * 32 + (col >> 2) * 16 + (row & 3) * 4 + (col & 3)) =
-                    __byte_perm((uint32_t)c.q0, (uint32_t)c.q1, 0x5410);
-        }
+        const AreaCode c = code_area(cv, pred2(S, cu, e, x, y), f, i, b0, b1);
+        *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
+        if (emit) *(uint32_t *)(emit + t * 64 + pos) = c.levels();
     }
 }
 
 // Chroma residual coding (reference src/encoder.c:429-475 qt_code_chroma):
 // 4x4 TUs, four (option, component, TU) jobs per warp, one on each quarter of
-// the area's lanes.  Option o, component c predicts from
+// the area's lanes, from warp `woff` on.  Option o, component c predicts from
 // S.cpred[cbase + 2*o + c]; results accumulate in slot o.
 __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, bool accum, bool wrec, int16_t *emit,
                                           int woff) {
@@ -676,10 +714,12 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, boo
     const int lxc = L.lx >> 1, lyc = L.ly >> 1;
     const int lane = threadIdx.x & 31, r = (lane >> 2) & 3, cc = 2 * (lane & 1);
     const int quarter = ((lane >> 3) & 2) | ((lane >> 1) & 1);
+    if (threadIdx.x == 0) OPCOUNT(3, J);
+    int base = 4 * (((threadIdx.x >> 5) + NW - woff) & (NW - 1));
+    if (base >= J) return;
     const uint4 f4 = S.frag[2][lane], i4 = S.frag[3][lane];
     const uint4 b0 = S.qparam[1].band[band_rc(4, r, cc)], b1 = S.qparam[1].band[band_rc(4, r, cc + 1)];
-    if (threadIdx.x == 0) OPCOUNT(3, J);
-    for (int base = 4 * (((threadIdx.x >> 5) + NW - woff) & (NW - 1)); base < J; base += 4 * NW) {
+    for (; base < J; base += 4 * NW) {
         const bool act = base + quarter < J;
         const int j = act ? base + quarter : 0;
         const int o = j >> (2 * ln + 1), c = (j >> (2 * ln)) & 1, t = j & ((1 << (2 * ln)) - 1);
@@ -688,19 +728,19 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, boo
         const uint32_t pv = *(const uint16_t *)(S.cpred[cbase + 2 * o + c] + y * cs + x);
         const AreaCode a = code_area(cv, pv, f4, i4, b0, b1);
         if (accum) {
-            uint32_t s = a.sums;    // of the quarter's eight lanes: index bits 0, 2 and 3
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            s += __shfl_xor_sync(0xffffffffu, s, 8);
-            const int bits = base_bits4(a, lane) + 2 * (int)(s & 1023u);
+            int d = a.sse, n = a.bits;    // of the quarter's eight lanes: index bits 0, 2 and 3
+            for (int m = 1; m < 16; m = m == 1 ? 4 : 2 * m) {
+                d += __shfl_xor_sync(0xffffffffu, d, m);
+                n += __shfl_xor_sync(0xffffffffu, n, m);
+            }
+            n += S.last_bits[last4(a, lane)];
             if (act && (lane & 13) == 0) {
-                atomicAdd(&S.acc_sse[o][0], (int)(s >> 10));
-                atomicAdd(&S.acc_bits[o][0], bits);
+                atomicAdd(&S.acc[o][0][0], d);
+                atomicAdd(&S.acc[o][0][1], n);
             }
         }
         if (act && wrec) *(uint16_t *)&RC(S, c, lxc + x, lyc + y) = (uint16_t)a.rec;
-        if (act && emit)
-            *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = __byte_perm((uint32_t)a.q0, (uint32_t)a.q1, 0x5410);
+        if (act && emit) *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = a.levels();
     }
 }
 
@@ -850,34 +890,31 @@ __device__ __noinline__ void luma_mc_slots(Smem &, const FrameParams &, const Le
 }
 
 __device__ void zero_acc(Smem &S) {
-    for (int i = threadIdx.x; i < NCAND * 2; i += NT) {
-        (&S.acc_sse[0][0])[i] = 0;
-        (&S.acc_bits[0][0])[i] = 0;
-    }
+    for (int i = threadIdx.x; i < NCAND * 4; i += NT) (&S.acc[0][0][0])[i] = 0;
     if (threadIdx.x == 0) { S.acc64 = 0; S.inexact = 0; }
 }
 
-// Sum over the CU of |orig - pred| per listed slot into acc_sse[slot][0]
+// Sum over the CU of |orig - pred| per listed slot into acc[slot][0][0]
 // (fast-preset SAD proxy): one warp per (candidate, 8x8 area).
 __device__ void sad_areas(Smem &S, const Leaf &L, const int *cl, int ncl) {
     const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
     const int lane = threadIdx.x & 31;
     for (int it = threadIdx.x >> 5; it < J; it += NW) {
-        const int slot = cl[it >> (2 * lt)] & CL_SLOT, t = it & ((1 << (2 * lt)) - 1);
+        const int e = cl[it >> (2 * lt)], t = it & ((1 << (2 * lt)) - 1);
         const int x = (t & ((1 << lt) - 1)) * 8 + 2 * (lane & 3), y = (t >> lt) * 8 + (lane >> 2);
         const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
-        const unsigned s = __reduce_add_sync(0xffffffffu, __vsadu4(cv, pred2(S, cu, slot, x, y)));
-        if (lane == 0) atomicAdd(&S.acc_sse[slot][0], (int)s);
+        const unsigned s = __reduce_add_sync(0xffffffffu, __vsadu4(cv, pred2(S, cu, e, x, y)));
+        if (lane == 0) atomicAdd(&S.acc[e & CL_SLOT][0][0], (int)s);
     }
 }
 
 __device__ __forceinline__ long long best_of(const Smem &S, int slot, bool use4, long long lambda,
                                              int &lb, int &dct) {
-    const long long d8 = S.acc_sse[slot][0];
-    const int b8 = S.acc_bits[slot][0];
+    const long long d8 = S.acc[slot][0][0];
+    const int b8 = S.acc[slot][0][1];
     if (use4) {
-        const long long d4 = S.acc_sse[slot][1];
-        const int b4 = S.acc_bits[slot][1];
+        const long long d4 = S.acc[slot][1][0];
+        const int b4 = S.acc[slot][1][1];
         if (d4 + lambda * b4 < d8 + lambda * b8) { lb = b4; dct = 0; return d4; }
     }
     lb = b8; dct = 1;
@@ -995,10 +1032,8 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
             if (use_cache) {
                 luma_from_cache(S, L, K_INTRA + nd.intra_mode, nd.dct_size);
             } else {
-                if (threadIdx.x == 0) S.cl2[0] = (K_INTRA + nd.intra_mode) | cl_size;
                 if (!from) build_refs(L);
-                else SYNC();
-                luma_areas(L, S.cl2, 1, false, true, el, 0);
+                luma_replay(L, cl_entry(K_INTRA + nd.intra_mode, cl_size), el);
             }
             SYNC();
         }
@@ -1044,11 +1079,8 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
         }
         if (!nd.skip) {
             const int src = from ? S.win_slot : 0;   // the decision's prediction is still in its slot
-            if (threadIdx.x == 0) {
-                if (!from) {
-                    S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
-                }
-                S.cl2[0] = src | cl_size;
+            if (!from && threadIdx.x == 0) {
+                S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
             }
             SYNC();
             // Chroma prediction does not depend on this leaf's luma, so both
@@ -1067,7 +1099,7 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
                     const int slots[1] = {0};
                     luma_mc_slots(S, P, L, 1, slots, false);
                 }
-                luma_areas(L, S.cl2, 1, false, true, el, 0);
+                luma_replay(L, src | cl_size, el);
                 chroma_areas(L, 1, 0, false, true, ec, mini(NW / 2, (cu * cu) >> 6));
             }
         } else {
@@ -1194,14 +1226,14 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         const bool m8 = merges >> lane & 1u;
         if (cand >> lane & 1u)
             S.cl[__popc(cand & ((1u << lane) - 1u))] =
-                lane | CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0);
+                cl_entry(lane, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
     }
     SYNC();
     if (fast) {
         sad_areas(S, L, S.cl, ncl);
         SYNC();
     } else {
-        luma_areas(L, S.cl, ncl, true, false, nullptr, 0);
+        luma_score(L, S.cl, ncl);
         SYNC();
         PHASE_D(3, L.depth);
         if (is_p) {
@@ -1260,7 +1292,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
             long long d = 0;
             if (!skip) {
                 if (fast) {
-                    const long long sad = S.acc_sse[lane][0];
+                    const long long sad = S.acc[lane][0][0];
                     d = (sad * sad) >> (2 * lg2i(cu));   // / (cu * cu), sad >= 0
                     bits += intra ? 8 : 3;
                 } else {
@@ -1299,9 +1331,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         if (cu <= 16) {
             luma_from_cache(S, L, K_INTRA + nd0.intra_mode, nd0.dct_size);
         } else {
-            if (tid == 0) S.cl2[0] = (K_INTRA + nd0.intra_mode) | (nd0.dct_size ? CL_8 : CL_4);
-            SYNC();
-            luma_areas(L, S.cl2, 1, false, true, nullptr, 0);
+            luma_replay(L, cl_entry(K_INTRA + nd0.intra_mode, nd0.dct_size ? CL_8 : CL_4), nullptr);
         }
         SYNC();
         if (P.ref_valid[0]) chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
@@ -1314,8 +1344,8 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         SYNC();
         if (tid == 0) {
             const long long lam = P.lambda;
-            const long long dmc = S.acc_sse[0][0], dcfl = S.acc_sse[1][0];
-            const int lbmc = S.acc_bits[0][0], lbcfl = S.acc_bits[1][0];
+            const long long dmc = S.acc[0][0][0], dcfl = S.acc[1][0][0];
+            const int lbmc = S.acc[0][0][1], lbcfl = S.acc[1][0][1];
             if (dcfl + lam * (lbcfl + 4) < dmc + lam * (lbmc + 1))
                 S.nodes[qt_index(L.depth, L.cx, L.cy)].ch_intra = 1;
         }
@@ -1635,12 +1665,14 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     }
 }
 
-// The transform fragments (forward and inverse, 8x8 and 4x4) of every lane,
-// once per CTA.
+// The transform fragments (forward and inverse, 8x8 and 4x4) of every lane and
+// the last-position bits, once per CTA.
 __device__ void init_fragments(Smem &S) {
     if (threadIdx.x < 128)
         S.frag[threadIdx.x >> 5][threadIdx.x & 31] =
             dct_fragment(threadIdx.x < 64 ? 8 : 4, (threadIdx.x >> 5) & 1, threadIdx.x & 31);
+    else if (threadIdx.x < 128 + 65)
+        S.last_bits[threadIdx.x - 128] = last_bits((int)threadIdx.x - 129);
 }
 
 // One CTA per CTU of one anti-diagonal (items[blockIdx.x]).
@@ -2082,7 +2114,7 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
         const int lg = lg2i(cu) - 1;
         for (int i = threadIdx.x; i < cu * cu / 2; i += NT)
             *(uint16_t *)(S.pred[0] + 2 * i) =
-                (uint16_t)intra2(S, cu, nd.intra_mode, 2 * (i & (cu / 2 - 1)), i >> lg);
+                (uint16_t)pred2(S, cu, cl_entry(K_INTRA + nd.intra_mode, 0), 2 * (i & (cu / 2 - 1)), i >> lg);
         SYNC();
     } else {
         int r1 = -1, r2 = -1;

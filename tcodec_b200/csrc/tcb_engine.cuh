@@ -30,13 +30,16 @@ enum {
 };
 constexpr int NPRED = 5;            // inter prediction buffers (slots 0..4)
 
-// Entry of a leaf's candidate list: the slot and which TU sizes are scored.
+// Entry of a leaf's candidate list: the slot, which TU sizes are scored, and
+// from bit 16 on an angular mode's displacement.
 enum {
     CL_SLOT = 0xFF,
     CL_8 = 0x100,       // one 8x8 TU per 8x8 area
     CL_4 = 0x200,       // four 4x4 TUs per 8x8 area
     CL_EXACT = 0x400    // note whether the prediction equals the source
 };
+
+constexpr int EDGE_BASE = 96, EDGE_LEN = 264;   // index 0 of S.edge; entries up to 2.5 * 64 + 2
 
 constexpr int QPOS = 7;               // quarter-sample positions per axis around an integer best: -3..3
 struct MeGroup {
@@ -83,19 +86,19 @@ struct Smem {
         alignas(16) uint32_t plane[PLANE_WORDS];
     };
     uint32_t cur_pair[64 * 32];      // leaf's source samples (x, x + cu / 2) as 16-bit lanes, for the searches
-    uint8_t ra[2 * 64 + 4], rl[2 * 64 + 4];     // index i+1 holds ref[i], i in -1..2N
+    uint8_t edge[2][EDGE_LEN];       // intra reference samples per direction (see build_refs)
     int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
     uint4 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
-    int acc_sse[NCAND][2];
-    int acc_bits[NCAND][2];
+    int acc[NCAND][2][2];      // per slot and TU size (8x8, 4x4): distortion, bits
+    int last_bits[65];         // last_bits(last) by last + 1
     long long acc64;
     int cl[NCAND];             // candidate list for job loops
-    int cl2[1];                // the one candidate a replay codes
     int cand_mvx[NPRED], cand_mvy[NPRED], cand_ref[NPRED], cand_ref2[NPRED];
     int dc;
+    int above0;                // first sample of the above run (the planar mode's corner)
     int inexact;               // the merge prediction of the current leaf differs from the source
     long long best_cost;
     int sao[3];

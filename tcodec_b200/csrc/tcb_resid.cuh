@@ -13,12 +13,14 @@
 //  * The first pass multiplies the residuals (|r| <= 255, exact in f16).  The
 //    later passes multiply intermediates t, |t| < 8192, split as 64 th + tl
 //    with 0 <= tl < 64: k = 16 holds [64 C | C] against [th; tl].
-//  * Every product is an integer and every accumulator starts at 1.5 * 2^23,
-//    so its bits are 0x4B400000 + sum as long as |sum| < 2^22.  Residuals of
-//    8-bit pictures have norm <= 2040, a non-zero level dequantises to at
-//    most 1.75 |c| (q eff + eff / 6 with q eff <= |c| + eff / 3 and
-//    eff <= 1.5 |c|), so no intermediate exceeds 3571 and no partial sum
-//    182 * 3571 < 2^20.
+//  * Every product is an integer and the accumulators start at about
+//    1.5 * 2^23, so their bits are a constant plus the sum while
+//    |sum| < 2^20.3.  Residuals of 8-bit pictures have norm <= 2040, a
+//    non-zero level dequantises to at most 1.75 |c| (q eff + eff / 6 with
+//    q eff <= |c| + eff / 3 and eff <= 1.5 |c|), so no intermediate exceeds
+//    3571 and no partial sum 182 * 3571 < 2^20.
+//  * The start values are chosen so that 128 Hi + Lo, modulo 2^32 (or 2^28
+//    where only bits 14..27 are used), is the rounded sum with no correction.
 //
 // Data layout: lane l owns row l >> 2, columns 2 (l & 3) and 2 (l & 3) + 1 of
 // the 8x8 area.  That is the C fragment of an m16n8 MMA (rows 0..7: the Ch
@@ -28,9 +30,9 @@
 // with block-diagonal matrices.
 //
 // Compared with eight (four) lanes per TU and rows exchanged through shared
-// memory: 150 instructions per area and type instead of about 250 per 8x8 TU
-// and 50 per 4x4 TU, in a serial chain of about 150 instead of 1000, and
-// 3 KB of code instead of 38 KB.
+// memory: about 110 instructions per area and type with its bit estimate
+// instead of about 300 per 8x8 TU and 90 per 4x4 TU, in a serial chain of the
+// same length instead of 1000, and 3 KB of code instead of 38 KB.
 //
 // Arithmetic follows reference src/transform.c:331-439 (dct4_point,
 // dct8_point2, tc_fdct*/tc_idct*_res), src/encoder.c:333-385 (rdoq_level1,
@@ -73,21 +75,25 @@ static inline cudaError_t upload_dct_tables() {
 
 struct QuantParams {
     int eff[4];
-    // Per band: {quant step | dequantiser bias (eff / 6) << 16, reciprocal,
-    // quantiser offset (eff / 3) | (eff <= 1) << 16, RDOQ threshold}.  A level
-    // of magnitude 1 dequantises to dq = eff + eff / 6 and is dropped when
+    // Per band: {reciprocal, quantiser offset times reciprocal, smallest |c|
+    // with a level, quant step | dequantiser bias (eff / 6) << 16}.  The level
+    // is (|c| + eff / 3) / eff, as the high word of |c| rcp + off rcp (a step
+    // of 1: reciprocal 2^32 - 1 and offset 1, which give |c|).  A level of
+    // magnitude 1 dequantises to dq = eff + eff / 6 and is dropped when
     // c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference
-    // src/encoder.c:333-355), i.e. when dq (2 |c| - dq) < lambda: for the
-    // |c| below ceil((dq + ceil(lambda / dq)) / 2).
+    // src/encoder.c:333-355), i.e. when dq (2 |c| - dq) < lambda: below
+    // ceil((dq + ceil(lambda / dq)) / 2), if that lies in level 1's range.
     uint4 band[4];
     __host__ __device__ void set_band(int b, int e, uint32_t r, long long lambda) {
-        const int dq = e + e / 6;
-        const long long thr = ((lambda + dq - 1) / dq + dq + 1) >> 1;
+        const int off = e / 3, dq = e + e / 6;
+        long long thr = ((lambda + dq - 1) / dq + dq + 1) >> 1;
+        if (thr > 2 * e - off) thr = 2 * e - off;
+        if (thr < e - off) thr = e - off;
         eff[b] = e;
-        band[b].x = (uint32_t)e | (uint32_t)(e / 6) << 16;
-        band[b].y = r;
-        band[b].z = (uint32_t)(e / 3) | (e <= 1 ? 1u << 16 : 0u);
-        band[b].w = (uint32_t)(thr < 0x7FFFFFFF ? thr : 0x7FFFFFFF);
+        band[b].x = e <= 1 ? 0xFFFFFFFFu : r;
+        band[b].y = e <= 1 ? 0xFFFFFFFFu : (uint32_t)off * r;
+        band[b].z = (uint32_t)thr;
+        band[b].w = (uint32_t)e | (uint32_t)(e / 6) << 16;
     }
 };
 
@@ -119,57 +125,72 @@ __device__ inline uint4 dct_fragment(int N, int inv, int lane) {
                       pack(cl[0], cl[1]));
 }
 
-constexpr float MMA_BIAS = 12582912.0f;                  // 1.5 * 2^23, bits 0x4B400000
-// -(0x4B400000 * 129) mod 2^32 plus the rounding term of the 14-bit shift
-constexpr uint32_t MMA_UNBIAS = 0u - 0x4B400000u * 129u + 8192u;
+// Accumulator start values.  With 0x4B400000 the bits of 1.5 * 2^23,
+// (bits(Hi) << 7) + bits(Lo) = 0xEB400000 + 128 dH + dL + sum (mod 2^32) for
+// starts 1.5 * 2^23 + dH and + dL; dL = 8192 rounds the 14-bit shift.
+//   EXACT: 128 dH = 2^32 - 0xEB400000, the word is sum + 8192;
+//   FIELD: 128 dH = 2^27 - 0xEB400000 (mod 2^28), bits 14..27 are the rounded
+//          result + 8192 (results within +-8191).
+constexpr float ACC_LO = 12582912.0f + 8192.0f;
+constexpr float ACC_EXACT = 12582912.0f + 2719744.0f, ACC_FIELD = 12582912.0f - 425984.0f;
 
-__device__ __forceinline__ void mma_k8(float d[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    d[0] = d[1] = d[2] = d[3] = MMA_BIAS;
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
+struct MmaSums {
+    float h0, h1, l0, l1;
+    __device__ __forceinline__ uint32_t x0() const { return (__float_as_uint(h0) << 7) + __float_as_uint(l0); }
+    __device__ __forceinline__ uint32_t x1() const { return (__float_as_uint(h1) << 7) + __float_as_uint(l1); }
+};
+__device__ __forceinline__ MmaSums mma_k8(uint32_t a0, uint32_t a1, uint32_t b0, float start) {
+    MmaSums d;
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%8,%8};"
+        : "=f"(d.h0), "=f"(d.h1), "=f"(d.l0), "=f"(d.l1) : "r"(a0), "r"(a1), "r"(b0), "f"(start), "f"(ACC_LO));
+    return d;
 }
-__device__ __forceinline__ void mma_k16(float d[4], const uint4 a, uint32_t b0, uint32_t b1) {
-    d[0] = d[1] = d[2] = d[3] = MMA_BIAS;
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
-}
-// Rounded 14-bit result of one position from its two partial sums (+ bias).
-template <int BIAS>
-__device__ __forceinline__ int mma_round(float hi, float lo) {
-    return (int)((__float_as_uint(hi) << 7) + __float_as_uint(lo) + (MMA_UNBIAS + (uint32_t)BIAS * 16384u)) >> 14;
+__device__ __forceinline__ MmaSums mma_k16(const uint4 a, uint32_t b0, uint32_t b1, float start) {
+    MmaSums d;
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%11,%11};"
+        : "=f"(d.h0), "=f"(d.h1), "=f"(d.l0), "=f"(d.l1)
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(start), "f"(ACC_LO));
+    return d;
 }
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
     const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
-// B fragment halves of two intermediates given as t + 8192 (0..16383):
-// hi = half2(t >> 6), lo = half2(t & 63).  0x6400 | v is the half 1024 + v.
-__device__ __forceinline__ void split_b(int t0, int t1, uint32_t &hi, uint32_t &lo) {
-    const uint32_t pk = __byte_perm((uint32_t)t0, (uint32_t)t1, 0x5410);
+// B fragment halves of two intermediates, each t + 8192 in the low 14 bits of
+// its 16-bit lane of pk (the two bits above are ignored): hi = half2(t >> 6),
+// lo = half2(t & 63).  0x6400 | v is the half 1024 + v.
+__device__ __forceinline__ void split_b(uint32_t pk, uint32_t &hi, uint32_t &lo) {
     lo = h2_sub((pk & 0x003F003Fu) | 0x64006400u, 0x64006400u);            // - 1024
-    hi = h2_sub(((pk >> 6) & 0x03FF03FFu) | 0x64006400u, 0x64806480u);     // - (1024 + 8192 / 64)
+    hi = h2_sub(((pk >> 6) & 0x00FF00FFu) | 0x64006400u, 0x64806480u);     // - (1024 + 8192 / 64)
+}
+__device__ __forceinline__ void split_sums(const MmaSums &d, uint32_t &hi, uint32_t &lo) {
+    split_b(__byte_perm(d.x0() >> 14, d.x1() << 2, 0x7610), hi, lo);
 }
 // Two 8-bit samples (low 16 bits of v) as half2(1024 + v0, 1024 + v1).
 __device__ __forceinline__ uint32_t bytes_h2(uint32_t v) { return __byte_perm(v, 0x64u, 0x4140); }
 
 // One coefficient: dead-zone quantiser with RDOQ-lite.  Returns the level's
-// magnitude; dq is the signed dequantised value.
+// magnitude; dq is the signed dequantised value + 8192.
 __device__ __forceinline__ int quant_one(int c, const uint4 b, int &dq) {
     const int a = absi(c);
-    const uint32_t n = (uint32_t)a + (b.z & 0xFFFFu);
-    int q = (int)(__umulhi(n, b.y) + n * (b.z >> 16));     // step <= 1: reciprocal 0, level n
-    if (q == 1 && a < (int)b.w) q = 0;
-    const int m = q ? q * (int)(b.x & 0xFFFFu) + (int)(b.x >> 16) : 0;
-    dq = c < 0 ? -m : m;
+    const bool zero = a < (int)b.z;
+    int q = (int)(((unsigned long long)(unsigned)a * b.x + b.y) >> 32);
+    int m = q * (int)(b.w & 0xFFFFu) + (int)(b.w >> 16);
+    q = zero ? 0 : q;
+    m = zero ? 0 : m;
+    dq = (c < 0 ? -m : m) + 8192;
     return q;
 }
 
 // What the warp knows of one coded area.
 struct AreaCode {
-    int q0, q1;        // this lane's signed levels
-    uint32_t rec;      // this lane's two reconstructed samples (low 16 bits)
-    uint32_t sums;     // this lane's SSE << 10 | bit lengths of its levels
+    int m0, m1;        // magnitudes of this lane's levels
+    int c0, c1;        // its coefficients (whose signs the levels have)
+    uint32_t rec;      // its two reconstructed samples (low 16 bits)
+    int sse, bits;     // its SSE; 2 bitlen + 3 summed over its non-zero levels
+    __device__ __forceinline__ uint32_t levels() const {   // two int16 levels
+        return __byte_perm((uint32_t)(c0 < 0 ? -m0 : m0), (uint32_t)(c1 < 0 ? -m1 : m1), 0x5410);
+    }
 };
 
 // Codes the area whose samples this lane holds two of: cv (source) and pv
@@ -178,53 +199,46 @@ struct AreaCode {
 __device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint4 f, const uint4 i, const uint4 b0,
                                               const uint4 b1) {
     AreaCode r;
-    float d[4];
     uint32_t hi, lo;
-    mma_k8(d, f.z, f.w, h2_sub(bytes_h2(cv), bytes_h2(pv)));
-    split_b(mma_round<8192>(d[0], d[2]), mma_round<8192>(d[1], d[3]), hi, lo);
-    mma_k16(d, f, hi, lo);
-    const int c0 = mma_round<0>(d[0], d[2]), c1 = mma_round<0>(d[1], d[3]);
+    split_sums(mma_k8(f.z, f.w, h2_sub(bytes_h2(cv), bytes_h2(pv)), ACC_FIELD), hi, lo);
+    MmaSums d = mma_k16(f, hi, lo, ACC_EXACT);
+    r.c0 = (int)d.x0() >> 14;
+    r.c1 = (int)d.x1() >> 14;
     int dq0, dq1;
-    const int m0 = quant_one(c0, b0, dq0), m1 = quant_one(c1, b1, dq1);
-    r.q0 = c0 < 0 ? -m0 : m0;
-    r.q1 = c1 < 0 ? -m1 : m1;
-    split_b(dq0 + 8192, dq1 + 8192, hi, lo);
-    mma_k16(d, i, hi, lo);
-    split_b(mma_round<8192>(d[0], d[2]), mma_round<8192>(d[1], d[3]), hi, lo);
-    mma_k16(d, i, hi, lo);
-    const int v0 = clampi((int)(pv & 0xFF) + mma_round<0>(d[0], d[2]), 0, 255);
-    const int v1 = clampi((int)(pv >> 8) + mma_round<0>(d[1], d[3]), 0, 255);
+    r.m0 = quant_one(r.c0, b0, dq0);
+    r.m1 = quant_one(r.c1, b1, dq1);
+    split_b(__byte_perm((uint32_t)dq0, (uint32_t)dq1, 0x5410), hi, lo);
+    split_sums(mma_k16(i, hi, lo, ACC_FIELD), hi, lo);
+    d = mma_k16(i, hi, lo, ACC_EXACT);
+    const int v0 = __viaddmin_s32_relu((int)(pv & 0xFF), (int)d.x0() >> 14, 255);   // clamped to 0..255
+    const int v1 = __viaddmin_s32_relu((int)(pv >> 8), (int)d.x1() >> 14, 255);
     const int e0 = (int)(cv & 0xFF) - v0, e1 = (int)(cv >> 8) - v1;
     r.rec = (uint32_t)v0 | (uint32_t)v1 << 8;
-    r.sums = ((uint32_t)(e0 * e0 + e1 * e1) << 10) + (uint32_t)(bitlen((unsigned)m0) + bitlen((unsigned)m1));
+    r.sse = e0 * e0 + e1 * e1;
+    r.bits = 2 * (bitlen((unsigned)r.m0) + bitlen((unsigned)r.m1)) + (r.m0 ? 3 : 0) + (r.m1 ? 3 : 0);
     return r;
 }
 
-// Bit estimate of a TU without its levels' bit lengths.  The reference counts
-// 1 + 2 nz, a level term (1 for a zero, 2 + 2 bitlen otherwise) for every
-// position up to the last and the last position's cost
-// (src/encoder.c:360-385): with B the sum of the bit lengths that is
-// 2 B + 2 + 3 nz + last + lastpos_cost(last), last = -1 for an empty TU.
-__device__ __forceinline__ int tu_base_bits(int nz, int last) { return 2 + 3 * nz + last + lastpos_cost(last); }
+// Rest of a TU's bit estimate.  The reference counts 1 + 2 nz, a level term (1
+// for a zero, 2 + 2 bitlen otherwise) for every position up to the last and
+// the last position's cost (src/encoder.c:360-385): over all levels that is
+// the sum of 2 bitlen + 3 over the non-zero ones plus last_bits(last),
+// last = -1 for an empty TU.
+__host__ __device__ __forceinline__ int last_bits(int last) { return 2 + last + lastpos_cost(last); }
 
-// The 8x8 TU of the area: raster position of (lane, e) is 2 lane + e.
-__device__ __forceinline__ int base_bits8(const AreaCode &c) {
-    const unsigned n0 = __ballot_sync(0xffffffffu, c.q0 != 0), n1 = __ballot_sync(0xffffffffu, c.q1 != 0);
-    const unsigned any = n0 | n1;
-    const int h = 31 - __clz((int)any);
-    const int last = any ? 2 * h + (int)((n1 >> h) & 1u) : -1;
-    return tu_base_bits(__popc(n0) + __popc(n1), last);
+// Last position + 1 of the area's 8x8 TU (0: empty): the raster position of
+// (lane, e) is 2 lane + e.
+__device__ __forceinline__ int last8(const AreaCode &c, int lane) {
+    return (int)__reduce_max_sync(0xffffffffu, c.m1 ? 2u * lane + 2u : c.m0 ? 2u * lane + 1u : 0u);
 }
 
-// The lane's 4x4 TU (lanes of a quarter share bits 4 and 1 of their index,
+// Of the lane's 4x4 TU (lanes of a quarter share bits 4 and 1 of their index,
 // and within it the raster position grows with the lane index).
-__device__ __forceinline__ int base_bits4(const AreaCode &c, int lane) {
+__device__ __forceinline__ int last4(const AreaCode &c, int lane) {
     const unsigned qm = ((lane & 2) ? 0xCCCCCCCCu : 0x33333333u) & ((lane & 16) ? 0xFFFF0000u : 0x0000FFFFu);
-    const unsigned n0 = __ballot_sync(0xffffffffu, c.q0 != 0) & qm, n1 = __ballot_sync(0xffffffffu, c.q1 != 0) & qm;
-    const unsigned any = n0 | n1;
+    const unsigned any = __ballot_sync(0xffffffffu, (c.m0 | c.m1) != 0) & qm, n1 = __ballot_sync(0xffffffffu, c.m1 != 0);
     const int h = 31 - __clz((int)any);
-    const int last = any ? ((h >> 2) & 3) * 4 + (h & 1) * 2 + (int)((n1 >> h) & 1u) : -1;
-    return tu_base_bits(__popc(n0) + __popc(n1), last);
+    return any ? ((h >> 2) & 3) * 4 + (h & 1) * 2 + 1 + (int)((n1 >> h) & 1u) : 0;
 }
 
 }  // namespace tcb
