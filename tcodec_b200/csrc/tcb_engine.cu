@@ -80,10 +80,15 @@ __device__ unsigned long long tcb_op_counts[4];
 #define OPCOUNT(k, v) do {} while (0)
 #endif
 
-// Barrier of motion-search group g (named barrier g + 1) of n threads.
-__device__ __forceinline__ void group_bar(int g, int n) {
-    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(n) : "memory");
-}
+// A motion-search group: index, thread in it, log2 of its threads (7 or 8).
+struct MeTeam {
+    int g, gt, lth;
+    __device__ __forceinline__ MeTeam(int lth_) : g(threadIdx.x >> lth_), gt(threadIdx.x & ((1 << lth_) - 1)), lth(lth_) {}
+    // the group's barrier (named barrier g + 1)
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(1 << lth) : "memory");
+    }
+};
 
 // Four bytes from any address.  Reads only the aligned words that hold
 // p[0..3], so a plane whose last row ends exactly at the end of its
@@ -205,9 +210,9 @@ struct MeBlock {
 // (reference sad_at).  Lane k of every warp returns point p0 + k's SAD.  The
 // results go through part[par], which flips per call: a thread only gets to
 // the next call's barrier after all have read this one's.
-__device__ __forceinline__ int batch_sads(Smem &S, int g, int gt, int nthr, int &par, const MeBlock &M, int pat, int p0,
-                                          int K, int bx, int by, int scale) {
-    const int lpc = nthr >> 3, k = gt / lpc, l = gt & (lpc - 1), lane = gt & 31;
+__device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, const MeBlock &M, int pat, int p0, int K, int bx,
+                                          int by, int scale) {
+    const int gt = T.gt, lpc = 1 << (T.lth - 3), k = gt >> (T.lth - 3), l = gt & (lpc - 1), lane = gt & 31;
     unsigned v = 0;
     bool in = false;
     if (gt == 0) OPCOUNT(0, K * M.blk * M.blk);
@@ -235,9 +240,9 @@ __device__ __forceinline__ int batch_sads(Smem &S, int g, int gt, int nthr, int 
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     v += __shfl_xor_sync(0xffffffffu, v, 1);
     if (lpc == 32) v += __shfl_xor_sync(0xffffffffu, v, 16);
-    int *part = S.me[g].part[par];
+    int *part = S.me[T.g].part[par];
     if (l == 0) part[k] = in ? (int)v : 0x7FFFFFFF;
-    group_bar(g, nthr);
+    T.sync();
     par ^= 1;
     return lane < K ? part[lane] : 0x7FFFFFFF;
 }
@@ -256,16 +261,22 @@ __device__ __forceinline__ int batch_sads(Smem &S, int g, int gt, int nthr, int 
 // the result.  Two tables alternate, so refilling one never races with a
 // lagging thread still reading the other.
 constexpr int WIN_RMAX = 5, WIN_NMAX = 2 * WIN_RMAX + 1, WIN_WORDS = WIN_NMAX * WIN_NMAX;
-static_assert(2 * WIN_WORDS <= plane_words(8), "SAD tables overflow the group's planes");
+// (they lie past what the planes of a block up to 16x16 and the
+// reconstruction cache occupy, which are in use at the same time)
+constexpr int WIN_AT = PLANE_WORDS - NGROUP * 2 * WIN_WORDS;
+static_assert(NGROUP * plane_words(16) <= WIN_AT && (offsetof(Smem, crec) - offsetof(Smem, plane) + sizeof(Smem::crec)) / 4 <= WIN_AT,
+              "SAD tables overlap the planes or the reconstruction cache");
+static_assert(NGROUP * plane_words(16) * 4 <= offsetof(Smem, crec) - offsetof(Smem, plane),
+              "intra scoring writes the reconstruction cache while the searches use the planes");
 static_assert(WIN_WORDS <= 128, "one table position per thread of the smallest group");
 
 __device__ __forceinline__ int window_radius(int r) { return r >= 2 && r <= WIN_RMAX ? r : 4; }
 
-__device__ __forceinline__ void fill_sad_window(int g, int gt, int nthr, int *tab, const MeBlock &M, int wx, int wy,
-                                                int R) {
-    const int N = 2 * R + 1, two = nthr >> 8, pos = gt >> two;
+__device__ __forceinline__ void fill_sad_window(const MeTeam &T, int *tab, const MeBlock &M, int wx, int wy, int R) {
+    const int N = 2 * R + 1, two = T.lth - 7, gt = T.gt, pos = gt >> two;
     if (gt == 0) OPCOUNT(0, N * N * M.blk * M.blk);
-    const int py = pos / N, x = wx + pos - py * N - R, y = wy + py - R;
+    // pos / N for pos < 128, N = 5, 7, 9, 11
+    const int py = pos * (N == 9 ? 7282 : N == 7 ? 9363 : N == 11 ? 5958 : 13108) >> 16, x = wx + pos - py * N - R, y = wy + py - R;
     const int rows = M.blk >> two, r0 = (gt & two) * rows;
     const bool in = pos < N * N && M.inside(x, y);
     unsigned v = 0;
@@ -281,7 +292,7 @@ __device__ __forceinline__ void fill_sad_window(int g, int gt, int nthr, int *ta
     }
     if (two) v += __shfl_xor_sync(0xffffffffu, v, 1);
     if (pos < N * N) tab[pos] = in ? (int)v : 0x7FFFFFFF;
-    group_bar(g, nthr);
+    T.sync();
 }
 
 // The integer stages of one search: large hexagon (6 points, 2 passes,
@@ -291,17 +302,18 @@ __device__ __forceinline__ void fill_sad_window(int g, int gt, int nthr, int *ta
 // at once, one lane per point; the first one that improves is the sequential
 // walk's next commit, and the points after it are scored again around it.
 // The first batch also takes the centre, whose SAD the search starts from.
-__device__ __noinline__ void me_integer(int g, int gt, int nthr, int id, const uint8_t *ref, int lx, int ly, int blk,
-                                        int center_x, int center_y, int sr) {
+__device__ __noinline__ void me_integer(const MeTeam T, int id, const uint8_t *ref, int lx, int ly, int blk, int center_x,
+                                        int center_y, int sr) {
     Smem &S = smem_state();
     ME_T0();
+    const int g = T.g, gt = T.gt;
     const MeBlock M = {ref, S.cur_y + ly * 64 + lx, g_fp.stride_y, g_fp.W, g_fp.H, blk};
     const int lane = gt & 31;
     int par = 0;
     int bx = clampi(center_x, 0, M.W - blk), by = clampi(center_y, 0, M.H - blk);
     int bsad = 0x7FFFFFFF;
     bool centre = true;
-    int *tab = (int *)S.plane + g * plane_words(8);
+    int *const tab0 = (int *)S.plane + WIN_AT + g * 2 * WIN_WORDS, *tab = tab0;
     int wx = 0, wy = 0, R = -1;         // table around (wx, wy); R < 0: none yet
     const int radius = window_radius(g_fp.search_window);
 #pragma unroll 1
@@ -324,7 +336,7 @@ __device__ __noinline__ void me_integer(int g, int gt, int nthr, int id, const u
                     if (act && !off) v = tab[y * (2 * R + 1) + x];
                 } else {
                     base = centre ? 0 : p0;
-                    v = batch_sads(S, g, gt, nthr, par, M, pat, base, npts + 1 - base, bx, by, scale);
+                    v = batch_sads(S, T, par, M, pat, base, npts + 1 - base, bx, by, scale);
                     if (centre) bsad = __shfl_sync(0xffffffffu, v, 0);
                     centre = false;
                 }
@@ -334,9 +346,9 @@ __device__ __noinline__ void me_integer(int g, int gt, int nthr, int id, const u
                 if (__shfl_sync(0xffffffffu, (int)off, f)) {
                     // off the table: refill it around the running best, as
                     // the sequential walk does on reaching this point
-                    tab = (int *)S.plane + g * plane_words(8) + (tab == (int *)S.plane + g * plane_words(8) ? WIN_WORDS : 0);
+                    tab = tab == tab0 ? tab0 + WIN_WORDS : tab0;
                     wx = bx; wy = by; R = radius;
-                    fill_sad_window(g, gt, nthr, tab, M, wx, wy, R);
+                    fill_sad_window(T, tab, M, wx, wy, R);
                     p0 = f;
                     continue;
                 }
@@ -379,10 +391,11 @@ __device__ __forceinline__ int plane_div(int i, int blk) {   // i / plane_stride
     return (int)((uint32_t)i * m >> 16);
 }
 
-__device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *area, const uint8_t *ref, int blk) {
+__device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, const uint8_t *ref, int blk) {
     Smem &S = smem_state();
     ME_T0();
     MeGroup &E = S.me[id];
+    const int g = T.g, gt = T.gt, nthr = 1 << T.lth;
     const int s = g_fp.stride_y, W = g_fp.W, H = g_fp.H, B = blk, half = B >> 1, ST = half + 6;
     const int bx = E.bx, by = E.by, lane = gt & 31, warp = gt >> 5, gw = nthr >> 5;
     uint32_t *pI = area, *pH = pI + (B + 6) * ST, *pV = pH + (B + 6) * ST, *pD = pV + (B + 1) * ST;
@@ -394,7 +407,7 @@ __device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *
         pI[i] = (uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16;
     }
     if (gt < QPOS * QPOS) E.tab[gt] = 0;
-    group_bar(g, nthr);
+    T.sync();
     // horizontal halves at columns bx - 1 .. (word j reads columns j .. j + 5)
     // of every row; vertical halves of rows by - 1 .. at columns bx - 1 ..
     for (int i = gt; i < (B + 6) * ST - 5; i += nthr)
@@ -403,12 +416,12 @@ __device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *
         const uint32_t *q = pI + i + 2;
         pV[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
     }
-    group_bar(g, nthr);
+    T.sync();
     for (int i = gt; i < (B + 1) * ST - 5; i += nthr) {
         const uint32_t *q = pH + i;
         pD[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
     }
-    group_bar(g, nthr);
+    T.sync();
 
     // Lane p (1..8) holds point p; the points' offsets as in pat_point.
     int ox = 0, oy = 0;
@@ -473,7 +486,7 @@ __device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *
                 acc = __reduce_add_sync(0xffffffffu, acc);
                 if (lane == 0) atomicAdd(&E.tab[(Y - 1) * QPOS + X - 1], (int)acc);
             }
-            group_bar(g, nthr);
+            T.sync();
             const unsigned long long mine = (need >> lane & 1u) ? 1ull << idx : 0ull;
             known |= (unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) << 32 |
                      __reduce_or_sync(0xffffffffu, (unsigned)mine);
@@ -491,41 +504,36 @@ __device__ __noinline__ void me_qpel(int g, int gt, int nthr, int id, uint32_t *
     if (gt == 0) { E.mvx = 4 * bx + ux - 3; E.mvy = 4 * by + uy - 3; E.best = bsad; }
 }
 
-// One search of a leaf: slot id (S.me index), reference plane, start.
-struct MeJob {
-    const uint8_t *ref;
-    int cx, cy;
+// The leaf's searches (bits of `mask`, search k on plane r_k from centre
+// (x_k, y_k)), one warp group each: integer stages, then the refinement.  Two
+// groups' planes fit for a 64x64 leaf, so there a third and fourth group wait
+// for the first and second to be done with theirs.  No barrier of the whole
+// CTA: the other warps score the intra modes meanwhile.
+struct MeStart {
+    const uint8_t *r0, *r1, *r2, *r3;
+    int x0, y0, x1, y1, x2, y2, x3, y3;
 };
-
-// The leaf's searches (bits of `mask`, jobs indexed by search id): integer
-// stages on one warp group each, then the refinement; a 64x64 leaf's planes
-// leave room for two refinements at a time.
-__device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, MeJob j0, MeJob j1, MeJob j2, MeJob j3, int sr) {
+__device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, const MeStart J, int sr, int lth) {
     Smem &S = smem_state();
-    const int cu = L.cu, half = cu >> 1, lgh = lg2i(half), n = __popc(mask);
-    for (int i = threadIdx.x; i < cu * half; i += NT) {
-        const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
-        S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
+    const int cu = L.cu, n = __popc(mask);
+    const MeTeam T(lth);
+    if (T.g >= n) return;
+    unsigned m = mask;          // the group's search
+    if (T.g > 0) m &= m - 1;
+    if (T.g > 1) m &= m - 1;
+    if (T.g > 2) m &= m - 1;
+    const int id = __ffs((int)m) - 1;
+    const uint8_t *ref = id == 0 ? J.r0 : id == 1 ? J.r1 : id == 2 ? J.r2 : J.r3;
+    me_integer(T, id, ref, L.lx, L.ly, cu, id == 0 ? J.x0 : id == 1 ? J.x1 : id == 2 ? J.x2 : J.x3,
+               id == 0 ? J.y0 : id == 1 ? J.y1 : id == 2 ? J.y2 : J.y3, sr);
+    T.sync();                   // S.me[id] is written by one thread
+    if (cu == 64 && T.g >= PLANES64)
+        asm volatile("bar.sync %0, %1;" ::"r"(NGROUP + 1 + T.g - PLANES64), "r"(2 << lth) : "memory");
+    me_qpel(T, id, S.plane + (cu == 64 ? T.g & (PLANES64 - 1) : T.g) * plane_words(cu), ref, cu);
+    if (cu == 64 && T.g + PLANES64 < n) {
+        T.sync();
+        asm volatile("bar.arrive %0, %1;" ::"r"(NGROUP + 1 + T.g), "r"(2 << lth) : "memory");
     }
-    auto nth = [&](int k) {
-        unsigned m = mask;
-        for (; k > 0; --k) m &= m - 1;
-        return m ? __ffs((int)m) - 1 : -1;
-    };
-    auto job = [&](int id) { return id == 0 ? j0 : id == 1 ? j1 : id == 2 ? j2 : j3; };
-    const int nthr = n <= 2 ? 256 : 128, g = threadIdx.x / nthr, gt = threadIdx.x & (nthr - 1);
-    if (g < n) {
-        const int id = nth(g);
-        const MeJob J = job(id);
-        me_integer(g, gt, nthr, id, J.ref, L.lx, L.ly, cu, J.cx, J.cy, sr);
-    }
-    SYNC();   // the SAD tables share the planes' memory
-    const int qthr = cu == 64 ? 256 : nthr, per = NT / qthr, q = threadIdx.x / qthr, qt = threadIdx.x & (qthr - 1);
-    for (int k = q; k < n; k += per) {
-        const int id = nth(k);
-        me_qpel(q, qt, qthr, id, S.plane + q * plane_words(cu), job(id).ref, cu);
-    }
-    SYNC();
 }
 
 // ====================================================================
@@ -608,16 +616,16 @@ __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, i
 // src/encoder.c:476-560; the four-TU form has an outer flag bit).  Keeps the
 // reconstructions of leaves up to 16x16.
 //
-// A warp codes a group of areas for every candidate of its stream.  Bound:
-// issue slots (four warps a scheduler).  Both TU sizes share one prediction
-// and run interleaved; what a lane adds up over its group's areas is reduced
-// once per candidate.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves:
-// larger ones would leave warps without a candidate in the last round (21
-// candidates: 11 rounds of 2 areas in 2 streams, 6 of 4 in 4).  An 8x8
-// leaf's single area is split by TU size instead, over 8 streams.
-__device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl) {
+// Warps take (candidate, group of areas) items from queue `queue` until it is
+// empty: on inter frames the intra modes are scored by the warps that no
+// search occupies, and by the others as their searches end.  Bound: issue
+// slots (four warps a scheduler).  Both TU sizes share one prediction and run
+// interleaved; what a lane adds up over its group's areas is reduced once per
+// item.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves; an 8x8 leaf's
+// single area is split by TU size instead.
+__device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, int queue) {
     Smem &S = smem_state();
-    const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt, warp = threadIdx.x >> 5;
+    const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
     const uint4 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
     const uint4 *bands = S.qparam[0].band;
@@ -628,12 +636,15 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl) {
 #endif
     const int lG = la == 6 ? 2 : la == 0 ? 0 : 1;            // log2 of a group's areas
     const int lg = la == 0 ? 1 : la - lG;                    // log2 of the groups (8x8: TU sizes)
-    const int group = warp & ((1 << lg) - 1), step = NW >> lg;
-    const int sizes = la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4;
-    const int t0 = la == 0 ? 0 : group << lG;
-    for (int k = warp >> lg; k < ncl; k += step) {
-        const int e = cl[k], slot = e & CL_SLOT, do_sizes = e & sizes;
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(&S.next[queue], 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= ncl << lg) break;
+        const int group = it & ((1 << lg) - 1);
+        const int e = cl[it >> lg], slot = e & CL_SLOT, do_sizes = e & (la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4);
         if (!do_sizes) continue;
+        const int t0 = la == 0 ? 0 : group << lG;
         int s8 = 0, n8 = 0, s4 = 0, n4 = 0;
         bool differs = false;
         for (int t = t0; t < t0 + (1 << lG); ++t) {
@@ -891,7 +902,7 @@ __device__ __noinline__ void luma_mc_slots(Smem &, const FrameParams &, const Le
 
 __device__ void zero_acc(Smem &S) {
     for (int i = threadIdx.x; i < NCAND * 4; i += NT) (&S.acc[0][0][0])[i] = 0;
-    if (threadIdx.x == 0) { S.acc64 = 0; S.inexact = 0; }
+    if (threadIdx.x == 0) { S.acc64 = 0; S.inexact = 0; S.next[0] = 0; S.next[1] = 0; }
 }
 
 // Sum over the CU of |orig - pred| per listed slot into acc[slot][0][0]
@@ -1143,6 +1154,21 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     int mvpx, mvpy;
     mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
     zero_acc(S);
+    // Candidate list: intra modes first (they can be scored before the
+    // searches are done), inter candidates after them.
+    const bool try_intra = key || cu <= 16 || medium;
+    const bool use4 = medium && cu <= 32;
+    const uint32_t modes = !try_intra ? 0u : P.preset == 0 ? 0x1041u : P.preset == 1 ? 0x9249u : 0x3FFFFu;
+    const int nintra = __popc(modes);
+    if (tid < 18 && (modes >> tid & 1u))
+        S.cl[__popc(modes & ((1u << tid) - 1u))] = cl_entry(K_INTRA + tid, CL_8 | (use4 ? CL_4 : 0));
+    if (!key) {
+        const int half = cu >> 1, lgh = lg2i(half);
+        for (int i = tid; i < cu * half; i += NT) {
+            const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
+            S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
+        }
+    }
     build_refs(L);
     PHASE_D(0, L.depth);
 
@@ -1166,10 +1192,12 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
                 if (!pg.intra) { has_tmp = true; tdx = pg.dx; tdy = pg.dy; }
             }
         }
-        const MeJob j0 = {P.ref_y[0], cx0, cy0}, j1 = {P.ref_y[1], cx0, cy0},
-                    j2 = {P.ref_y[0], (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2},
-                    j3 = {P.ref_y[0], (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2};
-        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, j0, j1, j2, j3, sr);
+        const MeStart J = {P.ref_y[0], P.ref_y[1], P.ref_y[0], P.ref_y[0], cx0, cy0, cx0, cy0,
+                           (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2,
+                           (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2};
+        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, J, sr, fast ? 8 : 7);
+        if (!fast) luma_score(L, S.cl, nintra, 0);
+        SYNC();
         PHASE_D(1, L.depth);
         if (has_glb && S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) has_glb = false;
         if (has_tmp && S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) has_tmp = false;
@@ -1192,8 +1220,11 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     } else if (is_b) {
         // Forward / backward searches (reference src/encoder.c:795-852).
         const int sr = fast ? 16 : 32;
-        const MeJob j0 = {P.ref_y[maxi(rf, 0)], cx0, cy0}, j1 = {P.ref_y[maxi(rb, 0)], cx0, cy0};
-        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, j0, j1, j0, j1, sr);
+        const uint8_t *f = P.ref_y[maxi(rf, 0)], *b = P.ref_y[maxi(rb, 0)];
+        const MeStart J = {f, b, f, b, cx0, cy0, cx0, cy0, cx0, cy0, cx0, cy0};
+        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, J, sr, fast ? 8 : 7);
+        if (!fast) luma_score(L, S.cl, nintra, 0);
+        SYNC();
         PHASE_D(1, L.depth);
         const uint32_t hf = rf >= 0, hb = rb >= 0, mrg = medium;
         cand = hf | hb << 1 | (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;
@@ -1216,24 +1247,22 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     }
 
     // ---- residual coding / SAD proxies for every candidate --------------
-    const bool try_intra = key || cu <= 16 || medium;
-    const bool use4 = medium && cu <= 32;
-    if (try_intra) cand |= (P.preset == 0 ? 0x1041u : P.preset == 1 ? 0x9249u : 0x3FFFFu) << K_INTRA;
-    const int ncl = __popc(cand);
     // slots 2..4 of a B leaf and the merge slot of a P leaf: 8x8 TUs only
     const uint32_t merges = is_b ? 0x1Cu : 1u << K_MRG;
-    if (tid < 32) {
-        const bool m8 = merges >> lane & 1u;
-        if (cand >> lane & 1u)
-            S.cl[__popc(cand & ((1u << lane) - 1u))] =
-                cl_entry(lane, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
+    const int ninter = __popc(cand);
+    if (tid < NPRED && (cand >> tid & 1u)) {
+        const bool m8 = merges >> tid & 1u;
+        S.cl[nintra + __popc(cand & ((1u << tid) - 1u))] =
+            cl_entry(tid, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
     }
+    cand |= modes << K_INTRA;
     SYNC();
     if (fast) {
-        sad_areas(S, L, S.cl, ncl);
+        sad_areas(S, L, S.cl, nintra + ninter);
         SYNC();
     } else {
-        luma_score(L, S.cl, ncl);
+        if (key) luma_score(L, S.cl, nintra, 0);
+        else luma_score(L, S.cl + nintra, ninter, 1);
         SYNC();
         PHASE_D(3, L.depth);
         if (is_p) {

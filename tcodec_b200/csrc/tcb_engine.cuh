@@ -1,6 +1,7 @@
 // tcb_engine.cuh — shared-memory layout and launch constants of the CTU
 // rate-distortion engine (one 512-thread CTA per 64x64 CTU).
 #pragma once
+#include <stddef.h>
 #include "tcb_common.cuh"
 #include "tcb_resid.cuh"
 
@@ -97,6 +98,7 @@ struct Smem {
     long long acc64;
     int cl[NCAND];             // candidate list for job loops
     int cand_mvx[NPRED], cand_mvy[NPRED], cand_ref[NPRED], cand_ref2[NPRED];
+    int next[2];               // work queues of luma_score: next item
     int dc;
     int above0;                // first sample of the above run (the planar mode's corner)
     int inexact;               // the merge prediction of the current leaf differs from the source
