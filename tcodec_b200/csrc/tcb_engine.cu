@@ -261,13 +261,10 @@ __device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, co
 // the result.  Two tables alternate, so refilling one never races with a
 // lagging thread still reading the other.
 constexpr int WIN_RMAX = 5, WIN_NMAX = 2 * WIN_RMAX + 1, WIN_WORDS = WIN_NMAX * WIN_NMAX;
-// (they lie past what the planes of a block up to 16x16 and the
-// reconstruction cache occupy, which are in use at the same time)
+// (they lie past the planes of blocks up to 16x16, which are in use at the
+// same time)
 constexpr int WIN_AT = PLANE_WORDS - NGROUP * 2 * WIN_WORDS;
-static_assert(NGROUP * plane_words(16) <= WIN_AT && (offsetof(Smem, crec) - offsetof(Smem, plane) + sizeof(Smem::crec)) / 4 <= WIN_AT,
-              "SAD tables overlap the planes or the reconstruction cache");
-static_assert(NGROUP * plane_words(16) * 4 <= offsetof(Smem, crec) - offsetof(Smem, plane),
-              "intra scoring writes the reconstruction cache while the searches use the planes");
+static_assert(NGROUP * plane_words(16) <= WIN_AT, "SAD tables overlap the planes");
 static_assert(WIN_WORDS <= 128, "one table position per thread of the smallest group");
 
 __device__ __forceinline__ int window_radius(int r) { return r >= 2 && r <= WIN_RMAX ? r : 4; }
@@ -613,8 +610,7 @@ __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, i
 
 // Scores the listed candidates: distortion and bits of one 8x8 TU, of four
 // 4x4 TUs, or of both per 8x8 area, added to the slots' sums (reference
-// src/encoder.c:476-560; the four-TU form has an outer flag bit).  Keeps the
-// reconstructions of leaves up to 16x16.
+// src/encoder.c:476-560; the four-TU form has an outer flag bit).
 //
 // Warps take (candidate, group of areas) items from queue `queue` until it is
 // empty: on inter frames the intra modes are scored by the warps that no
@@ -648,7 +644,7 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
         int s8 = 0, n8 = 0, s4 = 0, n4 = 0;
         bool differs = false;
         for (int t = t0; t < t0 + (1 << lG); ++t) {
-            const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row, at = y * cu + x;
+            const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
             const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
             const uint32_t pv = pred2(S, cu, e, x, y);
             differs |= pv != cv;
@@ -657,14 +653,12 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
                 n8 += c.bits;
                 const int b = S.last_bits[last8(c, lane)];
                 if (lane == 0) n8 += b;
-                if (la <= 2) *(uint16_t *)(S.crec[slot][0] + at) = (uint16_t)c.rec;
             };
             auto add4 = [&](const AreaCode &c) {
                 s4 += c.sse;
                 n4 += c.bits;
                 const int b = S.last_bits[last4(c, lane)];
                 if ((lane & 13) == 0) n4 += b;
-                if (la <= 2) *(uint16_t *)(S.crec[slot][1] + at) = (uint16_t)c.rec;
             };
             if (do_sizes == (CL_8 | CL_4)) {
                 const AreaCode c8 = code_area(cv, pv, f8, i8, b80, b81);
@@ -710,17 +704,70 @@ __device__ __noinline__ void luma_replay(const Leaf L, int e, int16_t *emit) {
         const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
         const AreaCode c = code_area(cv, pred2(S, cu, e, x, y), f, i, b0, b1);
         *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
-        if (emit) *(uint32_t *)(emit + t * 64 + pos) = c.levels();
+        *(uint32_t *)(emit + t * 64 + pos) = c.levels();
     }
 }
 
-// Chroma residual coding (reference src/encoder.c:429-475 qt_code_chroma):
-// 4x4 TUs, four (option, component, TU) jobs per warp, one on each quarter of
-// the area's lanes, from warp `woff` on.  Option o, component c predicts from
-// S.cpred[cbase + 2*o + c]; results accumulate in slot o.
-__device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, bool accum, bool wrec, int16_t *emit,
-                                          int woff) {
+// Chroma DC value and chroma-from-luma model of component c of a leaf, by one
+// warp, from its reconstructed neighbours (reference src/predict.c:364-462).
+// At most 64 neighbour pairs of 8-bit samples: every sum and product stays
+// under 2^29 (n * sum(la * cv) <= 64 * 64 * 255^2), so 32-bit integers give
+// the reference's int64 values.
+__device__ __noinline__ void chroma_model(const Leaf L, int c) {
     Smem &S = smem_state();
+    const int cs = L.cu >> 1, lxc = L.lx >> 1, lyc = L.ly >> 1, lane = threadIdx.x & 31;
+    const bool up = L.py > 0, left = L.px > 0;
+    int sl = 0, sc = 0, slc = 0, sl2 = 0;
+    for (int i = lane; i < cs; i += 32) {
+        if (up) {
+            const int la = (RY(S, L.lx + 2 * i, L.ly - 1) + RY(S, L.lx + 2 * i + 1, L.ly - 1) + 1) >> 1;
+            const int cv = RC(S, c, lxc + i, lyc - 1);
+            sl += la; sc += cv; slc += la * cv; sl2 += la * la;
+        }
+        if (left) {
+            const int la = (RY(S, L.lx - 2, L.ly + 2 * i) + RY(S, L.lx - 1, L.ly + 2 * i) +
+                            RY(S, L.lx - 2, L.ly + 2 * i + 1) + RY(S, L.lx - 1, L.ly + 2 * i + 1) + 2) >> 2;
+            const int cv = RC(S, c, lxc - 1, lyc + i);
+            sl += la; sc += cv; slc += la * cv; sl2 += la * la;
+        }
+    }
+    const int n = (up ? cs : 0) + (left ? cs : 0);
+    sl = (int)__reduce_add_sync(0xffffffffu, (unsigned)sl);
+    sc = (int)__reduce_add_sync(0xffffffffu, (unsigned)sc);
+    slc = (int)__reduce_add_sync(0xffffffffu, (unsigned)slc);
+    sl2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)sl2);
+    if (lane == 0) {
+        const int cov = n * slc - sl * sc, vl = n * sl2 - sl * sl;
+        int ash = 3;
+        if (n > 0 && vl > 0 && cov != 0) {
+            const unsigned q = (unsigned)vl / (unsigned)(cov < 0 ? -cov : cov);
+            const int sh = q < 1 ? 2 : 31 - __clz((int)q);
+            ash = sh < 2 ? 2 : (sh > 5 ? 5 : sh);
+        }
+        S.cdc[c] = n ? (sc + n / 2) >> lg2i(n) : 128;   // n: cs or 2 cs
+        S.cfl_sign[c] = cov >= 0 ? 1 : -1;
+        S.cfl_shift[c] = ash;
+    }
+}
+
+// A leaf's chroma prediction: DC, CfL (DC plus the scaled difference of the
+// collocated luma from its 4x4 mean), or motion compensation, bi-predictive
+// with the mirrored vector when r2 >= 0 (reference src/encoder.c:673-699).
+enum { CH_DC, CH_CFL, CH_MC };
+struct ChromaPred {
+    int kind, r1, r2, mvx, mvy;
+};
+
+// Chroma coding (reference src/encoder.c:429-475 qt_code_chroma): 4x4 TUs,
+// four (option, component, TU) jobs per warp, one on each quarter of the
+// area's lanes, from warp `woff` on; predictions are formed in registers (a
+// TU is one 4x4 tile, so its CfL mean is a sum over the quarter's lanes).
+// One option (nopt 1): prediction K, reconstruction into the tile, levels to
+// `emit`.  Two: K and CfL, distortion and bits to S.cacc, reconstruction and
+// levels of both to S.cpred / S.clev.
+__device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPred K, int16_t *emit, int woff) {
+    Smem &S = smem_state();
+    const FrameParams &P = g_fp;
     const int cs = L.cu >> 1, ln = lg2i(cs) - 2, J = nopt << (2 * ln + 1);
     const int lxc = L.lx >> 1, lyc = L.ly >> 1;
     const int lane = threadIdx.x & 31, r = (lane >> 2) & 3, cc = 2 * (lane & 1);
@@ -736,22 +783,55 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, int cbase, boo
         const int o = j >> (2 * ln + 1), c = (j >> (2 * ln)) & 1, t = j & ((1 << (2 * ln)) - 1);
         const int x = (t & ((1 << ln) - 1)) * 4 + cc, y = (t >> ln) * 4 + r;
         const uint32_t cv = *(const uint16_t *)(S.cur_c[c] + (lyc + y) * 32 + lxc + x);
-        const uint32_t pv = *(const uint16_t *)(S.cpred[cbase + 2 * o + c] + y * cs + x);
+        uint32_t pv = (uint32_t)S.cdc[c] * 0x101u;
+        if (K.kind == CH_CFL || nopt == 2) {
+            const uint32_t l0 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y);
+            const uint32_t l1 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y + 1);
+            const int a0 = (int)__dp4a(l0, 0x0101u, __dp4a(l1, 0x0101u, 2u)) >> 2;
+            const int a1 = (int)__dp4a(l0, 0x01010000u, __dp4a(l1, 0x01010000u, 2u)) >> 2;
+            int m = a0 + a1;
+            m += __shfl_xor_sync(0xffffffffu, m, 1);
+            m += __shfl_xor_sync(0xffffffffu, m, 4);
+            m += __shfl_xor_sync(0xffffffffu, m, 8);
+            m = (m + 8) >> 4;
+            if (K.kind == CH_CFL || o == 1) {
+                const int dc = S.cdc[c], sg = S.cfl_sign[c], sh = S.cfl_shift[c];
+                pv = (uint32_t)__viaddmin_s32_relu(dc, sg * ((a0 - m) >> sh), 255) |
+                     (uint32_t)__viaddmin_s32_relu(dc, sg * ((a1 - m) >> sh), 255) << 8;
+            }
+        }
+        if (K.kind == CH_MC && o == 0) {
+            const int Wc = P.W >> 1, Hc = P.H >> 1;
+            pv = 0;
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+                int v = chroma_mc_at(c ? P.ref_cr[K.r1] : P.ref_cb[K.r1], P.stride_c, Wc, Hc, K.mvx, K.mvy, x + e, y);
+                if (K.r2 >= 0)
+                    v = (v + chroma_mc_at(c ? P.ref_cr[K.r2] : P.ref_cb[K.r2], P.stride_c, Wc, Hc, -K.mvx, -K.mvy, x + e, y) + 1) >> 1;
+                pv |= (uint32_t)v << (8 * e);
+            }
+        }
+        __syncwarp();
         const AreaCode a = code_area(cv, pv, f4, i4, b0, b1);
-        if (accum) {
+        if (nopt == 2) {
             int d = a.sse, n = a.bits;    // of the quarter's eight lanes: index bits 0, 2 and 3
             for (int m = 1; m < 16; m = m == 1 ? 4 : 2 * m) {
                 d += __shfl_xor_sync(0xffffffffu, d, m);
                 n += __shfl_xor_sync(0xffffffffu, n, m);
             }
             n += S.last_bits[last4(a, lane)];
-            if (act && (lane & 13) == 0) {
-                atomicAdd(&S.acc[o][0][0], d);
-                atomicAdd(&S.acc[o][0][1], n);
+            if (act) {
+                if ((lane & 13) == 0) {
+                    atomicAdd(&S.cacc[o][0], d);
+                    atomicAdd(&S.cacc[o][1], n);
+                }
+                *(uint16_t *)(S.cpred[2 * o + c] + y * cs + x) = (uint16_t)a.rec;
+                *(uint32_t *)(S.clev[2 * o + c] + t * 16 + r * 4 + cc) = a.levels();
             }
+        } else if (act) {
+            *(uint16_t *)&RC(S, c, lxc + x, lyc + y) = (uint16_t)a.rec;
+            *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = a.levels();
         }
-        if (act && wrec) *(uint16_t *)&RC(S, c, lxc + x, lyc + y) = (uint16_t)a.rec;
-        if (act && emit) *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = a.levels();
     }
 }
 
@@ -902,6 +982,7 @@ __device__ __noinline__ void luma_mc_slots(Smem &, const FrameParams &, const Le
 
 __device__ void zero_acc(Smem &S) {
     for (int i = threadIdx.x; i < NCAND * 4; i += NT) (&S.acc[0][0][0])[i] = 0;
+    if (threadIdx.x < 4) S.cacc[threadIdx.x >> 1][threadIdx.x & 1] = 0;
     if (threadIdx.x == 0) { S.acc64 = 0; S.inexact = 0; S.next[0] = 0; S.next[1] = 0; }
 }
 
@@ -1007,56 +1088,52 @@ __device__ __noinline__ void chroma_mc_bi(Smem &, const FrameParams &, const Lea
 }
 
 // ====================================================================
-// Leaf coding of a decided node: replay in the decide pass, syntax-order
-// coefficient emission in the write pass (reference src/encoder.c:587-781).
+// Leaf coding of a decided node (reference src/encoder.c:587-781): its
+// reconstruction into the tile and its levels into the CTU's record, where
+// the leaf's place is 96 levels per coded 8x8 cell before it in z-order
+// (close_gaps moves the levels up when skipped leaves leave gaps).  A 32x32 or
+// 16x16 leaf's levels wait in shared memory until it has won against its
+// split.  The last time a leaf of the final tree is coded leaves the record's
+// values, so no pass over the final tree is needed.
+// `decided`: the decision has just been made; its reference samples, chroma
+// model and inter predictions are still in shared memory, and an intra leaf's
+// chroma prediction is still to be chosen (src/encoder.c:1194-1221).
 // ====================================================================
-// The winner's luma reconstruction from the decide pass's cache (leaves up
-// to 16x16): the same samples its residual job produced when it was scored.
-__device__ void luma_from_cache(Smem &S, const Leaf &L, int slot, bool dct8) {
-    const int cu = L.cu;
-    const uint8_t *src = S.crec[slot][dct8 ? 0 : 1];
-    const int lg = lg2i(cu);
-    for (int i = threadIdx.x; i < cu * cu; i += NT) {
-        const int y = i >> lg, x = i & (cu - 1);
-        RY(S, L.lx + x, L.ly + y) = src[i];
-    }
-}
-
-// `from`: 0 codes the node from its record alone; 1 replays the winner of the
-// decision just made (its references, inter predictions and, up to 16x16, its
-// reconstruction are still in shared memory); 2 as 1 with the luma
-// reconstruction already in the tile.
-__device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L, bool emit, CtuOut *out, int from) {
+__device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
-    const Node nd = S.nodes[qt_index(L.depth, L.cx, L.cy)];
+    Node &node = S.nodes[qt_index(L.depth, L.cx, L.cy)];
+    const Node nd = node;
     int mvpx, mvpy;
     mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
-    const int cu = L.cu;
-    int16_t *el = emit ? out->coef + S.ncoef : nullptr;
-    int16_t *ec = emit ? el + cu * cu : nullptr;
-    const bool use_cache = from && P.preset >= 2 && cu <= 16;
+    const int cu = L.cu, cs = cu >> 1;
+    int16_t *el = L.depth == 1 ? S.lev1 : L.depth == 2 ? S.lev2 : S.coef + 96 * S.zoff[L.cy * 8 + L.cx];
+    int16_t *ec = el + cu * cu;
     const int cl_size = nd.dct_size ? CL_8 : CL_4;
-    bool coded = true;
     if (nd.intra) {
-        if (from < 2) {
-            if (use_cache) {
-                luma_from_cache(S, L, K_INTRA + nd.intra_mode, nd.dct_size);
-            } else {
-                if (!from) build_refs(L);
-                luma_replay(L, cl_entry(K_INTRA + nd.intra_mode, cl_size), el);
-            }
+        if (!decided) {
+            if (threadIdx.x >= NT - 64) chroma_model(L, (threadIdx.x >> 5) & 1);
+            build_refs(L);
+        }
+        luma_replay(L, cl_entry(K_INTRA + nd.intra_mode, cl_size), el);
+        SYNC();
+        const ChromaPred mc = {P.ref_valid[0] ? CH_MC : CH_DC, 0, -1, mvpx + L.px * 4, mvpy + L.py * 4};
+        if (decided && P.preset >= 2) {
+            chroma_areas(L, 2, mc, nullptr, 0);
             SYNC();
-        }
-        if (nd.ch_intra) {
-            chroma_dc_pred(S, L, 0);
-            cfl_blend(S, L, 0);
-        } else if (P.ref_valid[0]) {
-            chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
+            const long long lam = P.lambda;
+            const int o = S.cacc[1][0] + lam * (S.cacc[1][1] + 4) < S.cacc[0][0] + lam * (S.cacc[0][1] + 1);
+            if (threadIdx.x == 0) node.ch_intra = (uint8_t)o;
+            const int lg = lg2i(cs);
+            for (int i = threadIdx.x; i < cs * cs; i += NT) {   // two samples of one component
+                const int c = i >> (2 * lg - 1), p = 2 * i & (cs * cs - 1), y = p >> lg, x = p & (cs - 1);
+                *(uint16_t *)&RC(S, c, (L.lx >> 1) + x, (L.ly >> 1) + y) = *(const uint16_t *)(S.cpred[2 * o + c] + p);
+                *(uint32_t *)(ec + 2 * i) = *(const uint32_t *)(S.clev[2 * o + c] + p);
+            }
         } else {
-            chroma_dc_pred(S, L, 0);
+            const ChromaPred cfl = {CH_CFL, 0, -1, 0, 0};
+            chroma_areas(L, 1, nd.ch_intra ? cfl : mc, ec, 0);
         }
-        chroma_areas(L, 1, 0, false, true, ec, 0);
     } else {
         int mvx, mvy;
         if (nd.merge || nd.skip) { mvx = mvpx + L.px * 4; mvy = mvpy + L.py * 4; }
@@ -1089,32 +1166,28 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
             cr1 = r1;
         }
         if (!nd.skip) {
-            const int src = from ? S.win_slot : 0;   // the decision's prediction is still in its slot
-            if (!from && threadIdx.x == 0) {
-                S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
-            }
-            SYNC();
-            // Chroma prediction does not depend on this leaf's luma, so both
-            // predictions are formed first and the luma and chroma residual
-            // jobs then run side by side on different warps.
-            if (nd.ch_intra || cflat) chroma_dc_pred(S, L, 0);
-            else chroma_mc_bi(S, P, L, cr1, cr2, mvx, mvy);
-            if (use_cache) {
-                luma_from_cache(S, L, src, nd.dct_size);
-                chroma_areas(L, 1, 0, false, true, ec, 0);
+            const int src = decided ? S.win_slot : 0;   // the decision's prediction is still in its slot
+            if (decided) {
+                SYNC();   // every thread has read the grid (mvp_at)
             } else {
-                if (!from && flat) {
+                if (threadIdx.x == 0) {
+                    S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
+                }
+                if (cflat && threadIdx.x >= NT - 64) chroma_model(L, (threadIdx.x >> 5) & 1);
+                SYNC();
+                if (flat) {
                     for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
                     SYNC();
-                } else if (!from) {
+                } else {
                     const int slots[1] = {0};
                     luma_mc_slots(S, P, L, 1, slots, false);
                 }
-                luma_replay(L, src | cl_size, el);
-                chroma_areas(L, 1, 0, false, true, ec, mini(NW / 2, (cu * cu) >> 6));
             }
+            // luma and chroma run side by side on different warps
+            const ChromaPred mc = {cflat ? CH_DC : CH_MC, cr1, cr2, mvx, mvy};
+            luma_replay(L, src | cl_size, el);
+            chroma_areas(L, 1, mc, ec, mini(NW / 2, (cu * cu) >> 6));
         } else {
-            coded = false;
             if (threadIdx.x == 0) {
                 S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = 0; S.cand_ref2[0] = -1;
             }
@@ -1123,15 +1196,6 @@ __device__ __noinline__ void leaf_code(Smem &, const FrameParams &, const Leaf L
             luma_mc_slots(S, P, L, 1, slots, true);
             if (P.fresh_skip && P.frame_type == 1 && P.ref_valid[0])
                 chroma_mc(S, P, L, 0, mvx, mvy, 0, true);
-        }
-    }
-    SYNC();
-    if (emit && coded && threadIdx.x == 0) {
-        S.ncoef += cu * cu + (cu * cu >> 1);
-        if (nd.dct_size) {
-            const int gc = cu >> 3;
-            for (int gy = 0; gy < gc; ++gy)
-                for (int gx = 0; gx < gc; ++gx) S.tu8mask |= 1ull << ((L.cy + gy) * 8 + L.cx + gx);
         }
     }
     grid_update(S, L, nd, mvpx, mvpy);
@@ -1169,6 +1233,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
             S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
         }
     }
+    if (tid >= NT - 64) chroma_model(L, (tid >> 5) & 1);
     build_refs(L);
     PHASE_D(0, L.depth);
 
@@ -1353,37 +1418,8 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     SYNC();
 
     PHASE_D(5, L.depth);
-    // ---- intra chroma choice: MC vs CfL-blended DC (src/encoder.c:1194-1221)
-    const Node nd0 = S.nodes[qt_index(L.depth, L.cx, L.cy)];
-    const bool luma_done = nd0.intra && medium;
-    if (luma_done) {
-        if (cu <= 16) {
-            luma_from_cache(S, L, K_INTRA + nd0.intra_mode, nd0.dct_size);
-        } else {
-            luma_replay(L, cl_entry(K_INTRA + nd0.intra_mode, nd0.dct_size ? CL_8 : CL_4), nullptr);
-        }
-        SYNC();
-        if (P.ref_valid[0]) chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
-        else chroma_dc_pred(S, L, 0);
-        chroma_dc_pred(S, L, 2);
-        cfl_blend(S, L, 2);
-        zero_acc(S);
-        SYNC();
-        chroma_areas(L, 2, 0, true, false, nullptr, 0);
-        SYNC();
-        if (tid == 0) {
-            const long long lam = P.lambda;
-            const long long dmc = S.acc[0][0][0], dcfl = S.acc[1][0][0];
-            const int lbmc = S.acc[0][0][1], lbcfl = S.acc[1][0][1];
-            if (dcfl + lam * (lbcfl + 4) < dmc + lam * (lbmc + 1))
-                S.nodes[qt_index(L.depth, L.cx, L.cy)].ch_intra = 1;
-        }
-        SYNC();
-    }
     const long long best = S.best_cost;
-    PHASE_D(6, L.depth);
-    // ---- replay of the winner ------------------------------------------
-    leaf_code(S, P, L, false, nullptr, luma_done ? 2 : 1);
+    leaf_code(L, true);
     PHASE_D(7, L.depth);
     return best;
 }
@@ -1400,7 +1436,7 @@ __device__ long long leaf_eval(Smem &S, const FrameParams &P, const Leaf &L, boo
     const int idx = qt_index(L.depth, L.cx, L.cy);
     if (cached) {
         const long long c = S.node_cost[idx];
-        leaf_code(S, P, L, false, nullptr, 0);
+        leaf_code(L, false);
         return c;
     }
     const long long c = leaf_decide(S, P, L);
@@ -1432,7 +1468,7 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
         const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
         snap<D>(S, L, 0, true);
         const long long parent = leaf_eval<D>(S, P, L, cached);
-        snap<D>(S, L, 1, true);
+        if constexpr (D > 0) snap<D>(S, L, 1, true);
         snap<D>(S, L, 0, false);
         long long child = 0;
         for (int q = 0; q < 4; ++q) {
@@ -1441,18 +1477,32 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
         }
         if (child <= parent) {
             if (threadIdx.x == 0) nd.split = 1;
-            snap<D>(S, L, 0, false);
-            // Children keep their split-test evaluation until one of them
-            // splits (its region then differs from the split test's state).
-            bool same_state = true;
-            for (int q = 0; q < 4; ++q) {
-                const int qx = cx + (q & 1) * h, qy = cy + (q >> 1) * h;
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, qx, qy, same_state);
-                if (S.nodes[qt_index(D + 1, qx, qy)].split) same_state = false;
+            if constexpr (D == 2) {
+                // 8x8 children split no further: the split test has left
+                // their final reconstruction, grid and levels
+                SYNC();
+            } else {
+                snap<D>(S, L, 0, false);
+                // Children keep their split-test evaluation until one of them
+                // splits (its region then differs from the split test's state).
+                bool same_state = true;
+                for (int q = 0; q < 4; ++q) {
+                    const int qx = cx + (q & 1) * h, qy = cy + (q >> 1) * h;
+                    qt_decide<D + 1>(S, P, ctu_x, ctu_y, qx, qy, same_state);
+                    if (S.nodes[qt_index(D + 1, qx, qy)].split) same_state = false;
+                }
             }
         } else {
             if (threadIdx.x == 0) nd.split = 0;
-            snap<D>(S, L, 1, false);
+            if constexpr (D == 0) {
+                snap<D>(S, L, 0, false);
+                leaf_code(L, false);
+            } else {
+                const uint2 *lev = (const uint2 *)(D == 1 ? S.lev1 : S.lev2);
+                uint2 *out = (uint2 *)(S.coef + 96 * S.zoff[cy * 8 + cx]);
+                for (int i = threadIdx.x; i < 24 * (64 >> (2 * D)); i += NT) out[i] = lev[i];
+                snap<D>(S, L, 1, false);
+            }
         }
     } else {
         if (!in_frame) return;
@@ -1463,23 +1513,65 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
     }
 }
 
-template <int D>
-__device__ void qt_write(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy, CtuOut *out) {
-    constexpr int cu = 64 >> D;
-    const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
-    const bool in_frame = px + cu <= P.W && py + cu <= P.H;
-    if constexpr (D < 3) {
-        constexpr int h = 4 >> D;
-        if (!in_frame || S.nodes[qt_index(D, cx, cy)].split) {
-            for (int q = 0; q < 4; ++q)
-                qt_write<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, out);
-            return;
+// The final tree's 8x8-TU mask, and its levels without the gaps of skipped
+// leaves (reference src/encoder.c:1450-1456 writes the leaves in z-order).
+__device__ __noinline__ void close_gaps(int ctu_x, int ctu_y, CtuOut *out) {
+    Smem &S = smem_state();
+    const int t = threadIdx.x;
+    const auto in_frame = [&](int cx, int cy, int cu) {
+        return ctu_x + cx * 8 + cu <= g_fp.W && ctu_y + cy * 8 + cu <= g_fp.H;
+    };
+    bool skip = false, tu8 = false, cell = false;
+    if (t < 64) {
+        const int cx = t & 7, cy = t >> 3;
+        cell = in_frame(cx, cy, 8);
+        for (int d = 0; cell && d < 4; ++d) {
+            const int m = ~((8 >> d) - 1), nx = cx & m, ny = cy & m;
+            const Node &nd = S.nodes[qt_index(d, nx, ny)];
+            if (d < 3 && (nd.split || !in_frame(nx, ny, 64 >> d))) continue;
+            skip = nd.skip;
+            tu8 = !skip && nd.dct_size;
+            break;
         }
-    } else {
-        if (!in_frame) return;
+        S.leaf_skip[t] = skip;
     }
-    const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-    leaf_code(S, P, L, true, out, 0);
+    const unsigned b8 = __ballot_sync(0xffffffffu, tu8);
+    if (t == 0 || t == 32) ((unsigned *)&S.tu8mask)[t >> 5] = b8;
+    const int ncells = __syncthreads_count(cell), nskip = __syncthreads_count(skip);
+    if (t == 0) S.ncoef = 96 * (ncells - nskip);
+    if (nskip) {
+        // every thread holds its levels before any is moved; a cell's levels
+        // move by the skipped cells before it
+        constexpr int PER = CTU_COEF_MAX / 4 / NT;
+        uint2 v[PER];
+        int to[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int u = t + k * NT, z = u / 24;      // 4 levels; cell in order of coding
+            to[k] = -1;
+            if (z < ncells) {
+                v[k] = *(const uint2 *)(out->coef + 4 * u);
+                int before = 0;
+                for (int i = 0; i < 64; ++i) {
+                    const int zi = S.zoff[i];
+                    if (S.leaf_skip[i] && zi < z) ++before;
+                    if (zi == z && in_frame(i & 7, i >> 3, 8) && !S.leaf_skip[i]) to[k] = 0;
+                }
+                if (to[k] == 0) to[k] = u - 24 * before;
+            }
+        }
+        SYNC();
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int u = t + k * NT;
+            if (u >= 24 * (ncells - nskip) && u < 24 * ncells) *(uint2 *)(out->coef + 4 * u) = make_uint2(0, 0);
+        }
+        // (a cell never moves past the end of the kept ones)
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (to[k] >= 0) *(uint2 *)(out->coef + 4 * to[k]) = v[k];
+    }
+    SYNC();
 }
 
 // ====================================================================
@@ -1641,7 +1733,17 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
         Node z = {};
         S.nodes[i] = z;
     }
-    if (threadIdx.x == 0) { S.ncoef = 0; S.tu8mask = 0; }
+    CtuOut *out = P.out + row * P.ctu_cols + col;
+    if (threadIdx.x == 0) S.coef = out->coef;
+    if (threadIdx.x < 64) {
+        // coded cells (whole 8x8 blocks of the frame) before the z-th cell of
+        // z-order, z = this thread
+        auto at = [](int z, int b) { return (z >> b & 1) | (z >> (b + 1) & 2) | (z >> (b + 2) & 4); };
+        int n = 0;
+        for (int z = 0; z < (int)threadIdx.x; ++z)
+            n += ctu_x + at(z, 0) * 8 + 8 <= P.W && ctu_y + at(z, 1) * 8 + 8 <= P.H;
+        S.zoff[at(threadIdx.x, 1) * 8 + at(threadIdx.x, 0)] = (uint16_t)n;
+    }
     SYNC();
 
     // Quantiser parameters in shared memory: every residual job reads them
@@ -1653,17 +1755,11 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     }
     SYNC();
 
-    // ---- decide, then write in syntax order ----------------------------
+    // ---- decide and code -------------------------------------------------
     PHASE_T0();
     qt_decide<0>(S, P, ctu_x, ctu_y, 0, 0, false);
     PHASE(8);
-    for (int i = threadIdx.x; i < 64; i += NT) {
-        S.grid[i].dx = 0; S.grid[i].dy = 0; S.grid[i].intra = 1;
-    }
-    SYNC();
-    CtuOut *out = P.out + row * P.ctu_cols + col;
-    qt_write<0>(S, P, ctu_x, ctu_y, 0, 0, out);
-    SYNC();
+    close_gaps(ctu_x, ctu_y, out);
     PHASE(9);
     // ---- in-loop filters ------------------------------------------------
     if (w == 64 && h == 64) deblock_tile(S, P.qp);

@@ -65,8 +65,9 @@ struct Smem {
     uint8_t cur_c[2][32 * 32];
     uint8_t rec_y[RY_H * RY_W];
     uint8_t rec_c[2][RC_H * RC_W];
-    // qt_split snapshots, per depth: luma, cb, cr, grid (pre / parent).
-    uint8_t snap_y0[2][64 * 64], snap_c0[2][2][32 * 32];
+    // qt_split snapshots, per depth: luma, cb, cr, grid (pre / parent; a
+    // 64x64 parent that wins is coded again instead).
+    uint8_t snap_y0[1][64 * 64], snap_c0[1][2][32 * 32];
     uint8_t snap_y1[2][32 * 32], snap_c1[2][2][16 * 16];
     uint8_t snap_y2[2][16 * 16], snap_c2[2][2][8 * 8];
     MvCell snap_g[3][2][64];
@@ -77,11 +78,11 @@ struct Smem {
         // after the searches of a leaf
         struct {
             alignas(16) uint8_t pred[NPRED][64 * 64];
+            // chroma predictions (decoder, skip check), or the two chroma
+            // options of an intra leaf: reconstruction and levels of option o,
+            // component c in [2 * o + c]
             uint8_t cpred[4][32 * 32];
-            // Luma reconstruction of every scored candidate of the current
-            // leaf (leaves up to 16x16), [slot][8x8 TUs, 4x4 TUs]: the replay
-            // of the winner copies it instead of coding the winner again.
-            uint8_t crec[NCAND][2][16 * 16];
+            int16_t clev[4][32 * 32];
         };
         // during them: SAD tables of the integer stages, then sample planes
         alignas(16) uint32_t plane[PLANE_WORDS];
@@ -94,6 +95,10 @@ struct Smem {
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
     int acc[NCAND][2][2];      // per slot and TU size (8x8, 4x4): distortion, bits
+    int cacc[2][2];            // per chroma option: distortion, bits
+    int cdc[2], cfl_sign[2], cfl_shift[2];   // chroma DC and CfL model of the current leaf, per component
+    uint16_t zoff[64];         // coded 8x8 cells before each cell of the CTU in z-order
+    uint8_t leaf_skip[64];     // the cell's leaf is skipped
     int last_bits[65];         // last_bits(last) by last + 1
     long long acc64;
     int cl[NCAND];             // candidate list for job loops
@@ -106,7 +111,10 @@ struct Smem {
     int sao[3];
     int band_sum[32], band_cnt[32], band_sq[32], band_new[32], band_cand[32];
     int ncoef;
-    unsigned long long tu8mask;
+    int16_t *coef;             // the CTU record's levels
+    // levels of a 32x32 / 16x16 leaf while its split is tried
+    alignas(8) int16_t lev1[32 * 48], lev2[16 * 24];
+    alignas(8) unsigned long long tu8mask;
 };
 
 }  // namespace tcb

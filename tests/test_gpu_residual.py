@@ -41,3 +41,27 @@ def test_residual_extremes_decode_to_the_encoders_picture(kind, qp, preset):
     for t, (got, want) in enumerate(zip(decoded, recons)):
         for k in range(3):
             assert np.array_equal(got[k], want[k]), (t, k)
+
+
+@pytest.mark.parametrize("w,h", [(64, 64), (72, 72), (200, 136)])
+def test_skipped_leaves_leave_no_gap_in_the_record(w, h):
+    """Half of each picture is the previous reconstruction (exact skips), the
+    other half changes: the levels of the coded leaves, placed in z-order,
+    must close up over the skipped ones."""
+    from tcodec_b200 import api, synth
+    lib = api.load_library()
+    frames = synth.moving_rects_clip(w, h, 4)
+    enc = api.Encoder(lib, api.make_config(lib, w, h, qp=27, preset=2, profile=1, keyframe_interval=1000))
+    packets, recons = [], []
+    try:
+        for t, f in enumerate(frames):
+            if t:
+                f = tuple(np.where(np.arange(p.shape[1])[None, :] < p.shape[1] // 2, r, p)
+                          for p, r in zip(f, recons[-1]))
+            packets.append(enc.encode(*f))
+            recons.append(enc.recon())
+    finally:
+        enc.close()
+    for t, (got, want) in enumerate(zip(api.decode_sequence(lib, packets), recons)):
+        for k in range(3):
+            assert np.array_equal(got[k], want[k]), (t, k)
