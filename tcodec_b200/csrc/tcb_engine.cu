@@ -388,37 +388,129 @@ __device__ __forceinline__ int plane_div(int i, int blk) {   // i / plane_stride
     return (int)((uint32_t)i * m >> 16);
 }
 
+// The planes of a block around its integer position (bx, by).
+struct Planes {
+    uint32_t *I, *H, *V, *D;
+    int B, ST;
+    __device__ __forceinline__ Planes(uint32_t *area, int blk) : B(blk), ST((blk >> 1) + 6) {
+        I = area;
+        H = I + (B + 6) * ST;
+        V = H + (B + 6) * ST;
+        D = V + (B + 1) * ST;
+    }
+    // Integer samples of rows by - 3 .., columns bx - 3 .. (clamped: samples
+    // outside the frame are never part of a point that is used); then, as
+    // asked for, horizontal halves at columns bx - 1 .. (word j reads columns
+    // j .. j + 5) of every row, vertical halves of rows by - 1 .. at columns
+    // bx - 1 .., and centre halves.  All threads of the team.
+    __device__ __forceinline__ void build(const MeTeam &T, const uint8_t *ref, int bx, int by, bool h, bool v,
+                                          bool d) const {
+        const int nthr = 1 << T.lth, half = B >> 1, s = g_fp.stride_y, W = g_fp.W, Hh = g_fp.H;
+        for (int i = T.gt; i < (B + 6) * ST; i += nthr) {
+            const int r = plane_div(i, B), x = bx - 3 + i - r * ST;
+            const uint8_t *row = ref + (size_t)clampi(by - 3 + r, 0, Hh - 1) * s;
+            I[i] = (uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16;
+        }
+        T.sync();
+        if (h)
+            for (int i = T.gt; i < (B + 6) * ST - 5; i += nthr)
+                H[i] = pair_six_tap(I[i], I[i + 1], I[i + 2], I[i + 3], I[i + 4], I[i + 5], PAIR_K_RAW);
+        if (v)
+            for (int i = T.gt; i < (B + 1) * ST - 2; i += nthr) {
+                const uint32_t *q = I + i + 2;
+                V[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
+            }
+        T.sync();
+        if (d) {
+            for (int i = T.gt; i < (B + 1) * ST - 5; i += nthr) {
+                const uint32_t *q = H + i;
+                D[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
+            }
+            T.sync();
+        }
+    }
+};
+// Position (X, Y) in quarter samples (0..7) from (bx - 1, by - 1): the two
+// columns h0, h1 and rows v0, v1 of the half-sample grid it averages.  Even
+// ones lie on samples (planes I, V), odd ones between (H, D); rows likewise
+// (I, H / V, D).  Integer samples carry no bias in their plane.
+struct PlanePoint {
+    const uint32_t *q00, *q01, *q10, *q11;
+    uint32_t b00, b01, b10, b11;
+    __device__ __forceinline__ PlanePoint(const Planes &A, int X, int Y, int y0) {
+        const int h0 = X >> 1, h1 = (X + 1) >> 1, v0 = Y >> 1, v1 = (Y + 1) >> 1;
+        auto at = [&](int v, int h) {
+            const uint32_t *q = (v & 1) ? ((h & 1) ? A.D : A.V) : ((h & 1) ? A.H + 2 * A.ST : A.I + 2 * A.ST + 2);
+            return q + ((v >> 1) + y0) * A.ST + (h >> 1);
+        };
+        q00 = at(v0, h0); q01 = at(v0, h1); q10 = at(v1, h0); q11 = at(v1, h1);
+        b00 = (v0 | h0) & 1 ? 0 : PAIR_B; b01 = (v0 | h1) & 1 ? 0 : PAIR_B;
+        b10 = (v1 | h0) & 1 ? 0 : PAIR_B; b11 = (v1 | h1) & 1 ? 0 : PAIR_B;
+    }
+    // the clamped samples of word o
+    __device__ __forceinline__ uint32_t value(int o) const {
+        const uint32_t t = pair_avg(q00[o] + b00, q01[o] + b01), b = pair_avg(q10[o] + b10, q11[o] + b11);
+        return pair_min(pair_max(pair_avg(t, b), PAIR_B), PAIR_B + 255u * 0x00010001u) - PAIR_B;
+    }
+};
+
+// The prediction at (X, Y) into dst (stride B), averaged with what is there
+// when `avg`.  All threads of the team.
+__device__ __forceinline__ void plane_pred(const MeTeam &T, const Planes &A, int X, int Y, uint8_t *dst, bool avg) {
+    const PlanePoint P(A, X, Y, 0);
+    const int half = A.B >> 1, lgh = lg2i(half);
+    for (int i = T.gt; i < A.B * half; i += 1 << T.lth) {
+        const int y = i >> lgh, x = i & (half - 1);
+        uint8_t *d = dst + y * A.B + x;
+        uint32_t v = P.value(y * A.ST + x);
+        if (avg) v = pair_avg(v, (uint32_t)d[0] | (uint32_t)d[half] << 16);
+        d[0] = (uint8_t)v;
+        d[half] = (uint8_t)(v >> 16);
+    }
+}
+
+// Luma prediction of a B x B block at the absolute quarter-sample vector
+// (mvx, mvy), sample by sample, by `nthr` threads (reference
+// src/motion.c:493-584); `avg` as in plane_pred.
+__device__ __noinline__ void mc_samples(int t, int nthr, const uint8_t *ref, int mvx, int mvy, int B, uint8_t *dst,
+                                        bool avg) {
+    LumaMC m;
+    m.init(ref, g_fp.stride_y, g_fp.W, g_fp.H, mvx, mvy, B);
+    const int lg = lg2i(B);
+    for (int i = t; i < B * B; i += nthr) {
+        const int v = m.at(i & (B - 1), i >> lg);
+        dst[i] = (uint8_t)(avg ? (v + dst[i] + 1) >> 1 : v);
+    }
+}
+
+// The same by a team with a plane area of its own: from planes where the
+// six-tap support lies inside the frame and the block is large enough to pay
+// for them.
+__device__ __noinline__ void mc_team(const MeTeam T, uint32_t *area, const uint8_t *ref, int mvx, int mvy, int B,
+                                     uint8_t *dst, bool avg) {
+    const int fx = mvx >> 2, fy = mvy >> 2, dx = mvx & 3, dy = mvy & 3;
+    if (area && B >= 16 && (dx | dy) && fx >= 2 && fy >= 2 && fx + B + 2 < g_fp.W && fy + B + 2 < g_fp.H) {
+        const Planes A(area, B);
+        A.build(T, ref, fx + 1, fy + 1, dx, dy, dx && dy);
+        plane_pred(T, A, dx, dy, dst, avg);
+    } else {
+        mc_samples(T.gt, 1 << T.lth, ref, mvx, mvy, B, dst, avg);
+    }
+    T.sync();
+}
+
+// Refines search `id` and leaves its prediction in S.pred[id].
 __device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, const uint8_t *ref, int blk) {
     Smem &S = smem_state();
     ME_T0();
     MeGroup &E = S.me[id];
-    const int g = T.g, gt = T.gt, nthr = 1 << T.lth;
-    const int s = g_fp.stride_y, W = g_fp.W, H = g_fp.H, B = blk, half = B >> 1, ST = half + 6;
-    const int bx = E.bx, by = E.by, lane = gt & 31, warp = gt >> 5, gw = nthr >> 5;
-    uint32_t *pI = area, *pH = pI + (B + 6) * ST, *pV = pH + (B + 6) * ST, *pD = pV + (B + 1) * ST;
-    // integer samples of rows by - 3 .., columns bx - 3 .. (clamped: samples
-    // outside the frame are never part of a point that is scored)
-    for (int i = gt; i < (B + 6) * ST; i += nthr) {
-        const int r = plane_div(i, B), x = bx - 3 + i - r * ST;
-        const uint8_t *row = ref + (size_t)clampi(by - 3 + r, 0, H - 1) * s;
-        pI[i] = (uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16;
-    }
+    const int g = T.g, gt = T.gt;
+    const int W = g_fp.W, H = g_fp.H, B = blk, half = B >> 1;
+    const int bx = E.bx, by = E.by, lane = gt & 31, warp = gt >> 5, gw = 1 << (T.lth - 5);
+    const Planes A(area, B);
+    const int ST = A.ST;
     if (gt < QPOS * QPOS) E.tab[gt] = 0;
-    T.sync();
-    // horizontal halves at columns bx - 1 .. (word j reads columns j .. j + 5)
-    // of every row; vertical halves of rows by - 1 .. at columns bx - 1 ..
-    for (int i = gt; i < (B + 6) * ST - 5; i += nthr)
-        pH[i] = pair_six_tap(pI[i], pI[i + 1], pI[i + 2], pI[i + 3], pI[i + 4], pI[i + 5], PAIR_K_RAW);
-    for (int i = gt; i < (B + 1) * ST - 2; i += nthr) {
-        const uint32_t *q = pI + i + 2;
-        pV[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
-    }
-    T.sync();
-    for (int i = gt; i < (B + 1) * ST - 5; i += nthr) {
-        const uint32_t *q = pH + i;
-        pD[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
-    }
-    T.sync();
+    A.build(T, ref, bx, by, true, true, true);
 
     // Lane p (1..8) holds point p; the points' offsets as in pat_point.
     int ox = 0, oy = 0;
@@ -449,29 +541,12 @@ __device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, con
                 const int y0 = ((it & ((1 << lsp) - 1)) * n) >> lgh;
                 unsigned acc = 0;
                 if (qfx >= 2 && qfy >= 2 && qfx + B + 2 < W && qfy + B + 2 < H) {
-                    // half-grid columns h0, h1 and rows v0, v1: even ones lie
-                    // on samples (planes I, V), odd ones between (H, D); rows
-                    // likewise (I, H / V, D)
-                    const int h0 = X >> 1, h1 = (X + 1) >> 1, v0 = Y >> 1, v1 = (Y + 1) >> 1;
-                    auto at = [&](int v, int h) {
-                        const uint32_t *q = (v & 1) ? ((h & 1) ? pD : pV) + (v >> 1) * ST
-                                                    : ((h & 1) ? pH + 2 * ST : pI + 2 * ST + 2) + (v >> 1) * ST;
-                        return q + (h >> 1) + y0 * ST;
-                    };
-                    // integer samples carry no bias in their plane
-                    const uint32_t *q00 = at(v0, h0), *q01 = at(v0, h1), *q10 = at(v1, h0), *q11 = at(v1, h1);
-                    const uint32_t b00 = (v0 | h0) & 1 ? 0 : PAIR_B, b01 = (v0 | h1) & 1 ? 0 : PAIR_B;
-                    const uint32_t b10 = (v1 | h0) & 1 ? 0 : PAIR_B, b11 = (v1 | h1) & 1 ? 0 : PAIR_B;
+                    const PlanePoint P(A, X, Y, y0);
 #pragma unroll 4
-                    for (int i = lane; i < n; i += 32) {
-                        const int o = (i >> lgh) * ST + (i & (half - 1));
-                        const uint32_t t = pair_avg(q00[o] + b00, q01[o] + b01);
-                        const uint32_t b = pair_avg(q10[o] + b10, q11[o] + b11);
-                        const uint32_t v = pair_min(pair_max(pair_avg(t, b), PAIR_B), PAIR_B + 255u * 0x00010001u) - PAIR_B;
-                        acc += __vsadu4(v, cur[i]);
-                    }
+                    for (int i = lane; i < n; i += 32)
+                        acc += __vsadu4(P.value((i >> lgh) * ST + (i & (half - 1))), cur[i]);
                 } else {
-                    const uint32_t *q = pI + (2 + (Y >> 2) + y0) * ST + 2 + (X >> 2);
+                    const uint32_t *q = A.I + (2 + (Y >> 2) + y0) * ST + 2 + (X >> 2);
                     const uint32_t dx = X & 3, dy = Y & 3, k2 = 0x00020002u;
                     for (int i = lane; i < n; i += 32) {
                         const int o = (i >> lgh) * ST + (i & (half - 1));
@@ -498,38 +573,74 @@ __device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, con
         p0 = f + 1;
     }
     ME_MARK(12);
-    if (gt == 0) { E.mvx = 4 * bx + ux - 3; E.mvy = 4 * by + uy - 3; E.best = bsad; }
+    // the prediction at the refined vector (an integer one, or one whose
+    // six-tap support is inside, is a plane point; else sample by sample)
+    const int mvx = 4 * bx + ux - 3, mvy = 4 * by + uy - 3, fx = mvx >> 2, fy = mvy >> 2;
+    if (!((mvx | mvy) & 3) || (fx >= 2 && fy >= 2 && fx + B + 2 < W && fy + B + 2 < H))
+        plane_pred(T, A, ux + 1, uy + 1, S.pred[id], false);
+    else
+        mc_samples(gt, 1 << T.lth, ref, mvx, mvy, B, S.pred[id], false);
+    if (gt == 0) { E.mvx = mvx; E.mvy = mvy; E.best = bsad; S.cand_mvx[id] = mvx; S.cand_mvy[id] = mvy; }
 }
 
 // The leaf's searches (bits of `mask`, search k on plane r_k from centre
-// (x_k, y_k)), one warp group each: integer stages, then the refinement.  Two
-// groups' planes fit for a 64x64 leaf, so there a third and fourth group wait
-// for the first and second to be done with theirs.  No barrier of the whole
-// CTA: the other warps score the intra modes meanwhile.
+// (x_k, y_k)), one warp group each: integer stages, refinement, prediction.
+// Two groups' planes fit for a 64x64 leaf, so there a third and fourth group
+// wait for the first and second to be done with theirs.  The merge
+// predictions at vector (mx, my) go to the groups without a search, or
+// follow one: P (slot 4): from r0; B: slot 3 from r0, slot 4 from r1, slot 2
+// their average with r1 at the mirrored vector (reference
+// src/encoder.c:642-647, 855-859); null planes are left out.  No barrier of
+// the whole CTA: the other warps score the intra modes meanwhile.
 struct MeStart {
     const uint8_t *r0, *r1, *r2, *r3;
     int x0, y0, x1, y1, x2, y2, x3, y3;
+    int mx, my;
 };
-__device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, const MeStart J, int sr, int lth) {
+__device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, const MeStart J, int sr, int lth, bool merges,
+                                         bool is_b) {
     Smem &S = smem_state();
     const int cu = L.cu, n = __popc(mask);
     const MeTeam T(lth);
-    if (T.g >= n) return;
-    unsigned m = mask;          // the group's search
-    if (T.g > 0) m &= m - 1;
-    if (T.g > 1) m &= m - 1;
-    if (T.g > 2) m &= m - 1;
-    const int id = __ffs((int)m) - 1;
-    const uint8_t *ref = id == 0 ? J.r0 : id == 1 ? J.r1 : id == 2 ? J.r2 : J.r3;
-    me_integer(T, id, ref, L.lx, L.ly, cu, id == 0 ? J.x0 : id == 1 ? J.x1 : id == 2 ? J.x2 : J.x3,
-               id == 0 ? J.y0 : id == 1 ? J.y1 : id == 2 ? J.y2 : J.y3, sr);
-    T.sync();                   // S.me[id] is written by one thread
-    if (cu == 64 && T.g >= PLANES64)
-        asm volatile("bar.sync %0, %1;" ::"r"(NGROUP + 1 + T.g - PLANES64), "r"(2 << lth) : "memory");
-    me_qpel(T, id, S.plane + (cu == 64 ? T.g & (PLANES64 - 1) : T.g) * plane_words(cu), ref, cu);
-    if (cu == 64 && T.g + PLANES64 < n) {
+    const int teams = NT >> lth;
+    uint32_t *area = cu == 64 ? (T.g < PLANES64 ? S.plane + T.g * plane_words(64) : nullptr)
+                              : S.plane + T.g * plane_words(cu);
+    if (T.g < n) {
+        unsigned m = mask;          // the group's search
+        if (T.g > 0) m &= m - 1;
+        if (T.g > 1) m &= m - 1;
+        if (T.g > 2) m &= m - 1;
+        const int id = __ffs((int)m) - 1;
+        const uint8_t *ref = id == 0 ? J.r0 : id == 1 ? J.r1 : id == 2 ? J.r2 : J.r3;
+        me_integer(T, id, ref, L.lx, L.ly, cu, id == 0 ? J.x0 : id == 1 ? J.x1 : id == 2 ? J.x2 : J.x3,
+                   id == 0 ? J.y0 : id == 1 ? J.y1 : id == 2 ? J.y2 : J.y3, sr);
+        T.sync();                   // S.me[id] is written by one thread
+        if (cu == 64 && T.g >= PLANES64)
+            asm volatile("bar.sync %0, %1;" ::"r"(NGROUP + 1 + T.g - PLANES64), "r"(2 << lth) : "memory");
+        me_qpel(T, id, S.plane + (cu == 64 ? T.g & (PLANES64 - 1) : T.g) * plane_words(cu), ref, cu);
+        if (cu == 64 && T.g + PLANES64 < n) {
+            T.sync();
+            asm volatile("bar.arrive %0, %1;" ::"r"(NGROUP + 1 + T.g), "r"(2 << lth) : "memory");
+        }
+        if (n < teams) return;      // free groups take the merges
+        if (cu == 64) area = nullptr;   // another group may be using it
+    }
+    if (!merges) return;
+    const int g0 = n < teams ? n : 0, ng = teams - g0;   // groups taking merges
+    for (int k = T.g - g0; k < (is_b ? 3 : 1); k += ng) {
         T.sync();
-        asm volatile("bar.arrive %0, %1;" ::"r"(NGROUP + 1 + T.g), "r"(2 << lth) : "memory");
+        if (!is_b) {
+            mc_team(T, area, J.r0, J.mx, J.my, cu, S.pred[K_MRG], false);
+        } else if (k == 0) {
+            if (J.r0 && J.r1) {
+                mc_team(T, area, J.r0, J.mx, J.my, cu, S.pred[K_B0 + 2], false);
+                mc_team(T, area, J.r1, -J.mx, -J.my, cu, S.pred[K_B0 + 2], true);
+            }
+        } else if (k == 1) {
+            if (J.r0) mc_team(T, area, J.r0, J.mx, J.my, cu, S.pred[K_B0 + 3], false);
+        } else if (J.r1) {
+            mc_team(T, area, J.r1, J.mx, J.my, cu, S.pred[K_B0 + 4], false);
+        }
     }
 }
 
@@ -617,9 +728,9 @@ __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, i
 // search occupies, and by the others as their searches end.  Bound: issue
 // slots (four warps a scheduler).  Both TU sizes share one prediction and run
 // interleaved; what a lane adds up over its group's areas is reduced once per
-// item.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves; an 8x8 leaf's
+// item.  Slots not in `mask` are left out.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves; an 8x8 leaf's
 // single area is split by TU size instead.
-__device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, int queue) {
+__device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, int queue, uint32_t mask) {
     Smem &S = smem_state();
     const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
@@ -639,7 +750,7 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
         if (it >= ncl << lg) break;
         const int group = it & ((1 << lg) - 1);
         const int e = cl[it >> lg], slot = e & CL_SLOT, do_sizes = e & (la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4);
-        if (!do_sizes) continue;
+        if (!do_sizes || !(mask >> slot & 1u)) continue;
         const int t0 = la == 0 ? 0 : group << lG;
         int s8 = 0, n8 = 0, s4 = 0, n4 = 0;
         bool differs = false;
@@ -950,34 +1061,21 @@ __device__ __noinline__ void chroma_mc(Smem &, const FrameParams &, const Leaf L
     SYNC();
 }
 
-// Luma MC of the listed (slot, ref, mv) predictions into S.pred[slot].
-// (to_rec: the one listed slot's prediction goes straight into the
-// reconstruction tile, as a skipped leaf's does.)
-__device__ __noinline__ void luma_mc_slots(Smem &, const FrameParams &, const Leaf L, int nslots,
-                                           const int *slots, bool to_rec) {
-    Smem &S = smem_state();
-    const FrameParams &P = g_fp;
-    const int cu = L.cu, n = cu * cu, lg = lg2i(cu);
-    for (int i = threadIdx.x; i < nslots * n; i += NT) {
-        const int k = i >> (2 * lg), p = i & (n - 1), y = p >> lg, x = p & (cu - 1);
-        const int slot = slots[k];
-        const int r2 = S.cand_ref2[slot];
-        int v = 0;
-        // Bi-prediction averages with the mirrored (negated absolute) MV on
-        // the second reference (reference src/encoder.c:642-647, 855-859).
-#pragma unroll 1
-        for (int h = 0; h < (r2 >= 0 ? 2 : 1); ++h) {
-            const int sgn = h ? -1 : 1;
-            LumaMC m;
-            m.init(P.ref_y[h ? r2 : S.cand_ref[slot]], P.stride_y, P.W, P.H, sgn * S.cand_mvx[slot],
-                   sgn * S.cand_mvy[slot], cu);
-            const int u = m.at(x, y);
-            v = h ? (v + u + 1) >> 1 : u;
-        }
-        if (to_rec) RY(S, L.lx + x, L.ly + y) = (uint8_t)v;
-        else S.pred[slot][p] = (uint8_t)v;
-    }
+// Luma prediction of a leaf into S.pred[0] from plane r1, averaged with r2 at
+// the mirrored vector unless null (reference src/encoder.c:642-647, 855-859).
+// By the whole CTA.
+__device__ void luma_mc(Smem &S, const Leaf &L, const uint8_t *r1, const uint8_t *r2, int mvx, int mvy) {
+    mc_samples(threadIdx.x, NT, r1, mvx, mvy, L.cu, S.pred[0], false);
     SYNC();
+    if (r2) {
+        mc_samples(threadIdx.x, NT, r2, -mvx, -mvy, L.cu, S.pred[0], true);
+        SYNC();
+    }
+}
+// A skipped leaf's luma: the prediction in S.pred[0].
+__device__ void copy_pred(Smem &S, const Leaf &L) {
+    const int lg = lg2i(L.cu);
+    for (int i = threadIdx.x; i < L.cu * L.cu; i += NT) RY(S, L.lx + (i & (L.cu - 1)), L.ly + (i >> lg)) = S.pred[0][i];
 }
 
 __device__ void zero_acc(Smem &S) {
@@ -988,11 +1086,13 @@ __device__ void zero_acc(Smem &S) {
 
 // Sum over the CU of |orig - pred| per listed slot into acc[slot][0][0]
 // (fast-preset SAD proxy): one warp per (candidate, 8x8 area).
-__device__ void sad_areas(Smem &S, const Leaf &L, const int *cl, int ncl) {
+__device__ void sad_areas(Smem &S, const Leaf &L, const int *cl, int ncl, uint32_t mask) {
     const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
     const int lane = threadIdx.x & 31;
     for (int it = threadIdx.x >> 5; it < J; it += NW) {
-        const int e = cl[it >> (2 * lt)], t = it & ((1 << (2 * lt)) - 1);
+        const int e = cl[it >> (2 * lt)];
+        if (!(mask >> (e & CL_SLOT) & 1u)) continue;
+        const int t = it & ((1 << (2 * lt)) - 1);
         const int x = (t & ((1 << lt) - 1)) * 8 + 2 * (lane & 3), y = (t >> lt) * 8 + (lane >> 2);
         const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
         const unsigned s = __reduce_add_sync(0xffffffffu, __vsadu4(cv, pred2(S, cu, e, x, y)));
@@ -1170,17 +1270,12 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
             if (decided) {
                 SYNC();   // every thread has read the grid (mvp_at)
             } else {
-                if (threadIdx.x == 0) {
-                    S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1; S.cand_ref2[0] = r2;
-                }
                 if (cflat && threadIdx.x >= NT - 64) chroma_model(L, (threadIdx.x >> 5) & 1);
-                SYNC();
                 if (flat) {
                     for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
                     SYNC();
                 } else {
-                    const int slots[1] = {0};
-                    luma_mc_slots(S, P, L, 1, slots, false);
+                    luma_mc(S, L, P.ref_y[r1], r2 >= 0 ? P.ref_y[r2] : nullptr, mvx, mvy);
                 }
             }
             // luma and chroma run side by side on different warps
@@ -1188,12 +1283,8 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
             luma_replay(L, src | cl_size, el);
             chroma_areas(L, 1, mc, ec, mini(NW / 2, (cu * cu) >> 6));
         } else {
-            if (threadIdx.x == 0) {
-                S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = 0; S.cand_ref2[0] = -1;
-            }
-            SYNC();
-            const int slots[1] = {0};
-            luma_mc_slots(S, P, L, 1, slots, true);
+            luma_mc(S, L, P.ref_y[0], nullptr, mvx, mvy);
+            copy_pred(S, L);
             if (P.fresh_skip && P.frame_type == 1 && P.ref_valid[0])
                 chroma_mc(S, P, L, 0, mvx, mvy, 0, true);
         }
@@ -1224,6 +1315,12 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     const bool use4 = medium && cu <= 32;
     const uint32_t modes = !try_intra ? 0u : P.preset == 0 ? 0x1041u : P.preset == 1 ? 0x9249u : 0x3FFFFu;
     const int nintra = __popc(modes);
+    // slots 2..4 of a B leaf and the merge slot of a P leaf: 8x8 TUs only
+    const uint32_t merges = is_b ? 0x1Cu : 1u << K_MRG;
+    if (tid >= 32 && tid < 32 + NPRED) {
+        const bool m8 = merges >> (tid - 32) & 1u;
+        S.cl[nintra + tid - 32] = cl_entry(tid - 32, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
+    }
     if (tid < 18 && (modes >> tid & 1u))
         S.cl[__popc(modes & ((1u << tid) - 1u))] = cl_entry(K_INTRA + tid, CL_8 | (use4 ? CL_4 : 0));
     if (!key) {
@@ -1259,75 +1356,37 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         }
         const MeStart J = {P.ref_y[0], P.ref_y[1], P.ref_y[0], P.ref_y[0], cx0, cy0, cx0, cy0,
                            (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2,
-                           (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2};
-        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, J, sr, fast ? 8 : 7);
-        if (!fast) luma_score(L, S.cl, nintra, 0);
+                           (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2, mvpx + L.px * 4, mvpy + L.py * 4};
+        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, J, sr, fast ? 8 : 7,
+                    medium, false);
+        if (!fast) luma_score(L, S.cl, nintra, 0, ~0u);
         SYNC();
         PHASE_D(1, L.depth);
         if (has_glb && S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) has_glb = false;
         if (has_tmp && S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) has_tmp = false;
         cand = 1u << K_ME0 | (uint32_t)has_me1 << K_ME1 | (uint32_t)has_glb << K_GLB | (uint32_t)has_tmp << K_TMP |
                (uint32_t)medium << K_MRG;
-        int slots[5], ns = 0;
-        for (int k = 0; k < NPRED; ++k)
-            if (cand >> k & 1u) slots[ns++] = k;
-        if (tid == 0) {
-            S.cand_mvx[K_ME0] = S.me[0].mvx; S.cand_mvy[K_ME0] = S.me[0].mvy; S.cand_ref[K_ME0] = 0;
-            S.cand_mvx[K_ME1] = S.me[1].mvx; S.cand_mvy[K_ME1] = S.me[1].mvy; S.cand_ref[K_ME1] = 1;
-            S.cand_mvx[K_GLB] = S.me[2].mvx; S.cand_mvy[K_GLB] = S.me[2].mvy; S.cand_ref[K_GLB] = 0;
-            S.cand_mvx[K_TMP] = S.me[3].mvx; S.cand_mvy[K_TMP] = S.me[3].mvy; S.cand_ref[K_TMP] = 0;
-            S.cand_mvx[K_MRG] = mvpx + L.px * 4; S.cand_mvy[K_MRG] = mvpy + L.py * 4; S.cand_ref[K_MRG] = 0;
-            for (int k = 0; k < NPRED; ++k) S.cand_ref2[k] = -1;
-        }
-        SYNC();
-        luma_mc_slots(S, P, L, ns, slots, false);
-        PHASE_D(2, L.depth);
     } else if (is_b) {
         // Forward / backward searches (reference src/encoder.c:795-852).
         const int sr = fast ? 16 : 32;
-        const uint8_t *f = P.ref_y[maxi(rf, 0)], *b = P.ref_y[maxi(rb, 0)];
-        const MeStart J = {f, b, f, b, cx0, cy0, cx0, cy0, cx0, cy0, cx0, cy0};
-        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, J, sr, fast ? 8 : 7);
-        if (!fast) luma_score(L, S.cl, nintra, 0);
+        const uint8_t *f = rf >= 0 ? P.ref_y[rf] : nullptr, *b = rb >= 0 ? P.ref_y[rb] : nullptr;
+        const MeStart J = {f, b, f, b, cx0, cy0, cx0, cy0, cx0, cy0, cx0, cy0, mvpx + L.px * 4, mvpy + L.py * 4};
+        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, J, sr, fast ? 8 : 7, medium, true);
+        if (!fast) luma_score(L, S.cl, nintra, 0, ~0u);
         SYNC();
         PHASE_D(1, L.depth);
         const uint32_t hf = rf >= 0, hb = rb >= 0, mrg = medium;
         cand = hf | hb << 1 | (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;
-        int slots[5], ns = 0;
-        for (int k = 0; k < NPRED; ++k)
-            if (cand >> k & 1u) slots[ns++] = k;
-        if (tid == 0) {
-            const int mmx = mvpx + L.px * 4, mmy = mvpy + L.py * 4;
-            for (int k = 0; k < NPRED; ++k) S.cand_ref2[k] = -1;
-            S.cand_mvx[K_B0 + 0] = S.me[0].mvx; S.cand_mvy[K_B0 + 0] = S.me[0].mvy; S.cand_ref[K_B0 + 0] = rf < 0 ? 0 : rf;
-            S.cand_mvx[K_B0 + 1] = S.me[1].mvx; S.cand_mvy[K_B0 + 1] = S.me[1].mvy; S.cand_ref[K_B0 + 1] = rb < 0 ? 0 : rb;
-            S.cand_mvx[K_B0 + 2] = mmx; S.cand_mvy[K_B0 + 2] = mmy; S.cand_ref[K_B0 + 2] = rf < 0 ? 0 : rf;
-            S.cand_ref2[K_B0 + 2] = rb;
-            S.cand_mvx[K_B0 + 3] = mmx; S.cand_mvy[K_B0 + 3] = mmy; S.cand_ref[K_B0 + 3] = rf < 0 ? 0 : rf;
-            S.cand_mvx[K_B0 + 4] = mmx; S.cand_mvy[K_B0 + 4] = mmy; S.cand_ref[K_B0 + 4] = rb < 0 ? 0 : rb;
-        }
-        SYNC();
-        luma_mc_slots(S, P, L, ns, slots, false);
-        PHASE_D(2, L.depth);
     }
 
     // ---- residual coding / SAD proxies for every candidate --------------
-    // slots 2..4 of a B leaf and the merge slot of a P leaf: 8x8 TUs only
-    const uint32_t merges = is_b ? 0x1Cu : 1u << K_MRG;
-    const int ninter = __popc(cand);
-    if (tid < NPRED && (cand >> tid & 1u)) {
-        const bool m8 = merges >> tid & 1u;
-        S.cl[nintra + __popc(cand & ((1u << tid) - 1u))] =
-            cl_entry(tid, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
-    }
     cand |= modes << K_INTRA;
-    SYNC();
     if (fast) {
-        sad_areas(S, L, S.cl, nintra + ninter);
+        sad_areas(S, L, S.cl, nintra + (key ? 0 : NPRED), cand);
         SYNC();
     } else {
-        if (key) luma_score(L, S.cl, nintra, 0);
-        else luma_score(L, S.cl + nintra, ninter, 1);
+        if (key) luma_score(L, S.cl, nintra, 0, ~0u);
+        else luma_score(L, S.cl + nintra, NPRED, 1, cand);
         SYNC();
         PHASE_D(3, L.depth);
         if (is_p) {
@@ -2254,13 +2313,8 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
         } else {
             r1 = (nd.ref_sel < MAX_REFS && P.ref_valid[nd.ref_sel]) ? nd.ref_sel : -1;
         }
-        if (threadIdx.x == 0) {
-            S.cand_mvx[0] = mvx; S.cand_mvy[0] = mvy; S.cand_ref[0] = r1 < 0 ? 0 : r1; S.cand_ref2[0] = r2;
-        }
-        SYNC();
         if (r1 >= 0) {
-            const int slots[1] = {0};
-            luma_mc_slots(S, P, L, 1, slots, false);
+            luma_mc(S, L, P.ref_y[r1], r2 >= 0 ? P.ref_y[r2] : nullptr, mvx, mvy);
         } else {
             for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
             SYNC();

@@ -74,22 +74,22 @@ struct Smem {
     MvCell grid[64];
     Node nodes[QT_NODES];
     long long node_cost[QT_NODES];
+    alignas(16) uint8_t pred[NPRED][64 * 64];
     union {
         // after the searches of a leaf
         struct {
-            alignas(16) uint8_t pred[NPRED][64 * 64];
             // chroma predictions (decoder, skip check), or the two chroma
             // options of an intra leaf: reconstruction and levels of option o,
             // component c in [2 * o + c]
-            uint8_t cpred[4][32 * 32];
+            alignas(16) uint8_t cpred[4][32 * 32];
             int16_t clev[4][32 * 32];
+            int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
         };
         // during them: SAD tables of the integer stages, then sample planes
         alignas(16) uint32_t plane[PLANE_WORDS];
     };
     uint32_t cur_pair[64 * 32];      // leaf's source samples (x, x + cu / 2) as 16-bit lanes, for the searches
     uint8_t edge[2][EDGE_LEN];       // intra reference samples per direction (see build_refs)
-    int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
     uint4 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
@@ -102,7 +102,7 @@ struct Smem {
     int last_bits[65];         // last_bits(last) by last + 1
     long long acc64;
     int cl[NCAND];             // candidate list for job loops
-    int cand_mvx[NPRED], cand_mvy[NPRED], cand_ref[NPRED], cand_ref2[NPRED];
+    int cand_mvx[NPRED], cand_mvy[NPRED];   // refined vectors of the searches
     int next[2];               // work queues of luma_score: next item
     int dc;
     int above0;                // first sample of the above run (the planar mode's corner)
