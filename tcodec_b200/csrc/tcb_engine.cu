@@ -734,10 +734,10 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
     Smem &S = smem_state();
     const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
-    const uint4 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
-    const uint4 *bands = S.qparam[0].band;
-    const uint4 b80 = bands[band_rc(8, row, col)], b81 = bands[band_rc(8, row, col + 1)];
-    const uint4 b40 = bands[band_rc(4, row & 3, col & 3)], b41 = bands[band_rc(4, row & 3, (col & 3) + 1)];
+    const uint2 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
+    const QuantParams &qp = S.qparam[0];
+    const QuantPos b80(qp, band_rc(8, row, col)), b81(qp, band_rc(8, row, col + 1));
+    const QuantPos b40(qp, band_rc(4, row & 3, col & 3)), b41(qp, band_rc(4, row & 3, (col & 3) + 1));
 #ifdef TCB_PHASE_PROFILE
     if (threadIdx.x < ncl) { OPCOUNT(2, cl[threadIdx.x] & CL_8 ? 1 << la : 0); OPCOUNT(3, cl[threadIdx.x] & CL_4 ? 4 << la : 0); }
 #endif
@@ -752,7 +752,8 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
         const int e = cl[it >> lg], slot = e & CL_SLOT, do_sizes = e & (la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4);
         if (!do_sizes || !(mask >> slot & 1u)) continue;
         const int t0 = la == 0 ? 0 : group << lG;
-        int s8 = 0, n8 = 0, s4 = 0, n4 = 0;
+        AreaSums s8, s4;
+        int n8 = 0, n4 = 0;      // last positions' bits
         bool differs = false;
         for (int t = t0; t < t0 + (1 << lG); ++t) {
             const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
@@ -760,14 +761,12 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
             const uint32_t pv = pred2(S, cu, e, x, y);
             differs |= pv != cv;
             auto add8 = [&](const AreaCode &c) {
-                s8 += c.sse;
-                n8 += c.bits;
+                s8.add(c);
                 const int b = S.last_bits[last8(c, lane)];
                 if (lane == 0) n8 += b;
             };
             auto add4 = [&](const AreaCode &c) {
-                s4 += c.sse;
-                n4 += c.bits;
+                s4.add(c);
                 const int b = S.last_bits[last4(c, lane)];
                 if ((lane & 13) == 0) n4 += b;
             };
@@ -785,11 +784,13 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
         if ((e & CL_EXACT) && __any_sync(0xffffffffu, differs)) S.inexact = 1;
         int v = 0;   // lanes 0..3: the four sums of the slot
         if (do_sizes & CL_8) {
-            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s8), b = (int)__reduce_add_sync(0xffffffffu, (unsigned)n8);
+            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s8.sse);
+            const int b = (int)__reduce_add_sync(0xffffffffu, (unsigned)(n8 + s8.bits()));
             v = lane == 0 ? a : lane == 1 ? b : 0;
         }
         if (do_sizes & CL_4) {
-            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s4), b = (int)__reduce_add_sync(0xffffffffu, (unsigned)n4);
+            const int a = (int)__reduce_add_sync(0xffffffffu, (unsigned)s4.sse);
+            const int b = (int)__reduce_add_sync(0xffffffffu, (unsigned)(n4 + s4.bits()));
             v = lane == 2 ? a : lane == 3 ? b + (1 << lG) : v;
         }
         if (lane < 4) atomicAdd(&S.acc[slot][0][0] + lane, v);
@@ -806,9 +807,9 @@ __device__ __noinline__ void luma_replay(const Leaf L, int e, int16_t *emit) {
     int t = threadIdx.x >> 5;
     if (t >= 1 << (2 * lt)) return;
     const bool d8 = e & CL_8;
-    const uint4 f = S.frag[d8 ? 0 : 2][lane], i = S.frag[d8 ? 1 : 3][lane];
-    const uint4 b0 = S.qparam[0].band[d8 ? band_rc(8, row, col) : band_rc(4, row & 3, col & 3)];
-    const uint4 b1 = S.qparam[0].band[d8 ? band_rc(8, row, col + 1) : band_rc(4, row & 3, (col & 3) + 1)];
+    const uint2 f = S.frag[d8 ? 0 : 2][lane], i = S.frag[d8 ? 1 : 3][lane];
+    const QuantPos b0(S.qparam[0], d8 ? band_rc(8, row, col) : band_rc(4, row & 3, col & 3));
+    const QuantPos b1(S.qparam[0], d8 ? band_rc(8, row, col + 1) : band_rc(4, row & 3, (col & 3) + 1));
     const int pos = d8 ? 2 * lane : (row >> 2) * 32 + (col >> 2) * 16 + (row & 3) * 4 + (col & 3);
     for (; t < 1 << (2 * lt); t += NW) {
         const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
@@ -886,8 +887,8 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
     if (threadIdx.x == 0) OPCOUNT(3, J);
     int base = 4 * (((threadIdx.x >> 5) + NW - woff) & (NW - 1));
     if (base >= J) return;
-    const uint4 f4 = S.frag[2][lane], i4 = S.frag[3][lane];
-    const uint4 b0 = S.qparam[1].band[band_rc(4, r, cc)], b1 = S.qparam[1].band[band_rc(4, r, cc + 1)];
+    const uint2 f4 = S.frag[2][lane], i4 = S.frag[3][lane];
+    const QuantPos b0(S.qparam[1], band_rc(4, r, cc)), b1(S.qparam[1], band_rc(4, r, cc + 1));
     for (; base < J; base += 4 * NW) {
         const bool act = base + quarter < J;
         const int j = act ? base + quarter : 0;
@@ -925,7 +926,9 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
         __syncwarp();
         const AreaCode a = code_area(cv, pv, f4, i4, b0, b1);
         if (nopt == 2) {
-            int d = a.sse, n = a.bits;    // of the quarter's eight lanes: index bits 0, 2 and 3
+            AreaSums u;
+            u.add(a);
+            int d = u.sse, n = u.bits();    // of the quarter's eight lanes: index bits 0, 2 and 3
             for (int m = 1; m < 16; m = m == 1 ? 4 : 2 * m) {
                 d += __shfl_xor_sync(0xffffffffu, d, m);
                 n += __shfl_xor_sync(0xffffffffu, n, m);
@@ -1809,8 +1812,8 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     // at fixed offsets.
     if (threadIdx.x < 8) {
         const int b = threadIdx.x & 3;
-        if (threadIdx.x < 4) S.qparam[0].set_band(b, P.eff_l[b], P.rcp_l[b], P.lambda);
-        else S.qparam[1].set_band(b, P.eff_c[b], P.rcp_c[b], P.lambda_c);
+        if (threadIdx.x < 4) S.qparam[0].set_band(b, P.eff_l[b], P.lambda);
+        else S.qparam[1].set_band(b, P.eff_c[b], P.lambda_c);
     }
     SYNC();
 

@@ -90,7 +90,7 @@ struct Smem {
     };
     uint32_t cur_pair[64 * 32];      // leaf's source samples (x, x + cu / 2) as 16-bit lanes, for the searches
     uint8_t edge[2][EDGE_LEN];       // intra reference samples per direction (see build_refs)
-    uint4 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
+    uint2 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)

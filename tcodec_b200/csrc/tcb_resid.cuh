@@ -9,18 +9,24 @@
 //
 //  * A matrix entry C (|C| <= 10703) is split as 128 Ch + Cl with
 //    |Ch| <= 84, |Cl| <= 64; the 16 rows of the A operand are the 8 rows of
-//    Ch and the 8 rows of Cl, so one MMA gives both partial sums.
-//  * The first pass multiplies the residuals (|r| <= 255, exact in f16).  The
-//    later passes multiply intermediates t, |t| < 8192, split as 64 th + tl
-//    with 0 <= tl < 64: k = 16 holds [64 C | C] against [th; tl].
-//  * Every product is an integer and the accumulators start at about
-//    1.5 * 2^23, so their bits are a constant plus the sum while
-//    |sum| < 2^20.3.  Residuals of 8-bit pictures have norm <= 2040, a
-//    non-zero level dequantises to at most 1.75 |c| (q eff + eff / 6 with
-//    q eff <= |c| + eff / 3 and eff <= 1.5 |c|), so no intermediate exceeds
-//    3571 and no partial sum 182 * 3571 < 2^20.
-//  * The start values are chosen so that 128 Hi + Lo, modulo 2^32 (or 2^28
-//    where only bits 14..27 are used), is the rounded sum with no correction.
+//    Ch and the 8 rows of Cl, so one MMA gives both partial sums Sh and Sl.
+//  * B operands are integers exact in f16 (|v| <= 2048): residuals
+//    (|r| <= 255), first-pass results (|t| <= 722), and dequantised levels
+//    and row-inverse results as f16(v) plus the remainder v - f16(v) (0 or
+//    +-1), against [C | C] with k = 16.
+//  * Every product and sum is an integer below 2^24, so f32 holds it exactly:
+//    residuals of 8-bit pictures have norm <= 2040, a non-zero level
+//    dequantises to at most 1.75 |c| (q eff + eff / 6 with q eff <= |c| +
+//    eff / 3 and eff <= 1.5 |c|), so no intermediate exceeds 3571 and no
+//    partial sum 182 * 3571 < 2^20.
+//  * The 14-bit rounding shift, floor((128 Sh + Sl + 8192) / 2^14), is taken
+//    in f32 with round-down adds of 1.5 * 2^23, whose last bit is 1 (the
+//    8192 is the accumulator's start value).
+//
+// Everything up to the reconstruction stays in f32: the FMA pipe issues one
+// instruction a cycle where the integer ALU issues one every two, and the
+// integer form of the same steps was bound by the latter (142 cycles a
+// scheduler per area and TU size; now about half).
 //
 // Data layout: lane l owns row l >> 2, columns 2 (l & 3) and 2 (l & 3) + 1 of
 // the 8x8 area.  That is the C fragment of an m16n8 MMA (rows 0..7: the Ch
@@ -30,9 +36,9 @@
 // with block-diagonal matrices.
 //
 // Compared with eight (four) lanes per TU and rows exchanged through shared
-// memory: about 110 instructions per area and type with its bit estimate
-// instead of about 300 per 8x8 TU and 90 per 4x4 TU, in a serial chain of the
-// same length instead of 1000, and 3 KB of code instead of 38 KB.
+// memory: about 100 instructions per area and type instead of about 300 per
+// 8x8 TU and 90 per 4x4 TU, in a serial chain of the same length instead of
+// 1000, and 3 KB of code instead of 38 KB.
 //
 // Arithmetic follows reference src/transform.c:331-439 (dct4_point,
 // dct8_point2, tc_fdct*/tc_idct*_res), src/encoder.c:333-385 (rdoq_level1,
@@ -75,25 +81,37 @@ static inline cudaError_t upload_dct_tables() {
 
 struct QuantParams {
     int eff[4];
-    // Per band: {reciprocal, quantiser offset times reciprocal, smallest |c|
-    // with a level, quant step | dequantiser bias (eff / 6) << 16}.  The level
-    // is (|c| + eff / 3) / eff, as the high word of |c| rcp + off rcp (a step
-    // of 1: reciprocal 2^32 - 1 and offset 1, which give |c|).  A level of
-    // magnitude 1 dequantises to dq = eff + eff / 6 and is dropped when
-    // c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference
+    // Per band: {1 / eff, (eff / 3 + 1/2) / eff, smallest |c| with a level,
+    // eff} and eff / 6, the dequantiser's bias.  The level is
+    // floor((|c| + eff / 3) / eff) = floor(|c| / eff + (eff / 3 + 1/2) / eff):
+    // the half keeps the sum 1 / (2 eff) away from every integer, far more
+    // than its f32 rounding (below 2^-22 of it, for |c| + eff / 3 < 2^13).  A
+    // level of magnitude 1 dequantises to dq = eff + eff / 6 and is dropped
+    // when c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference
     // src/encoder.c:333-355), i.e. when dq (2 |c| - dq) < lambda: below
     // ceil((dq + ceil(lambda / dq)) / 2), if that lies in level 1's range.
-    uint4 band[4];
-    __host__ __device__ void set_band(int b, int e, uint32_t r, long long lambda) {
+    float4 band[4];
+    float bias[4];
+    __host__ __device__ void set_band(int b, int e, long long lambda) {
         const int off = e / 3, dq = e + e / 6;
         long long thr = ((lambda + dq - 1) / dq + dq + 1) >> 1;
         if (thr > 2 * e - off) thr = 2 * e - off;
         if (thr < e - off) thr = e - off;
         eff[b] = e;
-        band[b].x = e <= 1 ? 0xFFFFFFFFu : r;
-        band[b].y = e <= 1 ? 0xFFFFFFFFu : (uint32_t)off * r;
-        band[b].z = (uint32_t)thr;
-        band[b].w = (uint32_t)e | (uint32_t)(e / 6) << 16;
+        band[b].x = 1.0f / (float)e;
+        band[b].y = ((float)off + 0.5f) / (float)e;
+        band[b].z = (float)thr;
+        band[b].w = (float)e;
+        bias[b] = (float)(e / 6);
+    }
+};
+// Quantiser of one position.
+struct QuantPos {
+    float r, off, thr, eff, bias;
+    __device__ __forceinline__ QuantPos(const QuantParams &q, int b) {
+        const float4 v = q.band[b];
+        r = v.x; off = v.y; thr = v.z; eff = v.w;
+        bias = q.bias[b];
     }
 };
 
@@ -103,9 +121,9 @@ struct QuantParams {
 __device__ __forceinline__ int band_rc(int N, int r, int c) { return freq_band(r * N + c, N * N); }
 
 // A fragments of the forward (inv 0) or inverse (inv 1) transform for this
-// lane: {64 Ch, 64 Cl, Ch, Cl} of matrix row lane >> 2, columns
-// 2 (lane & 3) + {0, 1}; N = 4: two 4x4 matrices on the diagonal.
-__device__ inline uint4 dct_fragment(int N, int inv, int lane) {
+// lane: {Ch, Cl} of matrix row lane >> 2, columns 2 (lane & 3) + {0, 1};
+// N = 4: two 4x4 matrices on the diagonal.
+__device__ inline uint2 dct_fragment(int N, int inv, int lane) {
     const int m = lane >> 2;
     float ch[2], cl[2];
     for (int e = 0; e < 2; ++e) {
@@ -121,101 +139,105 @@ __device__ inline uint4 dct_fragment(int N, int inv, int lane) {
         const __half2 v = __floats2half2_rn(a, b);
         return *reinterpret_cast<const uint32_t *>(&v);
     };
-    return make_uint4(pack(64.f * ch[0], 64.f * ch[1]), pack(64.f * cl[0], 64.f * cl[1]), pack(ch[0], ch[1]),
-                      pack(cl[0], cl[1]));
+    return make_uint2(pack(ch[0], ch[1]), pack(cl[0], cl[1]));
 }
-
-// Accumulator start values.  With 0x4B400000 the bits of 1.5 * 2^23,
-// (bits(Hi) << 7) + bits(Lo) = 0xEB400000 + 128 dH + dL + sum (mod 2^32) for
-// starts 1.5 * 2^23 + dH and + dL; dL = 8192 rounds the 14-bit shift.
-//   EXACT: 128 dH = 2^32 - 0xEB400000, the word is sum + 8192;
-//   FIELD: 128 dH = 2^27 - 0xEB400000 (mod 2^28), bits 14..27 are the rounded
-//          result + 8192 (results within +-8191).
-constexpr float ACC_LO = 12582912.0f + 8192.0f;
-constexpr float ACC_EXACT = 12582912.0f + 2719744.0f, ACC_FIELD = 12582912.0f - 425984.0f;
 
 struct MmaSums {
-    float h0, h1, l0, l1;
-    __device__ __forceinline__ uint32_t x0() const { return (__float_as_uint(h0) << 7) + __float_as_uint(l0); }
-    __device__ __forceinline__ uint32_t x1() const { return (__float_as_uint(h1) << 7) + __float_as_uint(l1); }
+    float h0, h1, l0, l1;    // Sh and Sl + 8192 of the lane's two positions
 };
-__device__ __forceinline__ MmaSums mma_k8(uint32_t a0, uint32_t a1, uint32_t b0, float start) {
+__device__ __forceinline__ MmaSums mma_k8(const uint2 a, uint32_t b0) {
     MmaSums d;
     asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%8,%8};"
-        : "=f"(d.h0), "=f"(d.h1), "=f"(d.l0), "=f"(d.l1) : "r"(a0), "r"(a1), "r"(b0), "f"(start), "f"(ACC_LO));
+        : "=f"(d.h0), "=f"(d.h1), "=f"(d.l0), "=f"(d.l1) : "r"(a.x), "r"(a.y), "r"(b0), "f"(0.0f), "f"(8192.0f));
     return d;
 }
-__device__ __forceinline__ MmaSums mma_k16(const uint4 a, uint32_t b0, uint32_t b1, float start) {
+__device__ __forceinline__ MmaSums mma_k16(const uint2 a, uint32_t b0, uint32_t b1) {
     MmaSums d;
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%11,%11};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%4,%5}, {%6,%7}, {%8,%8,%9,%9};"
         : "=f"(d.h0), "=f"(d.h1), "=f"(d.l0), "=f"(d.l1)
-        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(start), "f"(ACC_LO));
+        : "r"(a.x), "r"(a.y), "r"(b0), "r"(b1), "f"(0.0f), "f"(8192.0f));
     return d;
+}
+constexpr float RND = 12582912.0f;     // 1.5 * 2^23, bits 0x4B400000
+// RND + floor((128 h + l) / 2^14): any sums, or (first pass) 128 |h| + |l| < 2^24.
+__device__ __forceinline__ float shift14(float h, float l) {
+    return __fmaf_rd(__fmaf_rd(l, 1.0f / 128, RND) + h, 1.0f / 128, RND - RND / 128);
+}
+__device__ __forceinline__ float shift14_small(float h, float l) {
+    return __fmaf_rd(__fmaf_rn(h, 128.0f, l), 1.0f / 16384, RND);
+}
+__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
+    const __half2 v = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&v);
 }
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
     const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
-// B fragment halves of two intermediates, each t + 8192 in the low 14 bits of
-// its 16-bit lane of pk (the two bits above are ignored): hi = half2(t >> 6),
-// lo = half2(t & 63).  0x6400 | v is the half 1024 + v.
-__device__ __forceinline__ void split_b(uint32_t pk, uint32_t &hi, uint32_t &lo) {
-    lo = h2_sub((pk & 0x003F003Fu) | 0x64006400u, 0x64006400u);            // - 1024
-    hi = h2_sub(((pk >> 6) & 0x00FF00FFu) | 0x64006400u, 0x64806480u);     // - (1024 + 8192 / 64)
-}
-__device__ __forceinline__ void split_sums(const MmaSums &d, uint32_t &hi, uint32_t &lo) {
-    split_b(__byte_perm(d.x0() >> 14, d.x1() << 2, 0x7610), hi, lo);
+// B operands of two integers within +-4095: f16 values and remainders.
+__device__ __forceinline__ void split_h2(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = pack_h2(a - __low2float(h), b - __high2float(h));
 }
 // Two 8-bit samples (low 16 bits of v) as half2(1024 + v0, 1024 + v1).
 __device__ __forceinline__ uint32_t bytes_h2(uint32_t v) { return __byte_perm(v, 0x64u, 0x4140); }
 
-// One coefficient: dead-zone quantiser with RDOQ-lite.  Returns the level's
-// magnitude; dq is the signed dequantised value + 8192.
-__device__ __forceinline__ int quant_one(int c, const uint4 b, int &dq) {
-    const int a = absi(c);
-    const bool zero = a < (int)b.z;
-    int q = (int)(((unsigned long long)(unsigned)a * b.x + b.y) >> 32);
-    int m = q * (int)(b.w & 0xFFFFu) + (int)(b.w >> 16);
-    q = zero ? 0 : q;
-    m = zero ? 0 : m;
-    dq = (c < 0 ? -m : m) + 8192;
-    return q;
-}
-
 // What the warp knows of one coded area.
 struct AreaCode {
-    int m0, m1;        // magnitudes of this lane's levels
-    int c0, c1;        // its coefficients (whose signs the levels have)
+    float z0, z1;      // 1 where this lane's level is non-zero, else 0
+    float q0, q1;      // magnitudes of its levels
+    float c0, c1;      // its coefficients (whose signs the levels have)
     uint32_t rec;      // its two reconstructed samples (low 16 bits)
-    int sse, bits;     // its SSE; 2 bitlen + 3 summed over its non-zero levels
+    int e0, e1;        // its reconstruction errors
     __device__ __forceinline__ uint32_t levels() const {   // two int16 levels
-        return __byte_perm((uint32_t)(c0 < 0 ? -m0 : m0), (uint32_t)(c1 < 0 ? -m1 : m1), 0x5410);
+        return __byte_perm(__float_as_uint(copysignf(q0, c0) + RND), __float_as_uint(copysignf(q1, c1) + RND), 0x5410);
     }
+};
+// A lane's sums over areas: SSE, exponents and number of non-zero levels.
+struct AreaSums {
+    int sse = 0;
+    unsigned exps = 0;
+    float nz = 0.0f;
+    __device__ __forceinline__ void add(const AreaCode &c) {
+        sse += c.e0 * c.e0 + c.e1 * c.e1;
+        exps += (__float_as_uint(c.q0) >> 23) + (__float_as_uint(c.q1) >> 23);
+        nz += c.z0 + c.z1;
+    }
+    // 2 bitlen + 3 over the non-zero levels: the exponent field of a level of
+    // bit length n is 126 + n, that of zero 0
+    __device__ __forceinline__ int bits() const { return 2 * (int)exps - 249 * (int)nz; }
 };
 
 // Codes the area whose samples this lane holds two of: cv (source) and pv
 // (prediction), 16 bits each, with the transform fragments f / i and the
-// quantiser bands b0 / b1 of the lane's two positions.  All 32 lanes.
-__device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint4 f, const uint4 i, const uint4 b0,
-                                              const uint4 b1) {
+// quantisers of the lane's two positions.  All 32 lanes.
+__device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint2 f, const uint2 i, const QuantPos &a,
+                                              const QuantPos &b) {
     AreaCode r;
+    MmaSums d = mma_k8(f, h2_sub(bytes_h2(cv), bytes_h2(pv)));
+    d = mma_k8(f, pack_h2(shift14_small(d.h0, d.l0) - RND, shift14_small(d.h1, d.l1) - RND));
+    r.c0 = shift14(d.h0, d.l0) - RND;
+    r.c1 = shift14(d.h1, d.l1) - RND;
+    // dead-zone quantiser with RDOQ-lite, centroid dequantiser
+    const float a0 = fabsf(r.c0), a1 = fabsf(r.c1);
+    r.z0 = a0 >= a.thr ? 1.0f : 0.0f;
+    r.z1 = a1 >= b.thr ? 1.0f : 0.0f;
+    r.q0 = (__fadd_rd(__fmaf_rn(a0, a.r, a.off), RND) - RND) * r.z0;
+    r.q1 = (__fadd_rd(__fmaf_rn(a1, b.r, b.off), RND) - RND) * r.z1;
     uint32_t hi, lo;
-    split_sums(mma_k8(f.z, f.w, h2_sub(bytes_h2(cv), bytes_h2(pv)), ACC_FIELD), hi, lo);
-    MmaSums d = mma_k16(f, hi, lo, ACC_EXACT);
-    r.c0 = (int)d.x0() >> 14;
-    r.c1 = (int)d.x1() >> 14;
-    int dq0, dq1;
-    r.m0 = quant_one(r.c0, b0, dq0);
-    r.m1 = quant_one(r.c1, b1, dq1);
-    split_b(__byte_perm((uint32_t)dq0, (uint32_t)dq1, 0x5410), hi, lo);
-    split_sums(mma_k16(i, hi, lo, ACC_FIELD), hi, lo);
-    d = mma_k16(i, hi, lo, ACC_EXACT);
-    const int v0 = __viaddmin_s32_relu((int)(pv & 0xFF), (int)d.x0() >> 14, 255);   // clamped to 0..255
-    const int v1 = __viaddmin_s32_relu((int)(pv >> 8), (int)d.x1() >> 14, 255);
-    const int e0 = (int)(cv & 0xFF) - v0, e1 = (int)(cv >> 8) - v1;
+    split_h2(__fmaf_rn(r.q0, a.eff, a.bias) * copysignf(r.z0, r.c0), __fmaf_rn(r.q1, b.eff, b.bias) * copysignf(r.z1, r.c1),
+             hi, lo);
+    d = mma_k16(i, hi, lo);
+    split_h2(shift14(d.h0, d.l0) - RND, shift14(d.h1, d.l1) - RND, hi, lo);
+    d = mma_k16(i, hi, lo);
+    // prediction + residual, clamped: the prediction carries minus the bits of RND
+    const uint32_t p0 = __byte_perm(pv, 0xB4C00000u, 0x7650), p1 = __byte_perm(pv, 0xB4C00000u, 0x7651);
+    const int v0 = __viaddmin_s32_relu((int)p0, __float_as_int(shift14(d.h0, d.l0)), 255);
+    const int v1 = __viaddmin_s32_relu((int)p1, __float_as_int(shift14(d.h1, d.l1)), 255);
+    r.e0 = (int)(cv & 0xFF) - v0;
+    r.e1 = (int)(cv >> 8) - v1;
     r.rec = (uint32_t)v0 | (uint32_t)v1 << 8;
-    r.sse = e0 * e0 + e1 * e1;
-    r.bits = 2 * (bitlen((unsigned)r.m0) + bitlen((unsigned)r.m1)) + (r.m0 ? 3 : 0) + (r.m1 ? 3 : 0);
     return r;
 }
 
@@ -229,14 +251,15 @@ __host__ __device__ __forceinline__ int last_bits(int last) { return 2 + last + 
 // Last position + 1 of the area's 8x8 TU (0: empty): the raster position of
 // (lane, e) is 2 lane + e.
 __device__ __forceinline__ int last8(const AreaCode &c, int lane) {
-    return (int)__reduce_max_sync(0xffffffffu, c.m1 ? 2u * lane + 2u : c.m0 ? 2u * lane + 1u : 0u);
+    return (int)__reduce_max_sync(0xffffffffu, c.z1 != 0.0f ? 2u * lane + 2u : c.z0 != 0.0f ? 2u * lane + 1u : 0u);
 }
 
 // Of the lane's 4x4 TU (lanes of a quarter share bits 4 and 1 of their index,
 // and within it the raster position grows with the lane index).
 __device__ __forceinline__ int last4(const AreaCode &c, int lane) {
     const unsigned qm = ((lane & 2) ? 0xCCCCCCCCu : 0x33333333u) & ((lane & 16) ? 0xFFFF0000u : 0x0000FFFFu);
-    const unsigned any = __ballot_sync(0xffffffffu, (c.m0 | c.m1) != 0) & qm, n1 = __ballot_sync(0xffffffffu, c.m1 != 0);
+    const unsigned any = __ballot_sync(0xffffffffu, c.z0 + c.z1 != 0.0f) & qm,
+                   n1 = __ballot_sync(0xffffffffu, c.z1 != 0.0f);
     const int h = 31 - __clz((int)any);
     return any ? ((h >> 2) & 3) * 4 + (h & 1) * 2 + 1 + (int)((n1 >> h) & 1u) : 0;
 }
