@@ -141,9 +141,10 @@ __device__ void mvp_at(const MvCell *grid, int cx, int cy, int &mx, int &my) {
     if (!ha) { ax = hb ? bx : cxv; ay = hb ? by : cyv; }
     if (!hb) { bx = ha ? ax : cxv; by = ha ? ay : cyv; }
     if (!hc) { cxv = ha ? ax : bx; cyv = ha ? ay : by; }
-    const long long qa = (long long)ax * ax + (long long)ay * ay;
-    const long long qb = (long long)bx * bx + (long long)by * by;
-    const long long qc = (long long)cxv * cxv + (long long)cyv * cyv;
+    // squared lengths of 16-bit vectors: at most 2^31
+    const uint32_t qa = (uint32_t)(ax * ax) + (uint32_t)(ay * ay);
+    const uint32_t qb = (uint32_t)(bx * bx) + (uint32_t)(by * by);
+    const uint32_t qc = (uint32_t)(cxv * cxv) + (uint32_t)(cyv * cyv);
     if (qb < qa && qb <= qc) { mx = bx; my = by; }
     else if (qc < qa && qc < qb) { mx = cxv; my = cyv; }
     else { mx = ax; my = ay; }
@@ -406,6 +407,7 @@ struct Planes {
     __device__ __forceinline__ void build(const MeTeam &T, const uint8_t *ref, int bx, int by, bool h, bool v,
                                           bool d) const {
         const int nthr = 1 << T.lth, half = B >> 1, s = g_fp.stride_y, W = g_fp.W, Hh = g_fp.H;
+#pragma unroll 2
         for (int i = T.gt; i < (B + 6) * ST; i += nthr) {
             const int r = plane_div(i, B), x = bx - 3 + i - r * ST;
             const uint8_t *row = ref + (size_t)clampi(by - 3 + r, 0, Hh - 1) * s;
@@ -413,15 +415,18 @@ struct Planes {
         }
         T.sync();
         if (h)
+#pragma unroll 2
             for (int i = T.gt; i < (B + 6) * ST - 5; i += nthr)
                 H[i] = pair_six_tap(I[i], I[i + 1], I[i + 2], I[i + 3], I[i + 4], I[i + 5], PAIR_K_RAW);
         if (v)
+#pragma unroll 2
             for (int i = T.gt; i < (B + 1) * ST - 2; i += nthr) {
                 const uint32_t *q = I + i + 2;
                 V[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
             }
         T.sync();
         if (d) {
+#pragma unroll 2
             for (int i = T.gt; i < (B + 1) * ST - 5; i += nthr) {
                 const uint32_t *q = H + i;
                 D[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
@@ -459,6 +464,7 @@ struct PlanePoint {
 __device__ __forceinline__ void plane_pred(const MeTeam &T, const Planes &A, int X, int Y, uint8_t *dst, bool avg) {
     const PlanePoint P(A, X, Y, 0);
     const int half = A.B >> 1, lgh = lg2i(half);
+#pragma unroll 2
     for (int i = T.gt; i < A.B * half; i += 1 << T.lth) {
         const int y = i >> lgh, x = i & (half - 1);
         uint8_t *d = dst + y * A.B + x;
@@ -471,14 +477,28 @@ __device__ __forceinline__ void plane_pred(const MeTeam &T, const Planes &A, int
 
 // Luma prediction of a B x B block at the absolute quarter-sample vector
 // (mvx, mvy), sample by sample, by `nthr` threads (reference
-// src/motion.c:493-584); `avg` as in plane_pred.
+// src/motion.c:493-584); `avg` as in plane_pred.  The per-sample form with its
+// edge fallbacks covers the block forms too: samples whose six-tap support is
+// inside the frame take the nine-anchor combination, which for a whole-sample
+// or one-direction phase gives the copy's and the one-direction filters'
+// values (their truncating division differs on negative sums only, which the
+// clamp maps to 0), and a whole-sample phase gives the copy everywhere.
 __device__ __noinline__ void mc_samples(int t, int nthr, const uint8_t *ref, int mvx, int mvy, int B, uint8_t *dst,
                                         bool avg) {
-    LumaMC m;
-    m.init(ref, g_fp.stride_y, g_fp.W, g_fp.H, mvx, mvy, B);
-    const int lg = lg2i(B);
+    const int s = g_fp.stride_y, W = g_fp.W, H = g_fp.H, dx = mvx & 3, dy = mvy & 3, lg = lg2i(B);
+#pragma unroll 1
     for (int i = t; i < B * B; i += nthr) {
-        const int v = m.at(i & (B - 1), i >> lg);
+        const int fx = (mvx >> 2) + (i & (B - 1)), fy = (mvy >> 2) + (i >> lg);
+        int v;
+        if (fx >= 2 && fx + 3 < W && fy >= 2 && fy + 3 < H) {
+            v = luma_hv(ref, s, fx, fy, dx, dy);
+        } else if (fx >= 0 && fy >= 0 && fx + 1 < W && fy + 1 < H) {
+            const uint8_t *p = ref + (size_t)fy * s + fx;
+            v = interp_qpel(interp_qpel(p[0], p[1], dx), interp_qpel(p[s], p[s + 1], dx), dy);
+        } else {
+            const int nx = clampi(fx + (dx >= 2 ? 1 : 0), 0, W - 1), ny = clampi(fy + (dy >= 2 ? 1 : 0), 0, H - 1);
+            v = ref[(size_t)ny * s + nx];
+        }
         dst[i] = (uint8_t)(avg ? (v + dst[i] + 1) >> 1 : v);
     }
 }
@@ -548,6 +568,7 @@ __device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, con
                 } else {
                     const uint32_t *q = A.I + (2 + (Y >> 2) + y0) * ST + 2 + (X >> 2);
                     const uint32_t dx = X & 3, dy = Y & 3, k2 = 0x00020002u;
+#pragma unroll 1
                     for (int i = lane; i < n; i += 32) {
                         const int o = (i >> lgh) * ST + (i & (half - 1));
                         const uint32_t t = ((q[o] * (4 - dx) + q[o + 1] * dx + k2) >> 2) & 0x00FF00FFu;
@@ -674,13 +695,12 @@ __device__ __noinline__ void build_refs(const Leaf L) {
         S.edge[horiz][EDGE_BASE + j] = (uint8_t)sample(horiz == (j > 0), j > 0 ? j : 1 - j);
     }
     if (threadIdx.x == 0) S.above0 = sample(false, 0);
-    SYNC();
-    if (threadIdx.x < 32) {
+    if (threadIdx.x >= NT - 96 && threadIdx.x < NT - 64) {
         // DC value (reference src/predict.c:140-161): samples 1..N of each run.
         int sum = 0;
-        for (int i = threadIdx.x + 1; i <= N; i += 32) sum += S.edge[0][EDGE_BASE + i] + S.edge[1][EDGE_BASE + i];
+        for (int i = (threadIdx.x & 31) + 1; i <= N; i += 32) sum += sample(false, i) + sample(true, i);
         sum = __reduce_add_sync(0xffffffffu, sum);
-        if (threadIdx.x == 0) S.dc = (sum + N) >> __ffs(N);   // / (2 N)
+        if ((threadIdx.x & 31) == 0) S.dc = (sum + N) >> __ffs(N);   // / (2 N)
     }
     SYNC();
 }
@@ -719,6 +739,10 @@ __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, i
     return intra2(S, cu, slot - K_INTRA, e >> 16, x, y);
 }
 
+__device__ __forceinline__ QuantLane quant_lane(const Smem &S, int type, int lane) {
+    return {S.quant[type][0][lane], S.quant[type][1][lane], S.quant[type][2][lane]};
+}
+
 // Scores the listed candidates: distortion and bits of one 8x8 TU, of four
 // 4x4 TUs, or of both per 8x8 area, added to the slots' sums (reference
 // src/encoder.c:476-560; the four-TU form has an outer flag bit).
@@ -735,9 +759,7 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
     const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
     const uint2 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
-    const QuantParams &qp = S.qparam[0];
-    const QuantPos b80(qp, band_rc(8, row, col)), b81(qp, band_rc(8, row, col + 1));
-    const QuantPos b40(qp, band_rc(4, row & 3, col & 3)), b41(qp, band_rc(4, row & 3, (col & 3) + 1));
+    const QuantLane q8 = quant_lane(S, 0, lane), q4 = quant_lane(S, 1, lane);
 #ifdef TCB_PHASE_PROFILE
     if (threadIdx.x < ncl) { OPCOUNT(2, cl[threadIdx.x] & CL_8 ? 1 << la : 0); OPCOUNT(3, cl[threadIdx.x] & CL_4 ? 4 << la : 0); }
 #endif
@@ -771,14 +793,14 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
                 if ((lane & 13) == 0) n4 += b;
             };
             if (do_sizes == (CL_8 | CL_4)) {
-                const AreaCode c8 = code_area(cv, pv, f8, i8, b80, b81);
-                const AreaCode c4 = code_area(cv, pv, f4, i4, b40, b41);
+                const AreaCode c8 = code_area(cv, pv, f8, i8, q8);
+                const AreaCode c4 = code_area(cv, pv, f4, i4, q4);
                 add8(c8);
                 add4(c4);
             } else if (do_sizes == CL_8) {
-                add8(code_area(cv, pv, f8, i8, b80, b81));
+                add8(code_area(cv, pv, f8, i8, q8));
             } else {
-                add4(code_area(cv, pv, f4, i4, b40, b41));
+                add4(code_area(cv, pv, f4, i4, q4));
             }
         }
         if ((e & CL_EXACT) && __any_sync(0xffffffffu, differs)) S.inexact = 1;
@@ -808,13 +830,12 @@ __device__ __noinline__ void luma_replay(const Leaf L, int e, int16_t *emit) {
     if (t >= 1 << (2 * lt)) return;
     const bool d8 = e & CL_8;
     const uint2 f = S.frag[d8 ? 0 : 2][lane], i = S.frag[d8 ? 1 : 3][lane];
-    const QuantPos b0(S.qparam[0], d8 ? band_rc(8, row, col) : band_rc(4, row & 3, col & 3));
-    const QuantPos b1(S.qparam[0], d8 ? band_rc(8, row, col + 1) : band_rc(4, row & 3, (col & 3) + 1));
+    const QuantLane q = quant_lane(S, d8 ? 0 : 1, lane);
     const int pos = d8 ? 2 * lane : (row >> 2) * 32 + (col >> 2) * 16 + (row & 3) * 4 + (col & 3);
     for (; t < 1 << (2 * lt); t += NW) {
         const int x = (t & ((1 << lt) - 1)) * 8 + col, y = (t >> lt) * 8 + row;
         const uint32_t cv = *(const uint16_t *)(S.cur_y + (L.ly + y) * 64 + L.lx + x);
-        const AreaCode c = code_area(cv, pred2(S, cu, e, x, y), f, i, b0, b1);
+        const AreaCode c = code_area(cv, pred2(S, cu, e, x, y), f, i, q);
         *(uint16_t *)&RY(S, L.lx + x, L.ly + y) = (uint16_t)c.rec;
         *(uint32_t *)(emit + t * 64 + pos) = c.levels();
     }
@@ -888,7 +909,7 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
     int base = 4 * (((threadIdx.x >> 5) + NW - woff) & (NW - 1));
     if (base >= J) return;
     const uint2 f4 = S.frag[2][lane], i4 = S.frag[3][lane];
-    const QuantPos b0(S.qparam[1], band_rc(4, r, cc)), b1(S.qparam[1], band_rc(4, r, cc + 1));
+    const QuantLane q = quant_lane(S, 2, lane);
     for (; base < J; base += 4 * NW) {
         const bool act = base + quarter < J;
         const int j = act ? base + quarter : 0;
@@ -924,7 +945,7 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
             }
         }
         __syncwarp();
-        const AreaCode a = code_area(cv, pv, f4, i4, b0, b1);
+        const AreaCode a = code_area(cv, pv, f4, i4, q);
         if (nopt == 2) {
             AreaSums u;
             u.add(a);
@@ -1089,7 +1110,8 @@ __device__ void zero_acc(Smem &S) {
 
 // Sum over the CU of |orig - pred| per listed slot into acc[slot][0][0]
 // (fast-preset SAD proxy): one warp per (candidate, 8x8 area).
-__device__ void sad_areas(Smem &S, const Leaf &L, const int *cl, int ncl, uint32_t mask) {
+__device__ __noinline__ void sad_areas(const Leaf L, const int *cl, int ncl, uint32_t mask) {
+    Smem &S = smem_state();
     const int cu = L.cu, lt = lg2i(cu) - 3, J = ncl << (2 * lt);
     const int lane = threadIdx.x & 31;
     for (int it = threadIdx.x >> 5; it < J; it += NW) {
@@ -1116,30 +1138,38 @@ __device__ __forceinline__ long long best_of(const Smem &S, int slot, bool use4,
     return d8;
 }
 
-// Snapshot / restore of a node's reconstruction and grid cells.
-template <int D>
-__device__ void snap(Smem &S, const Leaf &L, int which, bool save) {
-    constexpr int cu = 64 >> D, cs = cu >> 1, gc = cu >> 3;
-    uint8_t *ys = D == 0 ? S.snap_y0[which] : D == 1 ? S.snap_y1[which] : S.snap_y2[which];
-    uint8_t *c0 = D == 0 ? S.snap_c0[which][0] : D == 1 ? S.snap_c1[which][0] : S.snap_c2[which][0];
-    uint8_t *c1 = D == 0 ? S.snap_c0[which][1] : D == 1 ? S.snap_c1[which][1] : S.snap_c2[which][1];
-    MvCell *gs = S.snap_g[D][which];
-    constexpr int lgu = 6 - D, lgs = 5 - D, lgg = 3 - D;
-    for (int i = threadIdx.x; i < cu * cu; i += NT) {
-        const int y = i >> lgu, x = i & (cu - 1);
-        if (save) ys[i] = RY(S, L.lx + x, L.ly + y); else RY(S, L.lx + x, L.ly + y) = ys[i];
+// Snapshot / restore of a node's reconstruction and grid cells (rows of a node
+// start on 8-byte addresses in luma, on 4-byte ones in chroma).  Compiled once
+// for all depths: the decide pass's code should stay in the instruction cache.
+//  to, from: snapshot the node is saved to, and the one it is then restored
+//  from (-1: none).
+__device__ __noinline__ void snap(const Leaf L, int to, int from) {
+    Smem &S = smem_state();
+    const int cu = L.cu, cs = cu >> 1, gc = cu >> 3, lg = lg2i(cu), d = L.depth;
+    const int size = 6 * cu * cu >> 2, step = d == 0 ? 0 : size;   // bytes; from snapshot 0 to 1
+    uint8_t *base = d == 0 ? S.snap0[0] : d == 1 ? S.snap1[0] : S.snap2[0];
+    const int ny = cu * cu >> 3, nc = cs * cs >> 2;
+    if (threadIdx.x < ny) {
+        const int i = threadIdx.x;
+        uint2 *t = (uint2 *)&RY(S, L.lx + (8 * i & (cu - 1)), L.ly + (8 * i >> lg));
+        if (to >= 0) *((uint2 *)(base + to * step) + i) = *t;
+        if (from >= 0) *t = *((uint2 *)(base + from * step) + i);
     }
-    for (int i = threadIdx.x; i < cs * cs; i += NT) {
-        const int y = i >> lgs, x = i & (cs - 1);
-        if (save) { c0[i] = RC(S, 0, (L.lx >> 1) + x, (L.ly >> 1) + y); c1[i] = RC(S, 1, (L.lx >> 1) + x, (L.ly >> 1) + y); }
-        else { RC(S, 0, (L.lx >> 1) + x, (L.ly >> 1) + y) = c0[i]; RC(S, 1, (L.lx >> 1) + x, (L.ly >> 1) + y) = c1[i]; }
+    if (threadIdx.x < 2 * nc) {
+        const int i = threadIdx.x, c = i >= nc, p = 4 * (i - c * nc);
+        uint32_t *t = (uint32_t *)&RC(S, c, (L.lx >> 1) + (p & (cs - 1)), (L.ly >> 1) + (p >> (lg - 1)));
+        if (to >= 0) *((uint32_t *)(base + to * step + cu * cu) + i) = *t;
+        if (from >= 0) *t = *((uint32_t *)(base + from * step + cu * cu) + i);
     }
-    for (int i = threadIdx.x; i < gc * gc; i += NT) {
-        const int y = i >> lgg, x = i & (gc - 1);
-        if (save) gs[i] = S.grid[(L.cy + y) * 8 + L.cx + x]; else S.grid[(L.cy + y) * 8 + L.cx + x] = gs[i];
+    if (threadIdx.x >= NT - gc * gc) {
+        const int i = threadIdx.x - (NT - gc * gc);
+        MvCell *g = &S.grid[(L.cy + (i >> (lg - 3))) * 8 + L.cx + (i & (gc - 1))];
+        if (to >= 0) S.snap_g[d][to][i] = *g;
+        if (from >= 0) *g = S.snap_g[d][from][i];
     }
     SYNC();
 }
+static_assert(NT >= 64 * 64 / 8, "a thread per 8 luma samples of a snapshot");
 
 // Grid update after a leaf (reference src/encoder.c:1279-1288 / 760-780).
 __device__ void grid_update(Smem &S, const Leaf &L, const Node &nd, int mvpx, int mvpy) {
@@ -1200,15 +1230,15 @@ __device__ __noinline__ void chroma_mc_bi(Smem &, const FrameParams &, const Lea
 // values, so no pass over the final tree is needed.
 // `decided`: the decision has just been made; its reference samples, chroma
 // model and inter predictions are still in shared memory, and an intra leaf's
-// chroma prediction is still to be chosen (src/encoder.c:1194-1221).
+// chroma prediction is still to be chosen (src/encoder.c:1194-1221);
+// (mvpx, mvpy) is its vector predictor.
 // ====================================================================
-__device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
+__device__ __noinline__ void leaf_code(const Leaf L, bool decided, int mvpx, int mvpy) {
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
     Node &node = S.nodes[qt_index(L.depth, L.cx, L.cy)];
     const Node nd = node;
-    int mvpx, mvpy;
-    mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
+    if (!decided) mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
     const int cu = L.cu, cs = cu >> 1;
     int16_t *el = L.depth == 1 ? S.lev1 : L.depth == 2 ? S.lev2 : S.coef + 96 * S.zoff[L.cy * 8 + L.cx];
     int16_t *ec = el + cu * cu;
@@ -1270,9 +1300,7 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
         }
         if (!nd.skip) {
             const int src = decided ? S.win_slot : 0;   // the decision's prediction is still in its slot
-            if (decided) {
-                SYNC();   // every thread has read the grid (mvp_at)
-            } else {
+            if (!decided) {
                 if (cflat && threadIdx.x >= NT - 64) chroma_model(L, (threadIdx.x >> 5) & 1);
                 if (flat) {
                     for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
@@ -1298,7 +1326,7 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided) {
 // ====================================================================
 // Leaf decision (reference src/encoder.c:784-1277).
 // ====================================================================
-__device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const Leaf L) {
+__device__ __noinline__ long long leaf_decide(const Leaf L) {
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
     const int cu = L.cu, tid = threadIdx.x, lane = tid & 31;
@@ -1385,7 +1413,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
     // ---- residual coding / SAD proxies for every candidate --------------
     cand |= modes << K_INTRA;
     if (fast) {
-        sad_areas(S, L, S.cl, nintra + (key ? 0 : NPRED), cand);
+        sad_areas(L, S.cl, nintra + (key ? 0 : NPRED), cand);
         SYNC();
     } else {
         if (key) luma_score(L, S.cl, nintra, 0, ~0u);
@@ -1428,11 +1456,10 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
         const int pos = lane < NPRED ? lane : (skip ? NPRED : lane + 1);
         const bool valid = (cand >> lane & 1u) ||
                            (skip && is_p && medium && P.ref_valid[0] && !S.inexact && S.acc64 == 0);
-        // extra bits: 6 for inter, 8 for the second reference, 8 for intra,
-        // 2 for skip, and the multiref syntax of a P leaf's searches
-        int extra = intra ? 8 : skip ? 2 : 6;
-        if (is_p && lane == K_ME1) extra = 8;
-        if (P.multiref && is_p) extra += (lane == K_ME0 || lane == K_TMP) ? 2 : lane == K_GLB ? 1 : 0;
+        // extra bits (a nibble per inter slot): 6, 8 for the second reference,
+        // and the multiref syntax of a P leaf's searches; 8 for intra, 2 for skip
+        const uint32_t ext = !is_p ? 0x66666u : P.multiref ? 0x68788u : 0x66686u;
+        const int extra = inter ? (int)(ext >> (4 * lane) & 15u) : skip ? 2 : 8;
         const int f_ref = is_b ? (lane == K_B0 + 1 || lane == K_B0 + 4) : lane == K_ME1;
         int f_dct = 1, f_mx = 0, f_my = 0, bits = extra;
         uint32_t kh = 0xFFFFFFFFu, kl = 0xFFFFFFFFu;
@@ -1481,7 +1508,7 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
 
     PHASE_D(5, L.depth);
     const long long best = S.best_cost;
-    leaf_code(L, true);
+    leaf_code(L, true, mvpx, mvpy);
     PHASE_D(7, L.depth);
     return best;
 }
@@ -1493,50 +1520,51 @@ __device__ __noinline__ long long leaf_decide(Smem &, const FrameParams &, const
 // split test) from exactly the state it sees now — every earlier sibling
 // kept the leaf decision it had then — so its decision (still in
 // S.nodes) and cost (S.node_cost) are reused and only the replay runs.
-template <int D>
-__device__ long long leaf_eval(Smem &S, const FrameParams &P, const Leaf &L, bool cached) {
+__device__ __noinline__ long long leaf_eval(const Leaf L, bool cached) {
+    Smem &S = smem_state();
     const int idx = qt_index(L.depth, L.cx, L.cy);
     if (cached) {
         const long long c = S.node_cost[idx];
-        leaf_code(L, false);
+        leaf_code(L, false, 0, 0);
         return c;
     }
-    const long long c = leaf_decide(S, P, L);
+    const long long c = leaf_decide(L);
     if (threadIdx.x == 0) S.node_cost[idx] = c;
     return c;
 }
 
+// One copy per depth, not inlined into each other: an unrolled tree would be
+// code that runs once per CTU and misses the instruction cache every time.
 template <int D>
-__device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy, bool cached) {
+__device__ __noinline__ void qt_decide(int ctu_x, int ctu_y, int cx, int cy, bool cached) {
+    Smem &S = smem_state();
+    const FrameParams &P = g_fp;
     constexpr int cu = 64 >> D;
     const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
     const bool in_frame = px + cu <= P.W && py + cu <= P.H;
     Node &nd = S.nodes[qt_index(D, cx, cy)];
     if constexpr (D < 3) {
         constexpr int h = 4 >> D;   // child offset in cells
-        if (!in_frame) {
-            for (int q = 0; q < 4; ++q)
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, false);
-            return;
-        }
         const int fast_leaf_depth = P.preset == 0 ? 3 : 2;
-        if (P.preset <= 1 && D < fast_leaf_depth) {
-            if (threadIdx.x == 0) nd.split = 1;
-            SYNC();
+        const bool pass = in_frame && P.preset <= 1 && D < fast_leaf_depth;
+        if (!in_frame || pass) {
+            if (pass) {
+                if (threadIdx.x == 0) nd.split = 1;
+                SYNC();
+            }
+#pragma unroll 1
             for (int q = 0; q < 4; ++q)
-                qt_decide<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, false);
+                qt_decide<D + 1>(ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, false);
             return;
         }
         const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-        snap<D>(S, L, 0, true);
-        const long long parent = leaf_eval<D>(S, P, L, cached);
-        if constexpr (D > 0) snap<D>(S, L, 1, true);
-        snap<D>(S, L, 0, false);
+        snap(L, 0, -1);
+        const long long parent = leaf_eval(L, cached);
+        snap(L, D > 0 ? 1 : -1, 0);
         long long child = 0;
-        for (int q = 0; q < 4; ++q) {
-            const Leaf C(P, ctu_x, ctu_y, D + 1, cx + (q & 1) * h, cy + (q >> 1) * h);
-            child += leaf_eval<D + 1>(S, P, C, false);
-        }
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q)
+            child += leaf_eval(Leaf(P, ctu_x, ctu_y, D + 1, cx + (q & 1) * h, cy + (q >> 1) * h), false);
         if (child <= parent) {
             if (threadIdx.x == 0) nd.split = 1;
             if constexpr (D == 2) {
@@ -1544,32 +1572,32 @@ __device__ void qt_decide(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, i
                 // their final reconstruction, grid and levels
                 SYNC();
             } else {
-                snap<D>(S, L, 0, false);
+                snap(L, -1, 0);
                 // Children keep their split-test evaluation until one of them
                 // splits (its region then differs from the split test's state).
                 bool same_state = true;
+#pragma unroll 1
                 for (int q = 0; q < 4; ++q) {
                     const int qx = cx + (q & 1) * h, qy = cy + (q >> 1) * h;
-                    qt_decide<D + 1>(S, P, ctu_x, ctu_y, qx, qy, same_state);
+                    qt_decide<D + 1>(ctu_x, ctu_y, qx, qy, same_state);
                     if (S.nodes[qt_index(D + 1, qx, qy)].split) same_state = false;
                 }
             }
         } else {
             if (threadIdx.x == 0) nd.split = 0;
             if constexpr (D == 0) {
-                snap<D>(S, L, 0, false);
-                leaf_code(L, false);
+                snap(L, -1, 0);
+                leaf_code(L, false, 0, 0);
             } else {
                 const uint2 *lev = (const uint2 *)(D == 1 ? S.lev1 : S.lev2);
                 uint2 *out = (uint2 *)(S.coef + 96 * S.zoff[cy * 8 + cx]);
                 for (int i = threadIdx.x; i < 24 * (64 >> (2 * D)); i += NT) out[i] = lev[i];
-                snap<D>(S, L, 1, false);
+                snap(L, -1, 1);
             }
         }
     } else {
         if (!in_frame) return;
-        const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-        leaf_eval<D>(S, P, L, cached);
+        leaf_eval(Leaf(P, ctu_x, ctu_y, D, cx, cy), cached);
         if (threadIdx.x == 0) nd.split = 0;
         SYNC();
     }
@@ -1795,6 +1823,18 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
         Node z = {};
         S.nodes[i] = z;
     }
+    // every lane's quantisers
+    if (threadIdx.x >= NT - 96) {
+        const int t = threadIdx.x - (NT - 96), type = t >> 5, lane = t & 31, r = lane >> 2, c = 2 * (lane & 3);
+        const int b0 = type ? band_rc(4, r & 3, c & 3) : band_rc(8, r, c);
+        const int b1 = type ? band_rc(4, r & 3, (c & 3) + 1) : band_rc(8, r, c + 1);
+        const int *eff = type == 2 ? P.eff_c : P.eff_l;
+        const long long lambda = type == 2 ? (long long)P.lambda_c : P.lambda;
+        const QuantLane q = QuantLane::make(QuantPos(eff[b0], lambda), QuantPos(eff[b1], lambda));
+        S.quant[type][0][lane] = q.a;
+        S.quant[type][1][lane] = q.b;
+        S.quant[type][2][lane] = q.c;
+    }
     CtuOut *out = P.out + row * P.ctu_cols + col;
     if (threadIdx.x == 0) S.coef = out->coef;
     if (threadIdx.x < 64) {
@@ -1808,18 +1848,9 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     }
     SYNC();
 
-    // Quantiser parameters in shared memory: every residual job reads them
-    // at fixed offsets.
-    if (threadIdx.x < 8) {
-        const int b = threadIdx.x & 3;
-        if (threadIdx.x < 4) S.qparam[0].set_band(b, P.eff_l[b], P.lambda);
-        else S.qparam[1].set_band(b, P.eff_c[b], P.lambda_c);
-    }
-    SYNC();
-
     // ---- decide and code -------------------------------------------------
     PHASE_T0();
-    qt_decide<0>(S, P, ctu_x, ctu_y, 0, 0, false);
+    qt_decide<0>(ctu_x, ctu_y, 0, 0, false);
     PHASE(8);
     close_gaps(ctu_x, ctu_y, out);
     PHASE(9);
@@ -2176,12 +2207,12 @@ tc_error_t tcb_debug_ctu_encode_frame_without_first(const tcb_frame_desc_t *desc
 // ====================================================================
 namespace tcb {
 
-__device__ __forceinline__ int dq_eff(const QuantParams &qp, int pos, int n) {
-    return qp.eff[freq_band(pos, n)];
+__device__ __forceinline__ int dq_eff(const int *eff, int pos, int n) {
+    return eff[freq_band(pos, n)];
 }
 
 // 8x8 TU from levels on an octet; writes pred + residual into the tile.
-__device__ void dec_luma8(Smem &S, const Leaf &L, const int16_t *lv, const QuantParams &qp) {
+__device__ void dec_luma8(Smem &S, const Leaf &L, const int16_t *lv, const int *qp) {
     const int cu = L.cu, ntu = cu >> 3, J = ntu * ntu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, oct = lane >> 3, l8 = lane & 7;
     int *scr = S.scratch[warp] + oct * 64;
@@ -2224,7 +2255,7 @@ __device__ void dec_luma8(Smem &S, const Leaf &L, const int16_t *lv, const Quant
 // 4x4 TUs from levels on quads.  Luma: per 8x8 TU four sub-blocks in
 // raster order; chroma (chroma_c >= 0): (cs/4)^2 TUs of that component.
 __device__ void dec_tu4(Smem &S, const Leaf &L, int chroma_c, const int16_t *lv,
-                        const QuantParams &qp) {
+                        const int *qp) {
     const int cu = L.cu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, l4 = lane & 3;
     int *scr = S.scratch[warp] + qd * 16;
@@ -2286,7 +2317,7 @@ __device__ void dec_tu4(Smem &S, const Leaf &L, int chroma_c, const int16_t *lv,
 // Decoder prediction reference choice (reference src/decoder.c:1628-1664,
 // 1697-1750); `flat` = no reference (128 / chroma DC).
 __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int16_t *coef,
-                         const QuantParams &ql, const QuantParams &qc) {
+                         const int *ql, const int *qc) {
     const Node nd = S.nodes[qt_index(L.depth, L.cx, L.cy)];
     int mvpx, mvpy;
     mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
@@ -2362,7 +2393,7 @@ __device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int
 
 template <int D>
 __device__ void qt_dec(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy,
-                       const int16_t *coef, const QuantParams &ql, const QuantParams &qc) {
+                       const int16_t *coef, const int *ql, const int *qc) {
     constexpr int cu = 64 >> D;
     const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
     const bool in_frame = px + cu <= P.W && py + cu <= P.H;
@@ -2413,14 +2444,9 @@ decode_kernel(const FrameParams *__restrict__ params, const int *__restrict__ it
     for (int i = threadIdx.x; i < QT_NODES; i += NT) S.nodes[i] = rec->nodes[i];
     if (threadIdx.x == 0) { S.ncoef = 0; S.tu8mask = rec->tu8mask; }
     SYNC();
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < 4; ++b) {   // the decoder reads the quantiser steps only
-            S.qparam[0].eff[b] = P.eff_l[b];
-            S.qparam[1].eff[b] = P.eff_c[b];
-        }
-    }
+    if (threadIdx.x < 8) S.eff[threadIdx.x >> 2][threadIdx.x & 3] = threadIdx.x < 4 ? P.eff_l[threadIdx.x] : P.eff_c[threadIdx.x & 3];
     SYNC();
-    const QuantParams &ql = S.qparam[0], &qc = S.qparam[1];
+    const int *ql = S.eff[0], *qc = S.eff[1];
     qt_dec<0>(S, P, ctu_x, ctu_y, 0, 0, rec->coef, ql, qc);
     SYNC();
     if (w == 64 && h == 64) deblock_tile(S, P.qp);

@@ -63,13 +63,12 @@ static_assert(NGROUP * plane_words(32) <= PLANE_WORDS && NGROUP * plane_words(16
 struct Smem {
     alignas(16) uint8_t cur_y[64 * 64];
     uint8_t cur_c[2][32 * 32];
-    uint8_t rec_y[RY_H * RY_W];
-    uint8_t rec_c[2][RC_H * RC_W];
+    alignas(16) uint8_t rec_y[RY_H * RY_W];
+    alignas(16) uint8_t rec_c[2][RC_H * RC_W];
     // qt_split snapshots, per depth: luma, cb, cr, grid (pre / parent; a
     // 64x64 parent that wins is coded again instead).
-    uint8_t snap_y0[1][64 * 64], snap_c0[1][2][32 * 32];
-    uint8_t snap_y1[2][32 * 32], snap_c1[2][2][16 * 16];
-    uint8_t snap_y2[2][16 * 16], snap_c2[2][2][8 * 8];
+    // [luma | cb | cr] of a node, 6 bytes per 4 luma samples
+    alignas(16) uint8_t snap0[1][6144], snap1[2][1536], snap2[2][384];
     MvCell snap_g[3][2][64];
     MvCell grid[64];
     Node nodes[QT_NODES];
@@ -92,7 +91,8 @@ struct Smem {
     uint8_t edge[2][EDGE_LEN];       // intra reference samples per direction (see build_refs)
     uint2 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
-    QuantParams qparam[2];     // luma, chroma quantiser of the current CTU
+    float4 quant[3][3][32];   // QuantLane parts per lane: luma 8x8, luma 4x4, chroma 4x4
+    int eff[2][4];            // decoder: quantiser steps of luma, chroma
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
     int acc[NCAND][2][2];      // per slot and TU size (8x8, 4x4): distortion, bits
     int cacc[2][2];            // per chroma option: distortion, bits

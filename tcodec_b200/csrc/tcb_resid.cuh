@@ -79,39 +79,36 @@ static inline cudaError_t upload_dct_tables() {
     return cudaMemcpyToSymbol(c_dct8, d8, sizeof(d8));
 }
 
-struct QuantParams {
-    int eff[4];
-    // Per band: {1 / eff, (eff / 3 + 1/2) / eff, smallest |c| with a level,
-    // eff} and eff / 6, the dequantiser's bias.  The level is
-    // floor((|c| + eff / 3) / eff) = floor(|c| / eff + (eff / 3 + 1/2) / eff):
-    // the half keeps the sum 1 / (2 eff) away from every integer, far more
-    // than its f32 rounding (below 2^-22 of it, for |c| + eff / 3 < 2^13).  A
-    // level of magnitude 1 dequantises to dq = eff + eff / 6 and is dropped
-    // when c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference
-    // src/encoder.c:333-355), i.e. when dq (2 |c| - dq) < lambda: below
-    // ceil((dq + ceil(lambda / dq)) / 2), if that lies in level 1's range.
-    float4 band[4];
-    float bias[4];
-    __host__ __device__ void set_band(int b, int e, long long lambda) {
-        const int off = e / 3, dq = e + e / 6;
-        long long thr = ((lambda + dq - 1) / dq + dq + 1) >> 1;
-        if (thr > 2 * e - off) thr = 2 * e - off;
-        if (thr < e - off) thr = e - off;
-        eff[b] = e;
-        band[b].x = 1.0f / (float)e;
-        band[b].y = ((float)off + 0.5f) / (float)e;
-        band[b].z = (float)thr;
-        band[b].w = (float)e;
-        bias[b] = (float)(e / 6);
-    }
-};
-// Quantiser of one position.
+// Quantiser of one coefficient position: 1 / eff, (eff / 3 + 1/2) / eff, the
+// smallest |c| with a level, eff, and eff / 6, the dequantiser's bias.  The
+// level is floor((|c| + eff / 3) / eff) = floor(|c| / eff + (eff / 3 + 1/2) /
+// eff): the half keeps the sum 1 / (2 eff) away from every integer, far more
+// than its f32 rounding (below 2^-22 of it, for |c| + eff / 3 < 2^13).  A level
+// of magnitude 1 dequantises to dq = eff + eff / 6 and is dropped when
+// c^2 + lambda < (|c| - dq)^2 + 2 lambda (reference src/encoder.c:333-355), i.e.
+// when dq (2 |c| - dq) < lambda: below ceil((dq + ceil(lambda / dq)) / 2), if
+// that lies in level 1's range.
 struct QuantPos {
     float r, off, thr, eff, bias;
-    __device__ __forceinline__ QuantPos(const QuantParams &q, int b) {
-        const float4 v = q.band[b];
-        r = v.x; off = v.y; thr = v.z; eff = v.w;
-        bias = q.bias[b];
+    __host__ __device__ QuantPos() {}
+    __host__ __device__ QuantPos(int e, long long lambda) {
+        const int o = e / 3, dq = e + e / 6;
+        long long t = ((lambda + dq - 1) / dq + dq + 1) >> 1;
+        if (t > 2 * e - o) t = 2 * e - o;
+        if (t < e - o) t = e - o;
+        r = 1.0f / (float)e;
+        off = ((float)o + 0.5f) / (float)e;
+        thr = (float)t;
+        eff = (float)e;
+        bias = (float)(e / 6);
+    }
+};
+// The quantisers of a lane's two positions, as laid out in shared memory.
+struct QuantLane {
+    float4 a, b, c;      // r, off, thr, eff of each position; both biases
+    __device__ __forceinline__ static QuantLane make(const QuantPos &p, const QuantPos &q) {
+        return {make_float4(p.r, p.off, p.thr, p.eff), make_float4(q.r, q.off, q.thr, q.eff),
+                make_float4(p.bias, q.bias, 0.0f, 0.0f)};
     }
 };
 
@@ -211,9 +208,9 @@ struct AreaSums {
 
 // Codes the area whose samples this lane holds two of: cv (source) and pv
 // (prediction), 16 bits each, with the transform fragments f / i and the
-// quantisers of the lane's two positions.  All 32 lanes.
-__device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint2 f, const uint2 i, const QuantPos &a,
-                                              const QuantPos &b) {
+// lane's quantisers.  All 32 lanes.
+__device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const uint2 f, const uint2 i,
+                                              const QuantLane &q) {
     AreaCode r;
     MmaSums d = mma_k8(f, h2_sub(bytes_h2(cv), bytes_h2(pv)));
     d = mma_k8(f, pack_h2(shift14_small(d.h0, d.l0) - RND, shift14_small(d.h1, d.l1) - RND));
@@ -221,12 +218,12 @@ __device__ __forceinline__ AreaCode code_area(uint32_t cv, uint32_t pv, const ui
     r.c1 = shift14(d.h1, d.l1) - RND;
     // dead-zone quantiser with RDOQ-lite, centroid dequantiser
     const float a0 = fabsf(r.c0), a1 = fabsf(r.c1);
-    r.z0 = a0 >= a.thr ? 1.0f : 0.0f;
-    r.z1 = a1 >= b.thr ? 1.0f : 0.0f;
-    r.q0 = (__fadd_rd(__fmaf_rn(a0, a.r, a.off), RND) - RND) * r.z0;
-    r.q1 = (__fadd_rd(__fmaf_rn(a1, b.r, b.off), RND) - RND) * r.z1;
+    r.z0 = a0 >= q.a.z ? 1.0f : 0.0f;
+    r.z1 = a1 >= q.b.z ? 1.0f : 0.0f;
+    r.q0 = (__fadd_rd(__fmaf_rn(a0, q.a.x, q.a.y), RND) - RND) * r.z0;
+    r.q1 = (__fadd_rd(__fmaf_rn(a1, q.b.x, q.b.y), RND) - RND) * r.z1;
     uint32_t hi, lo;
-    split_h2(__fmaf_rn(r.q0, a.eff, a.bias) * copysignf(r.z0, r.c0), __fmaf_rn(r.q1, b.eff, b.bias) * copysignf(r.z1, r.c1),
+    split_h2(__fmaf_rn(r.q0, q.a.w, q.c.x) * copysignf(r.z0, r.c0), __fmaf_rn(r.q1, q.b.w, q.c.y) * copysignf(r.z1, r.c1),
              hi, lo);
     d = mma_k16(i, hi, lo);
     split_h2(shift14(d.h0, d.l0) - RND, shift14(d.h1, d.l1) - RND, hi, lo);
