@@ -409,7 +409,7 @@ tc_error_t DecImpl::legacy_body(const uint8_t *data, size_t size, Reader &bs, co
     if (cudaMemcpyAsync(d_lblk, h_lblk, sizeof(legacy::LBlock) * nblk, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return TC_ERR_INTERNAL;
     for (size_t d = 0; d < ldiag_off.size(); ++d)
-        if (launch_legacy_ctus(F, d_litems + ldiag_off[d], ldiag_cnt[d], false, st) != cudaSuccess)
+        if (launch_legacy_decode(F, d_litems + ldiag_off[d], ldiag_cnt[d], st) != cudaSuccess)
             return TC_ERR_INTERNAL;
     return TC_OK;
 }

@@ -189,7 +189,6 @@ bool EncImpl::init(const tc_config_t &c) {
         legacy = true;
         const int threads = c.threads > 0 ? c.threads : 4;
         legacy_wpp = ctu_rows > 1 && threads > 1 && !c.enable_entropy_coded;
-        CK(upload_legacy_tables());
         CK(dmalloc(&d_lblk, sizeof(legacy::LBlock) * (size_t)nctu * legacy::BLOCKS));
         CK(pinned_alloc(&h_lblk, sizeof(legacy::LBlock) * (size_t)nctu * legacy::BLOCKS));
         std::vector<int> litems;
@@ -475,7 +474,7 @@ tc_error_t EncImpl::launch_legacy() {
             return TC_ERR_INTERNAL;
     }
     for (size_t d = 0; d < ldiag_off.size(); ++d)
-        if (launch_legacy_ctus(lframe, d_litems + ldiag_off[d], ldiag_cnt[d], true, st) != cudaSuccess)
+        if (launch_legacy_encode(lframe, d_litems + ldiag_off[d], ldiag_cnt[d], st) != cudaSuccess)
             return TC_ERR_INTERNAL;
     kernel_launches += (long long)ldiag_off.size();
     if (timing) cudaEventRecord(ev1, st);

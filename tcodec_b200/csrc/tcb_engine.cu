@@ -1980,10 +1980,17 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
     }
 }
 
+namespace legacy {
+__global__ void legacy_encode_kernel(const LFrame F, const int *__restrict__ items);
+}
+
 cudaError_t init_engine_tables() {
     cudaError_t e = upload_dct_tables();
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(ctu_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(Smem));
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(legacy::legacy_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(Smem));
     if (e != cudaSuccess) return e;
     if (CTAS_PER_SM > 1) {   // room for CTAS_PER_SM CTUs' shared memory per SM
@@ -2483,6 +2490,8 @@ cudaError_t launch_decode_items(const FrameParams *d_params, const int *d_items,
 }
 
 }  // namespace tcb
+
+#include "tcb_legacy_enc.cuh"
 
 #ifdef TCB_PHASE_PROFILE
 // Profiling builds only: read and reset the phase cycle counters.

@@ -1,5 +1,6 @@
-// tcb_legacy.cu — device side of the legacy (v0 / v1) 8x8 block path
-// (reference src/encoder.c:1526-2361, src/decoder.c:260-683).
+// tcb_legacy.cu — reconstruction of the legacy (v0 / v1) 8x8 block path from
+// parsed records (reference src/decoder.c:260-683); the encoder runs on the
+// CTU engine's parts (tcb_legacy_enc.cuh).
 //
 // One warp per CTU.  A CTU reads the reconstruction of its left, above and
 // above-right neighbours (intra references, including the above-right 8
@@ -28,12 +29,12 @@ __device__ __forceinline__ int ldct8(int k, int n) { return c_ldct8[k][n]; }
 namespace tcb {
 namespace legacy {
 
-__global__ void __launch_bounds__(32) legacy_ctu_kernel(LFrame F, const int *items, int n, int enc) {
+__global__ void __launch_bounds__(32) legacy_decode_kernel(LFrame F, const int *items, int n) {
     __shared__ LState S;
     const int it = blockIdx.x;
     if (it >= n) return;
     const int v = items[it];
-    code_ctu(S, F, v >> 10, v & 1023, enc != 0);
+    code_ctu(S, F, v >> 10, v & 1023, false);
 }
 
 }  // namespace legacy
@@ -62,9 +63,9 @@ cudaError_t upload_legacy_tables() {
     return cudaSuccess;
 }
 
-cudaError_t launch_legacy_ctus(const legacy::LFrame &F, const int *d_items, int n, bool encode, cudaStream_t st) {
+cudaError_t launch_legacy_decode(const legacy::LFrame &F, const int *d_items, int n, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    legacy::legacy_ctu_kernel<<<n, 32, 0, st>>>(F, d_items, n, encode ? 1 : 0);
+    legacy::legacy_decode_kernel<<<n, 32, 0, st>>>(F, d_items, n);
     return cudaGetLastError();
 }
 

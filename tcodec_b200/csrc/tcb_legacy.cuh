@@ -25,7 +25,7 @@ namespace legacy {
 #ifdef __CUDACC__
 #define LG_FN __device__ __forceinline__
 #define LG_TABLE static __constant__
-#define LG_NOINL __device__ __noinline__
+#define LG_NOINL static __device__ __noinline__
 constexpr int NL = 32;
 LG_FN int lane_id() { return threadIdx.x & 31; }
 LG_FN int team_sum(int v) { return (int)__reduce_add_sync(0xffffffffu, (unsigned)v); }
