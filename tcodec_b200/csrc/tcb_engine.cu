@@ -211,8 +211,8 @@ struct MeBlock {
 // (reference sad_at).  Lane k of every warp returns point p0 + k's SAD.  The
 // results go through part[par], which flips per call: a thread only gets to
 // the next call's barrier after all have read this one's.
-__device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, const MeBlock &M, int pat, int p0, int K, int bx,
-                                          int by, int scale) {
+__device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, const MeBlock &M, int pat, int p0, int K,
+                                          int bx, int by, int scale) {
     const int gt = T.gt, lpc = 1 << (T.lth - 3), k = gt >> (T.lth - 3), l = gt & (lpc - 1), lane = gt & 31;
     unsigned v = 0;
     bool in = false;
@@ -228,7 +228,7 @@ __device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, co
                 if (l < 8) v = sad8(r + (size_t)l * M.s, *(const uint2 *)(M.cur + l * 64), 0);
             } else {
                 const int lc = lg2i(M.blk) - 4, n = M.blk << lc;
-#pragma unroll 2
+#pragma unroll 4
                 for (int c = l; c < n; c += lpc) {
                     const int row = c >> lc, xo = (c & ((1 << lc) - 1)) * 16;
                     v = sad16(r + (size_t)row * M.s + xo, *(const uint4 *)(M.cur + row * 64 + xo), v);
@@ -260,21 +260,29 @@ __device__ __forceinline__ int batch_sads(Smem &S, const MeTeam &T, int &par, co
 // walk (order of candidates, first-improvement commits) is that of the
 // batched stages, on the same SAD values, so R changes the speed and never
 // the result.  Two tables alternate, so refilling one never races with a
-// lagging thread still reading the other.
-constexpr int WIN_RMAX = 5, WIN_NMAX = 2 * WIN_RMAX + 1, WIN_WORDS = WIN_NMAX * WIN_NMAX;
-// (they lie past the planes of blocks up to 16x16, which are in use at the
-// same time)
-constexpr int WIN_AT = PLANE_WORDS - NGROUP * 2 * WIN_WORDS;
-static_assert(NGROUP * plane_words(16) <= WIN_AT, "SAD tables overlap the planes");
-static_assert(WIN_WORDS <= 128, "one table position per thread of the smallest group");
-
+// lagging thread still reading the other.  The first one, around the start,
+// is filled along with the first batch.
+//
+// A walk is a chain of look-ups, about a dozen a search, and that chain is
+// what a small block's search takes: one minimum over (point, SAD + 1) keys
+// finds the next event, with "off the table" stored as 0 so that it passes
+// the same comparison, and a ring of such entries instead of bounds checks.
 __device__ __forceinline__ int window_radius(int r) { return r >= 2 && r <= WIN_RMAX ? r : 4; }
+__device__ __forceinline__ int win_index(int dx, int dy, int R) { return (dy + R + 2) * WIN_SIDE + dx + R + 2; }
 
-__device__ __forceinline__ void fill_sad_window(const MeTeam &T, int *tab, const MeBlock &M, int wx, int wy, int R) {
+// "Off the table" everywhere; once per CTU (a fill writes the positions of its
+// radius, the same for the whole CTU).
+__device__ void init_windows(Smem &S) {
+    for (int i = threadIdx.x; i < NGROUP * 2 * WIN_WORDS; i += NT)
+        S.me[i / (2 * WIN_WORDS)].win[0][i % (2 * WIN_WORDS)] = 0;
+}
+
+__device__ __forceinline__ void fill_sad_window(const MeTeam &T, uint16_t *tab, const MeBlock &M, int wx, int wy, int R) {
     const int N = 2 * R + 1, two = T.lth - 7, gt = T.gt, pos = gt >> two;
     if (gt == 0) OPCOUNT(0, N * N * M.blk * M.blk);
     // pos / N for pos < 128, N = 5, 7, 9, 11
-    const int py = pos * (N == 9 ? 7282 : N == 7 ? 9363 : N == 11 ? 5958 : 13108) >> 16, x = wx + pos - py * N - R, y = wy + py - R;
+    const int py = pos * (N == 9 ? 7282 : N == 7 ? 9363 : N == 11 ? 5958 : 13108) >> 16, px = pos - py * N;
+    const int x = wx + px - R, y = wy + py - R;
     const int rows = M.blk >> two, r0 = (gt & two) * rows;
     const bool in = pos < N * N && M.inside(x, y);
     unsigned v = 0;
@@ -289,8 +297,7 @@ __device__ __forceinline__ void fill_sad_window(const MeTeam &T, int *tab, const
         }
     }
     if (two) v += __shfl_xor_sync(0xffffffffu, v, 1);
-    if (pos < N * N) tab[pos] = in ? (int)v : 0x7FFFFFFF;
-    T.sync();
+    if (pos < N * N) tab[(py + 2) * WIN_SIDE + px + 2] = in ? (uint16_t)(v + 1) : (uint16_t)0xFFFF;
 }
 
 // The integer stages of one search: large hexagon (6 points, 2 passes,
@@ -309,55 +316,91 @@ __device__ __noinline__ void me_integer(const MeTeam T, int id, const uint8_t *r
     const int lane = gt & 31;
     int par = 0;
     int bx = clampi(center_x, 0, M.W - blk), by = clampi(center_y, 0, M.H - blk);
+    int wx = bx, wy = by;               // table around (wx, wy)
+    uint16_t *const tab0 = S.me[g].win[0], *tab = tab0;
+    const int R = window_radius(g_fp.search_window);
+    if (blk <= 16) fill_sad_window(T, tab, M, wx, wy, R);
     int bsad = 0x7FFFFFFF;
     bool centre = true;
-    int *const tab0 = (int *)S.plane + WIN_AT + g * 2 * WIN_WORDS, *tab = tab0;
-    int wx = 0, wy = 0, R = -1;         // table around (wx, wy); R < 0: none yet
-    const int radius = window_radius(g_fp.search_window);
+    // batched stages: the large hexagon, from 32x32 on all three
 #pragma unroll 1
-    for (int pat = 0; pat < 3; ++pat) {
+    for (int pat = 0; pat < (blk <= 16 ? 1 : 3); ++pat) {
         const int npts = pat == 2 ? 4 : 6, scale = pat == 0 ? maxi(1, sr / 4) : 1;
-        const bool table = pat > 0 && blk <= 16;
-        int ldx = 0, ldy = 0;           // this lane's pattern point (lanes 1..npts)
-        if (lane <= npts) pat_point(pat, lane, ldx, ldy);
 #pragma unroll 1
         for (int it = 0; it < pat + 2; ++it) {
             bool improved = false;
             int p0 = 1;
             while (p0 <= npts) {
-                int v = 0x7FFFFFFF, base = 0;   // lane's SAD; lane of point 0
-                bool off = false;
-                if (table) {
-                    const bool act = lane >= p0 && lane <= npts;
-                    const int x = bx + ldx - wx + R, y = by + ldy - wy + R;
-                    off = act && (R < 0 || x < 0 || x > 2 * R || y < 0 || y > 2 * R);
-                    if (act && !off) v = tab[y * (2 * R + 1) + x];
-                } else {
-                    base = centre ? 0 : p0;
-                    v = batch_sads(S, T, par, M, pat, base, npts + 1 - base, bx, by, scale);
-                    if (centre) bsad = __shfl_sync(0xffffffffu, v, 0);
-                    centre = false;
-                }
-                const unsigned ev = __ballot_sync(0xffffffffu, off || v < bsad);
-                if (!ev) break;                   // no point of this pass improves
-                const int f = __ffs(ev) - 1;
-                if (__shfl_sync(0xffffffffu, (int)off, f)) {
-                    // off the table: refill it around the running best, as
-                    // the sequential walk does on reaching this point
-                    tab = tab == tab0 ? tab0 + WIN_WORDS : tab0;
-                    wx = bx; wy = by; R = radius;
-                    fill_sad_window(T, tab, M, wx, wy, R);
-                    p0 = f;
-                    continue;
-                }
-                bsad = __shfl_sync(0xffffffffu, v, f);
-                bx += scale * __shfl_sync(0xffffffffu, ldx, f + base);
-                by += scale * __shfl_sync(0xffffffffu, ldy, f + base);
+                const int base = centre ? 0 : p0;                  // lane k: point base + k
+                const int v = batch_sads(S, T, par, M, pat, base, npts + 1 - base, bx, by, scale);
+                if (centre) bsad = __shfl_sync(0xffffffffu, v, 0);
+                centre = false;
+                // SADs are below 2^20: the first improving point has the smallest key
+                const unsigned k = __reduce_min_sync(0xffffffffu, v < bsad ? (unsigned)lane << 20 | (unsigned)v : 0xFFFFFFFFu);
+                if (k == 0xFFFFFFFFu) break;                       // no point of this pass improves
+                const int f = base + (int)(k >> 20);
+                int dx, dy;
+                pat_point(pat, f, dx, dy);
+                bsad = (int)(k & 0xFFFFFu);
+                bx += dx * scale;
+                by += dy * scale;
                 improved = true;
-                p0 = f + base + 1;
+                p0 = f + 1;
             }
             if (!improved) break;
         }
+    }
+    if (blk <= 16) {
+        int c = win_index(bx - wx, by - wy, R), b1 = bsad + 1;
+        if (bx - wx > R || bx - wx < -R || by - wy > R || by - wy < -R) {
+            tab = tab0 + WIN_WORDS;
+            wx = bx; wy = by;
+            c = win_index(0, 0, R);
+            fill_sad_window(T, tab, M, wx, wy, R);
+            T.sync();
+        }
+#pragma unroll 1
+        for (int pat = 1; pat < 3; ++pat) {
+            const int npts = pat == 1 ? 6 : 4;
+            int ldx, ldy;               // this lane's pattern point (lanes 1..npts)
+            pat_point(pat, mini(lane, 6), ldx, ldy);
+            const int loff = ldy * WIN_SIDE + ldx;
+#pragma unroll 1
+            for (int it = 0; it < pat + 2; ++it) {
+                bool improved = false;
+                int p0 = 1;
+                while (p0 <= npts) {
+                    unsigned key = 0xFFFFFFFFu;
+                    if (lane >= p0 && lane <= npts) {
+                        const int v = tab[c + loff];
+                        if (v < b1) key = (unsigned)lane << 16 | (unsigned)v;
+                    }
+                    key = __reduce_min_sync(0xffffffffu, key);
+                    if (key == 0xFFFFFFFFu) break;
+                    const int f = (int)(key >> 16), v = (int)(key & 0xFFFFu);
+                    if (v == 0) {
+                        // off the table: refill it around the running best, as
+                        // the sequential walk does on reaching this point
+                        tab = tab == tab0 ? tab0 + WIN_WORDS : tab0;
+                        wx = bx; wy = by;
+                        c = win_index(0, 0, R);
+                        fill_sad_window(T, tab, M, wx, wy, R);
+                        T.sync();
+                        p0 = f;
+                        continue;
+                    }
+                    int dx, dy;
+                    pat_point(pat, f, dx, dy);
+                    b1 = v;
+                    bx += dx; by += dy;
+                    c += dy * WIN_SIDE + dx;
+                    improved = true;
+                    p0 = f + 1;
+                }
+                if (!improved) break;
+            }
+        }
+        bsad = b1 - 1;
     }
     ME_MARK(11);
     if (gt == 0) { S.me[id].bx = bx; S.me[id].by = by; S.me[id].best = bsad; }
@@ -389,7 +432,9 @@ __device__ __forceinline__ int plane_div(int i, int blk) {   // i / plane_stride
     return (int)((uint32_t)i * m >> 16);
 }
 
-// The planes of a block around its integer position (bx, by).
+// The planes of a block around its integer position (bx, by), every sample
+// biased by 208 (integer samples too: 208..463 are in the range the six-tap
+// is exact for, see pair_six_tap).
 struct Planes {
     uint32_t *I, *H, *V, *D;
     int B, ST;
@@ -411,18 +456,18 @@ struct Planes {
         for (int i = T.gt; i < (B + 6) * ST; i += nthr) {
             const int r = plane_div(i, B), x = bx - 3 + i - r * ST;
             const uint8_t *row = ref + (size_t)clampi(by - 3 + r, 0, Hh - 1) * s;
-            I[i] = (uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16;
+            I[i] = ((uint32_t)__ldg(row + clampi(x, 0, W - 1)) | (uint32_t)__ldg(row + clampi(x + half, 0, W - 1)) << 16) + PAIR_B;
         }
         T.sync();
         if (h)
 #pragma unroll 2
             for (int i = T.gt; i < (B + 6) * ST - 5; i += nthr)
-                H[i] = pair_six_tap(I[i], I[i + 1], I[i + 2], I[i + 3], I[i + 4], I[i + 5], PAIR_K_RAW);
+                H[i] = pair_six_tap(I[i], I[i + 1], I[i + 2], I[i + 3], I[i + 4], I[i + 5], PAIR_K_HALF);
         if (v)
 #pragma unroll 2
             for (int i = T.gt; i < (B + 1) * ST - 2; i += nthr) {
                 const uint32_t *q = I + i + 2;
-                V[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_RAW);
+                V[i] = pair_six_tap(q[0], q[ST], q[2 * ST], q[3 * ST], q[4 * ST], q[5 * ST], PAIR_K_HALF);
             }
         T.sync();
         if (d) {
@@ -438,10 +483,10 @@ struct Planes {
 // Position (X, Y) in quarter samples (0..7) from (bx - 1, by - 1): the two
 // columns h0, h1 and rows v0, v1 of the half-sample grid it averages.  Even
 // ones lie on samples (planes I, V), odd ones between (H, D); rows likewise
-// (I, H / V, D).  Integer samples carry no bias in their plane.
+// (I, H / V, D).
 struct PlanePoint {
     const uint32_t *q00, *q01, *q10, *q11;
-    uint32_t b00, b01, b10, b11;
+    bool four;               // both directions average two values; else q00 and q11 do
     __device__ __forceinline__ PlanePoint(const Planes &A, int X, int Y, int y0) {
         const int h0 = X >> 1, h1 = (X + 1) >> 1, v0 = Y >> 1, v1 = (Y + 1) >> 1;
         auto at = [&](int v, int h) {
@@ -449,14 +494,16 @@ struct PlanePoint {
             return q + ((v >> 1) + y0) * A.ST + (h >> 1);
         };
         q00 = at(v0, h0); q01 = at(v0, h1); q10 = at(v1, h0); q11 = at(v1, h1);
-        b00 = (v0 | h0) & 1 ? 0 : PAIR_B; b01 = (v0 | h1) & 1 ? 0 : PAIR_B;
-        b10 = (v1 | h0) & 1 ? 0 : PAIR_B; b11 = (v1 | h1) & 1 ? 0 : PAIR_B;
+        four = X & Y & 1;
     }
-    // the clamped samples of word o
-    __device__ __forceinline__ uint32_t value(int o) const {
-        const uint32_t t = pair_avg(q00[o] + b00, q01[o] + b01), b = pair_avg(q10[o] + b10, q11[o] + b11);
-        return pair_min(pair_max(pair_avg(t, b), PAIR_B), PAIR_B + 255u * 0x00010001u) - PAIR_B;
+    __device__ __forceinline__ static uint32_t finish(uint32_t v) {   // clamped, bias removed
+        return pair_min(pair_max(v, PAIR_B), PAIR_B + 255u * 0x00010001u) - PAIR_B;
     }
+    // the samples of word o
+    __device__ __forceinline__ uint32_t value4(int o) const {
+        return finish(pair_avg(pair_avg(q00[o], q01[o]), pair_avg(q10[o], q11[o])));
+    }
+    __device__ __forceinline__ uint32_t value2(int o) const { return finish(pair_avg(q00[o], q11[o])); }
 };
 
 // The prediction at (X, Y) into dst (stride B), averaged with what is there
@@ -468,7 +515,7 @@ __device__ __forceinline__ void plane_pred(const MeTeam &T, const Planes &A, int
     for (int i = T.gt; i < A.B * half; i += 1 << T.lth) {
         const int y = i >> lgh, x = i & (half - 1);
         uint8_t *d = dst + y * A.B + x;
-        uint32_t v = P.value(y * A.ST + x);
+        uint32_t v = P.four ? P.value4(y * A.ST + x) : P.value2(y * A.ST + x);
         if (avg) v = pair_avg(v, (uint32_t)d[0] | (uint32_t)d[half] << 16);
         d[0] = (uint8_t)v;
         d[half] = (uint8_t)(v >> 16);
@@ -529,68 +576,79 @@ __device__ __noinline__ void me_qpel(const MeTeam T, int id, uint32_t *area, con
     const int bx = E.bx, by = E.by, lane = gt & 31, warp = gt >> 5, gw = 1 << (T.lth - 5);
     const Planes A(area, B);
     const int ST = A.ST;
-    if (gt < QPOS * QPOS) E.tab[gt] = 0;
+    if (gt < QPOS * QPOS) E.tab[gt] = make_int4(0, 0, 0, 0);
     A.build(T, ref, bx, by, true, true, true);
 
-    // Lane p (1..8) holds point p; the points' offsets as in pat_point.
-    int ox = 0, oy = 0;
-    if (lane >= 1 && lane <= 8) {
-        const uint32_t px = 0x79798879u, py = 0x77997988u;   // (+-1, 0), (0, +-1), then the corners
-        ox = (int)(px >> (4 * (lane - 1)) & 15u) - 8;
-        oy = (int)(py >> (4 * (lane - 1)) & 15u) - 8;
-    }
+    // Lane p (1..8) holds point p; the points' offsets a nibble each (value +
+    // 8): (+-1, 0), (0, +-1), then the corners.
+    constexpr uint32_t PX = 0x79798879u, PY = 0x77997988u;
+    const bool point = lane >= 1 && lane <= 8;
+    const int sh = 4 * (lane - 1) & 31;
+    const int ox = (int)(PX >> sh & 15u) - 8, oy = (int)(PY >> sh & 15u) - 8;
     int ux = 3, uy = 3, bsad = E.best, p0 = 1;     // running best: quarter-sample offset + 3
+    // Positions scored so far.  Kept in registers, the same in every warp: a
+    // warp that looked at the table instead could already see what a faster
+    // one has written for the next round, and their barriers would not match.
     unsigned long long known = 0;
+    const bool inner = bx >= 3 && by >= 3 && bx + B + 2 < W && by + B + 2 < H;   // every point is a plane point
 #pragma unroll 1
     for (;;) {
         const int cx = ux + ox, cy = uy + oy, fx = (4 * bx + cx - 3) >> 2, fy = (4 * by + cy - 3) >> 2;
-        const bool act = lane >= p0 && lane <= 8 && fx >= 0 && fy >= 0 && fx + B + 1 <= W && fy + B + 1 <= H;
+        const bool act = point && lane >= p0 && (inner || (fx >= 0 && fy >= 0 && fx + B + 1 <= W && fy + B + 1 <= H));
         const int idx = act ? cy * QPOS + cx : 0;
         const unsigned need = __ballot_sync(0xffffffffu, act && !(known >> idx & 1ull));
         if (need) {
+            const unsigned long long mine = act ? 1ull << idx : 0ull;
+            known |= (unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) << 32 |
+                     __reduce_or_sync(0xffffffffu, (unsigned)mine);
             const int K = __popc(need), lsp = B >= 32 ? 2 : 0, n = (B * half) >> lsp, lgh = lg2i(half);
             if (gt == 0) OPCOUNT(1, K * B * B);
+#pragma unroll 1
             for (int it = warp; it < K << lsp; it += gw) {
                 unsigned m = need;
                 for (int j = it >> lsp; j > 0; --j) m &= m - 1;
-                const int f = __ffs(m) - 1;
-                const int X = __shfl_sync(0xffffffffu, cx, f) + 1, Y = __shfl_sync(0xffffffffu, cy, f) + 1;
+                const int fs = 4 * (__ffs((int)m) - 2), part = it & ((1 << lsp) - 1);
                 // position in quarter samples from (bx - 1, by - 1): 1..7
+                const int X = ux + (int)(PX >> fs & 15u) - 7, Y = uy + (int)(PY >> fs & 15u) - 7;
                 const int qfx = bx - 1 + (X >> 2), qfy = by - 1 + (Y >> 2);
-                const uint32_t *cur = S.cur_pair + (it & ((1 << lsp) - 1)) * n;
-                const int y0 = ((it & ((1 << lsp) - 1)) * n) >> lgh;
+                const uint32_t *cur = S.cur_pair + part * n;
+                const int y0 = (part * n) >> lgh;
                 unsigned acc = 0;
-                if (qfx >= 2 && qfy >= 2 && qfx + B + 2 < W && qfy + B + 2 < H) {
+                if (inner || (qfx >= 2 && qfy >= 2 && qfx + B + 2 < W && qfy + B + 2 < H)) {
                     const PlanePoint P(A, X, Y, y0);
+                    if (P.four) {
 #pragma unroll 4
-                    for (int i = lane; i < n; i += 32)
-                        acc += __vsadu4(P.value((i >> lgh) * ST + (i & (half - 1))), cur[i]);
+                        for (int i = lane; i < n; i += 32)
+                            acc += __vsadu4(P.value4((i >> lgh) * ST + (i & (half - 1))), cur[i]);
+                    } else {
+#pragma unroll 4
+                        for (int i = lane; i < n; i += 32)
+                            acc += __vsadu4(P.value2((i >> lgh) * ST + (i & (half - 1))), cur[i]);
+                    }
                 } else {
                     const uint32_t *q = A.I + (2 + (Y >> 2) + y0) * ST + 2 + (X >> 2);
                     const uint32_t dx = X & 3, dy = Y & 3, k2 = 0x00020002u;
 #pragma unroll 1
                     for (int i = lane; i < n; i += 32) {
                         const int o = (i >> lgh) * ST + (i & (half - 1));
-                        const uint32_t t = ((q[o] * (4 - dx) + q[o + 1] * dx + k2) >> 2) & 0x00FF00FFu;
-                        const uint32_t b = ((q[o + ST] * (4 - dx) + q[o + ST + 1] * dx + k2) >> 2) & 0x00FF00FFu;
+                        const uint32_t t = (((q[o] - PAIR_B) * (4 - dx) + (q[o + 1] - PAIR_B) * dx + k2) >> 2) & 0x00FF00FFu;
+                        const uint32_t b = (((q[o + ST] - PAIR_B) * (4 - dx) + (q[o + ST + 1] - PAIR_B) * dx + k2) >> 2) & 0x00FF00FFu;
                         acc += __vsadu4(((t * (4 - dy) + b * dy + k2) >> 2) & 0x00FF00FFu, cur[i]);
                     }
                 }
                 acc = __reduce_add_sync(0xffffffffu, acc);
-                if (lane == 0) atomicAdd(&E.tab[(Y - 1) * QPOS + X - 1], (int)acc);
+                if (lane == 0) ((int *)&E.tab[(Y - 1) * QPOS + X - 1])[part] = (int)acc;
             }
             T.sync();
-            const unsigned long long mine = (need >> lane & 1u) ? 1ull << idx : 0ull;
-            known |= (unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) << 32 |
-                     __reduce_or_sync(0xffffffffu, (unsigned)mine);
         }
-        const int v = act ? E.tab[idx] : 0x7FFFFFFF;
-        const unsigned ev = __ballot_sync(0xffffffffu, v < bsad);
-        if (!ev) break;
-        const int f = __ffs(ev) - 1;
-        bsad = __shfl_sync(0xffffffffu, v, f);
-        ux = __shfl_sync(0xffffffffu, cx, f);
-        uy = __shfl_sync(0xffffffffu, cy, f);
+        const int4 e = E.tab[idx];
+        const int v = e.x + e.y + e.z + e.w;       // below 2^20
+        const unsigned k = __reduce_min_sync(0xffffffffu, act && v < bsad ? (unsigned)lane << 20 | (unsigned)v : 0xFFFFFFFFu);
+        if (k == 0xFFFFFFFFu) break;
+        const int f = (int)(k >> 20), fs = 4 * (f - 1);
+        bsad = (int)(k & 0xFFFFFu);
+        ux += (int)(PX >> fs & 15u) - 8;
+        uy += (int)(PY >> fs & 15u) - 8;
         p0 = f + 1;
     }
     ME_MARK(12);
@@ -1835,6 +1893,7 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
         S.quant[type][1][lane] = q.b;
         S.quant[type][2][lane] = q.c;
     }
+    init_windows(S);
     CtuOut *out = P.out + row * P.ctu_cols + col;
     if (threadIdx.x == 0) S.coef = out->coef;
     if (threadIdx.x < 64) {

@@ -42,10 +42,16 @@ enum {
 
 constexpr int EDGE_BASE = 96, EDGE_LEN = 264;   // index 0 of S.edge; entries up to 2.5 * 64 + 2
 
+// SAD tables of the integer stages of blocks up to 16x16: positions within R
+// (2..WIN_RMAX) of the window's centre, and a ring of 2 around them that
+// says "off the table".
+constexpr int WIN_RMAX = 5, WIN_SIDE = 2 * WIN_RMAX + 5, WIN_WORDS = WIN_SIDE * WIN_SIDE;
+
 constexpr int QPOS = 7;               // quarter-sample positions per axis around an integer best: -3..3
-struct MeGroup {
+struct alignas(16) MeGroup {
     int part[2][8];         // SADs of a batch of candidates, double-buffered (see batch_sads)
-    int tab[QPOS * QPOS];   // SADs of the quarter-sample positions scored so far
+    int4 tab[QPOS * QPOS];  // SADs of the quarter-sample positions scored, by quarters of the block
+    uint16_t win[2][WIN_WORDS];   // two SAD tables: SAD + 1, 0 off the table, 0xFFFF outside the frame
     int bx, by;             // integer best
     int mvx, mvy, best;
 };
@@ -84,7 +90,7 @@ struct Smem {
             int16_t clev[4][32 * 32];
             int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
         };
-        // during them: SAD tables of the integer stages, then sample planes
+        // during them: sample planes
         alignas(16) uint32_t plane[PLANE_WORDS];
     };
     uint32_t cur_pair[64 * 32];      // leaf's source samples (x, x + cu / 2) as 16-bit lanes, for the searches

@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(NT, 1) legacy_encode_kernel(const LFrame F, co
     const int w = mini(64, W - ox), h = mini(64, H - oy), wc = w >> 1, hc = h >> 1;
     if (tid == 0) { g_fp.W = W; g_fp.H = H; g_fp.stride_y = F.sy; g_fp.search_window = 0; }
     init_fragments(S);
+    init_windows(S);
     if (tid >= 128 && tid < 192) E.wht[(tid - 128) >> 5][lane] = wht_fragment(tid < 160 ? 8 : 4, lane);
     if (tid >= NT - 96) {
         const int k = (tid - (NT - 96)) >> 5, r = lane >> 2, c = 2 * (lane & 3);
