@@ -36,6 +36,53 @@ uint64_t now_ns() {
     return (uint64_t)t.tv_sec * 1000000000ull + (uint64_t)t.tv_nsec;
 }
 
+// Replaces the coded vector differences of a CTU's leaves by absolute
+// quarter-sample vectors (16-bit, wrapping as in reference
+// src/decoder.c:1560-1600): the predictor is the shortest of the left, above
+// and above-right neighbours' vectors (src/motion.c:119-170), which chains
+// every leaf to the one before, so it is done here, where the leaves are in
+// order anyway, and the device takes them in any order.
+void resolve_vectors(CtuOut &o, int ctu_x, int ctu_y, int W, int H) {
+    struct Cell { int dx, dy; bool ok; } grid[64];
+    for (Cell &g : grid) g.ok = false;
+    for (int z = 0; z < 64;) {
+        const int cx = (z & 1) | (z >> 1 & 2) | (z >> 2 & 4), cy = (z >> 1 & 1) | (z >> 2 & 2) | (z >> 3 & 4);
+        int d = 0;
+        for (; d < 3; ++d) {   // the largest node that starts here, is inside the frame and not split
+            const int gc = 8 >> d, m = gc - 1;
+            if (!(cx & m) && !(cy & m) && ctu_x + 8 * (cx + gc) <= W && ctu_y + 8 * (cy + gc) <= H &&
+                !o.nodes[qt_index(d, cx, cy)].split)
+                break;
+        }
+        const int gc = 8 >> d;
+        if (ctu_x + 8 * (cx + gc) <= W && ctu_y + 8 * (cy + gc) <= H) {
+            Node &nd = o.nodes[qt_index(d, cx, cy)];
+            Cell a = {0, 0, false}, b = a, c = a;
+            if (cx > 0) a = grid[cy * 8 + cx - 1];
+            if (cy > 0) b = grid[cy * 8 + cx - 8];
+            if (cy > 0 && cx < 7) c = grid[cy * 8 + cx - 7];
+            int mx = 0, my = 0;
+            if (a.ok || b.ok || c.ok) {
+                if (!a.ok) a = b.ok ? b : c;
+                if (!b.ok) b = a;
+                if (!c.ok) c = a;
+                auto len = [](const Cell &g) { return (uint32_t)(g.dx * g.dx) + (uint32_t)(g.dy * g.dy); };
+                const uint32_t qa = len(a), qb = len(b), qc = len(c);
+                const Cell &p = qb < qa && qb <= qc ? b : qc < qa && qc < qb ? c : a;
+                mx = p.dx; my = p.dy;
+            }
+            const bool own = !(nd.skip || nd.merge);
+            const Cell g = {(int16_t)(mx + (own ? nd.mvd_x : 0)), (int16_t)(my + (own ? nd.mvd_y : 0)), !nd.intra};
+            for (int y = 0; y < gc; ++y)
+                for (int x = 0; x < gc; ++x) grid[(cy + y) * 8 + cx + x] = g;
+            const bool add = own && !nd.intra;
+            nd.mvd_x = (int16_t)(mx + (ctu_x + cx * 8) * 4 + (add ? nd.mvd_x : 0));
+            nd.mvd_y = (int16_t)(my + (ctu_y + cy * 8) * 4 + (add ? nd.mvd_y : 0));
+        }
+        z += 64 >> (2 * d);
+    }
+}
+
 }  // namespace
 
 namespace tcb {
@@ -51,6 +98,7 @@ struct DecImpl {
     int dpb_poc[TC_REF_FRAMES] = {-1, -1, -1, -1};
     std::vector<DevFrame> spare;      // free device frames
     CtuOut *d_rec = nullptr, *h_rec = nullptr;
+    int *h_status = nullptr;          // the kernels' status word, behind h_rec
     // Legacy (v0 / v1) streams: block records and the wavefront of
     // diagonals c + 2r (see tcb_legacy.cu).
     legacy::LBlock *d_lblk = nullptr, *h_lblk = nullptr;
@@ -111,7 +159,8 @@ struct DecImpl {
         rows = (h + 63) / 64;
         if (!alloc_frame(cur)) return false;
         if (dev_alloc(&d_rec, sizeof(CtuOut) * cols * rows) != cudaSuccess) return false;
-        if (pinned_alloc(&h_rec, sizeof(CtuOut) * cols * rows) != cudaSuccess) return false;
+        if (pinned_alloc(&h_rec, sizeof(CtuOut) * (cols * rows + 1)) != cudaSuccess) return false;
+        h_status = (int *)(h_rec + cols * rows);
         std::vector<int> items;
         diag_off.clear(); diag_cnt.clear();
         for (int d = 0; d < rows + cols - 1; ++d) {
@@ -122,6 +171,7 @@ struct DecImpl {
             }
             diag_cnt.push_back((int)items.size() - diag_off.back());
         }
+        items.push_back(0);   // the kernels' status word
         if (dev_alloc(&d_items, sizeof(int) * items.size()) != cudaSuccess) return false;
         cudaMemcpy(d_items, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice);
         std::vector<int> litems;
@@ -238,6 +288,7 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
                 p.o = h_rec + row * cols + col;
                 p.ctu(row, col);
                 if (r.error) return false;
+                resolve_vectors(*p.o, col * 64, row * 64, W, H);
             }
         return true;
     };
@@ -333,8 +384,10 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
         cudaMemcpyAsync(d_rec, h_rec, sizeof(CtuOut) * nctu, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return TC_ERR_INTERNAL;
     for (size_t d = 0; d < diag_off.size(); ++d)
-        if (launch_decode_items(d_params, d_items + diag_off[d], diag_cnt[d], st) != cudaSuccess)
+        if (launch_decode_items(d_params, d_items + diag_off[d], diag_cnt[d], d_items + nctu, st) != cudaSuccess)
             return TC_ERR_INTERNAL;
+    if (cudaMemcpyAsync(h_status, d_items + nctu, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+        return TC_ERR_INTERNAL;
     }   // v2 stream
     // DPB: slot 3 falls out and its buffer takes a copy of the
     // reconstruction into slot 0 (another buffer when slot 3 is empty, taken
@@ -354,6 +407,10 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
         return TC_ERR_INTERNAL;
     dpb[0] = nf; dpb_ok[0] = 1; dpb_poc[0] = hdr.frame_num;
     if (!d2h(out, cur)) return TC_ERR_INTERNAL;
+    if (!legacy_stream && *h_status != 0) {   // an area gave up waiting
+        cudaMemset(d_items + rows * cols, 0, sizeof(int));
+        return TC_ERR_INTERNAL;
+    }
     const uint64_t t_rec = now_ns();
     if (profile) { prof[0] += t_parse1 - t_parse0; prof[2] += t_rec - t_parse1; }
     if (hdr.has_ext) {

@@ -101,10 +101,12 @@ __device__ __forceinline__ uint32_t ld4u(const uint8_t *p) {
     return __funnelshift_r(lo, __ldg(w + 1), (uint32_t)(a & 3) * 8);
 }
 
-__device__ __forceinline__ uint8_t &RY(Smem &S, int x, int y) {
+template <class T>
+__device__ __forceinline__ uint8_t &RY(T &S, int x, int y) {
     return S.rec_y[(y + RY_OY) * RY_W + x + RY_OX];
 }
-__device__ __forceinline__ uint8_t &RC(Smem &S, int c, int x, int y) {
+template <class T>
+__device__ __forceinline__ uint8_t &RC(T &S, int c, int x, int y) {
     return S.rec_c[c][(y + RC_OY) * RC_W + x + RC_OX];
 }
 
@@ -522,6 +524,17 @@ __device__ __forceinline__ void plane_pred(const MeTeam &T, const Planes &A, int
     }
 }
 
+// One interpolated luma sample (reference src/motion.c:269-304).
+__device__ __forceinline__ int mc_sample(const uint8_t *ref, int s, int W, int H, int fx, int fy, int dx, int dy) {
+    if (fx >= 2 && fx + 3 < W && fy >= 2 && fy + 3 < H) return luma_hv(ref, s, fx, fy, dx, dy);
+    if (fx >= 0 && fy >= 0 && fx + 1 < W && fy + 1 < H) {
+        const uint8_t *p = ref + (size_t)fy * s + fx;
+        return interp_qpel(interp_qpel(p[0], p[1], dx), interp_qpel(p[s], p[s + 1], dx), dy);
+    }
+    const int nx = clampi(fx + (dx >= 2 ? 1 : 0), 0, W - 1), ny = clampi(fy + (dy >= 2 ? 1 : 0), 0, H - 1);
+    return ref[(size_t)ny * s + nx];
+}
+
 // Luma prediction of a B x B block at the absolute quarter-sample vector
 // (mvx, mvy), sample by sample, by `nthr` threads (reference
 // src/motion.c:493-584); `avg` as in plane_pred.  The per-sample form with its
@@ -536,16 +549,7 @@ __device__ __noinline__ void mc_samples(int t, int nthr, const uint8_t *ref, int
 #pragma unroll 1
     for (int i = t; i < B * B; i += nthr) {
         const int fx = (mvx >> 2) + (i & (B - 1)), fy = (mvy >> 2) + (i >> lg);
-        int v;
-        if (fx >= 2 && fx + 3 < W && fy >= 2 && fy + 3 < H) {
-            v = luma_hv(ref, s, fx, fy, dx, dy);
-        } else if (fx >= 0 && fy >= 0 && fx + 1 < W && fy + 1 < H) {
-            const uint8_t *p = ref + (size_t)fy * s + fx;
-            v = interp_qpel(interp_qpel(p[0], p[1], dx), interp_qpel(p[s], p[s + 1], dx), dy);
-        } else {
-            const int nx = clampi(fx + (dx >= 2 ? 1 : 0), 0, W - 1), ny = clampi(fy + (dy >= 2 ? 1 : 0), 0, H - 1);
-            v = ref[(size_t)ny * s + nx];
-        }
+        const int v = mc_sample(ref, s, W, H, fx, fy, dx, dy);
         dst[i] = (uint8_t)(avg ? (v + dst[i] + 1) >> 1 : v);
     }
 }
@@ -766,17 +770,18 @@ __device__ __noinline__ void build_refs(const Leaf L) {
 // Intra prediction samples (x, y) and (x + 1, y) of an N x N leaf in the low
 // two bytes; disp is the mode's angular displacement (the per-sample form is
 // intra_at; reference src/predict.c:117-340).
-__device__ __forceinline__ uint32_t intra2(const Smem &S, int N, int mode, int disp, int x, int y) {
+__device__ __forceinline__ uint32_t intra2(const uint8_t (*edge)[EDGE_LEN], int above0, int dc, int N, int mode, int disp,
+                                           int x, int y) {
     if (mode == 0) {
-        const uint8_t *ra = S.edge[0] + EDGE_BASE;
-        const int sh = __ffs(N), l = S.edge[1][EDGE_BASE + y + 1], c = S.above0;
+        const uint8_t *ra = edge[0] + EDGE_BASE;
+        const int sh = __ffs(N), l = edge[1][EDGE_BASE + y + 1], c = above0;
         const int v0 = (ra[x + 1] * (N - 1 - y) + l * (N - 1 - x) + c * (x + y) + N) >> sh;
         const int v1 = (ra[x + 2] * (N - 1 - y) + l * (N - 2 - x) + c * (x + 1 + y) + N) >> sh;
         return (uint32_t)mini(v0, 255) | (uint32_t)mini(v1, 255) << 8;
     }
-    if (mode == 1 || mode > 17) return (uint32_t)S.dc * 0x101u;
+    if (mode == 1 || mode > 17) return (uint32_t)dc * 0x101u;
     const bool vert = mode < 9;
-    const uint8_t *E = S.edge[vert ? 0 : 1] + EDGE_BASE + 1;
+    const uint8_t *E = edge[vert ? 0 : 1] + EDGE_BASE + 1;
     const int p0 = vert ? (x << 5) + y * disp : (y << 5) + x * disp, p1 = p0 + (vert ? 32 : disp);
     const uint8_t *e0 = E + (p0 >> 5) + (p0 >> 31), *e1 = E + (p1 >> 5) + (p1 >> 31);
     const int a0 = e0[0], b0 = e0[1], a1 = e1[0], b1 = e1[1];
@@ -794,7 +799,7 @@ __device__ __forceinline__ int cl_entry(int slot, int sizes) {
 __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, int y) {
     const int slot = e & CL_SLOT;
     if (slot < NPRED) return *(const uint16_t *)(S.pred[slot] + y * cu + x);
-    return intra2(S, cu, slot - K_INTRA, e >> 16, x, y);
+    return intra2(S.edge, S.above0, S.dc, cu, slot - K_INTRA, e >> 16, x, y);
 }
 
 __device__ __forceinline__ QuantLane quant_lane(const Smem &S, int type, int lane) {
@@ -904,8 +909,8 @@ __device__ __noinline__ void luma_replay(const Leaf L, int e, int16_t *emit) {
 // At most 64 neighbour pairs of 8-bit samples: every sum and product stays
 // under 2^29 (n * sum(la * cv) <= 64 * 64 * 255^2), so 32-bit integers give
 // the reference's int64 values.
-__device__ __noinline__ void chroma_model(const Leaf L, int c) {
-    Smem &S = smem_state();
+template <class T>
+__device__ __forceinline__ ChromaModel chroma_stats(T &S, const Leaf L, int c) {
     const int cs = L.cu >> 1, lxc = L.lx >> 1, lyc = L.ly >> 1, lane = threadIdx.x & 31;
     const bool up = L.py > 0, left = L.px > 0;
     int sl = 0, sc = 0, slc = 0, sl2 = 0;
@@ -927,18 +932,37 @@ __device__ __noinline__ void chroma_model(const Leaf L, int c) {
     sc = (int)__reduce_add_sync(0xffffffffu, (unsigned)sc);
     slc = (int)__reduce_add_sync(0xffffffffu, (unsigned)slc);
     sl2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)sl2);
-    if (lane == 0) {
-        const int cov = n * slc - sl * sc, vl = n * sl2 - sl * sl;
-        int ash = 3;
-        if (n > 0 && vl > 0 && cov != 0) {
-            const unsigned q = (unsigned)vl / (unsigned)(cov < 0 ? -cov : cov);
-            const int sh = q < 1 ? 2 : 31 - __clz((int)q);
-            ash = sh < 2 ? 2 : (sh > 5 ? 5 : sh);
-        }
-        S.cdc[c] = n ? (sc + n / 2) >> lg2i(n) : 128;   // n: cs or 2 cs
-        S.cfl_sign[c] = cov >= 0 ? 1 : -1;
-        S.cfl_shift[c] = ash;
+    const int cov = n * slc - sl * sc, vl = n * sl2 - sl * sl;
+    int ash = 3;
+    if (n > 0 && vl > 0 && cov != 0) {
+        const unsigned q = (unsigned)vl / (unsigned)(cov < 0 ? -cov : cov);
+        const int sh = q < 1 ? 2 : 31 - __clz((int)q);
+        ash = sh < 2 ? 2 : (sh > 5 ? 5 : sh);
     }
+    return {n ? (sc + n / 2) >> lg2i(n) : 128, cov >= 0 ? 1 : -1, ash};   // n: cs or 2 cs
+}
+__device__ __noinline__ void chroma_model(const Leaf L, int c) {
+    Smem &S = smem_state();
+    const ChromaModel m = chroma_stats(S, L, c);
+    if ((threadIdx.x & 31) == 0) S.cmodel[c] = m;
+}
+
+// CfL prediction of chroma samples (x, y), (x + 1, y) of a leaf: the model's DC
+// plus the scaled difference of the collocated luma from the mean of the 4x4
+// tile, whose eight lanes (index bits 0, 2 and 3) call this together.
+template <class T>
+__device__ __forceinline__ uint32_t cfl_pair(T &S, const Leaf &L, const ChromaModel &M, int x, int y) {
+    const uint32_t l0 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y);
+    const uint32_t l1 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y + 1);
+    const int a0 = (int)__dp4a(l0, 0x0101u, __dp4a(l1, 0x0101u, 2u)) >> 2;
+    const int a1 = (int)__dp4a(l0, 0x01010000u, __dp4a(l1, 0x01010000u, 2u)) >> 2;
+    int m = a0 + a1;
+    m += __shfl_xor_sync(0xffffffffu, m, 1);
+    m += __shfl_xor_sync(0xffffffffu, m, 4);
+    m += __shfl_xor_sync(0xffffffffu, m, 8);
+    m = (m + 8) >> 4;
+    return (uint32_t)__viaddmin_s32_relu(M.dc, M.sign * ((a0 - m) >> M.shift), 255) |
+           (uint32_t)__viaddmin_s32_relu(M.dc, M.sign * ((a1 - m) >> M.shift), 255) << 8;
 }
 
 // A leaf's chroma prediction: DC, CfL (DC plus the scaled difference of the
@@ -974,22 +998,11 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
         const int o = j >> (2 * ln + 1), c = (j >> (2 * ln)) & 1, t = j & ((1 << (2 * ln)) - 1);
         const int x = (t & ((1 << ln) - 1)) * 4 + cc, y = (t >> ln) * 4 + r;
         const uint32_t cv = *(const uint16_t *)(S.cur_c[c] + (lyc + y) * 32 + lxc + x);
-        uint32_t pv = (uint32_t)S.cdc[c] * 0x101u;
+        const ChromaModel M = S.cmodel[c];
+        uint32_t pv = (uint32_t)M.dc * 0x101u;
         if (K.kind == CH_CFL || nopt == 2) {
-            const uint32_t l0 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y);
-            const uint32_t l1 = *(const uint32_t *)&RY(S, L.lx + 2 * x, L.ly + 2 * y + 1);
-            const int a0 = (int)__dp4a(l0, 0x0101u, __dp4a(l1, 0x0101u, 2u)) >> 2;
-            const int a1 = (int)__dp4a(l0, 0x01010000u, __dp4a(l1, 0x01010000u, 2u)) >> 2;
-            int m = a0 + a1;
-            m += __shfl_xor_sync(0xffffffffu, m, 1);
-            m += __shfl_xor_sync(0xffffffffu, m, 4);
-            m += __shfl_xor_sync(0xffffffffu, m, 8);
-            m = (m + 8) >> 4;
-            if (K.kind == CH_CFL || o == 1) {
-                const int dc = S.cdc[c], sg = S.cfl_sign[c], sh = S.cfl_shift[c];
-                pv = (uint32_t)__viaddmin_s32_relu(dc, sg * ((a0 - m) >> sh), 255) |
-                     (uint32_t)__viaddmin_s32_relu(dc, sg * ((a1 - m) >> sh), 255) << 8;
-            }
+            const uint32_t v = cfl_pair(S, L, M, x, y);
+            if (K.kind == CH_CFL || o == 1) pv = v;
         }
         if (K.kind == CH_MC && o == 0) {
             const int Wc = P.W >> 1, Hc = P.H >> 1;
@@ -1026,104 +1039,6 @@ __device__ __noinline__ void chroma_areas(const Leaf L, int nopt, const ChromaPr
             *(uint32_t *)(emit + c * cs * cs + t * 16 + r * 4 + cc) = a.levels();
         }
     }
-}
-
-// Chroma DC predictor (reference src/predict.c:364-379) into cpred[dst+c].
-__device__ __noinline__ void chroma_dc_pred(Smem &, const Leaf L, int dst) {
-    Smem &S = smem_state();
-    const int cs = L.cu >> 1, lxc = L.lx >> 1, lyc = L.ly >> 1;
-    const bool ha = L.py > 0, hl = L.px > 0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp < 2) {
-        const int c = warp;
-        int sum = 0;
-        for (int i = lane; i < cs; i += 32) {
-            if (ha) sum += RC(S, c, lxc + i, lyc - 1);
-            if (hl) sum += RC(S, c, lxc - 1, lyc + i);
-        }
-        sum = __reduce_add_sync(0xffffffffu, sum);
-        const int n = (ha ? cs : 0) + (hl ? cs : 0);
-        if (lane == 0) S.sao[c] = n ? (sum + n / 2) >> lg2i(n) : 128;   // n: cs or 2 cs
-    }
-    SYNC();
-    const int lg2 = 2 * lg2i(cs);
-    for (int i = threadIdx.x; i < 2 * cs * cs; i += NT) {
-        const int c = i >> lg2;
-        S.cpred[dst + c][i & ((1 << lg2) - 1)] = (uint8_t)S.sao[c];
-    }
-    SYNC();
-}
-
-// Chroma-from-luma blend over the DC prediction in cpred[dst+c]
-// (reference src/predict.c:390-462), reading fresh reconstructed luma.
-__device__ __noinline__ void cfl_blend(Smem &, const Leaf L, int dst) {
-    Smem &S = smem_state();
-    const int cs = L.cu >> 1, lxc = L.lx >> 1, lyc = L.ly >> 1;
-    const bool up = L.py > 0, left = L.px > 0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int s_sign[2], s_shift[2];
-    if (warp < 2) {
-        // At most 64 neighbour pairs of 8-bit samples: every sum and product
-        // below stays under 2^29 (n * sum(la * cv) <= 64 * 64 * 255^2), so
-        // 32-bit integers give the reference's int64 values.
-        const int c = warp;
-        int sl = 0, sc = 0, slc = 0, sl2 = 0;
-        for (int i = lane; i < cs; i += 32) {
-            if (up) {
-                const int la = (RY(S, L.lx + 2 * i, L.ly - 1) + RY(S, L.lx + 2 * i + 1, L.ly - 1) + 1) >> 1;
-                const int cv = RC(S, c, lxc + i, lyc - 1);
-                sl += la; sc += cv; slc += la * cv; sl2 += la * la;
-            }
-            if (left) {
-                const int la = (RY(S, L.lx - 2, L.ly + 2 * i) + RY(S, L.lx - 1, L.ly + 2 * i) +
-                                RY(S, L.lx - 2, L.ly + 2 * i + 1) + RY(S, L.lx - 1, L.ly + 2 * i + 1) + 2) >> 2;
-                const int cv = RC(S, c, lxc - 1, lyc + i);
-                sl += la; sc += cv; slc += la * cv; sl2 += la * la;
-            }
-        }
-        const int n = (up ? cs : 0) + (left ? cs : 0);
-        sl = (int)__reduce_add_sync(0xffffffffu, (unsigned)sl);
-        sc = (int)__reduce_add_sync(0xffffffffu, (unsigned)sc);
-        slc = (int)__reduce_add_sync(0xffffffffu, (unsigned)slc);
-        sl2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)sl2);
-        if (lane == 0) {
-            const int sign = (n == 0 || n * slc >= sl * sc) ? 1 : -1;
-            int ash = 3;
-            const int cov = n * slc - sl * sc, vl = n * sl2 - sl * sl;
-            if (n > 0 && vl > 0 && cov != 0) {
-                const unsigned q = (unsigned)vl / (unsigned)(cov < 0 ? -cov : cov);
-                const int sh = q < 1 ? 2 : 31 - __clz((int)q);
-                ash = sh < 2 ? 2 : (sh > 5 ? 5 : sh);
-            }
-            s_sign[c] = sign;
-            s_shift[c] = ash;
-        }
-    }
-    // The 2x2-averaged collocated luma of every chroma position, then its
-    // mean per 4x4 chroma tile, into the residual jobs' scratch (idle here).
-    const int nt = cs >> 2, lgs = lg2i(cs), lgt = lgs - 2;
-    int *la = &S.scratch[0][0];              // cs * cs entries
-    int *tile = la + 32 * 32;                // nt * nt entries
-    for (int i = threadIdx.x; i < cs * cs; i += NT) {
-        const int X = L.lx + 2 * (i & (cs - 1)), Y = L.ly + 2 * (i >> lgs);
-        la[i] = (RY(S, X, Y) + RY(S, X + 1, Y) + RY(S, X, Y + 1) + RY(S, X + 1, Y + 1) + 2) >> 2;
-    }
-    SYNC();
-    for (int t = threadIdx.x; t < nt * nt; t += NT) {
-        const int *q = la + ((t >> lgt) << 2) * cs + ((t & (nt - 1)) << 2);
-        int sum = 0;
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy) sum += q[yy * cs] + q[yy * cs + 1] + q[yy * cs + 2] + q[yy * cs + 3];
-        tile[t] = (sum + 8) >> 4;            // sum >= 0
-    }
-    SYNC();
-    for (int i = threadIdx.x; i < 2 * cs * cs; i += NT) {
-        const int c = i >> (2 * lgs), p = i & ((1 << (2 * lgs)) - 1), y = p >> lgs, x = p & (cs - 1);
-        const int avg = tile[(y >> 2) * nt + (x >> 2)];
-        uint8_t &d = S.cpred[dst + c][p];
-        d = (uint8_t)clampi((int)d + s_sign[c] * ((la[p] - avg) >> s_shift[c]), 0, 255);
-    }
-    SYNC();
 }
 
 // Chroma MC of both components into cpred[dst+c] (or straight into the
@@ -1260,22 +1175,6 @@ __device__ __forceinline__ int dpb_bwd(const FrameParams &P) {
     for (int i = 0; i < MAX_REFS; ++i)
         if (P.ref_valid[i] && P.ref_poc[i] >= 0 && P.ref_poc[i] > P.poc && P.ref_poc[i] < bp) { bp = P.ref_poc[i]; best = i; }
     return best;
-}
-
-// Chroma MC of both components, averaged over two references when r2 >= 0
-// (second reference with the mirrored MV; reference src/encoder.c:673-699).
-__device__ __noinline__ void chroma_mc_bi(Smem &, const FrameParams &, const Leaf L, int r1, int r2, int mvx, int mvy) {
-    Smem &S = smem_state();
-    const FrameParams &P = g_fp;
-    const int cs = L.cu >> 1, Wc = P.W >> 1, Hc = P.H >> 1, lgs = lg2i(cs);
-    for (int i = threadIdx.x; i < 2 * cs * cs; i += NT) {
-        const int c = i >> (2 * lgs), p = i & ((1 << (2 * lgs)) - 1), y = p >> lgs, x = p & (cs - 1);
-        int v = chroma_mc_at(c ? P.ref_cr[r1] : P.ref_cb[r1], P.stride_c, Wc, Hc, mvx, mvy, x, y);
-        if (r2 >= 0)
-            v = (v + chroma_mc_at(c ? P.ref_cr[r2] : P.ref_cb[r2], P.stride_c, Wc, Hc, -mvx, -mvy, x, y) + 1) >> 1;
-        S.cpred[c][p] = (uint8_t)v;
-    }
-    SYNC();
 }
 
 // ====================================================================
@@ -1725,8 +1624,8 @@ __device__ __noinline__ void close_gaps(int ctu_x, int ctu_y, CtuOut *out) {
 // ====================================================================
 // In-loop filters on the CTU tile.
 // ====================================================================
-__device__ __noinline__ void deblock_tile(Smem &, int qp) {
-    Smem &S = smem_state();
+template <class T>
+__device__ __forceinline__ void deblock_on(T &S, int qp) {
     const int tc = clampi(qp / 3, 1, 10);
     const int cqp = clampi(qp - 1, 0, 63), ctc = clampi(cqp / 4, 1, 6);
     // Luma vertical edges x = 4..60 and chroma (Cb) vertical edges x = 4..28.
@@ -1775,6 +1674,8 @@ __device__ __noinline__ void deblock_tile(Smem &, int qp) {
     }
     SYNC();
 }
+
+__device__ __noinline__ void deblock_tile(Smem &, int qp) { deblock_on(smem_state(), qp); }
 
 // Luma SAO band offset: choose (reference src/filter.c:269-319), rate gate
 // (src/encoder.c:1473-1493) and apply (src/filter.c:251-266).
@@ -2264,292 +2165,7 @@ tc_error_t tcb_debug_ctu_encode_frame_without_first(const tcb_frame_desc_t *desc
 
 }  // extern "C"
 
-// ====================================================================
-// Decoder reconstruction (reference src/decoder.c:1521-1816): the same
-// wavefront of CTAs rebuilds each CTU from its parsed record — prediction
-// exactly as the encoder's write pass, residual from the transmitted
-// levels.  Levels come from an arbitrary bitstream, so the second inverse
-// pass accumulates in 64 bits.
-// ====================================================================
-namespace tcb {
-
-__device__ __forceinline__ int dq_eff(const int *eff, int pos, int n) {
-    return eff[freq_band(pos, n)];
-}
-
-// 8x8 TU from levels on an octet; writes pred + residual into the tile.
-__device__ void dec_luma8(Smem &S, const Leaf &L, const int16_t *lv, const int *qp) {
-    const int cu = L.cu, ntu = cu >> 3, J = ntu * ntu;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, oct = lane >> 3, l8 = lane & 7;
-    int *scr = S.scratch[warp] + oct * 64;
-    for (int base = 0; base < J; base += NW * 4) {
-        const int t = base + warp * 4 + oct;
-        const int t0 = t < J ? t : 0, ty0 = t0 / ntu, tx0 = t0 - ty0 * ntu;
-        const bool act = t < J && ((S.tu8mask >> ((L.cy + ty0) * 8 + L.cx + tx0)) & 1);
-        const int tt = act ? t : 0, ty = tt / ntu, tx = tt - ty * ntu;
-        int row[8];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            const int pos = l8 * 8 + n;
-            row[n] = (int16_t)dequant_coeff(act ? lv[tt * 64 + pos] : 0, dq_eff(qp, pos, 64));
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            int acc = 0;
-#pragma unroll
-            for (int n = 0; n < 8; ++n) acc += c_dct8[n][k] * row[n];
-            scr[l8 * 8 + k] = (acc + 8192) >> 14;
-        }
-        __syncwarp();
-        long long col[8];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) col[n] = scr[n * 8 + l8];
-        __syncwarp();
-        const int x = tx * 8 + l8;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            long long acc = 0;
-#pragma unroll
-            for (int n = 0; n < 8; ++n) acc += (long long)c_dct8[n][k] * col[n];
-            const int r = (int16_t)(int)((acc + 8192) >> 14);
-            const int y = ty * 8 + k;
-            if (act) RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(S.pred[0][y * cu + x] + r, 0, 255);
-        }
-    }
-}
-
-// 4x4 TUs from levels on quads.  Luma: per 8x8 TU four sub-blocks in
-// raster order; chroma (chroma_c >= 0): (cs/4)^2 TUs of that component.
-__device__ void dec_tu4(Smem &S, const Leaf &L, int chroma_c, const int16_t *lv,
-                        const int *qp) {
-    const int cu = L.cu;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, l4 = lane & 3;
-    int *scr = S.scratch[warp] + qd * 16;
-    const int cs = cu >> 1;
-    const int J = chroma_c >= 0 ? (cs >> 2) * (cs >> 2) : (cu >> 3) * (cu >> 3) * 4;
-    for (int base = 0; base < J; base += NW * 8) {
-        const int j = base + warp * 8 + qd;
-        bool act = j < J;
-        if (act && chroma_c < 0) {
-            const int ntu = cu >> 3, t = j >> 2;
-            act = !((S.tu8mask >> ((L.cy + t / ntu) * 8 + L.cx + t % ntu)) & 1);
-        }
-        const int jj = act ? j : 0;
-        int sx, sy;
-        if (chroma_c >= 0) {
-            const int nt = cs >> 2, ty = jj / nt, tx = jj - ty * nt;
-            sx = tx * 4; sy = ty * 4;
-        } else {
-            const int ntu = cu >> 3, t = jj >> 2, q = jj & 3, ty = t / ntu, tx = t - ty * ntu;
-            sx = tx * 8 + (q & 1) * 4; sy = ty * 8 + (q & 2) * 2;
-        }
-        int row[4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int pos = l4 * 4 + n;
-            row[n] = (int16_t)dequant_coeff(act ? lv[jj * 16 + pos] : 0, dq_eff(qp, pos, 16));
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            int acc = 0;
-#pragma unroll
-            for (int n = 0; n < 4; ++n) acc += c_dct4[n][k] * row[n];
-            scr[l4 * 4 + k] = (acc + 8192) >> 14;
-        }
-        __syncwarp();
-        long long col[4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) col[n] = scr[n * 4 + l4];
-        __syncwarp();
-        const int x = sx + l4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            long long acc = 0;
-#pragma unroll
-            for (int n = 0; n < 4; ++n) acc += (long long)c_dct4[n][k] * col[n];
-            const int r = (int16_t)(int)((acc + 8192) >> 14);
-            const int y = sy + k;
-            if (!act) continue;
-            if (chroma_c >= 0) {
-                const int v = clampi((int)S.cpred[chroma_c][y * cs + x] + r, 0, 255);
-                RC(S, chroma_c, (L.lx >> 1) + x, (L.ly >> 1) + y) = (uint8_t)v;
-            } else {
-                RY(S, L.lx + x, L.ly + y) = (uint8_t)clampi(S.pred[0][y * cu + x] + r, 0, 255);
-            }
-        }
-    }
-}
-
-// Decoder prediction reference choice (reference src/decoder.c:1628-1664,
-// 1697-1750); `flat` = no reference (128 / chroma DC).
-__device__ void dec_leaf(Smem &S, const FrameParams &P, const Leaf &L, const int16_t *coef,
-                         const int *ql, const int *qc) {
-    const Node nd = S.nodes[qt_index(L.depth, L.cx, L.cy)];
-    int mvpx, mvpy;
-    mvp_at(S.grid, L.cx, L.cy, mvpx, mvpy);
-    const int cu = L.cu;
-    const int16_t *el = coef + S.ncoef, *ec = el + cu * cu;
-    const bool use_mvd = !(nd.skip || nd.merge || nd.intra);
-    const int mvx = (int16_t)(mvpx + L.px * 4 + (use_mvd ? nd.mvd_x : 0));
-    const int mvy = (int16_t)(mvpy + L.py * 4 + (use_mvd ? nd.mvd_y : 0));
-    const bool bidir = P.frame_type == 2;
-    if (nd.intra) {
-        build_refs(L);
-        const int lg = lg2i(cu) - 1;
-        for (int i = threadIdx.x; i < cu * cu / 2; i += NT)
-            *(uint16_t *)(S.pred[0] + 2 * i) =
-                (uint16_t)pred2(S, cu, cl_entry(K_INTRA + nd.intra_mode, 0), 2 * (i & (cu / 2 - 1)), i >> lg);
-        SYNC();
-    } else {
-        int r1 = -1, r2 = -1;
-        if (bidir) {
-            const int rf = dpb_fwd(P), rb = dpb_bwd(P);
-            if ((nd.bi || nd.skip) && rf >= 0 && rb >= 0) { r1 = rf; r2 = rb; }
-            else {
-                int r = nd.bi ? rf : (nd.ref_sel ? rb : rf);
-                if (r < 0) r = rf >= 0 ? rf : rb;
-                r1 = r;
-            }
-        } else {
-            r1 = (nd.ref_sel < MAX_REFS && P.ref_valid[nd.ref_sel]) ? nd.ref_sel : -1;
-        }
-        if (r1 >= 0) {
-            luma_mc(S, L, P.ref_y[r1], r2 >= 0 ? P.ref_y[r2] : nullptr, mvx, mvy);
-        } else {
-            for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
-            SYNC();
-        }
-    }
-    if (nd.skip) {
-        for (int i = threadIdx.x; i < cu * cu; i += NT) {
-            const int y = i / cu, x = i - y * cu;
-            RY(S, L.lx + x, L.ly + y) = S.pred[0][i];
-        }
-        SYNC();
-        if (P.fresh_skip && P.frame_type == 1 && P.ref_valid[0]) chroma_mc(S, P, L, 0, mvx, mvy, 0, true);
-        grid_update(S, L, nd, mvpx, mvpy);
-        return;
-    }
-    // Luma residual: each 8x8 region carries its own TU-size flag.
-    dec_luma8(S, L, el, ql);
-    dec_tu4(S, L, -1, el, ql);
-    SYNC();
-    // Chroma prediction.
-    if (nd.intra) {
-        if (nd.ch_intra) { chroma_dc_pred(S, L, 0); cfl_blend(S, L, 0); }
-        else if (P.ref_valid[0]) chroma_mc(S, P, L, 0, mvx, mvy, 0, false);
-        else chroma_dc_pred(S, L, 0);
-    } else if (bidir && nd.bi) {
-        const int cf = dpb_fwd(P), cbw = dpb_bwd(P);
-        if (cf >= 0 && cbw >= 0) chroma_mc_bi(S, P, L, cf, cbw, mvx, mvy);
-        else if (cf >= 0 || cbw >= 0) chroma_mc_bi(S, P, L, cf >= 0 ? cf : cbw, -1, mvx, mvy);
-        else chroma_dc_pred(S, L, 0);
-    } else {
-        int r = (nd.ref_sel < MAX_REFS && P.ref_valid[nd.ref_sel]) ? nd.ref_sel : -1;
-        if (bidir) r = nd.ref_sel ? dpb_bwd(P) : dpb_fwd(P);
-        if (r >= 0) chroma_mc_bi(S, P, L, r, -1, mvx, mvy);
-        else chroma_dc_pred(S, L, 0);
-    }
-    dec_tu4(S, L, 0, ec, qc);
-    dec_tu4(S, L, 1, ec + (cu >> 1) * (cu >> 1), qc);
-    SYNC();
-    if (threadIdx.x == 0) S.ncoef += cu * cu + (cu * cu >> 1);
-    grid_update(S, L, nd, mvpx, mvpy);
-}
-
-template <int D>
-__device__ void qt_dec(Smem &S, const FrameParams &P, int ctu_x, int ctu_y, int cx, int cy,
-                       const int16_t *coef, const int *ql, const int *qc) {
-    constexpr int cu = 64 >> D;
-    const int px = ctu_x + cx * 8, py = ctu_y + cy * 8;
-    const bool in_frame = px + cu <= P.W && py + cu <= P.H;
-    if constexpr (D < 3) {
-        constexpr int h = 4 >> D;
-        if (!in_frame || S.nodes[qt_index(D, cx, cy)].split) {
-            for (int q = 0; q < 4; ++q)
-                qt_dec<D + 1>(S, P, ctu_x, ctu_y, cx + (q & 1) * h, cy + (q >> 1) * h, coef, ql, qc);
-            return;
-        }
-    } else {
-        if (!in_frame) return;
-    }
-    const Leaf L(P, ctu_x, ctu_y, D, cx, cy);
-    dec_leaf(S, P, L, coef, ql, qc);
-}
-
-__global__ void __launch_bounds__(NT, CTAS_PER_SM)
-decode_kernel(const FrameParams *__restrict__ params, const int *__restrict__ items) {
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    Smem &S = *reinterpret_cast<Smem *>(smem_raw);
-    FrameParams &P = g_fp;   // the shared helpers (MC, chroma) read the frame from g_fp
-    const int item = items[blockIdx.x];
-    const int sid = item >> 20, row = (item >> 10) & 1023, col = item & 1023;
-    if (threadIdx.x == 0) P = params[sid];
-    SYNC();
-    const int ctu_x = col * 64, ctu_y = row * 64;
-    const int w = mini(64, P.W - ctu_x), h = mini(64, P.H - ctu_y);
-    const int wc = w >> 1, hc = h >> 1;
-    const CtuOut *rec = P.out + row * P.ctu_cols + col;
-    // Border from the frame being rebuilt; interior starts from the
-    // persistent reconstruction buffer (stale samples are only ever read
-    // by streams that skip with stale chroma, as in the reference).
-    for (int i = threadIdx.x; i < 65 * 66; i += NT) {
-        const int y = i / 66 - 1, x = i % 66 - 2;
-        if (ctu_y + y >= 0 && ctu_x + x >= 0 && y < h && x < w)
-            RY(S, x, y) = P.rec_y[(size_t)(ctu_y + y) * P.stride_y + ctu_x + x];
-    }
-    for (int i = threadIdx.x; i < 2 * 33 * 33; i += NT) {
-        const int c = i / (33 * 33), p = i - c * 33 * 33, y = p / 33 - 1, x = p % 33 - 1;
-        const uint8_t *src = c ? P.rec_cr : P.rec_cb;
-        if ((ctu_y >> 1) + y >= 0 && (ctu_x >> 1) + x >= 0 && y < hc && x < wc)
-            RC(S, c, x, y) = src[(size_t)((ctu_y >> 1) + y) * P.stride_c + (ctu_x >> 1) + x];
-    }
-    for (int i = threadIdx.x; i < 64; i += NT) {
-        S.grid[i].dx = 0; S.grid[i].dy = 0; S.grid[i].intra = 1; S.grid[i].pad = 0;
-    }
-    for (int i = threadIdx.x; i < QT_NODES; i += NT) S.nodes[i] = rec->nodes[i];
-    if (threadIdx.x == 0) { S.ncoef = 0; S.tu8mask = rec->tu8mask; }
-    SYNC();
-    if (threadIdx.x < 8) S.eff[threadIdx.x >> 2][threadIdx.x & 3] = threadIdx.x < 4 ? P.eff_l[threadIdx.x] : P.eff_c[threadIdx.x & 3];
-    SYNC();
-    const int *ql = S.eff[0], *qc = S.eff[1];
-    qt_dec<0>(S, P, ctu_x, ctu_y, 0, 0, rec->coef, ql, qc);
-    SYNC();
-    if (w == 64 && h == 64) deblock_tile(S, P.qp);
-    if (rec->sao_has) {
-        const int band = clampi(rec->sao_band, 0, 31), off = clampi(rec->sao_offset, -7, 7);
-        for (int i = threadIdx.x; i < w * h; i += NT) {
-            const int y = div_p2(i, w), x = i - y * w;
-            uint8_t &p = RY(S, x, y);
-            if ((p >> 3) == band) p = (uint8_t)clampi(p + off, 0, 255);
-        }
-        SYNC();
-    }
-    for (int i = threadIdx.x; i < w * h; i += NT) {
-        const int y = div_p2(i, w), x = i - y * w;
-        P.rec_y[(size_t)(ctu_y + y) * P.stride_y + ctu_x + x] = RY(S, x, y);
-    }
-    for (int i = threadIdx.x; i < 2 * wc * hc; i += NT) {
-        const int c = div_p2(i, wc * hc), p = i - c * wc * hc, y = div_p2(p, wc), x = p - y * wc;
-        uint8_t *dst = c ? P.rec_cr : P.rec_cb;
-        dst[(size_t)((ctu_y >> 1) + y) * P.stride_c + (ctu_x >> 1) + x] = RC(S, c, x, y);
-    }
-}
-
-cudaError_t init_decode_tables() {
-    return cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(Smem));
-}
-
-cudaError_t launch_decode_items(const FrameParams *d_params, const int *d_items, int n,
-                                cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    decode_kernel<<<n, NT, sizeof(Smem), st>>>(d_params, d_items);
-    return cudaGetLastError();
-}
-
-}  // namespace tcb
-
+#include "tcb_decode.cuh"
 #include "tcb_legacy_enc.cuh"
 
 #ifdef TCB_PHASE_PROFILE

@@ -66,6 +66,11 @@ constexpr int PLANE_WORDS = PLANES64 * plane_words(64);
 static_assert(NGROUP * plane_words(32) <= PLANE_WORDS && NGROUP * plane_words(16) <= PLANE_WORDS,
               "every group's planes fit below 64x64");
 
+// Chroma DC value and chroma-from-luma model of a leaf's component.
+struct ChromaModel {
+    int dc, sign, shift;
+};
+
 struct Smem {
     alignas(16) uint8_t cur_y[64 * 64];
     uint8_t cur_c[2][32 * 32];
@@ -83,12 +88,11 @@ struct Smem {
     union {
         // after the searches of a leaf
         struct {
-            // chroma predictions (decoder, skip check), or the two chroma
+            // chroma predictions (skip check), or the two chroma
             // options of an intra leaf: reconstruction and levels of option o,
             // component c in [2 * o + c]
             alignas(16) uint8_t cpred[4][32 * 32];
             int16_t clev[4][32 * 32];
-            int scratch[NW][256];     // decoder: rows of 4 octets x 64 or 8 quads x 16 ints per warp
         };
         // during them: sample planes
         alignas(16) uint32_t plane[PLANE_WORDS];
@@ -98,11 +102,10 @@ struct Smem {
     uint2 frag[4][32];        // transform fragments per lane: forward 8x8, inverse 8x8, forward 4x4, inverse 4x4
     MeGroup me[NGROUP];
     float4 quant[3][3][32];   // QuantLane parts per lane: luma 8x8, luma 4x4, chroma 4x4
-    int eff[2][4];            // decoder: quantiser steps of luma, chroma
     int win_slot;              // candidate slot of the last scan's winner (-1: skip)
     int acc[NCAND][2][2];      // per slot and TU size (8x8, 4x4): distortion, bits
     int cacc[2][2];            // per chroma option: distortion, bits
-    int cdc[2], cfl_sign[2], cfl_shift[2];   // chroma DC and CfL model of the current leaf, per component
+    ChromaModel cmodel[2];     // chroma DC and CfL model of the current leaf, per component
     uint16_t zoff[64];         // coded 8x8 cells before each cell of the CTU in z-order
     uint8_t leaf_skip[64];     // the cell's leaf is skipped
     int last_bits[65];         // last_bits(last) by last + 1

@@ -1,9 +1,9 @@
 """The encoder's residual path at the ends of its ranges: saturated
 residuals (0 against 255), flat pictures, and quantiser steps from 1 (level =
 coefficient) to above every coefficient, with leaves of every size and both
-TU sizes.  The decoder rebuilds every picture from the packets through its
-own transforms (64-bit second pass, no matrix instructions), so its pictures
-must equal the encoder's reconstructions sample for sample."""
+TU sizes.  The decoder rebuilds every picture from the packets, so its pictures
+must equal the encoder's reconstructions sample for sample (its transforms
+are checked against 64-bit integers in test_gpu_decode_areas.py)."""
 import numpy as np
 import pytest
 
