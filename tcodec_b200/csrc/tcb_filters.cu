@@ -15,15 +15,15 @@
 // read once and written at most once.  Deblocking filters two edge
 // positions per instruction on packed 16-bit lanes (tcb_deblock_pairs.cuh).
 //
-// SAO statistics without atomics: every thread owns two 16-pixel row
-// segments (kept in registers for the whole CTU) and a private column of a
-// [row][thread] table in shared memory, so its read-modify-writes never
-// conflict.  A table word packs count and difference sum as
-// count * 65536 + sum of (256 + o - r), which one integer add per pixel
-// maintains exactly (tcb_sao_decide.cuh: SAO_BIAS, sao_unpack); the rows and increments of a
+// SAO statistics: the CTA keeps a [row][32] table in shared memory, column =
+// lane, and every sample adds one word with a shared-memory add that returns
+// nothing.  The lanes of a warp always hit different banks, and a column takes
+// the 128 samples of one lane of each warp.  A word packs count and difference
+// sum as count * 65536 + sum of (256 + o - r), exact for 128 samples
+// (tcb_sao_decide.cuh: SAO_BIAS); the rows and increments of a
 // word's four pixels come from a few word operations (sao_rows4,
-// sao_incr4), leaving a lane extract, an address and the read-modify-write
-// per pixel.  Rows are the 30 inner bands plus the 16 single
+// sao_incr4), leaving a lane extract, an address and the add per pixel.  Rows
+// are the 30 inner bands plus the 16 single
 // sample values of bands 0 and 31, where an offset can clip; the SSE of
 // every band after its offset then follows in closed form, clipping
 // included (tcb_sao_decide.cuh), with no second pass over the pixels.
@@ -44,8 +44,7 @@ namespace tcb {
 namespace {
 
 // Threads per CTA (one CTU each) are a template parameter: deblocking 64,
-// 128 or 256, SAO 64 or 128 (its statistics table holds one column per
-// thread; 256 would pass the 48 KB of static shared memory); the autotuner
+// 128 or 256, SAO 64 or 128; the autotuner
 // times each per frame size, 128 without tuning.  Small
 // CTAs let many CTUs' loads be in flight per SM while other CTUs of the
 // same SM filter.
@@ -62,6 +61,19 @@ __device__ __forceinline__ int find_frame(const int *off, int n, int g) {
     return lo;
 }
 
+// The frame and CTU of this CTA.  Frames of one size are launched as a grid
+// (columns, rows, frames), which needs neither the search nor a division;
+// other groups as one row of CTAs (grid3 0).
+struct CtuAt {
+    int k, x, y;
+};
+template <class Cols>
+__device__ __forceinline__ CtuAt ctu_at(const int *off, int n, int grid3, Cols cols_of) {
+    if (grid3) return {(int)blockIdx.z, (int)blockIdx.x, (int)blockIdx.y};
+    const int k = find_frame(off, n, blockIdx.x), local = blockIdx.x - off[k], cols = cols_of(k);
+    return {k, local % cols, local / cols};
+}
+
 __device__ __forceinline__ bool aligned16(const void *p, int stride) {
     return (((uintptr_t)p) & 15) == 0 && (stride & 15) == 0;
 }
@@ -74,10 +86,9 @@ __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
     constexpr int NPIECE = (384 + DFT - 1) / DFT;   // 16-byte pieces per thread (384 per CTU)
     __shared__ __align__(16) uint8_t ty[64 * 64];
     __shared__ __align__(16) uint8_t tc[2][32 * 32];
-    const int k = find_frame(J.ctu_off, J.n, blockIdx.x);
-    const DeblockFrame &F = J.f[k];
-    const int local = blockIdx.x - J.ctu_off[k], cols = F.W >> 6;
-    const int x0 = (local % cols) << 6, y0 = (local / cols) << 6;
+    const CtuAt at = ctu_at(J.ctu_off, J.n, J.grid3, [&](int k) { return J.f[k].W >> 6; });
+    const DeblockFrame &F = J.f[at.k];
+    const int x0 = at.x << 6, y0 = at.y << 6;
     const int t = threadIdx.x;
     uint8_t *gy = F.y + (size_t)y0 * F.sy + x0;
     uint8_t *const gcb = F.cb + (size_t)(y0 >> 1) * F.sc + (x0 >> 1), *const gcr = F.cr + (size_t)(y0 >> 1) * F.sc + (x0 >> 1);
@@ -159,7 +170,7 @@ __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
 struct DeblockTmaJobs {            // passed as a __grid_constant__ kernel parameter (about 12.7 KB)
     static constexpr int MAX = 32;
     CUtensorMap ty[MAX], tcb[MAX], tcr[MAX];
-    int n;
+    int n, grid3;
     int ctu_off[MAX + 1];
     int cols[MAX], qp[MAX];
 };
@@ -189,9 +200,8 @@ __global__ void __launch_bounds__(DFT) deblock_tma_kernel(const __grid_constant_
     __shared__ __align__(128) uint8_t ty[64 * 64];
     __shared__ __align__(128) uint8_t tc[2][32 * 32];
     __shared__ __align__(8) uint64_t bar;
-    const int k = find_frame(J.ctu_off, J.n, blockIdx.x);
-    const int local = blockIdx.x - J.ctu_off[k];
-    const int x0 = (local % J.cols[k]) << 6, y0 = (local / J.cols[k]) << 6;
+    const CtuAt at = ctu_at(J.ctu_off, J.n, J.grid3, [&](int k) { return J.cols[k]; });
+    const int k = at.k, x0 = at.x << 6, y0 = at.y << 6;
     const int t = threadIdx.x;
     const uint32_t b = smem_addr(&bar);
     if (t == 0) {
@@ -247,31 +257,29 @@ __device__ __forceinline__ int byte_i(const uint4 &v, int i) {
     return byte_k(w, i & 3);
 }
 
-// One sample pair into the thread's statistics column: the word of the
+// One sample pair into a statistics column: the word of the
 // sample's row (sao_row_of, computed: a lookup table would add a shared
 // load with bank conflicts to every pixel) gains 65536 + SAO_BIAS + o - r.
-template <int SFT>
 __device__ __forceinline__ void sao_count(int *col, int r, int o) {
-    col[sao_row_of(r) * SFT] += 65536 + (int)SAO_BIAS + o - r;
+    atomicAdd(&col[sao_row_of(r) * 32], 65536 + (int)SAO_BIAS + o - r);
 }
 
+// Bound: the integer ALU (about 2,300 instructions of a warp per CTU, a third
+// of them the adds and addresses of the statistics).  A column per thread
+// instead of per lane took four times the zeroing and row totals, and the
+// offset on 16-bit pairs twice the instructions of whole words: 3,060 per CTU.
 template <int SFT>
 __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
     constexpr int NSEG = 256 / SFT;           // 16-pixel segments per thread
-    static_assert(SFT == 64 || SFT == 128, "SAO CTA: 256 16-pixel segments per CTU, table within 48 KB");
-    // G columns of the table are summed before unpacking: a column holds
-    // at most 16 * NSEG samples, and a sum of words splits exactly up to
-    // 128 (sao_unpack).
-    constexpr int G = NSEG <= 2 ? 4 : 2;
+    static_assert(SFT == 64 || SFT == 128, "SAO CTA: 256 16-pixel segments per CTU");
     constexpr int TPR = SFT >= 2 * SAO_ROWS ? 2 : 1;   // threads summing one row
-    __shared__ __align__(16) int hist[SAO_ROWS][SFT];   // count * 65536 + sum of (256 + org - rec), per thread
+    __shared__ __align__(16) int hist[SAO_ROWS][32];   // count * 65536 + sum of (256 + org - rec), per lane
     __shared__ int row_cnt[SAO_ROWS], row_sum[SAO_ROWS];
     __shared__ int red[SFT / 32];
     __shared__ int dec[3];
-    const int k = find_frame(J.ctu_off, J.n, blockIdx.x);
-    const SaoFrame &F = J.f[k];
-    const int local = blockIdx.x - J.ctu_off[k], cols = (F.W + 63) >> 6;
-    const int x0 = (local % cols) << 6, y0 = (local / cols) << 6;
+    const CtuAt at = ctu_at(J.ctu_off, J.n, J.grid3, [&](int k) { return (J.f[k].W + 63) >> 6; });
+    const SaoFrame &F = J.f[at.k];
+    const int x0 = at.x << 6, y0 = at.y << 6;
     const int w = min(64, F.W - x0), h = min(64, F.H - y0);
     const int t = threadIdx.x;
     // segment j of this thread: row (t + j*SFT) >> 2, columns 16 * ((t + j*SFT) & 3)
@@ -308,11 +316,11 @@ __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
             ov[j] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
         }
     }
-    for (int i = t; i < SAO_ROWS * SFT / 4; i += SFT) ((int4 *)&hist[0][0])[i] = make_int4(0, 0, 0, 0);
+    for (int i = t; i < SAO_ROWS * 32 / 4; i += SFT) ((int4 *)&hist[0][0])[i] = make_int4(0, 0, 0, 0);
     __syncthreads();
     // ---- pass 1: per-row (count, sum) and the unfiltered SSE (|d|^2 four
     // pixels at a time; padding bytes are zero in both vectors)
-    int *col = &hist[0][t];
+    int *col = &hist[0][t & 31];
     int base = 0;
 #pragma unroll
     for (int j = 0; j < NSEG; ++j) {
@@ -330,41 +338,36 @@ __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
                 uint32_t even, odd;
                 sao_incr4(rw[q], ow[q], even, odd);
                 // shared-memory atomic adds with no result: one instruction
-                // per sample instead of a load / add / store chain (the
-                // column is private, so they never contend)
-                atomicAdd(&col[(rows & 0xFF) * SFT], (int)sao_lane_lo(even));
-                atomicAdd(&col[((rows >> 8) & 0xFF) * SFT], (int)sao_lane_lo(odd));
-                atomicAdd(&col[((rows >> 16) & 0xFF) * SFT], (int)sao_lane_hi(even));
-                atomicAdd(&col[(rows >> 24) * SFT], (int)sao_lane_hi(odd));
+                // per sample instead of a load / add / store chain
+                atomicAdd(&col[(rows & 0xFF) * 32], (int)sao_lane_lo(even));
+                atomicAdd(&col[((rows >> 8) & 0xFF) * 32], (int)sao_lane_lo(odd));
+                atomicAdd(&col[((rows >> 16) & 0xFF) * 32], (int)sao_lane_hi(even));
+                atomicAdd(&col[(rows >> 24) * 32], (int)sao_lane_hi(odd));
             }
         } else {
-            for (int i = 0; i < nvalid[j]; ++i) sao_count<SFT>(col, byte_i(rv[j], i), byte_i(ov[j], i));
+            for (int i = 0; i < nvalid[j]; ++i) sao_count(col, byte_i(rv[j], i), byte_i(ov[j], i));
         }
     }
     const int bsum = __reduce_add_sync(0xffffffffu, (unsigned)base);
     if ((t & 31) == 0) red[t >> 5] = bsum;
     __syncthreads();
-    // ---- row totals: TPR threads per row, summing G columns at a time
-    // (16-byte loads) before unpacking
+    // ---- row totals: TPR threads per row.  The words' sum and the sum of
+    // their low halves give both totals (4096 samples stay below 2^28 and 2^22)
     if (t < TPR * SAO_ROWS) {
         const int row = t / TPR, part = t % TPR;
-        const int4 *p = (const int4 *)&hist[row][part * (SFT / TPR)];
-        int cnt = 0, sum = 0;
-        auto unpack = [&](int x) { sao_unpack((uint32_t)x, cnt, sum); };
+        const int4 *p = (const int4 *)&hist[row][part * (32 / TPR)];
+        int all = 0, sum = 0;
         // start each thread at its own 16-byte column group: the rows are
-        // 128 words apart, so unrotated every lane would read the same banks
-        constexpr int NV = SFT / TPR / 4;
+        // 32 words apart, so unrotated every lane would read the same banks
+        constexpr int NV = 32 / TPR / 4;
         const int rot = (row * TPR + part) % NV;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int4 v = p[(i + rot) % NV];
-            if (G == 4) {
-                unpack(v.x + v.y + v.z + v.w);
-            } else {
-                unpack(v.x + v.y);
-                unpack(v.z + v.w);
-            }
+            all += v.x + v.y + v.z + v.w;
+            sum += (v.x & 0xFFFF) + (v.y & 0xFFFF) + (v.z & 0xFFFF) + (v.w & 0xFFFF);
         }
+        int cnt = (all - sum) >> 16;
         sum -= (int)SAO_BIAS * cnt;
         if (TPR == 2) {
             cnt += __shfl_xor_sync(0xffffffffu, cnt, 1);
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
             dec[1] = has ? bb : 0;
             dec[2] = has ? cand : 0;
             if (F.params) {
-                int16_t *pp = F.params + 3 * local;
+                int16_t *pp = F.params + 3 * (at.y * ((F.W + 63) >> 6) + at.x);
                 pp[0] = (int16_t)dec[0]; pp[1] = (int16_t)dec[1]; pp[2] = (int16_t)dec[2];
             }
         }
@@ -403,10 +406,13 @@ __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
     __syncthreads();
     // ---- apply: bytes of the chosen band (exact per-byte test: band
     // indices are <= 31, so adding 0x7F sets bit 7 of every nonzero byte
-    // without carries), offset on pairs; only segments with a hit are
-    // written
+    // without carries).  Where no sample of the band can leave 0..255 the
+    // offset is added to the hit bytes of a whole word at once (each byte's
+    // result is a byte, so nothing carries between them); bands 0 and 31 go
+    // by clamped pairs.  Only segments with a hit are written.
     if (dec[0]) {
         const uint32_t bandx4 = (uint32_t)dec[1] * 0x01010101u, one = 0x00010001u;
+        const bool clips = dec[1] == 0 || dec[1] == 31;
         const uint32_t add = (uint32_t)(dec[2] + 128) * one, lo = 128u * one, hi = (128u + 255u) * one;
 #pragma unroll
         for (int j = 0; j < NSEG; ++j) {
@@ -416,15 +422,19 @@ __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint32_t tq = ((wv[q] >> 3) & 0x1F1F1F1Fu) ^ bandx4;
-                hit[q] = ~(tq + 0x7F7F7F7Fu) & 0x80808080u;
+                hit[q] = (~(tq + 0x7F7F7F7Fu) >> 7) & 0x01010101u;
                 any |= hit[q] != 0;
             }
             if (!any) continue;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
+                if (!clips) {
+                    wv[q] += hit[q] * (uint32_t)dec[2];
+                    continue;
+                }
                 const uint32_t a = pair_min(pair_max(pair_lo(wv[q]) + add, lo), hi) - lo;
                 const uint32_t b = pair_min(pair_max(pair_hi(wv[q]) + add, lo), hi) - lo;
-                const uint32_t m = (hit[q] >> 7) * 0xFFu;
+                const uint32_t m = hit[q] * 0xFFu;
                 wv[q] = (pair_pack(a, b) & m) | (wv[q] & ~m);
             }
             const int sg = t + j * SFT, row = sg >> 2, c0 = (sg & 3) * 16;
@@ -482,6 +492,15 @@ unsigned int tma_waits_expired() {
 
 namespace {
 
+// Grid of a launch over m frames (see ctu_at): three-dimensional when they have
+// one size.
+template <class Frame>
+dim3 ctu_grid(const Frame *f, int m, int total, int cols, int rows, int &grid3) {
+    grid3 = 1;
+    for (int j = 1; j < m; ++j) grid3 &= f[j].W == f[0].W && f[j].H == f[0].H;
+    return grid3 ? dim3(cols, rows, m) : dim3(total);
+}
+
 cudaError_t launch_group_tma(const DeblockFrame *frames, int m, cudaStream_t st, int threads) {
     DeblockTmaJobs J;
     memset(&J, 0, sizeof(J));
@@ -500,9 +519,10 @@ cudaError_t launch_group_tma(const DeblockFrame *frames, int m, cudaStream_t st,
     J.n = m;
     J.ctu_off[m] = total;
     if (total == 0) return cudaSuccess;
-    if (threads == 64) deblock_tma_kernel<64><<<total, 64, 0, st>>>(J);
-    else if (threads == 256) deblock_tma_kernel<256><<<total, 256, 0, st>>>(J);
-    else deblock_tma_kernel<128><<<total, 128, 0, st>>>(J);
+    const dim3 grid = ctu_grid(frames, m, total, frames[0].W >> 6, frames[0].H >> 6, J.grid3);
+    if (threads == 64) deblock_tma_kernel<64><<<grid, 64, 0, st>>>(J);
+    else if (threads == 256) deblock_tma_kernel<256><<<grid, 256, 0, st>>>(J);
+    else deblock_tma_kernel<128><<<grid, 128, 0, st>>>(J);
     return cudaGetLastError();
 }
 
@@ -517,9 +537,10 @@ cudaError_t launch_group_vec(const DeblockFrame *frames, int m, cudaStream_t st,
     }
     J.ctu_off[m] = total;
     if (total == 0) return cudaSuccess;
-    if (threads == 64) deblock_frames_kernel<64><<<total, 64, 0, st>>>(J);
-    else if (threads == 256) deblock_frames_kernel<256><<<total, 256, 0, st>>>(J);
-    else deblock_frames_kernel<128><<<total, 128, 0, st>>>(J);
+    const dim3 grid = ctu_grid(frames, m, total, frames[0].W >> 6, frames[0].H >> 6, J.grid3);
+    if (threads == 64) deblock_frames_kernel<64><<<grid, 64, 0, st>>>(J);
+    else if (threads == 256) deblock_frames_kernel<256><<<grid, 256, 0, st>>>(J);
+    else deblock_frames_kernel<128><<<grid, 128, 0, st>>>(J);
     return cudaGetLastError();
 }
 
@@ -557,8 +578,9 @@ cudaError_t launch_sao_frames(const SaoFrame *frames, int n, cudaStream_t st, in
         }
         J.ctu_off[J.n] = total;
         if (total > 0) {
-            if (threads == 64) sao_frames_kernel<64><<<total, 64, 0, st>>>(J);
-            else sao_frames_kernel<128><<<total, 128, 0, st>>>(J);
+            const dim3 grid = ctu_grid(J.f, J.n, total, (J.f[0].W + 63) >> 6, (J.f[0].H + 63) >> 6, J.grid3);
+            if (threads == 64) sao_frames_kernel<64><<<grid, 64, 0, st>>>(J);
+            else sao_frames_kernel<128><<<grid, 128, 0, st>>>(J);
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }

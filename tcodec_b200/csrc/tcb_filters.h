@@ -16,7 +16,7 @@ struct DeblockFrame {
 };
 struct DeblockJobs {
     static constexpr int MAX = 32;
-    int n;
+    int n, grid3;              // grid3: frames of one size, CTAs in a 3D grid
     int ctu_off[MAX + 1];      // first CTA of each frame (full CTUs only)
     DeblockFrame f[MAX];
 };
@@ -30,7 +30,7 @@ struct SaoFrame {
 };
 struct SaoJobs {
     static constexpr int MAX = 32;
-    int n;
+    int n, grid3;
     int ctu_off[MAX + 1];
     SaoFrame f[MAX];
 };
