@@ -11,8 +11,8 @@
 //                          (present, band, offset) of every CTU.
 //
 // Both are byte kernels: one 128-thread CTA per CTU, the tile moved with
-// 16-byte loads and stores (a byte path serves unaligned planes), each byte
-// read once and written at most once.  Deblocking filters two edge
+// 16-byte loads and stores (or the widest the planes' alignment allows), each
+// byte read once and written at most once.  Deblocking filters two edge
 // positions per instruction on packed 16-bit lanes (tcb_deblock_pairs.cuh).
 //
 // SAO statistics: the CTA keeps a [row][32] table in shared memory, column =
@@ -50,7 +50,7 @@ namespace {
 // same SM filter.
 
 // The frame whose CTA range [off[k], off[k+1]) holds CTA g (binary search
-// over the n <= 32 frames of a launch; off[0] = 0 <= g).
+// over the n frames of a launch; off[0] = 0 <= g).
 __device__ __forceinline__ int find_frame(const int *off, int n, int g) {
     int lo = 0, hi = n - 1;
     while (lo < hi) {
@@ -78,9 +78,45 @@ __device__ __forceinline__ bool aligned16(const void *p, int stride) {
     return (((uintptr_t)p) & 15) == 0 && (stride & 15) == 0;
 }
 
+// 16 bytes at any address: one vector where it is aligned, else the aligned
+// words that hold them (each holds at least one of the bytes, so all are
+// readable) and funnel shifts; and their store with the widest accesses the
+// address allows.
+__device__ __forceinline__ uint4 load16(const uint8_t *p) {
+    const uintptr_t a = (uintptr_t)p;
+    if ((a & 15) == 0) return __ldcs((const uint4 *)p);
+    const uint32_t *w = (const uint32_t *)(a & ~(uintptr_t)3), sh = (uint32_t)(a & 3) * 8;
+    const uint32_t w0 = __ldcs(w), w1 = __ldcs(w + 1), w2 = __ldcs(w + 2), w3 = __ldcs(w + 3), w4 = sh ? __ldcs(w + 4) : 0;
+    return make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh),
+                      __funnelshift_r(w3, w4, sh));
+}
+__device__ __forceinline__ void store16(uint8_t *p, const uint4 v) {
+    const uintptr_t a = (uintptr_t)p;
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    if ((a & 15) == 0) __stcs((uint4 *)p, v);
+    else if ((a & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) __stcs((uint32_t *)p + i, w[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t h = w[i >> 1] >> (16 * (i & 1));
+            if ((a & 1) == 0) ((uint16_t *)p)[i] = (uint16_t)h;
+            else { p[2 * i] = (uint8_t)h; p[2 * i + 1] = (uint8_t)(h >> 8); }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- deblock
 
-template <int DFT>
+// Bound: for a full grid the memory, for a launch of few CTUs the latency of
+// one: load, the two phases, store.  FINE splits the phases into one edge pair
+// (vertical) and one word column (horizontal) per item, 640 and 296 items,
+// instead of a row and 16 columns, 96 and 116 items of eight times the work.
+// One 320x240 frame (15 CTUs), called back to back: 10.5 us with the coarse
+// items, 7.7 fine, of which 7 are the call and the launch.  64 frames of 68x64:
+// 24.6 us byte by byte in two launches, 7.8 with words and in one.
+template <int DFT, bool FINE>
 __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
     static_assert(DFT >= 32 && DFT % 32 == 0, "whole warps");
     constexpr int NPIECE = (384 + DFT - 1) / DFT;   // 16-byte pieces per thread (384 per CTU)
@@ -93,20 +129,19 @@ __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
     uint8_t *gy = F.y + (size_t)y0 * F.sy + x0;
     uint8_t *const gcb = F.cb + (size_t)(y0 >> 1) * F.sc + (x0 >> 1), *const gcr = F.cr + (size_t)(y0 >> 1) * F.sc + (x0 >> 1);
     auto gc = [&](int c) { return c ? gcr : gcb; };   // a select, not an indexed (local-memory) array
-    const bool vec = aligned16(F.y, F.sy) && aligned16(F.cb, F.sc) && aligned16(F.cr, F.sc);
     // ---- load: 16-byte pieces 0..255 luma (row p>>2, segment p&3),
     // 256..383 chroma (plane, row, segment); all issued before any use
-    if (vec) {
+    {
         uint4 v[NPIECE];
 #pragma unroll
         for (int j = 0; j < NPIECE; ++j) {
             const int p = t + j * DFT;
             if (p >= 384) break;
             if (p < 256) {
-                v[j] = __ldcs((const uint4 *)(gy + (size_t)(p >> 2) * F.sy + (p & 3) * 16));
+                v[j] = load16(gy + (size_t)(p >> 2) * F.sy + (p & 3) * 16);
             } else {
                 const int q = p - 256, c = q >> 6, r = (q >> 1) & 31, sg = q & 1;
-                v[j] = __ldcs((const uint4 *)(gc(c) + (size_t)r * F.sc + sg * 16));
+                v[j] = load16(gc(c) + (size_t)r * F.sc + sg * 16);
             }
         }
 #pragma unroll
@@ -119,12 +154,6 @@ __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
                 *(uint4 *)&tc[c][r * 32 + sg * 16] = v[j];
             }
         }
-    } else {
-        for (int i = t; i < 64 * 64; i += DFT) ty[i] = gy[(size_t)(i >> 6) * F.sy + (i & 63)];
-        for (int i = t; i < 2 * 32 * 32; i += DFT) {
-            const int c = i >> 10, p = i & 1023;
-            tc[c][p] = gc(c)[(size_t)(p >> 5) * F.sc + (p & 31)];
-        }
     }
     __syncthreads();
     // ---- vertical edges, then horizontal edges, as independent items
@@ -132,28 +161,27 @@ __global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
     // luma items of 16 columns and 56 chroma items of 4
     DeblockQp q;
     q.init(F.qp);
-    for (int i = t; i < DEBLOCK_VERT_ROWS; i += DFT) deblock_vert_rows(ty, tc[0], i, q);
-    __syncthreads();
-    for (int i = t; i < deblock_horiz_wide_items<4>(); i += DFT) deblock_horiz_wide<4>(ty, tc[0], tc[1], i, q);
+    if (FINE) {
+#pragma unroll
+        for (int i = t; i < DEBLOCK_VERT_ITEMS; i += DFT) deblock_vert(ty, tc[0], i, q);
+        __syncthreads();
+        for (int i = t; i < deblock_horiz_wide_items<1>(); i += DFT) deblock_horiz_wide<1>(ty, tc[0], tc[1], i, q);
+    } else {
+        for (int i = t; i < DEBLOCK_VERT_ROWS; i += DFT) deblock_vert_rows(ty, tc[0], i, q);
+        __syncthreads();
+        for (int i = t; i < deblock_horiz_wide_items<4>(); i += DFT) deblock_horiz_wide<4>(ty, tc[0], tc[1], i, q);
+    }
     __syncthreads();
     // ---- store
-    if (vec) {
 #pragma unroll
-        for (int j = 0; j < NPIECE; ++j) {
-            const int p = t + j * DFT;
-            if (p >= 384) break;
-            if (p < 256) {
-                __stcs((uint4 *)(gy + (size_t)(p >> 2) * F.sy + (p & 3) * 16), *(const uint4 *)&ty[p * 16]);
-            } else {
-                const int q = p - 256, c = q >> 6, r = (q >> 1) & 31, sg = q & 1;
-                __stcs((uint4 *)(gc(c) + (size_t)r * F.sc + sg * 16), *(const uint4 *)&tc[c][r * 32 + sg * 16]);
-            }
-        }
-    } else {
-        for (int i = t; i < 64 * 64; i += DFT) gy[(size_t)(i >> 6) * F.sy + (i & 63)] = ty[i];
-        for (int i = t; i < 2 * 32 * 32; i += DFT) {
-            const int c = i >> 10, p = i & 1023;
-            gc(c)[(size_t)(p >> 5) * F.sc + (p & 31)] = tc[c][p];
+    for (int j = 0; j < NPIECE; ++j) {
+        const int p = t + j * DFT;
+        if (p >= 384) break;
+        if (p < 256) {
+            store16(gy + (size_t)(p >> 2) * F.sy + (p & 3) * 16, *(const uint4 *)&ty[p * 16]);
+        } else {
+            const int q = p - 256, c = q >> 6, r = (q >> 1) & 31, sg = q & 1;
+            store16(gc(c) + (size_t)r * F.sc + sg * 16, *(const uint4 *)&tc[c][r * 32 + sg * 16]);
         }
     }
 }
@@ -268,6 +296,7 @@ __device__ __forceinline__ void sao_count(int *col, int r, int o) {
 // of them the adds and addresses of the statistics).  A column per thread
 // instead of per lane took four times the zeroing and row totals, and the
 // offset on 16-bit pairs twice the instructions of whole words: 3,060 per CTU.
+// 64 planes of 1920x1080: 139 us so, 87 now (398 MB, 4.6 TB/s).
 template <int SFT>
 __global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
     constexpr int NSEG = 256 / SFT;           // 16-pixel segments per thread
@@ -538,9 +567,12 @@ cudaError_t launch_group_vec(const DeblockFrame *frames, int m, cudaStream_t st,
     J.ctu_off[m] = total;
     if (total == 0) return cudaSuccess;
     const dim3 grid = ctu_grid(frames, m, total, frames[0].W >> 6, frames[0].H >> 6, J.grid3);
-    if (threads == 64) deblock_frames_kernel<64><<<grid, 64, 0, st>>>(J);
-    else if (threads == 256) deblock_frames_kernel<256><<<grid, 256, 0, st>>>(J);
-    else deblock_frames_kernel<128><<<grid, 128, 0, st>>>(J);
+    // Few CTUs: at most one per SM, so a CTU's latency is the launch's time.
+    constexpr int SMS = 148;
+    if (threads == 64) deblock_frames_kernel<64, false><<<grid, 64, 0, st>>>(J);
+    else if (threads == 256) deblock_frames_kernel<256, false><<<grid, 256, 0, st>>>(J);
+    else if (threads == 0 && total <= SMS) deblock_frames_kernel<320, true><<<grid, 320, 0, st>>>(J);
+    else deblock_frames_kernel<128, false><<<grid, 128, 0, st>>>(J);
     return cudaGetLastError();
 }
 
@@ -551,11 +583,11 @@ cudaError_t launch_deblock_frames(const DeblockFrame *frames, int n, cudaStream_
     // group meets the tensor-map alignment; 16-byte vector loads otherwise
     const bool want_tma = (variant & TCB_STAGING_TMA) != 0;
     const int threads = variant & ~TCB_STAGING_TMA;
-    static_assert((int)DeblockJobs::MAX == (int)DeblockTmaJobs::MAX, "one group size");
     for (int i = 0; i < n;) {
-        const int m = n - i < DeblockJobs::MAX ? n - i : DeblockJobs::MAX;
+        int m = n - i < DeblockTmaJobs::MAX ? n - i : DeblockTmaJobs::MAX;
         bool tma = want_tma && tensor_map_encoder() != nullptr;
         for (int j = 0; tma && j < m; ++j) tma = tma_ok(frames[i + j]);
+        if (!tma && !want_tma) m = n - i < DeblockJobs::MAX ? n - i : DeblockJobs::MAX;
         const cudaError_t e = tma ? launch_group_tma(frames + i, m, st, threads)
                                   : launch_group_vec(frames + i, m, st, threads);
         if (e != cudaSuccess) return e;

@@ -15,7 +15,7 @@ struct DeblockFrame {
     int W, H, sy, sc, qp;
 };
 struct DeblockJobs {
-    static constexpr int MAX = 32;
+    static constexpr int MAX = 64;
     int n, grid3;              // grid3: frames of one size, CTAs in a 3D grid
     int ctu_off[MAX + 1];      // first CTA of each frame (full CTUs only)
     DeblockFrame f[MAX];
@@ -29,7 +29,7 @@ struct SaoFrame {
     int16_t *params;           // 3 per CTU: present, band, offset (may be NULL)
 };
 struct SaoJobs {
-    static constexpr int MAX = 32;
+    static constexpr int MAX = 64;
     int n, grid3;
     int ctu_off[MAX + 1];
     SaoFrame f[MAX];

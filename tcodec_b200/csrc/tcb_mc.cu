@@ -33,7 +33,7 @@ struct McFrame {
     int W, H, sy, sc;
 };
 struct McJobs {                      // passed by value as the kernel parameter
-    static constexpr int MAX = 32;
+    static constexpr int MAX = 64;
     int n;
     int cta_off[MAX + 1];            // first CTA of each frame
     McFrame f[MAX];
