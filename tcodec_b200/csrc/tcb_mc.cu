@@ -9,11 +9,11 @@
 // neighbouring blocks, so its loads and stores are contiguous runs): thread
 // h produces luma columns 4h..4h+3 of the block and chroma plane h (Cb, Cr).
 // The six-tap and bilinear paths run on packed sample pairs
-// (tcb_mc_pairs.cuh) for planes whose stride is a multiple of 4 bytes;
-// blocks near the frame edge, and planes with other strides, take the
-// per-sample arithmetic of the CTU engine (tcb_pixel.cuh), so predictions
-// equal the encoder's; a CTA queues those blocks and all of its threads
-// share their samples after its packed blocks (McEdge below).
+// (tcb_mc_pairs.cuh), with one alignment per block for planes whose stride is a
+// multiple of 4 bytes and one per row for others.  Blocks near the frame edge
+// give the edge-safe arithmetic of the CTU engine (tcb_pixel.cuh), so
+// predictions equal the encoder's; a CTA queues those blocks and all of its
+// threads share them after its packed blocks (McEdge below).
 #include <cuda_runtime.h>
 
 #include "../../include/tcodec_b200.h"
@@ -41,7 +41,9 @@ struct McJobs {                      // passed by value as the kernel parameter
 
 // Threads per CTA are a template parameter (64, 128 or 256; the autotuner
 // times each per frame size, 256 without tuning); the register budget is
-// cut for 768 resident threads per SM (80 registers).
+// cut for 1,024 resident threads per SM (64 registers, a few spilled): the
+// six-tap path is bound by latency, and 16 frames of 1280x720 with random
+// vectors take 58.5 us so, 61.1 with 768 threads and 80 registers.
 constexpr int MC_DEFAULT_THREADS = 256;
 
 // Four bytes v to dst, only the first w of them at a clipped block edge.
@@ -55,7 +57,7 @@ __device__ __forceinline__ void store4(uint8_t *dst, uint32_t v, int w) {
 
 template <int DX, int DY>
 __device__ __forceinline__ void luma_fixed(const uint8_t *ref, int s, int fx, int fy, int h, uint32_t out[8]) {
-    mc_luma_six_tap(ref, s, fx, fy, h, PairPhaseFixed<DX, DY>(), out);
+    mc_luma_six_tap<PairPhaseFixed<DX, DY>>(ref, s, fx, fy, h, PairPhaseFixed<DX, DY>(), out);
 }
 // The full six-tap block with its quarter phase (dx * 4 + dy, 1..15) fixed.
 __device__ __forceinline__ void luma_six_tap_fixed(const uint8_t *ref, int s, int fx, int fy, int h, int phase,
@@ -79,12 +81,18 @@ __device__ __forceinline__ void luma_six_tap_fixed(const uint8_t *ref, int s, in
     }
 }
 
-// The per-sample edge-safe path costs 30-40 times the packed one.  A block
-// that needs it would hold its whole warp (16 blocks) for that long, so its
-// threads only queue it in shared memory; once the CTA's packed blocks are
-// done, all MT threads share the queued blocks' samples, one sample each.
-// (Sharing within the warp instead, without the CTA barrier, measured 5 %
-// slower on random vectors.)
+// Blocks whose six-tap support leaves the frame (and chroma blocks whose
+// coordinates clamp) cost several times the packed ones and would hold their
+// whole warp (16 blocks) for that long, so their threads only queue them in
+// shared memory; once the CTA's packed blocks are done, all MT threads share
+// them.  Few are taken sample by sample, up to MC_SAMPLE_ROUNDS rounds of the
+// CTA, for the shortest chain; more row by row, four samples from one window
+// of clamped samples at a quarter of the instructions a sample (a CTU row along
+// the top edge of a picture is all edge blocks, and its CTA was the whole
+// launch's time: one 1824x926 frame with a global vector took 47.8 us, now
+// 22.6).  Random vectors, 16 frames of 1280x720: 60.7 us with the rule, 64.6
+// with rows only.
+constexpr int MC_SAMPLE_ROUNDS = 2;
 struct McEdge {
     int h, X, Y, mvx, mvy;
     __device__ __forceinline__ McEdge(const McFrame &F, int g) {
@@ -99,34 +107,43 @@ struct McEdge {
 };
 
 // The queued half blocks (entries: thread indices within the CTA, whose
-// first element is g0), one sample per thread: luma 32 per entry (4 columns
-// x 8 rows), chroma 16 (the 4x4 block of plane h).  Not inlined, so that
+// first element is g0): luma 32 samples or 8 rows of four per entry, chroma 4
+// rows (of the 4x4 block of plane h).  Not inlined, so that
 // its registers do not add to the packed path's; the frame comes by value,
 // as an address into the kernel parameter would copy every frame to the
 // stack.
 template <int MT>
 __device__ __noinline__ void mc_edge_samples(const McFrame F, int g0, const uint16_t *q_luma, int n_luma,
                                              const uint16_t *q_chroma, int n_chroma) {
-    const int nl = n_luma * 32, nc = n_chroma * 16;
-    for (int i = threadIdx.x; i < nl; i += MT) {
-        const McEdge B(F, g0 + q_luma[i >> 5]);
-        const int c = i & 3, y = (i >> 2) & 7, x = B.X + 4 * B.h + c;
+    const int nl = n_luma * 8, nc = n_chroma * 4;
+    if (4 * nl <= MC_SAMPLE_ROUNDS * MT) {
+        for (int i = threadIdx.x; i < 4 * nl; i += MT) {
+            const McEdge B(F, g0 + q_luma[i >> 5]);
+            const int c = i & 3, y = (i >> 2) & 7, x = B.X + 4 * B.h + c;
+            if (x < F.W && B.Y + y < F.H)
+                F.py[(size_t)(B.Y + y) * F.sy + x] = (uint8_t)interp_luma_safe(
+                    F.ry, F.sy, F.W, F.H, (B.mvx >> 2) + 4 * B.h + c, (B.mvy >> 2) + y, B.mvx & 3, B.mvy & 3);
+        }
+    } else for (int i = threadIdx.x; i < nl; i += MT) {
+        const McEdge B(F, g0 + q_luma[i >> 3]);
+        const int y = i & 7, x = B.X + 4 * B.h;
         if (x < F.W && B.Y + y < F.H)
-            F.py[(size_t)(B.Y + y) * F.sy + x] = (uint8_t)interp_luma_safe(
-                F.ry, F.sy, F.W, F.H, (B.mvx >> 2) + 4 * B.h + c, (B.mvy >> 2) + y, B.mvx & 3, B.mvy & 3);
+            store4(F.py + (size_t)(B.Y + y) * F.sy + x,
+                   mc_luma_edge_row(F.ry, F.sy, F.W, F.H, B.mvx >> 2, B.mvy >> 2, B.h, y, B.mvx & 3, B.mvy & 3),
+                   min(4, F.W - x));
     }
     for (int i = threadIdx.x; i < nc; i += MT) {
-        const McEdge B(F, g0 + q_chroma[i >> 4]);
-        const int Wc = F.W >> 1, Hc = F.H >> 1, c = i & 3, y = (i >> 2) & 3;
-        const int x = (B.X >> 1) + c, yy = (B.Y >> 1) + y;
+        const McEdge B(F, g0 + q_chroma[i >> 2]);
+        const int Wc = F.W >> 1, Hc = F.H >> 1, y = i & 3, x = B.X >> 1, yy = (B.Y >> 1) + y;
         if (x < Wc && yy < Hc)
-            (B.h ? F.pcr : F.pcb)[(size_t)yy * F.sc + x] =
-                (uint8_t)chroma_mc_at(B.h ? F.rcr : F.rcb, F.sc, Wc, Hc, B.mvx, B.mvy, c, y);
+            store4((B.h ? F.pcr : F.pcb) + (size_t)yy * F.sc + x,
+                   mc_chroma_edge_row(B.h ? F.rcr : F.rcb, F.sc, Wc, Hc, B.mvx >> 3, B.mvy >> 3, y, B.mvx & 7, B.mvy & 7),
+                   min(4, Wc - x));
     }
 }
 
 template <int MT>
-__global__ void __launch_bounds__(MT, 768 / MT) mc_frames_kernel(McJobs J) {
+__global__ void __launch_bounds__(MT, 1024 / MT) mc_frames_kernel(McJobs J) {
     __shared__ uint16_t q_luma[MT], q_chroma[MT];   // threads whose block takes the per-sample path
     __shared__ int n_luma, n_chroma;
     if (threadIdx.x == 0) n_luma = n_chroma = 0;
@@ -150,7 +167,11 @@ __global__ void __launch_bounds__(MT, 768 / MT) mc_frames_kernel(McJobs J) {
         if (dx == 0 && dy == 0 && fx >= 0 && fy >= 0 && fx + 8 <= F.W && fy + 8 <= F.H) {
 #pragma unroll
             for (int y = 0; y < 8; ++y) out[y] = mc_load4(F.ry + (size_t)(fy + y) * F.sy + fx + 4 * h);
-        } else if ((dx | dy) != 0 && fx >= 2 && fx + 10 < F.W && fy >= 2 && fy + 10 < F.H && (F.sy & 3) == 0) {
+        } else if ((dx | dy) != 0 && fx >= 2 && fx + 10 < F.W && fy >= 2 && fy + 10 < F.H && (F.sy & 3) != 0) {
+            PairPhase ph;
+            ph.init(dx, dy);
+            mc_luma_six_tap<PairPhase, false>(F.ry, F.sy, fx, fy, h, ph, out);
+        } else if ((dx | dy) != 0 && fx >= 2 && fx + 10 < F.W && fy >= 2 && fy + 10 < F.H) {
             // Blocks of one warp that share the phase (coherent motion) take
             // the path specialised for it; mixed phases take the selecting one.
             const int phase = dx * 4 + dy;
@@ -160,7 +181,7 @@ __global__ void __launch_bounds__(MT, 768 / MT) mc_frames_kernel(McJobs J) {
             } else {
                 PairPhase ph;
                 ph.init(dx, dy);
-                mc_luma_six_tap(F.ry, F.sy, fx, fy, h, ph, out);
+                mc_luma_six_tap<PairPhase>(F.ry, F.sy, fx, fy, h, ph, out);
             }
         } else {
             q_luma[atomicAdd(&n_luma, 1)] = (uint16_t)threadIdx.x;
@@ -176,9 +197,10 @@ __global__ void __launch_bounds__(MT, 768 / MT) mc_frames_kernel(McJobs J) {
         // ---- chroma: plane h, the 4x4 block at (X/2, Y/2)
         const int Wc = F.W >> 1, Hc = F.H >> 1, cx = X >> 1, cy = Y >> 1;
         const int xi = mvx >> 3, yi = mvy >> 3;
-        if (xi >= 0 && xi + 4 < Wc && yi >= 0 && yi + 4 < Hc && (F.sc & 3) == 0) {
+        if (xi >= 0 && xi + 4 < Wc && yi >= 0 && yi + 4 < Hc) {
             uint32_t cout[4];
-            mc_chroma_bilinear(h ? F.rcr : F.rcb, F.sc, xi, yi, mvx & 7, mvy & 7, cout);
+            if (F.sc & 3) mc_chroma_bilinear<false>(h ? F.rcr : F.rcb, F.sc, xi, yi, mvx & 7, mvy & 7, cout);
+            else mc_chroma_bilinear(h ? F.rcr : F.rcb, F.sc, xi, yi, mvx & 7, mvy & 7, cout);
             const int wc = min(4, Wc - cx), hc = min(4, Hc - cy);
             uint8_t *dst = (h ? F.pcr : F.pcb) + (size_t)cy * F.sc + cx;
 #pragma unroll
