@@ -34,6 +34,13 @@ namespace tcb {
 
 #define SYNC() __syncthreads()
 
+// Code size: what a leaf runs through once stays in the instruction cache only
+// if all of it fits (straight-line code costs 2 cycles an instruction below
+// 32 KB, 3 below 128 KB and 9 beyond), so loops of a few iterations are kept
+// rolled: the compiler's unrolling by four had the functions of a leaf decision
+// at 170 KB, now 125 KB (a key frame of 1280x720 22.7 -> 22.0 ms, a P frame of
+// 1920x1080 61.0 -> 59.5).
+
 // Optional per-phase cycle counters (build with -DTCB_PHASE_PROFILE); thread
 // 0 of each CTA accumulates clock64() deltas into tcb_phase_cycles[].
 #ifdef TCB_PHASE_PROFILE
@@ -751,6 +758,7 @@ __device__ __noinline__ void build_refs(const Leaf L) {
         if (left) return hl ? RY(S, L.lx - 1, L.ly + j) : (ha ? RY(S, L.lx, L.ly - 1) : 128);
         return ha ? RY(S, L.lx + j, L.ly - 1) : (hl ? RY(S, L.lx - 1, L.ly) : 128);
     };
+#pragma unroll 1
     for (int i = threadIdx.x; i < 2 * n; i += NT) {
         const bool horiz = i >= n;
         const int j = (horiz ? i - n : i) - 3 * N / 2;
@@ -760,6 +768,7 @@ __device__ __noinline__ void build_refs(const Leaf L) {
     if (threadIdx.x >= NT - 96 && threadIdx.x < NT - 64) {
         // DC value (reference src/predict.c:140-161): samples 1..N of each run.
         int sum = 0;
+#pragma unroll 1
         for (int i = (threadIdx.x & 31) + 1; i <= N; i += 32) sum += sample(false, i) + sample(true, i);
         sum = __reduce_add_sync(0xffffffffu, sum);
         if ((threadIdx.x & 31) == 0) S.dc = (sum + N) >> __ffs(N);   // / (2 N)
@@ -914,6 +923,7 @@ __device__ __forceinline__ ChromaModel chroma_stats(T &S, const Leaf L, int c) {
     const int cs = L.cu >> 1, lxc = L.lx >> 1, lyc = L.ly >> 1, lane = threadIdx.x & 31;
     const bool up = L.py > 0, left = L.px > 0;
     int sl = 0, sc = 0, slc = 0, sl2 = 0;
+#pragma unroll 1
     for (int i = lane; i < cs; i += 32) {
         if (up) {
             const int la = (RY(S, L.lx + 2 * i, L.ly - 1) + RY(S, L.lx + 2 * i + 1, L.ly - 1) + 1) >> 1;
@@ -1048,6 +1058,7 @@ __device__ __noinline__ void chroma_mc(Smem &, const FrameParams &, const Leaf L
     Smem &S = smem_state();
     const FrameParams &P = g_fp;
     const int cs = L.cu >> 1, Wc = P.W >> 1, Hc = P.H >> 1, lgs = lg2i(cs);
+#pragma unroll 1
     for (int i = threadIdx.x; i < 2 * cs * cs; i += NT) {
         const int c = i >> (2 * lgs), p = i & ((1 << (2 * lgs)) - 1), y = p >> lgs, x = p & (cs - 1);
         const uint8_t *ref = c ? P.ref_cr[refi] : P.ref_cb[refi];
@@ -1072,6 +1083,7 @@ __device__ void luma_mc(Smem &S, const Leaf &L, const uint8_t *r1, const uint8_t
 // A skipped leaf's luma: the prediction in S.pred[0].
 __device__ void copy_pred(Smem &S, const Leaf &L) {
     const int lg = lg2i(L.cu);
+#pragma unroll 1
     for (int i = threadIdx.x; i < L.cu * L.cu; i += NT) RY(S, L.lx + (i & (L.cu - 1)), L.ly + (i >> lg)) = S.pred[0][i];
 }
 
@@ -1147,6 +1159,7 @@ static_assert(NT >= 64 * 64 / 8, "a thread per 8 luma samples of a snapshot");
 // Grid update after a leaf (reference src/encoder.c:1279-1288 / 760-780).
 __device__ void grid_update(Smem &S, const Leaf &L, const Node &nd, int mvpx, int mvpy) {
     const int gc = L.cu >> 3, lgg = lg2i(gc);
+#pragma unroll 1
     for (int i = threadIdx.x; i < gc * gc; i += NT) {
         const int y = i >> lgg, x = i & (gc - 1);
         MvCell &g = S.grid[(L.cy + y) * 8 + L.cx + x];
@@ -1215,6 +1228,7 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided, int mvpx, int
             const int o = S.cacc[1][0] + lam * (S.cacc[1][1] + 4) < S.cacc[0][0] + lam * (S.cacc[0][1] + 1);
             if (threadIdx.x == 0) node.ch_intra = (uint8_t)o;
             const int lg = lg2i(cs);
+#pragma unroll 1
             for (int i = threadIdx.x; i < cs * cs; i += NT) {   // two samples of one component
                 const int c = i >> (2 * lg - 1), p = 2 * i & (cs * cs - 1), y = p >> lg, x = p & (cs - 1);
                 *(uint16_t *)&RC(S, c, (L.lx >> 1) + x, (L.ly >> 1) + y) = *(const uint16_t *)(S.cpred[2 * o + c] + p);
@@ -1260,6 +1274,7 @@ __device__ __noinline__ void leaf_code(const Leaf L, bool decided, int mvpx, int
             if (!decided) {
                 if (cflat && threadIdx.x >= NT - 64) chroma_model(L, (threadIdx.x >> 5) & 1);
                 if (flat) {
+#pragma unroll 1
                     for (int i = threadIdx.x; i < cu * cu; i += NT) S.pred[0][i] = 128;
                     SYNC();
                 } else {
@@ -1313,6 +1328,7 @@ __device__ __noinline__ long long leaf_decide(const Leaf L) {
         S.cl[__popc(modes & ((1u << tid) - 1u))] = cl_entry(K_INTRA + tid, CL_8 | (use4 ? CL_4 : 0));
     if (!key) {
         const int half = cu >> 1, lgh = lg2i(half);
+#pragma unroll 1
         for (int i = tid; i < cu * half; i += NT) {
             const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
             S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
@@ -1384,6 +1400,7 @@ __device__ __noinline__ long long leaf_decide(const Leaf L) {
                 chroma_mc(S, P, L, 0, mvpx + L.px * 4, mvpy + L.py * 4, 0, false);
                 const int cs = cu >> 1;
                 long long ac = 0;
+#pragma unroll 1
                 for (int p = tid; p < cs * cs; p += NT) {
                     const int y = p >> lg2i(cs), x = p & (cs - 1);
                     const int db = (int)S.cur_c[0][((L.ly >> 1) + y) * 32 + (L.lx >> 1) + x] - (int)S.cpred[0][p];
@@ -1548,6 +1565,7 @@ __device__ __noinline__ void qt_decide(int ctu_x, int ctu_y, int cx, int cy, boo
             } else {
                 const uint2 *lev = (const uint2 *)(D == 1 ? S.lev1 : S.lev2);
                 uint2 *out = (uint2 *)(S.coef + 96 * S.zoff[cy * 8 + cx]);
+#pragma unroll 1
                 for (int i = threadIdx.x; i < 24 * (64 >> (2 * D)); i += NT) out[i] = lev[i];
                 snap(L, -1, 1);
             }
