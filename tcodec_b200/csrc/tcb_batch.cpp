@@ -225,9 +225,16 @@ tc_error_t enqueue_step(tcb_batch *b, const std::vector<int> &part, const std::v
     if (b->timing && cudaEventRecordWithFlags(b->ev0, b->st, evf) != cudaSuccess) return TC_ERR_INTERNAL;
     const bool persistent = b->encs[part[0]]->impl->persistent;
     if (persistent) {
+        int ready = 0;                // CTUs in work at once
+        bool searching = false;
+        for (int s : part) {
+            const EncImpl &e = *b->encs[s]->impl;
+            ready += std::min(e.ctu_cols, e.ctu_rows);
+            searching = searching || e.cfg.preset >= 2;
+        }
         if (cudaMemsetAsync(b->d_ctrl, 0, 2 * sizeof(int), b->st) != cudaSuccess ||
-            launch_ctu_persistent(b->d_params, b->d_items, (int)b->h_items.size(), b->d_ctrl, b->num_sms, b->st) !=
-                cudaSuccess)
+            launch_ctu_persistent(b->d_params, b->d_items, (int)b->h_items.size(), b->d_ctrl, b->num_sms,
+                                  searching ? ready : 0, b->st) != cudaSuccess)
             return TC_ERR_INTERNAL;
         b->kernel_launches += 1;
     } else {

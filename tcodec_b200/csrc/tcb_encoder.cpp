@@ -486,7 +486,8 @@ tc_error_t EncImpl::launch_own() {
     if (timing) cudaEventRecord(ev0, st);
     if (persistent) {
         if (cudaMemsetAsync(d_ctrl, 0, 2 * sizeof(int), st) != cudaSuccess ||
-            launch_ctu_persistent(d_params, d_items, ctu_cols * ctu_rows, d_ctrl, num_sms, st) != cudaSuccess)
+            launch_ctu_persistent(d_params, d_items, ctu_cols * ctu_rows, d_ctrl, num_sms,
+                                  cfg.preset >= 2 ? std::min(ctu_cols, ctu_rows) : 0, st) != cudaSuccess)
             return TC_ERR_INTERNAL;
         kernel_launches += 1;
     } else {

@@ -160,6 +160,105 @@ __device__ void mvp_at(const MvCell *grid, int cx, int cy, int &mx, int &my) {
 }
 
 // ====================================================================
+// Helper CTAs.  One stream's wavefront keeps at most min(columns, rows) CTUs
+// going, a fraction of the SMs.  Launches that leave SMs idle run clusters of
+// two or four CTAs: the first encodes the CTU, and for every leaf decision the
+// others take their share of the motion searches and of the scoring of the
+// intra modes.  They work on their own copy of the source tile, are sent the
+// leaf and its intra reference samples, claim scoring items from the first
+// CTA's queue, add to its sums and write predictions and vectors into its
+// shared memory; nothing else crosses.  What is computed, and from what, does
+// not depend on who computes it.
+//
+// Protocol: the first CTA writes cmd (and the samples) into a helper's shared
+// memory, then its cmd_seq; the helper answers every command by adding 1 to
+// the first CTA's acks once its results are written.  The first CTA waits for
+// all acks of a command before it sends the next.  Waits are bounded; one that
+// gives up reports an error (ctrl[1]) and the CTA goes on, or (helper) to the
+// cluster barrier that ends the kernel, so no shared memory is released
+// while another CTA may still write to it.
+//
+// Leaves from 32x32 on only (at 16x16 the round trip, about 3,000 cycles, takes
+// what the shares give).  A 64x64 / 32x32 leaf of a P frame with four searches
+// takes 199,000 / 86,000 cycles alone and 98,000 / 60,000 with three helpers,
+// bound by the longest search.
+// ====================================================================
+enum HelpCmd { HELP_EXIT, HELP_CTU, HELP_LEAF };
+
+__device__ __forceinline__ Smem *peer_smem(int rank) {
+    uint64_t p;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(p) : "l"(&smem_state()), "r"(rank));
+    return (Smem *)p;
+}
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ int cluster_size() {
+    int r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    SYNC();
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_fence() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+__device__ __forceinline__ int ld_acquire_cluster(const int *p) {
+    int v;
+    asm volatile("ld.acquire.cluster.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// The last warp sends a command (c0: HelpCmd) to every helper; a leaf's with
+// its intra reference samples.  The caller has seen all earlier acks.
+__device__ __noinline__ void send_command(int c0, int c1, int c2, int c3, int c4, int c5) {
+    Smem &S = smem_state();
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) S.ack_goal += S.helpers;
+    if (threadIdx.x < NT - 32) return;
+    const int seq = S.cmd_sent + 1, n = S.helpers;
+    __syncwarp();
+#pragma unroll 1
+    for (int r = 1; r <= n; ++r) {
+        Smem *H = peer_smem(r);
+        if (c0 == HELP_LEAF) {
+#pragma unroll 1
+            for (int i = lane; i < 2 * EDGE_LEN / 4; i += 32) ((uint32_t *)H->edge)[i] = ((const uint32_t *)S.edge)[i];
+            if (lane == 0) { H->dc = S.dc; H->above0 = S.above0; }
+        }
+        if (lane < 6) H->cmd[lane] = lane == 0 ? c0 : lane == 1 ? c1 : lane == 2 ? c2 : lane == 3 ? c3 : lane == 4 ? c4 : c5;
+    }
+    cluster_fence();
+    __syncwarp();
+    if (lane == 0) {
+        S.cmd_sent = seq;
+#pragma unroll 1
+        for (int r = 1; r <= n; ++r)
+            asm volatile("st.release.cluster.s32 [%0], %1;" ::"l"(&peer_smem(r)->cmd_seq), "r"(seq) : "memory");
+    }
+}
+// Thread 0 waits for the helpers' acks; a barrier of the CTA follows.
+__device__ __forceinline__ void wait_helpers(Smem &S) {
+    if (threadIdx.x != 0 || S.helpers == 0) return;
+    const int goal = S.ack_goal;
+    for (int i = 0; i < (1 << 24); ++i)
+        if (ld_acquire_cluster(&S.acks) >= goal) return;
+    atomicExch(S.error, 1);
+}
+// A helper's answer: everything its threads have written is the first CTA's
+// to read.
+__device__ __forceinline__ void acknowledge() {
+    cluster_fence();
+    SYNC();
+    if (threadIdx.x == 0) {
+        cluster_fence();
+        atomicAdd(&peer_smem(0)->acks, 1);
+    }
+}
+
+// ====================================================================
 // Motion search on one warp group (reference src/motion.c:384-485): the
 // integer stages (me_integer), then, once every search of the leaf is done
 // with them, the quarter-sample refinement (me_qpel).  A group is 128
@@ -735,6 +834,76 @@ __device__ __noinline__ void me_searches(const Leaf L, uint32_t mask, const MeSt
 }
 
 // ====================================================================
+// Reference selection for B-frames (reference src/encoder.c:204-228):
+// forward = largest POC below the current one, backward = smallest above.
+// ====================================================================
+__device__ __forceinline__ int dpb_fwd(const FrameParams &P) {
+    int best = -1, bp = -1;
+    for (int i = 0; i < MAX_REFS; ++i)
+        if (P.ref_valid[i] && P.ref_poc[i] >= 0 && P.ref_poc[i] < P.poc && P.ref_poc[i] > bp) { bp = P.ref_poc[i]; best = i; }
+    return best;
+}
+__device__ __forceinline__ int dpb_bwd(const FrameParams &P) {
+    int best = -1, bp = 0x7FFFFFFF;
+    for (int i = 0; i < MAX_REFS; ++i)
+        if (P.ref_valid[i] && P.ref_poc[i] >= 0 && P.ref_poc[i] > P.poc && P.ref_poc[i] < bp) { bp = P.ref_poc[i]; best = i; }
+    return best;
+}
+
+// The searches of a leaf (reference src/encoder.c:795-852, 862-933): bit k of
+// `mask` is search k of `J`.
+struct LeafSearch {
+    uint32_t mask;
+    int sr;
+    MeStart J;
+};
+__device__ __forceinline__ LeafSearch leaf_searches(const Leaf &L, int mvpx, int mvpy) {
+    const FrameParams &P = g_fp;
+    const bool fast = P.preset <= 1;
+    const int cx0 = (mvpx + L.px * 4) >> 2, cy0 = (mvpy + L.py * 4) >> 2, mx = mvpx + L.px * 4, my = mvpy + L.py * 4;
+    if (P.frame_type == 2) {
+        const int rf = dpb_fwd(P), rb = dpb_bwd(P);
+        const uint8_t *f = rf >= 0 ? P.ref_y[rf] : nullptr, *b = rb >= 0 ? P.ref_y[rb] : nullptr;
+        return {(uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, fast ? 16 : 32,
+                {f, b, f, b, cx0, cy0, cx0, cy0, cx0, cy0, cx0, cy0, mx, my}};
+    }
+    const bool me1 = !fast && P.multiref && P.ref_valid[1];
+    const bool glb = !fast && P.glob_valid && (P.glob_x > 16 || P.glob_x < -16 || P.glob_y > 16 || P.glob_y < -16);
+    bool tmp = false;
+    int tdx = 0, tdy = 0;
+    if (!fast && P.ref_valid[0] && P.prev_valid) {
+        const int fx = L.px >> 3, fy = L.py >> 3;
+        if (fx < P.grid_w && fy < P.grid_h) {
+            const MvCell pg = P.prev_grid[fy * P.grid_w + fx];
+            if (!pg.intra) { tmp = true; tdx = pg.dx; tdy = pg.dy; }
+        }
+    }
+    return {1u | (uint32_t)me1 << 1 | (uint32_t)glb << 2 | (uint32_t)tmp << 3, fast ? 16 : 24,
+            {P.ref_y[0], P.ref_y[1], P.ref_y[0], P.ref_y[0], cx0, cy0, cx0, cy0, (L.px * 4 + P.glob_x) >> 2,
+             (L.py * 4 + P.glob_y) >> 2, (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2, mx, my}};
+}
+// The searches CTA `rank` of n takes, in turn.
+__device__ __forceinline__ uint32_t search_share(uint32_t mask, int rank, int n) {
+    uint32_t mine = 0;
+    for (int j = 0; mask; mask &= mask - 1, j = j + 1 == n ? 0 : j + 1)
+        if (j == rank) mine |= mask & -mask;
+    return mine;
+}
+// log2 of a team's threads for a CTA's share.
+__device__ __forceinline__ int search_team(uint32_t share, int helpers) {
+    return g_fp.preset <= 1 || (helpers && __popc(share) <= 2) ? 8 : 7;
+}
+// The leaf's source samples as pairs, for the searches.
+__device__ __forceinline__ void pair_source(Smem &S, const Leaf &L) {
+    const int half = L.cu >> 1, lgh = lg2i(half);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < L.cu * half; i += NT) {
+        const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
+        S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
+    }
+}
+
+// ====================================================================
 // Leaf helpers
 // ====================================================================
 
@@ -804,6 +973,15 @@ __device__ __forceinline__ int cl_entry(int slot, int sizes) {
     const int m = slot - K_INTRA;
     return slot | sizes | (m > 1 && m < 18 ? (int)c_ang_disp[m] * 65536 : 0);
 }
+// The intra modes a preset tries, as the first entries of the candidate list.
+__device__ __forceinline__ uint32_t intra_modes(int preset) {
+    return preset == 0 ? 0x1041u : preset == 1 ? 0x9249u : 0x3FFFFu;
+}
+__device__ __forceinline__ void list_intra(Smem &S, uint32_t modes, bool use4) {
+    const int tid = threadIdx.x;
+    if (tid < 18 && (modes >> tid & 1u))
+        S.cl[__popc(modes & ((1u << tid) - 1u))] = cl_entry(K_INTRA + tid, CL_8 | (use4 ? CL_4 : 0));
+}
 // Prediction samples (x, y) and (x + 1, y), x even, of a candidate (list entry e).
 __device__ __forceinline__ uint32_t pred2(const Smem &S, int cu, int e, int x, int y) {
     const int slot = e & CL_SLOT;
@@ -826,8 +1004,14 @@ __device__ __forceinline__ QuantLane quant_lane(const Smem &S, int type, int lan
 // interleaved; what a lane adds up over its group's areas is reduced once per
 // item.  Slots not in `mask` are left out.  Groups of 4, 2, 2, 1 areas for 64x64 .. 8x8 leaves; an 8x8 leaf's
 // single area is split by TU size instead.
+template <bool HELP>
 __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, int queue, uint32_t mask) {
     Smem &S = smem_state();
+    Smem *const M = HELP ? peer_smem(0) : nullptr;      // a helper's queue and sums are the first CTA's
+    // the next item: a helper asks for it one item ahead
+    const int lane_ = threadIdx.x & 31;
+    auto claim = [&] { return lane_ == 0 ? HELP ? atomicAdd(&M->next[queue], 1) : atomicAdd(&S.next[queue], 1) : 0; };
+    int ahead = HELP ? claim() : 0;
     const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
     const uint2 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
@@ -838,10 +1022,9 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
     const int lG = la == 6 ? 2 : la == 0 ? 0 : 1;            // log2 of a group's areas
     const int lg = la == 0 ? 1 : la - lG;                    // log2 of the groups (8x8: TU sizes)
     for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(&S.next[queue], 1);
-        it = __shfl_sync(0xffffffffu, it, 0);
+        const int it = __shfl_sync(0xffffffffu, HELP ? ahead : claim(), 0);
         if (it >= ncl << lg) break;
+        if (HELP) ahead = claim();
         const int group = it & ((1 << lg) - 1);
         const int e = cl[it >> lg], slot = e & CL_SLOT, do_sizes = e & (la == 0 ? (group ? CL_4 : CL_8) : CL_8 | CL_4);
         if (!do_sizes || !(mask >> slot & 1u)) continue;
@@ -887,7 +1070,7 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
             const int b = (int)__reduce_add_sync(0xffffffffu, (unsigned)(n4 + s4.bits()));
             v = lane == 2 ? a : lane == 3 ? b + (1 << lG) : v;
         }
-        if (lane < 4) atomicAdd(&S.acc[slot][0][0] + lane, v);
+        if (lane < 4) atomicAdd((HELP ? M : &S)->acc[slot][0] + lane, v);
     }
 }
 
@@ -1174,23 +1357,6 @@ __device__ void grid_update(Smem &S, const Leaf &L, const Node &nd, int mvpx, in
 }
 
 // ====================================================================
-// Reference selection for B-frames (reference src/encoder.c:204-228):
-// forward = largest POC below the current one, backward = smallest above.
-// ====================================================================
-__device__ __forceinline__ int dpb_fwd(const FrameParams &P) {
-    int best = -1, bp = -1;
-    for (int i = 0; i < MAX_REFS; ++i)
-        if (P.ref_valid[i] && P.ref_poc[i] >= 0 && P.ref_poc[i] < P.poc && P.ref_poc[i] > bp) { bp = P.ref_poc[i]; best = i; }
-    return best;
-}
-__device__ __forceinline__ int dpb_bwd(const FrameParams &P) {
-    int best = -1, bp = 0x7FFFFFFF;
-    for (int i = 0; i < MAX_REFS; ++i)
-        if (P.ref_valid[i] && P.ref_poc[i] >= 0 && P.ref_poc[i] > P.poc && P.ref_poc[i] < bp) { bp = P.ref_poc[i]; best = i; }
-    return best;
-}
-
-// ====================================================================
 // Leaf coding of a decided node (reference src/encoder.c:587-781): its
 // reconstruction into the tile and its levels into the CTU's record, where
 // the leaf's place is 96 levels per coded 8x8 cell before it in z-order
@@ -1316,7 +1482,7 @@ __device__ __noinline__ long long leaf_decide(const Leaf L) {
     // searches are done), inter candidates after them.
     const bool try_intra = key || cu <= 16 || medium;
     const bool use4 = medium && cu <= 32;
-    const uint32_t modes = !try_intra ? 0u : P.preset == 0 ? 0x1041u : P.preset == 1 ? 0x9249u : 0x3FFFFu;
+    const uint32_t modes = !try_intra ? 0u : intra_modes(P.preset);
     const int nintra = __popc(modes);
     // slots 2..4 of a B leaf and the merge slot of a P leaf: 8x8 TUs only
     const uint32_t merges = is_b ? 0x1Cu : 1u << K_MRG;
@@ -1324,63 +1490,35 @@ __device__ __noinline__ long long leaf_decide(const Leaf L) {
         const bool m8 = merges >> (tid - 32) & 1u;
         S.cl[nintra + tid - 32] = cl_entry(tid - 32, CL_8 | (use4 && !m8 ? CL_4 : 0) | (is_p && m8 ? CL_EXACT : 0));
     }
-    if (tid < 18 && (modes >> tid & 1u))
-        S.cl[__popc(modes & ((1u << tid) - 1u))] = cl_entry(K_INTRA + tid, CL_8 | (use4 ? CL_4 : 0));
-    if (!key) {
-        const int half = cu >> 1, lgh = lg2i(half);
-#pragma unroll 1
-        for (int i = tid; i < cu * half; i += NT) {
-            const uint8_t *c = S.cur_y + (L.ly + (i >> lgh)) * 64 + L.lx + (i & (half - 1));
-            S.cur_pair[i] = (uint32_t)c[0] | (uint32_t)c[half] << 16;
-        }
-    }
+    list_intra(S, modes, use4);
+    if (!key) pair_source(S, L);
     if (tid >= NT - 64) chroma_model(L, (tid >> 5) & 1);
     build_refs(L);
+    const int helpers = fast || cu < 32 ? 0 : S.helpers;
+    if (helpers) send_command(HELP_LEAF, L.depth, L.cx, L.cy, mvpx, mvpy);
     PHASE_D(0, L.depth);
 
     // ---- candidate set -------------------------------------------------
     // Present slots, one bit each: inter candidates 0..4, intra modes from
     // K_INTRA on.
     uint32_t cand = 0;
-    bool has_glb = false, has_tmp = false, has_me1 = false;
-    int tdx = 0, tdy = 0;
-    const int rf = is_b ? dpb_fwd(P) : -1, rb = is_b ? dpb_bwd(P) : -1;
-    const int cx0 = (mvpx + L.px * 4) >> 2, cy0 = (mvpy + L.py * 4) >> 2;
-    if (is_p) {
-        const int sr = fast ? 16 : 24;
-        has_me1 = !fast && P.multiref && P.ref_valid[1];
-        has_glb = !fast && P.glob_valid &&
-                  (P.glob_x > 16 || P.glob_x < -16 || P.glob_y > 16 || P.glob_y < -16);
-        if (!fast && P.ref_valid[0] && P.prev_valid) {
-            const int fx = L.px >> 3, fy = L.py >> 3;
-            if (fx < P.grid_w && fy < P.grid_h) {
-                const MvCell pg = P.prev_grid[fy * P.grid_w + fx];
-                if (!pg.intra) { has_tmp = true; tdx = pg.dx; tdy = pg.dy; }
-            }
+    if (!key) {
+        const LeafSearch M = leaf_searches(L, mvpx, mvpy);
+        const uint32_t share = helpers ? search_share(M.mask, 0, helpers + 1) : M.mask;
+        me_searches(L, share, M.J, M.sr, search_team(share, helpers), medium, is_b);
+        if (!fast) luma_score<false>(L, S.cl, nintra, 0, ~0u);
+        if (helpers) wait_helpers(S);
+        SYNC();
+        PHASE_D(1, L.depth);
+        cand = M.mask;
+        if (is_p) {
+            if (S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) cand &= ~(1u << K_GLB);
+            if (S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) cand &= ~(1u << K_TMP);
+            cand |= (uint32_t)medium << K_MRG;
+        } else {
+            const uint32_t mrg = medium, hf = M.mask & 1u, hb = M.mask >> 1;
+            cand |= (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;
         }
-        const MeStart J = {P.ref_y[0], P.ref_y[1], P.ref_y[0], P.ref_y[0], cx0, cy0, cx0, cy0,
-                           (L.px * 4 + P.glob_x) >> 2, (L.py * 4 + P.glob_y) >> 2,
-                           (L.px * 4 + tdx) >> 2, (L.py * 4 + tdy) >> 2, mvpx + L.px * 4, mvpy + L.py * 4};
-        me_searches(L, 1u | (uint32_t)has_me1 << 1 | (uint32_t)has_glb << 2 | (uint32_t)has_tmp << 3, J, sr, fast ? 8 : 7,
-                    medium, false);
-        if (!fast) luma_score(L, S.cl, nintra, 0, ~0u);
-        SYNC();
-        PHASE_D(1, L.depth);
-        if (has_glb && S.me[2].mvx == S.me[0].mvx && S.me[2].mvy == S.me[0].mvy) has_glb = false;
-        if (has_tmp && S.me[3].mvx == S.me[0].mvx && S.me[3].mvy == S.me[0].mvy) has_tmp = false;
-        cand = 1u << K_ME0 | (uint32_t)has_me1 << K_ME1 | (uint32_t)has_glb << K_GLB | (uint32_t)has_tmp << K_TMP |
-               (uint32_t)medium << K_MRG;
-    } else if (is_b) {
-        // Forward / backward searches (reference src/encoder.c:795-852).
-        const int sr = fast ? 16 : 32;
-        const uint8_t *f = rf >= 0 ? P.ref_y[rf] : nullptr, *b = rb >= 0 ? P.ref_y[rb] : nullptr;
-        const MeStart J = {f, b, f, b, cx0, cy0, cx0, cy0, cx0, cy0, cx0, cy0, mvpx + L.px * 4, mvpy + L.py * 4};
-        me_searches(L, (uint32_t)(rf >= 0) | (uint32_t)(rb >= 0) << 1, J, sr, fast ? 8 : 7, medium, true);
-        if (!fast) luma_score(L, S.cl, nintra, 0, ~0u);
-        SYNC();
-        PHASE_D(1, L.depth);
-        const uint32_t hf = rf >= 0, hb = rb >= 0, mrg = medium;
-        cand = hf | hb << 1 | (mrg & hf & hb) << 2 | (mrg & hf) << 3 | (mrg & hb) << 4;
     }
 
     // ---- residual coding / SAD proxies for every candidate --------------
@@ -1389,8 +1527,12 @@ __device__ __noinline__ long long leaf_decide(const Leaf L) {
         sad_areas(L, S.cl, nintra + (key ? 0 : NPRED), cand);
         SYNC();
     } else {
-        if (key) luma_score(L, S.cl, nintra, 0, ~0u);
-        else luma_score(L, S.cl + nintra, NPRED, 1, cand);
+        if (key) {
+            luma_score<false>(L, S.cl, nintra, 0, ~0u);
+            if (helpers) wait_helpers(S);
+        } else {
+            luma_score<false>(L, S.cl + nintra, NPRED, 1, cand);
+        }
         SYNC();
         PHASE_D(3, L.depth);
         if (is_p) {
@@ -1755,6 +1897,105 @@ __device__ __noinline__ void sao_tile(Smem &, int w, int h, int lambda_sao) {
     SYNC();
 }
 
+// Bound of a neighbour wait, in back-off iterations (sleeps of 32 ns
+// doubling to 2,048 ns): the default 2^22 is about 8.6 s, far above a
+// CTU's encode time even when the GPU is time-shared.  Per device; set by
+// tcb_set_neighbor_wait_limit.
+__device__ long long g_neighbor_wait_limit = 1ll << 22;
+
+// What a CTU's searches and scoring work from: its source luma, every lane's
+// quantisers, empty SAD tables.
+__device__ void load_luma(Smem &S, const FrameParams &P, int ctu_x, int ctu_y) {
+    const int w = mini(64, P.W - ctu_x), h = mini(64, P.H - ctu_y);
+    for (int i = threadIdx.x; i < 64 * 64; i += NT) {
+        const int y = i >> 6, x = i & 63;
+        S.cur_y[i] = (x < w && y < h) ? P.cur_y[(size_t)(ctu_y + y) * P.stride_y + ctu_x + x] : 0;
+    }
+    if (threadIdx.x >= NT - 96) {
+        const int t = threadIdx.x - (NT - 96), type = t >> 5, lane = t & 31, r = lane >> 2, c = 2 * (lane & 3);
+        const int b0 = type ? band_rc(4, r & 3, c & 3) : band_rc(8, r, c);
+        const int b1 = type ? band_rc(4, r & 3, (c & 3) + 1) : band_rc(8, r, c + 1);
+        const int *eff = type == 2 ? P.eff_c : P.eff_l;
+        const long long lambda = type == 2 ? (long long)P.lambda_c : P.lambda;
+        const QuantLane q = QuantLane::make(QuantPos(eff[b0], lambda), QuantPos(eff[b1], lambda));
+        S.quant[type][0][lane] = q.a;
+        S.quant[type][1][lane] = q.b;
+        S.quant[type][2][lane] = q.c;
+    }
+    init_windows(S);
+}
+
+// A helper's part of a leaf decision (see leaf_decide).
+__device__ __noinline__ void help_leaf(const Leaf L, int mvpx, int mvpy) {
+    Smem &S = smem_state();
+    const FrameParams &P = g_fp;
+    const int rank = cluster_rank(), n = cluster_size();
+    const uint32_t modes = intra_modes(P.preset);
+    list_intra(S, modes, L.cu <= 32);
+    uint32_t share = 0;
+    if (P.frame_type != 0) {
+        const LeafSearch M = leaf_searches(L, mvpx, mvpy);
+        share = search_share(M.mask, rank, n);
+        if (share) {
+            pair_source(S, L);
+            SYNC();
+            const int lth = search_team(share, n - 1);
+            me_searches(L, share, M.J, M.sr, lth, false, false);
+            // the team's search to the first CTA
+            const MeTeam T(lth);
+            if (T.g < __popc(share)) {
+                uint32_t m = share;
+                for (int i = 0; i < T.g; ++i) m &= m - 1;
+                const int id = __ffs((int)m) - 1;
+                T.sync();
+                Smem *A = peer_smem(0);
+                for (int i = T.gt; i < L.cu * L.cu / 16; i += 1 << lth)
+                    ((uint4 *)A->pred[id])[i] = ((const uint4 *)S.pred[id])[i];
+                if (T.gt == 0) {
+                    A->me[id].mvx = S.me[id].mvx; A->me[id].mvy = S.me[id].mvy;
+                    A->cand_mvx[id] = S.cand_mvx[id]; A->cand_mvy[id] = S.cand_mvy[id];
+                }
+            }
+        }
+    }
+    if (!share) SYNC();
+    luma_score<true>(L, S.cl, __popc(modes), 0, ~0u);
+}
+
+// A helper's life: commands until HELP_EXIT.
+__device__ void help(Smem &S, const FrameParams *__restrict__ params, int *ctrl) {
+    int ctu_x = 0, ctu_y = 0;
+    for (int seq = 1;; ++seq) {
+        bool got = false;
+        if (threadIdx.x == 0) {
+            // far longer than the first CTA waits for its neighbours
+            const long long limit = 4 * g_neighbor_wait_limit + (1ll << 24);
+            unsigned ns = 32;
+            for (long long i = 0; i < limit && !got; ++i) {
+                got = ld_acquire_cluster(&S.cmd_seq) >= seq;
+                if (!got && i > 4096) {
+                    __nanosleep(ns);
+                    if (ns < 1024) ns <<= 1;
+                }
+            }
+            if (!got) atomicExch(&ctrl[1], 1);
+        }
+        if (!__syncthreads_or(got)) return;
+        const int c0 = S.cmd[0], c1 = S.cmd[1], c2 = S.cmd[2], c3 = S.cmd[3], c4 = S.cmd[4], c5 = S.cmd[5];
+        if (c0 == HELP_EXIT) return;
+        if (c0 == HELP_CTU) {
+            if (threadIdx.x == 0) g_fp = params[c1 >> 20];
+            SYNC();
+            ctu_x = (c1 & 1023) * 64;
+            ctu_y = (c1 >> 10 & 1023) * 64;
+            load_luma(S, g_fp, ctu_x, ctu_y);
+        } else {
+            help_leaf(Leaf(g_fp, ctu_x, ctu_y, c1, c2, c3), c4, c5);
+        }
+        acknowledge();
+    }
+}
+
 // ====================================================================
 // The CTU kernel.  items[i] = (stream << 20) | (row << 10) | col.
 // ====================================================================
@@ -1763,10 +2004,7 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
     const int w = mini(64, P.W - ctu_x), h = mini(64, P.H - ctu_y);
     const int wc = w >> 1, hc = h >> 1;
     // ---- load source and the filtered neighbour border ----------------
-    for (int i = threadIdx.x; i < 64 * 64; i += NT) {
-        const int y = i >> 6, x = i & 63;
-        S.cur_y[i] = (x < w && y < h) ? P.cur_y[(size_t)(ctu_y + y) * P.stride_y + ctu_x + x] : 0;
-    }
+    load_luma(S, P, ctu_x, ctu_y);
     for (int i = threadIdx.x; i < 2 * 32 * 32; i += NT) {
         const int c = i >> 10, p = i & 1023, y = p >> 5, x = p & 31;
         const uint8_t *src = c ? P.cur_cr : P.cur_cb;
@@ -1800,19 +2038,6 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
         Node z = {};
         S.nodes[i] = z;
     }
-    // every lane's quantisers
-    if (threadIdx.x >= NT - 96) {
-        const int t = threadIdx.x - (NT - 96), type = t >> 5, lane = t & 31, r = lane >> 2, c = 2 * (lane & 3);
-        const int b0 = type ? band_rc(4, r & 3, c & 3) : band_rc(8, r, c);
-        const int b1 = type ? band_rc(4, r & 3, (c & 3) + 1) : band_rc(8, r, c + 1);
-        const int *eff = type == 2 ? P.eff_c : P.eff_l;
-        const long long lambda = type == 2 ? (long long)P.lambda_c : P.lambda;
-        const QuantLane q = QuantLane::make(QuantPos(eff[b0], lambda), QuantPos(eff[b1], lambda));
-        S.quant[type][0][lane] = q.a;
-        S.quant[type][1][lane] = q.b;
-        S.quant[type][2][lane] = q.c;
-    }
-    init_windows(S);
     CtuOut *out = P.out + row * P.ctu_cols + col;
     if (threadIdx.x == 0) S.coef = out->coef;
     if (threadIdx.x < 64) {
@@ -1824,6 +2049,7 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
             n += ctu_x + at(z, 0) * 8 + 8 <= P.W && ctu_y + at(z, 1) * 8 + 8 <= P.H;
         S.zoff[at(threadIdx.x, 1) * 8 + at(threadIdx.x, 0)] = (uint16_t)n;
     }
+    wait_helpers(S);      // they have loaded the CTU too
     SYNC();
 
     // ---- decide and code -------------------------------------------------
@@ -1880,6 +2106,7 @@ ctu_kernel(const FrameParams *__restrict__ params, const int *__restrict__ items
     const int item = items[blockIdx.x];
     if (threadIdx.x == 0) P = params[item >> 20];
     init_fragments(S);
+    if (threadIdx.x == 0) S.helpers = 0;
     SYNC();
     encode_ctu(S, P, (item >> 10) & 1023, item & 1023);
 }
@@ -1892,12 +2119,6 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
 __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-
-// Bound of a neighbour wait, in back-off iterations (sleeps of 32 ns
-// doubling to 2,048 ns): the default 2^22 is about 8.6 s, far above a
-// CTU's encode time even when the GPU is time-shared.  Per device; set by
-// tcb_set_neighbor_wait_limit.
-__device__ long long g_neighbor_wait_limit = 1ll << 22;
 
 // Persistent wavefront: a resident grid pulls CTUs from a queue laid out in
 // topological (anti-diagonal) order and starts each one as soon as its
@@ -1913,6 +2134,20 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
     FrameParams &P = g_fp;
     __shared__ int s_item;
     init_fragments(S);    // visible to all after the first item's barrier
+    const int helpers = cluster_size() - 1;
+    if (threadIdx.x == 0) {
+        S.helpers = helpers;
+        S.cmd_sent = S.cmd_seq = S.acks = S.ack_goal = 0;
+        S.error = ctrl + 1;
+    }
+    if (helpers) {
+        cluster_barrier();    // every CTA's counters are set
+        if (cluster_rank() > 0) {
+            help(S, params, ctrl);
+            cluster_barrier();
+            return;
+        }
+    }
 #ifdef TCB_PHASE_PROFILE
     const long long k0 = clock64();   // residency of the CTA (slot 14); neighbour waits in slot 13
 #endif
@@ -1930,6 +2165,7 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
             break;
         }
         const int row = (item >> 10) & 1023, col = item & 1023;
+        if (helpers) send_command(HELP_CTU, item, 0, 0, 0, 0);
         if (threadIdx.x == 0) {
             P = params[item >> 20];
             const int epoch = P.epoch;
@@ -1955,6 +2191,11 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
         __threadfence();
         SYNC();
         if (threadIdx.x == 0) st_release(P.done + row * P.ctu_cols + col, P.epoch);
+    }
+    if (helpers) {
+        send_command(HELP_EXIT, 0, 0, 0, 0, 0);
+        SYNC();
+        cluster_barrier();
     }
 }
 
@@ -2028,7 +2269,7 @@ cudaError_t encode_frame_with_scratch(const FrameParams &P0, uint8_t *scratch, c
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     return launch_ctu_persistent((const FrameParams *)(scratch + SCR_PARAMS), items + first, nctu - first, ctrl,
-                                 sms, st);
+                                 sms, P.preset >= 2 ? mini(P.ctu_cols, P.ctu_rows) : 0, st);
 }
 
 // Constant tables and kernel attributes, once per device.
@@ -2047,10 +2288,33 @@ cudaError_t ensure_device_tables() {
     return cudaSuccess;
 }
 
+// `ready`: CTUs that can be in work at once, 0 if the frames' leaves leave
+// nothing for helper CTAs.  Clusters of four where the CTUs in work leave SMs
+// for them, of two where only for one helper each; up to twice as many clusters
+// as CTUs in work, because a cluster that has dequeued a CTU waits with it
+// for its neighbours, and no more, to leave the other SMs to other streams.  With 17 CTUs in work (1920x1080) a P frame takes 59.9 ms
+// with single CTAs, 56.0 with clusters of two, 54.2 with four, 56.5 with six
+// (then 24 clusters), and 56.4 with four but only 17 clusters; 32 such streams
+// fill the SMs with single CTAs.
 cudaError_t launch_ctu_persistent(const FrameParams *d_params, const int *d_items, int n, int *d_ctrl,
-                                  int grid, cudaStream_t st) {
+                                  int grid, int ready, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     grid *= CTAS_PER_SM;
+    const int size = ready <= 0 ? 1 : 4 * ready <= grid ? 4 : 2 * ready <= grid ? 2 : 1;
+    if (size > 1) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim = {(unsigned)size, 1, 1};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(size * mini(mini(grid / size, 2 * ready), n)));
+        cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = sizeof(Smem);
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, ctu_persistent_kernel, d_params, d_items, n, d_ctrl) == cudaSuccess) return cudaSuccess;
+        cudaGetLastError();    // no room for a cluster on this device or partition: single CTAs
+    }
     ctu_persistent_kernel<<<grid < n ? grid : n, NT, sizeof(Smem), st>>>(d_params, d_items, n, d_ctrl);
     return cudaGetLastError();
 }

@@ -124,6 +124,12 @@ struct Smem {
     // levels of a 32x32 / 16x16 leaf while its split is tried
     alignas(8) int16_t lev1[32 * 48], lev2[16 * 24];
     alignas(8) unsigned long long tu8mask;
+    // helper CTAs (see HelpCmd): their number; commands sent, and (helper)
+    // received; acknowledgements received and expected
+    int helpers;
+    int *error;                // set to 1 when a wait gives up
+    int cmd_sent, cmd_seq, acks, ack_goal;
+    int cmd[6];
 };
 
 }  // namespace tcb

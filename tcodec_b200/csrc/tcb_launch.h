@@ -14,7 +14,7 @@ size_t ctu_smem_bytes();
 cudaError_t launch_decode_items(const FrameParams *d_params, const int *d_items, int n, int *d_status,
                                 cudaStream_t st);
 cudaError_t launch_ctu_persistent(const FrameParams *d_params, const int *d_items, int n, int *d_ctrl,
-                                  int grid, cudaStream_t st);
+                                  int grid, int ready, cudaStream_t st);
 cudaError_t launch_ctu_items(const FrameParams *d_params, const int *d_items, int n, cudaStream_t st);
 struct GlobJob {
     const uint8_t *cur, *ref;
