@@ -366,10 +366,11 @@ LG_FN void chroma_block(LState &S, const LFrame &F, bool enc, const uint8_t *ori
 // tc_deblock_ctu).  Every filtered edge only moves p0 / q0 (the strength is
 // never above 2), and the samples one edge writes are never read by another
 // edge of the same pass, so each pass runs all its edges at once.
-LG_FN void deblock_ctu(const LFrame &F, int ox, int oy) {
-    const int L = lane_id(), qp = F.qp, s = F.sy;
+template <class Sync>
+LG_FN void deblock_ctu(const LFrame &F, int ox, int oy, int t, int nt, Sync sync) {
+    const int qp = F.qp, s = F.sy;
     const int tcl = clampi(qp / 3, 1, 10);
-    for (int it = L; it < 64 * 15; it += NL) {           // vertical luma edges: row x edge
+    for (int it = t; it < 64 * 15; it += nt) {           // vertical luma edges: row x edge
         const int row = it / 15, x = ox + (it % 15 + 1) * 4;
         uint8_t *p = F.rec_y + (size_t)(oy + row) * s + x;
         const int p1 = p[-2], p0 = p[-1], q0 = p[0], q1 = p[1];
@@ -377,8 +378,8 @@ LG_FN void deblock_ctu(const LFrame &F, int ox, int oy) {
         p[-1] = (uint8_t)weak_filter(p1, p0, q0, q1, tcl);
         p[0] = (uint8_t)weak_filter(q1, q0, p0, p1, tcl);
     }
-    team_sync();
-    for (int it = L; it < 64 * 15; it += NL) {           // horizontal luma edges: column x edge
+    sync();
+    for (int it = t; it < 64 * 15; it += nt) {           // horizontal luma edges: column x edge
         const int col = it / 15, y = oy + (it % 15 + 1) * 4;
         uint8_t *p = F.rec_y + (size_t)y * s + ox + col;
         const int p1 = p[-2 * s], p0 = p[-s], q0 = p[0], q1 = p[s];
@@ -386,9 +387,9 @@ LG_FN void deblock_ctu(const LFrame &F, int ox, int oy) {
         p[-s] = (uint8_t)weak_filter(p1, p0, q0, q1, tcl);
         p[0] = (uint8_t)weak_filter(q1, q0, p0, p1, tcl);
     }
-    team_sync();
+    sync();
     const int cqp = clampi(qp - 1, 0, 63), tcc = clampi(cqp / 4, 1, 6), sc = F.sc;
-    for (int it = L; it < 32 * 7; it += NL) {            // vertical chroma edges (Cb only)
+    for (int it = t; it < 32 * 7; it += nt) {            // vertical chroma edges (Cb only)
         const int row = it / 7, x = ox / 2 + (it % 7 + 1) * 4;
         uint8_t *p = F.rec_cb + (size_t)(oy / 2 + row) * sc + x;
         const int p0 = p[-1], q0 = p[0];
@@ -397,8 +398,8 @@ LG_FN void deblock_ctu(const LFrame &F, int ox, int oy) {
         p[-1] = (uint8_t)clampi(p0 + d, 0, 255);
         p[0] = (uint8_t)clampi(q0 - d, 0, 255);
     }
-    team_sync();
-    for (int it = L; it < 32 * 7; it += NL) {            // horizontal chroma edges (Cr's strength for both)
+    sync();
+    for (int it = t; it < 32 * 7; it += nt) {            // horizontal chroma edges (Cr's strength for both)
         const int col = it / 7, y = oy / 2 + (it % 7 + 1) * 4, x = ox / 2 + col;
         uint8_t *r = F.rec_cr + (size_t)y * sc + x, *b = F.rec_cb + (size_t)y * sc + x;
         const int p0 = r[0], q0 = r[sc], pb = b[0], qb = b[sc];
@@ -410,7 +411,7 @@ LG_FN void deblock_ctu(const LFrame &F, int ox, int oy) {
         b[0] = (uint8_t)clampi(pb + d, 0, 255);
         b[sc] = (uint8_t)clampi(qb - d, 0, 255);
     }
-    team_sync();
+    sync();
 }
 
 // Evaluate one transform type for the residual: forward transform,
@@ -582,9 +583,9 @@ LG_NOINL void encode_block(LState &S, const LFrame &F, int bi, int fx, int fy, L
     team_sync();
 }
 
-// Reconstruct one 8x8 block from its parsed record (reference
+// Luma of one 8x8 block from its parsed record (reference
 // src/decoder.c:260-650 decode_block, after parsing).
-LG_NOINL void decode_block(LState &S, const LFrame &F, int fx, int fy, const LBlock &in) {
+LG_NOINL void decode_luma(LState &S, const LFrame &F, int fx, int fy, const LBlock &in) {
     const int L = lane_id(), sy = F.sy, W = F.W, H = F.H, ftype = F.frame_type;
     const bool intra = in.mode == 2, skip = in.mode == 0 || in.mode == 3;
     if (intra) {
@@ -619,11 +620,13 @@ LG_NOINL void decode_block(LState &S, const LFrame &F, int fx, int fy, const LBl
             F.rec_y[(size_t)(fy + (i >> 3)) * sy + fx + (i & 7)] = (uint8_t)clampi((int)S.pred[i] + S.inv[i], 0, 255);
     }
     team_sync();
-    const bool cfl = intra;   // intra blocks are never skip / merge
-    int16_t lv[32];
-    for (int i = 0; i < 32; ++i) lv[i] = in.chroma[i];
-    chroma_block(S, F, false, nullptr, F.rec_cb, fx, fy, cfl, lv);
-    chroma_block(S, F, false, nullptr, F.rec_cr, fx, fy, cfl, lv + 16);
+}
+// One component of its chroma, after its luma (intra blocks, never skip or
+// merge, predict from it; no component reads the other).
+LG_FN void decode_chroma(LState &S, const LFrame &F, int comp, int fx, int fy, const LBlock &in) {
+    int16_t lv[16];
+    for (int i = 0; i < 16; ++i) lv[i] = in.chroma[16 * comp + i];
+    chroma_block(S, F, false, nullptr, comp ? F.rec_cr : F.rec_cb, fx, fy, in.mode == 2, lv);
 }
 
 // One CTU: its blocks in raster order, then deblocking when the CTU lies
@@ -644,9 +647,12 @@ LG_FN void code_ctu(LState &S, const LFrame &F, int row, int col, bool enc) {
         const int fx = ox + (b & 7) * 8, fy = oy + (b >> 3) * 8;
         if (fx + 8 > F.W || fy + 8 > F.H) continue;
         if (enc) encode_block(S, F, b, fx, fy, blk[b]);
-        else if (blk[b].coded) decode_block(S, F, fx, fy, blk[b]);
+        else if (blk[b].coded) {
+            decode_luma(S, F, fx, fy, blk[b]);
+            for (int c = 0; c < 2; ++c) decode_chroma(S, F, c, fx, fy, blk[b]);
+        }
     }
-    if (ox + 64 <= F.W && oy + 64 <= F.H) deblock_ctu(F, ox, oy);
+    if (ox + 64 <= F.W && oy + 64 <= F.H) deblock_ctu(F, ox, oy, L, NL, [] { team_sync(); });
 }
 
 }  // namespace legacy
