@@ -113,11 +113,12 @@ __device__ __forceinline__ void store16(uint8_t *p, const uint4 v) {
 // one: load, the two phases, store.  FINE splits the phases into one edge pair
 // (vertical) and one word column (horizontal) per item, 640 and 296 items,
 // instead of a row and 16 columns, 96 and 116 items of eight times the work.
-// One 320x240 frame (15 CTUs), called back to back: 10.5 us with the coarse
-// items, 7.7 fine, of which 7 are the call and the launch.  64 frames of 68x64:
-// 24.6 us byte by byte in two launches, 7.8 with words and in one.
-template <int DFT, bool FINE>
-__global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs J) {
+// 64 frames of 152x94 (128 CTUs): 10.7 us with the coarse items, 8.4 fine; of
+// 68x64: 24.6 us byte by byte in two launches, 8.1 with words and in one.  One
+// 320x240 frame, called back to back, takes 6.9 us either way (start of the
+// call to the launch; 7.9 with one parameter block for 32 frames).
+template <int DFT, bool FINE, int N>
+__global__ void __launch_bounds__(DFT) deblock_frames_kernel(DeblockJobs<N> J) {
     static_assert(DFT >= 32 && DFT % 32 == 0, "whole warps");
     constexpr int NPIECE = (384 + DFT - 1) / DFT;   // 16-byte pieces per thread (384 per CTU)
     __shared__ __align__(16) uint8_t ty[64 * 64];
@@ -297,8 +298,8 @@ __device__ __forceinline__ void sao_count(int *col, int r, int o) {
 // instead of per lane took four times the zeroing and row totals, and the
 // offset on 16-bit pairs twice the instructions of whole words: 3,060 per CTU.
 // 64 planes of 1920x1080: 139 us so, 87 now (398 MB, 4.6 TB/s).
-template <int SFT>
-__global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs J) {
+template <int SFT, int N>
+__global__ void __launch_bounds__(SFT) sao_frames_kernel(SaoJobs<N> J) {
     constexpr int NSEG = 256 / SFT;           // 16-pixel segments per thread
     static_assert(SFT == 64 || SFT == 128, "SAO CTA: 256 16-pixel segments per CTU");
     constexpr int TPR = SFT >= 2 * SAO_ROWS ? 2 : 1;   // threads summing one row
@@ -555,8 +556,9 @@ cudaError_t launch_group_tma(const DeblockFrame *frames, int m, cudaStream_t st,
     return cudaGetLastError();
 }
 
+template <int N>
 cudaError_t launch_group_vec(const DeblockFrame *frames, int m, cudaStream_t st, int threads) {
-    DeblockJobs J;
+    DeblockJobs<N> J;
     J.n = m;
     int total = 0;
     for (int j = 0; j < m; ++j) {
@@ -569,10 +571,10 @@ cudaError_t launch_group_vec(const DeblockFrame *frames, int m, cudaStream_t st,
     const dim3 grid = ctu_grid(frames, m, total, frames[0].W >> 6, frames[0].H >> 6, J.grid3);
     // Few CTUs: at most one per SM, so a CTU's latency is the launch's time.
     constexpr int SMS = 148;
-    if (threads == 64) deblock_frames_kernel<64, false><<<grid, 64, 0, st>>>(J);
-    else if (threads == 256) deblock_frames_kernel<256, false><<<grid, 256, 0, st>>>(J);
-    else if (threads == 0 && total <= SMS) deblock_frames_kernel<320, true><<<grid, 320, 0, st>>>(J);
-    else deblock_frames_kernel<128, false><<<grid, 128, 0, st>>>(J);
+    if (threads == 64) deblock_frames_kernel<64, false, N><<<grid, 64, 0, st>>>(J);
+    else if (threads == 256) deblock_frames_kernel<256, false, N><<<grid, 256, 0, st>>>(J);
+    else if (threads == 0 && total <= SMS) deblock_frames_kernel<320, true, N><<<grid, 320, 0, st>>>(J);
+    else deblock_frames_kernel<128, false, N><<<grid, 128, 0, st>>>(J);
     return cudaGetLastError();
 }
 
@@ -587,35 +589,45 @@ cudaError_t launch_deblock_frames(const DeblockFrame *frames, int n, cudaStream_
         int m = n - i < DeblockTmaJobs::MAX ? n - i : DeblockTmaJobs::MAX;
         bool tma = want_tma && tensor_map_encoder() != nullptr;
         for (int j = 0; tma && j < m; ++j) tma = tma_ok(frames[i + j]);
-        if (!tma && !want_tma) m = n - i < DeblockJobs::MAX ? n - i : DeblockJobs::MAX;
+        if (!want_tma) m = n - i < MANY_FRAMES ? n - i : MANY_FRAMES;
         const cudaError_t e = tma ? launch_group_tma(frames + i, m, st, threads)
-                                  : launch_group_vec(frames + i, m, st, threads);
+                              : m <= FEW_FRAMES ? launch_group_vec<FEW_FRAMES>(frames + i, m, st, threads)
+                                                : launch_group_vec<MANY_FRAMES>(frames + i, m, st, threads);
         if (e != cudaSuccess) return e;
         i += m;
     }
     return cudaSuccess;
 }
 
+namespace {
+
+template <int N>
+cudaError_t launch_sao_group(const SaoFrame *frames, int m, cudaStream_t st, int threads) {
+    SaoJobs<N> J;
+    J.n = m;
+    int total = 0;
+    for (int j = 0; j < m; ++j) {
+        J.f[j] = frames[j];
+        J.ctu_off[j] = total;
+        total += ((frames[j].W + 63) >> 6) * ((frames[j].H + 63) >> 6);
+    }
+    J.ctu_off[m] = total;
+    if (total == 0) return cudaSuccess;
+    const dim3 grid = ctu_grid(frames, m, total, (frames[0].W + 63) >> 6, (frames[0].H + 63) >> 6, J.grid3);
+    if (threads == 64) sao_frames_kernel<64, N><<<grid, 64, 0, st>>>(J);
+    else sao_frames_kernel<128, N><<<grid, 128, 0, st>>>(J);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_sao_frames(const SaoFrame *frames, int n, cudaStream_t st, int threads) {
     for (int i = 0; i < n;) {
-        SaoJobs J;
-        J.n = 0;
-        int total = 0;
-        while (i < n && J.n < SaoJobs::MAX) {
-            J.f[J.n] = frames[i];
-            J.ctu_off[J.n] = total;
-            total += ((frames[i].W + 63) >> 6) * ((frames[i].H + 63) >> 6);
-            ++J.n;
-            ++i;
-        }
-        J.ctu_off[J.n] = total;
-        if (total > 0) {
-            const dim3 grid = ctu_grid(J.f, J.n, total, (J.f[0].W + 63) >> 6, (J.f[0].H + 63) >> 6, J.grid3);
-            if (threads == 64) sao_frames_kernel<64><<<grid, 64, 0, st>>>(J);
-            else sao_frames_kernel<128><<<grid, 128, 0, st>>>(J);
-            const cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return e;
-        }
+        const int m = n - i < MANY_FRAMES ? n - i : MANY_FRAMES;
+        const cudaError_t e = m <= FEW_FRAMES ? launch_sao_group<FEW_FRAMES>(frames + i, m, st, threads)
+                                              : launch_sao_group<MANY_FRAMES>(frames + i, m, st, threads);
+        if (e != cudaSuccess) return e;
+        i += m;
     }
     return cudaSuccess;
 }

@@ -32,8 +32,9 @@ struct McFrame {
     const int16_t *mv;
     int W, H, sy, sc;
 };
+template <int N>                     // FEW_FRAMES or MANY_FRAMES
 struct McJobs {                      // passed by value as the kernel parameter
-    static constexpr int MAX = 64;
+    static constexpr int MAX = N;
     int n;
     int cta_off[MAX + 1];            // first CTA of each frame
     McFrame f[MAX];
@@ -142,8 +143,8 @@ __device__ __noinline__ void mc_edge_samples(const McFrame F, int g0, const uint
     }
 }
 
-template <int MT>
-__global__ void __launch_bounds__(MT, 1024 / MT) mc_frames_kernel(McJobs J) {
+template <int MT, int N>
+__global__ void __launch_bounds__(MT, 1024 / MT) mc_frames_kernel(McJobs<N> J) {
     __shared__ uint16_t q_luma[MT], q_chroma[MT];   // threads whose block takes the per-sample path
     __shared__ int n_luma, n_chroma;
     if (threadIdx.x == 0) n_luma = n_chroma = 0;
@@ -214,30 +215,36 @@ __global__ void __launch_bounds__(MT, 1024 / MT) mc_frames_kernel(McJobs J) {
     if (n_luma | n_chroma) mc_edge_samples<MT>(F, g0, q_luma, n_luma, q_chroma, n_chroma);
 }
 
+template <int N>
+cudaError_t launch_mc_group(const tcb_mc_frame_t *frames, int m, cudaStream_t st, int MT) {
+    McJobs<N> J;
+    J.n = m;
+    int total = 0;
+    for (int j = 0; j < m; ++j) {
+        const tcb_mc_frame_t &f = frames[j];
+        J.f[j] = {f.ref_y, f.ref_cb, f.ref_cr, f.pred_y, f.pred_cb, f.pred_cr, f.mv,
+                  f.width, f.height, f.stride_y, f.stride_c};
+        J.cta_off[j] = total;
+        const int blocks = ((f.width + 7) >> 3) * ((f.height + 7) >> 3);
+        total += (2 * blocks + MT - 1) / MT;
+    }
+    J.cta_off[m] = total;
+    if (MT == 64) mc_frames_kernel<64, N><<<total, 64, 0, st>>>(J);
+    else if (MT == 128) mc_frames_kernel<128, N><<<total, 128, 0, st>>>(J);
+    else mc_frames_kernel<256, N><<<total, 256, 0, st>>>(J);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_mc_frames(const tcb_mc_frame_t *frames, int n, cudaStream_t st, int threads) {
     const int MT = (threads == 64 || threads == 128) ? threads : MC_DEFAULT_THREADS;
     for (int i = 0; i < n;) {
-        McJobs J;
-        J.n = 0;
-        int total = 0;
-        while (i < n && J.n < McJobs::MAX) {
-            const tcb_mc_frame_t &f = frames[i];
-            J.f[J.n] = {f.ref_y, f.ref_cb, f.ref_cr, f.pred_y, f.pred_cb, f.pred_cr, f.mv,
-                        f.width, f.height, f.stride_y, f.stride_c};
-            J.cta_off[J.n] = total;
-            const int blocks = ((f.width + 7) >> 3) * ((f.height + 7) >> 3);
-            total += (2 * blocks + MT - 1) / MT;
-            ++J.n;
-            ++i;
-        }
-        J.cta_off[J.n] = total;
-        if (MT == 64) mc_frames_kernel<64><<<total, 64, 0, st>>>(J);
-        else if (MT == 128) mc_frames_kernel<128><<<total, 128, 0, st>>>(J);
-        else mc_frames_kernel<256><<<total, 256, 0, st>>>(J);
-        const cudaError_t e = cudaGetLastError();
+        const int m = n - i < MANY_FRAMES ? n - i : MANY_FRAMES;
+        const cudaError_t e = m <= FEW_FRAMES ? launch_mc_group<FEW_FRAMES>(frames + i, m, st, MT)
+                                              : launch_mc_group<MANY_FRAMES>(frames + i, m, st, MT);
         if (e != cudaSuccess) return e;
+        i += m;
     }
     return cudaSuccess;
 }
