@@ -74,7 +74,6 @@ struct FrameParams {
     int lambda_c;                              // chroma RDOQ lambda
     int lambda_sao;                            // SAO gate lambda
     int eff_l[4], eff_c[4];                    // per-band quant steps
-    uint32_t rcp_l[4], rcp_c[4];               // exact reciprocals of eff
     int32_t *err;                              // device error word
     int *done;                                 // per-CTU publish flags (persistent wavefront)
     int epoch;                                 // value this frame publishes in `done`
@@ -112,27 +111,7 @@ TCB_HD int qt_index(int depth, int cx, int cy) {
     return base + ((cy >> shift) << depth) + (cx >> shift);
 }
 
-// Dead-zone quantizer (reference tcodec_common.h:232-238) with the divide
-// replaced by an exact reciprocal: for eff in [2, 2^13] and numerators
-// below 2^16, umulhi(n, floor(2^32/eff) + 1) == n / eff (checked
-// exhaustively by the oracle tests).  eff == 1 is the identity.
-TCB_HD uint32_t quant_rcp(int eff) {
-    return eff <= 1 ? 0u : (uint32_t)(0x100000000ull / (uint32_t)eff + 1ull);
-}
-TCB_HD int udiv_rcp(uint32_t n, int eff, uint32_t rcp) {
-#ifdef __CUDA_ARCH__
-    return eff <= 1 ? (int)n : (int)__umulhi(n, rcp);
-#else
-    return eff <= 1 ? (int)n : (int)(((uint64_t)n * rcp) >> 32);
-#endif
-}
-TCB_HD int quant_coeff(int c, int eff, uint32_t rcp) {
-    const int off = eff / 3;
-    if (c > 0) return udiv_rcp((uint32_t)(c + off), eff, rcp);
-    if (c < 0) return -udiv_rcp((uint32_t)(-c + off), eff, rcp);
-    return 0;
-}
-// Centroid dequantizer (reference tcodec_common.h:240-246).
+// Dequantizer (reference tcodec_common.h:240-246).
 TCB_HD int dequant_coeff(int q, int eff) {
     const int bias = eff / 6;
     return q > 0 ? q * eff + bias : (q < 0 ? q * eff - bias : 0);

@@ -396,8 +396,8 @@ tc_error_t EncImpl::stage_b() {
     P.lambda_c = tc_lambda_host(P.qp_c);
     P.lambda_sao = tc_lambda_host(qp);
     for (int b = 0; b < 4; ++b) {
-        P.eff_l[b] = eff_scale(qp, b); P.rcp_l[b] = quant_rcp(P.eff_l[b]);
-        P.eff_c[b] = eff_scale(P.qp_c, b); P.rcp_c[b] = quant_rcp(P.eff_c[b]);
+        P.eff_l[b] = eff_scale(qp, b);
+        P.eff_c[b] = eff_scale(P.qp_c, b);
     }
     P.err = d_err;
     P.done = d_done;
@@ -794,8 +794,8 @@ bool tcb::frame_params_from_desc(const tcb_frame_desc_t &d, FrameParams &P) {
     P.lambda_c = tc_lambda_host(P.qp_c);
     P.lambda_sao = tc_lambda_host(d.qp);
     for (int b = 0; b < 4; ++b) {
-        P.eff_l[b] = eff_scale(d.qp, b); P.rcp_l[b] = quant_rcp(P.eff_l[b]);
-        P.eff_c[b] = eff_scale(P.qp_c, b); P.rcp_c[b] = quant_rcp(P.eff_c[b]);
+        P.eff_l[b] = eff_scale(d.qp, b);
+        P.eff_c[b] = eff_scale(P.qp_c, b);
     }
     P.search_window = engine_tuning(d.width, d.height).search_window;
     return true;

@@ -5,14 +5,13 @@
 // shared memory:
 //
 //   decide pass  recursive quadtree RDO (reference src/encoder.c:1292-1397
-//                qt_split) over leaves (src/encoder.c:562-1290 qt_leaf);
-//                inside a leaf all candidates run concurrently: four motion
-//                searches on four warp groups, then every (candidate, TU
-//                size, TU) residual coding job on octets / quads of lanes,
-//                then an in-order strict-< scan that reproduces the
-//                reference's first-minimum tie rule;
-//   write pass   replays the chosen tree in z-order, emitting quantised
-//                coefficients (src/encoder.c:1450-1456);
+//                qt_split) over leaves (src/encoder.c:562-1290 qt_leaf):
+//                inside a leaf the motion searches run on warp groups while
+//                the other warps score the intra modes, an 8x8 area a warp on
+//                the matrix instructions; then an in-order strict-< scan
+//                reproduces the reference's first-minimum tie rule, and the
+//                winner is coded into the tile and the CTU's record
+//                (src/encoder.c:1450-1456);
 //   filters      deblocking of the CTU's inner edges (src/filter.c:175-237)
 //                and the luma SAO band-offset choice, rate gate and
 //                application (src/filter.c:245-319, src/encoder.c:1463-1506);
@@ -20,8 +19,8 @@
 //                CTU record the host range coder consumes.
 //
 // CTUs of one frame run as an anti-diagonal wavefront: CTU (r, c) reads the
-// filtered reconstruction of (r, c-1), (r-1, c) and (r-1, c-1) only, so all
-// CTUs with the same r + c are independent and go in one launch.
+// filtered reconstruction of (r, c-1), (r-1, c) and (r-1, c-1) only.  Where that
+// leaves SMs idle, helper CTAs share the large leaves of a CTU (see below).
 #include <mutex>
 
 #include "tcb_engine.cuh"
