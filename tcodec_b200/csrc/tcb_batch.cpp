@@ -95,7 +95,9 @@ std::vector<cudaGraphNode_t> graph_nodes(cudaGraph_t g) {
     return nodes;
 }
 
-// FNV-1a over the node types and kernel functions of a captured graph.
+// FNV-1a over the node types, kernel functions and cluster sizes of a captured
+// graph (an executable graph takes new kernel parameters, but no new cluster
+// size, which follows the streams of a step).
 uint64_t graph_signature(const std::vector<cudaGraphNode_t> &nodes) {
     uint64_t h = 1469598103934665603ull;
     auto mix = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
@@ -108,6 +110,12 @@ uint64_t graph_signature(const std::vector<cudaGraphNode_t> &nodes) {
             cudaKernelNodeParams kp;
             if (cudaGraphKernelNodeGetParams(nd, &kp) != cudaSuccess) return 0;
             mix((uint64_t)(uintptr_t)kp.func);
+            cudaLaunchAttributeValue at = {};
+            if (cudaGraphKernelNodeGetAttribute(nd, cudaLaunchAttributeClusterDimension, &at) != cudaSuccess) {
+                cudaGetLastError();
+                at.clusterDim.x = 0;
+            }
+            mix((uint64_t)at.clusterDim.x);
         }
     }
     return h;

@@ -1968,7 +1968,7 @@ __device__ void help(Smem &S, const FrameParams *__restrict__ params, int *ctrl)
         bool got = false;
         if (threadIdx.x == 0) {
             // far longer than the first CTA waits for its neighbours
-            const long long limit = 4 * g_neighbor_wait_limit + (1ll << 24);
+            const long long w = g_neighbor_wait_limit, limit = w < 1ll << 60 ? 4 * w + (1ll << 24) : w;
             unsigned ns = 32;
             for (long long i = 0; i < limit && !got; ++i) {
                 got = ld_acquire_cluster(&S.cmd_seq) >= seq;

@@ -54,3 +54,25 @@ def test_mixed_presets_share_a_clustered_launch():
     cfgs = [api.make_config(lib, w, h, qp=30, preset=p, profile=1, keyframe_interval=1000) for w, h, p in shapes]
     for got, cfg, clip in zip(_batch(lib, cfgs, clips), cfgs, clips):
         assert got == api.encode_sequence(lib, cfg, clip)
+
+
+def test_replayed_graphs_follow_the_cluster_size():
+    """Steps with the same nodes whose streams ask for clusters in one step and
+    for single CTAs in the next."""
+    from tcodec_b200 import api
+    lib = api.load_library()
+    shapes = [(128, 128, 2), (128, 128, 0), (320, 256, 2)]
+    clips = [_clip(w, h, 4, w) for w, h, _ in shapes]
+    cfgs = [api.make_config(lib, w, h, qp=30, preset=p, profile=0, keyframe_interval=1) for w, h, p in shapes]
+    batch = api.BatchEncoder(lib, cfgs)
+    batch.set_graphs(True)
+    got = [[] for _ in cfgs]
+    try:
+        for t in range(4):
+            for turn in range(3):
+                packets = batch.encode([clips[i][t] if i == turn else None for i in range(3)])
+                got[turn].append(packets[turn])
+    finally:
+        batch.close()
+    for g, cfg, clip in zip(got, cfgs, clips):
+        assert g == api.encode_sequence(lib, cfg, clip)
