@@ -1008,11 +1008,11 @@ __device__ __noinline__ void luma_score(const Leaf L, const int *cl, int ncl, in
     Smem &S = smem_state();
     Smem *const M = HELP ? peer_smem(0) : nullptr;      // a helper's queue and sums are the first CTA's
     // the next item: a helper asks for it one item ahead
-    const int lane_ = threadIdx.x & 31;
-    auto claim = [&] { return lane_ == 0 ? HELP ? atomicAdd(&M->next[queue], 1) : atomicAdd(&S.next[queue], 1) : 0; };
+    const int lane = threadIdx.x & 31;
+    auto claim = [&] { return lane == 0 ? HELP ? atomicAdd(&M->next[queue], 1) : atomicAdd(&S.next[queue], 1) : 0; };
     int ahead = HELP ? claim() : 0;
     const int cu = L.cu, lt = lg2i(cu) - 3, la = 2 * lt;
-    const int lane = threadIdx.x & 31, row = lane >> 2, col = 2 * (lane & 3);
+    const int row = lane >> 2, col = 2 * (lane & 3);
     const uint2 f8 = S.frag[0][lane], i8 = S.frag[1][lane], f4 = S.frag[2][lane], i4 = S.frag[3][lane];
     const QuantLane q8 = quant_lane(S, 0, lane), q4 = quant_lane(S, 1, lane);
 #ifdef TCB_PHASE_PROFILE
