@@ -293,7 +293,7 @@ typedef struct tcb_mc_frame {
  * 4x4 chroma blocks predicted from the reference at the block's vector,
  * exactly as tc_inter_predict / tc_inter_predict_chroma (reference
  * src/motion.c:493-632) with an 8x8 block; samples beyond the frame are not
- * written.  One launch per 32 frames. */
+ * written.  One launch per 64 frames. */
 tc_error_t tcb_mc_frames(const tcb_mc_frame_t *frames, int n, void *stream);
 
 /* One frame for the standalone in-loop filters.  Device pointers; the
@@ -311,7 +311,7 @@ typedef struct tcb_filter_frame {
 /* Deblocking of the internal 4-pixel edges of every full 64x64 CTU of n
  * frames (partial CTUs at the right / bottom border are left alone, as in
  * the reference): replaces tc_deblock_ctu (reference src/filter.c:23-237)
- * as called per CTU at src/encoder.c:1457-1458.  One launch per 32 frames. */
+ * as called per CTU at src/encoder.c:1457-1458.  One launch per 64 frames (32 with TMA staging). */
 tc_error_t tcb_deblock_frames(const tcb_filter_frame_t *frames, int n, void *stream);
 
 /* Luma SAO band offset of every CTU of n frames: choose
