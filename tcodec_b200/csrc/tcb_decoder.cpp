@@ -88,8 +88,12 @@ void resolve_vectors(CtuOut &o, int ctu_x, int ctu_y, int W, int H) {
 namespace tcb {
 
 struct DecImpl {
-    int W = 0, H = 0;                 // decoder geometry (dec->width/height)
-    int fw = 0, fh = 0, sy = 0, sc = 0, cols = 0, rows = 0;   // allocated frame geometry
+    // The size callers are told (tc_decoder_get_info): the one given at
+    // creation, else the first packet's.  It does not follow later packets.
+    int W = 0, H = 0;
+    // The size of the packet at hand, which the buffers, the parser and the
+    // kernels all go by.
+    int fw = 0, fh = 0, sy = 0, sc = 0, cols = 0, rows = 0;
     int device = 0;
     cudaStream_t st = nullptr;
     DevFrame cur;                     // persistent reconstruction target
@@ -156,7 +160,9 @@ struct DecImpl {
         cols = (w + 63) / 64;
         rows = (h + 63) / 64;
         if (!alloc_frame(cur)) return false;
-        out = tcb_host_frame_alloc(w, h, 1);
+        // room for the size callers are told: a smaller picture lies in its
+        // upper left corner
+        out = tcb_host_frame_alloc(std::max(w, std::min(W, TC_MAX_WIDTH)), std::max(h, std::min(H, TC_MAX_HEIGHT)), 1);
         return out != nullptr;
     }
     // Records and work lists of the kind of stream at hand, on its first packet:
@@ -247,6 +253,11 @@ struct DecImpl {
                 tc_frame_buf_t *f = disp_frames[i];
                 const int cw = (disp_out->width < f->width ? disp_out->width : f->width);
                 const int chh = (disp_out->height < f->height ? disp_out->height : f->height);
+                if (cw < disp_out->width || chh < disp_out->height) {   // nothing of an earlier, larger picture
+                    memset(disp_out->y, 0, (size_t)disp_out->stride_y * disp_out->height);
+                    memset(disp_out->cb, 0, (size_t)disp_out->stride_c * (disp_out->height / 2));
+                    memset(disp_out->cr, 0, (size_t)disp_out->stride_c * (disp_out->height / 2));
+                }
                 for (int r = 0; r < chh; ++r) memcpy(disp_out->y + (size_t)r * disp_out->stride_y, f->y + (size_t)r * f->stride_y, cw);
                 for (int r = 0; r < chh / 2; ++r) {
                     memcpy(disp_out->cb + (size_t)r * disp_out->stride_c, f->cb + (size_t)r * f->stride_c, cw / 2);
@@ -310,7 +321,7 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
                 p.o = h_rec + row * cols + col;
                 p.ctu(row, col);
                 if (r.error) return false;
-                resolve_vectors(*p.o, col * 64, row * 64, W, H);
+                resolve_vectors(*p.o, col * 64, row * 64, fw, fh);
             }
         return true;
     };
@@ -380,7 +391,7 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
     // ---- device reconstruction ------------------------------------------
     FrameParams P;
     memset(&P, 0, sizeof(P));
-    P.W = W; P.H = H; P.stride_y = sy; P.stride_c = sc; P.ctu_cols = cols; P.ctu_rows = rows;
+    P.W = fw; P.H = fh; P.stride_y = sy; P.stride_c = sc; P.ctu_cols = cols; P.ctu_rows = rows;
     P.rec_y = cur.y; P.rec_cb = cur.cb; P.rec_cr = cur.cr;
     for (int i = 0; i < MAX_REFS; ++i) {
         P.ref_valid[i] = dpb_ok[i];
