@@ -256,7 +256,9 @@ tc_error_t tcb_ctu_frame_result(const void *scratch, void *stream);
 tc_error_t tcb_ctu_frame_result_static(void *stream);
 
 /* Bound of a CTU's wait for a neighbour's publish flag, in back-off
- * iterations of at most 2,048 ns each; default 2^22 (about 8.6 s).  Set
+ * iterations of at most 2,048 ns each; default 2^22 (about 8.6 s).  The
+ * wait for the CTAs that help with a CTU has the same bound, after some
+ * milliseconds of polling.  Set
  * for the current device; applies to every CTU-engine launch on it
  * (frame entry points, encoders, batches, served sessions) that starts
  * afterwards.  spins < 1 returns TC_ERR_PARAM. */
@@ -270,6 +272,15 @@ tc_error_t tcb_get_neighbor_wait_limit(long long *spins);
  * usable.  Frames of at least 2 CTUs. */
 tc_error_t tcb_debug_ctu_encode_frame_without_first(const tcb_frame_desc_t *desc, void *scratch,
                                                     size_t scratch_bytes, void *stream);
+
+/* Test hook: tcb_ctu_encode_frame in which the first of the CTAs that help
+ * with a CTU (presets from MEDIUM on, frames that leave SMs idle) leaves at
+ * its `commands`-th command (>= 1) without an answer.  The wait for it runs
+ * out once per CTA group (bounded, see above), the frame is finished without
+ * helpers and tcb_ctu_frame_result reports TC_ERR_INTERNAL; the device
+ * context stays usable. */
+tc_error_t tcb_debug_ctu_encode_frame_helper_quits(const tcb_frame_desc_t *desc, void *scratch,
+                                                   size_t scratch_bytes, void *stream, int commands);
 
 /* Test hook: the next n device or pinned-host allocations of the library
  * succeed and the one after fails, once (n < 0: none).  Returns the count

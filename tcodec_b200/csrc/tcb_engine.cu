@@ -170,11 +170,18 @@ __device__ void mvp_at(const MvCell *grid, int cx, int cy, int &mx, int &my) {
 // not depend on who computes it.
 //
 // Protocol: the first CTA writes cmd (and the samples) into a helper's shared
-// memory, then its cmd_seq; the helper answers every command by adding 1 to
-// the first CTA's acks once its results are written.  The first CTA waits for
-// all acks of a command before it sends the next.  Waits are bounded; one that
-// gives up reports an error (ctrl[1]) and the CTA goes on, or (helper) to the
-// cluster barrier that ends the kernel, so no shared memory is released
+// memory, then its cmd_seq, one more than the command before; the helper
+// answers by adding 1 to the first CTA's acks once its results are written.
+// The first CTA waits for all acks of a command before it sends the next, so a
+// helper never reads a command that is being written.  CMD_LEAVE in cmd_seq
+// ends a helper; no other word goes with it.
+//
+// Waits are bounded.  If the first CTA's gives up it reports an error (ctrl[1])
+// and is without helpers from then on: it sends no command any more, only
+// CMD_LEAVE at its end, because a late helper may still be at the last one
+// (its results land in bounds, in a frame that is an error by then).  A helper
+// whose wait gives up, or that finds anything but the next command, leaves.
+// Every CTA ends at a barrier of the cluster, so no shared memory is released
 // while another CTA may still write to it.
 //
 // Leaves from 32x32 on only (at 16x16 the round trip, about 3,000 cycles, takes
@@ -182,7 +189,18 @@ __device__ void mvp_at(const MvCell *grid, int cx, int cy, int &mx, int &my) {
 // takes 199,000 / 86,000 cycles alone and 98,000 / 60,000 with three helpers,
 // bound by the longest search.
 // ====================================================================
-enum HelpCmd { HELP_EXIT, HELP_CTU, HELP_LEAF };
+enum HelpCmd { HELP_CTU, HELP_LEAF };
+constexpr int CMD_LEAVE = 0x7FFFFFFF;
+
+// Bound of a neighbour wait, in back-off iterations (sleeps of 32 ns
+// doubling to 2,048 ns): the default 2^22 is about 8.6 s, far above a
+// CTU's encode time even when the GPU is time-shared.  Per device; set by
+// tcb_set_neighbor_wait_limit.
+__device__ long long g_neighbor_wait_limit = 1ll << 22;
+// Waits inside a CTU or a cluster poll this often before they begin to sleep
+// and count towards that limit (some milliseconds; the longest share of a leaf
+// takes 0.1 ms).
+constexpr int WAIT_POLLS = 1 << 16;
 
 __device__ __forceinline__ Smem *peer_smem(int rank) {
     uint64_t p;
@@ -238,13 +256,31 @@ __device__ __noinline__ void send_command(int c0, int c1, int c2, int c3, int c4
             asm volatile("st.release.cluster.s32 [%0], %1;" ::"l"(&peer_smem(r)->cmd_seq), "r"(seq) : "memory");
     }
 }
+// The helpers' end.  By the last warp.
+__device__ __noinline__ void send_leave() {
+    if (threadIdx.x < NT - 32) return;
+    const int r = threadIdx.x & 31;
+    if (r > 0 && r < cluster_size())
+        asm volatile("st.release.cluster.s32 [%0], %1;" ::"l"(&peer_smem(r)->cmd_seq), "r"(CMD_LEAVE) : "memory");
+}
 // Thread 0 waits for the helpers' acks; a barrier of the CTA follows.
+__device__ __noinline__ void wait_helpers_slowly(Smem &S, int goal) {
+    const long long limit = g_neighbor_wait_limit;
+    unsigned ns = 32;
+    for (long long i = 0; i < limit; ++i) {
+        if (ld_acquire_cluster(&S.acks) >= goal) return;
+        __nanosleep(ns);
+        if (ns < 1024) ns <<= 1;
+    }
+    atomicExch(S.error, 1);
+    S.helpers = 0;
+}
 __device__ __forceinline__ void wait_helpers(Smem &S) {
     if (threadIdx.x != 0 || S.helpers == 0) return;
     const int goal = S.ack_goal;
-    for (int i = 0; i < (1 << 24); ++i)
+    for (int i = 0; i < WAIT_POLLS; ++i)
         if (ld_acquire_cluster(&S.acks) >= goal) return;
-    atomicExch(S.error, 1);
+    wait_helpers_slowly(S, goal);
 }
 // A helper's answer: everything its threads have written is the first CTA's
 // to read.
@@ -1896,12 +1932,6 @@ __device__ __noinline__ void sao_tile(Smem &, int w, int h, int lambda_sao) {
     SYNC();
 }
 
-// Bound of a neighbour wait, in back-off iterations (sleeps of 32 ns
-// doubling to 2,048 ns): the default 2^22 is about 8.6 s, far above a
-// CTU's encode time even when the GPU is time-shared.  Per device; set by
-// tcb_set_neighbor_wait_limit.
-__device__ long long g_neighbor_wait_limit = 1ll << 22;
-
 // What a CTU's searches and scoring work from: its source luma, every lane's
 // quantisers, empty SAD tables.
 __device__ void load_luma(Smem &S, const FrameParams &P, int ctu_x, int ctu_y) {
@@ -1961,27 +1991,26 @@ __device__ __noinline__ void help_leaf(const Leaf L, int mvpx, int mvpy) {
     luma_score<true>(L, S.cl, __popc(modes), 0, ~0u);
 }
 
-// A helper's life: commands until HELP_EXIT.
+// A helper's life: commands until CMD_LEAVE.
 __device__ void help(Smem &S, const FrameParams *__restrict__ params, int *ctrl) {
     int ctu_x = 0, ctu_y = 0;
     for (int seq = 1;; ++seq) {
-        bool got = false;
+        int got = 0;
         if (threadIdx.x == 0) {
             // far longer than the first CTA waits for its neighbours
             const long long w = g_neighbor_wait_limit, limit = w < 1ll << 60 ? 4 * w + (1ll << 24) : w;
             unsigned ns = 32;
-            for (long long i = 0; i < limit && !got; ++i) {
-                got = ld_acquire_cluster(&S.cmd_seq) >= seq;
-                if (!got && i > 4096) {
+            for (long long i = 0; i < limit && got < seq; ++i) {
+                got = ld_acquire_cluster(&S.cmd_seq);
+                if (got < seq && i > 4096) {
                     __nanosleep(ns);
                     if (ns < 1024) ns <<= 1;
                 }
             }
-            if (!got) atomicExch(&ctrl[1], 1);
+            if (got < seq) atomicExch(&ctrl[1], 1);
         }
-        if (!__syncthreads_or(got)) return;
+        if (!__syncthreads_or(got == seq)) return;
         const int c0 = S.cmd[0], c1 = S.cmd[1], c2 = S.cmd[2], c3 = S.cmd[3], c4 = S.cmd[4], c5 = S.cmd[5];
-        if (c0 == HELP_EXIT) return;
         if (c0 == HELP_CTU) {
             if (threadIdx.x == 0) g_fp = params[c1 >> 20];
             SYNC();
@@ -1991,6 +2020,8 @@ __device__ void help(Smem &S, const FrameParams *__restrict__ params, int *ctrl)
         } else {
             help_leaf(Leaf(g_fp, ctu_x, ctu_y, c1, c2, c3), c4, c5);
         }
+        // (test hook: the first helper leaves without an answer)
+        if (g_fp.helper_quits && seq >= g_fp.helper_quits && cluster_rank() == 1) return;
         acknowledge();
     }
 }
@@ -2133,13 +2164,13 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
     FrameParams &P = g_fp;
     __shared__ int s_item;
     init_fragments(S);    // visible to all after the first item's barrier
-    const int helpers = cluster_size() - 1;
+    const bool cluster = cluster_size() > 1;
     if (threadIdx.x == 0) {
-        S.helpers = helpers;
+        S.helpers = cluster_size() - 1;
         S.cmd_sent = S.cmd_seq = S.acks = S.ack_goal = 0;
         S.error = ctrl + 1;
     }
-    if (helpers) {
+    if (cluster) {
         cluster_barrier();    // every CTA's counters are set
         if (cluster_rank() > 0) {
             help(S, params, ctrl);
@@ -2164,7 +2195,7 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
             break;
         }
         const int row = (item >> 10) & 1023, col = item & 1023;
-        if (helpers) send_command(HELP_CTU, item, 0, 0, 0, 0);
+        if (S.helpers) send_command(HELP_CTU, item, 0, 0, 0, 0);
         if (threadIdx.x == 0) {
             P = params[item >> 20];
             const int epoch = P.epoch;
@@ -2191,9 +2222,8 @@ ctu_persistent_kernel(const FrameParams *__restrict__ params, const int *__restr
         SYNC();
         if (threadIdx.x == 0) st_release(P.done + row * P.ctu_cols + col, P.epoch);
     }
-    if (helpers) {
-        send_command(HELP_EXIT, 0, 0, 0, 0, 0);
-        SYNC();
+    if (cluster) {
+        send_leave();
         cluster_barrier();
     }
 }
@@ -2254,8 +2284,11 @@ __global__ void frame_setup_kernel(FrameParams P, uint8_t *__restrict__ scratch)
 // and nothing is copied from host memory.  `first` > 0 leaves the queue's
 // first items out (the wait-expiry test hook: their publish flags are
 // never set, so their neighbours' bounded waits run out).
-cudaError_t encode_frame_with_scratch(const FrameParams &P0, uint8_t *scratch, cudaStream_t st, int first) {
+// `helper_quits`: see FrameParams.
+cudaError_t encode_frame_with_scratch(const FrameParams &P0, uint8_t *scratch, cudaStream_t st, int first,
+                                      int helper_quits = 0) {
     FrameParams P = P0;
+    P.helper_quits = helper_quits;
     const int nctu = P.ctu_cols * P.ctu_rows;
     int *ctrl = (int *)(scratch + SCR_CTRL), *done = (int *)(scratch + SCR_DONE), *items = done + nctu;
     P.done = done;
@@ -2430,6 +2463,16 @@ tc_error_t tcb_set_neighbor_wait_limit(long long spins) {
 tc_error_t tcb_get_neighbor_wait_limit(long long *spins) {
     if (!spins) return TC_ERR_PARAM;
     return cudaMemcpyFromSymbol(spins, tcb::g_neighbor_wait_limit, sizeof(*spins)) == cudaSuccess
+               ? TC_OK : TC_ERR_INTERNAL;
+}
+
+tc_error_t tcb_debug_ctu_encode_frame_helper_quits(const tcb_frame_desc_t *desc, void *scratch, size_t scratch_bytes,
+                                                   void *stream, int commands) {
+    tcb::FrameParams P;
+    if (!desc || !scratch || commands < 1 || !tcb::frame_params_from_desc(*desc, P)) return TC_ERR_PARAM;
+    if (scratch_bytes < tcb::scratch_bytes_for(P.ctu_cols * P.ctu_rows)) return TC_ERR_PARAM;
+    if (tcb::ensure_device_tables() != cudaSuccess) return TC_ERR_INTERNAL;
+    return tcb::encode_frame_with_scratch(P, (uint8_t *)scratch, (cudaStream_t)stream, 0, commands) == cudaSuccess
                ? TC_OK : TC_ERR_INTERNAL;
 }
 
