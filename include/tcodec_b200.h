@@ -257,8 +257,9 @@ tc_error_t tcb_ctu_frame_result_static(void *stream);
 
 /* Bound of a CTU's wait for a neighbour's publish flag, in back-off
  * iterations of at most 2,048 ns each; default 2^22 (about 8.6 s).  The
- * wait for the CTAs that help with a CTU has the same bound, after some
- * milliseconds of polling.  Set
+ * waits for the CTAs that help with a CTU and, in the decoder, for the areas
+ * an intra area reads have the same bound, after some milliseconds of polling
+ * and with shorter sleeps.  Set
  * for the current device; applies to every CTU-engine launch on it
  * (frame entry points, encoders, batches, served sessions) that starts
  * afterwards.  spins < 1 returns TC_ERR_PARAM. */
@@ -281,6 +282,12 @@ tc_error_t tcb_debug_ctu_encode_frame_without_first(const tcb_frame_desc_t *desc
  * context stays usable. */
 tc_error_t tcb_debug_ctu_encode_frame_helper_quits(const tcb_frame_desc_t *desc, void *scratch,
                                                    size_t scratch_bytes, void *stream, int commands);
+
+/* Test hook: in the next v2 packet of a decoder the first 8x8 area of every
+ * CTU never counts as done, so areas of intra leaves beside it give up waiting
+ * (bounded, see tcb_set_neighbor_wait_limit).  tc_decoder_decode then returns
+ * TC_ERR_INTERNAL with the decoder as it was before the packet. */
+tc_error_t tcb_debug_decoder_lose_area(tc_decoder_t *dec);
 
 /* Test hook: the next n device or pinned-host allocations of the library
  * succeed and the one after fails, once (n < 0: none).  Returns the count

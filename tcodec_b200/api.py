@@ -374,6 +374,8 @@ def bind_b200(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.tcb_debug_ctu_encode_frame_helper_quits.argtypes = [ctypes.POINTER(FrameDesc), vp, ctypes.c_size_t, vp,
                                                             ctypes.c_int]
     lib.tcb_debug_ctu_encode_frame_helper_quits.restype = ctypes.c_int
+    lib.tcb_debug_decoder_lose_area.argtypes = [vp]
+    lib.tcb_debug_decoder_lose_area.restype = ctypes.c_int
     lib.tcb_debug_fail_allocations_after.argtypes = [ctypes.c_longlong]
     lib.tcb_debug_fail_allocations_after.restype = ctypes.c_longlong
     for fn in (lib.tcb_deblock_frames, lib.tcb_sao_frames):

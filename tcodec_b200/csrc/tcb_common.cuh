@@ -78,6 +78,7 @@ struct FrameParams {
     int *done;                                 // per-CTU publish flags (persistent wavefront)
     int epoch;                                 // value this frame publishes in `done`
     int search_window;                         // radius (2..5) of the search's SAD tables (engine tuning)
+    int lose_area;                             // test hook: the first area of each decoded CTU never counts as done
     int helper_quits;                          // test hook: a cluster's first helper CTA leaves at this command, unanswered (0: never)
 };
 

@@ -44,18 +44,20 @@ struct DecSmem {
     int scratch[NW][64];
 };
 
-// Waits until the cells [x0, x1) x [y0, y1) are done.  They come earlier in
-// z-order, so their warps are already running; the bound only guards against
-// a fault elsewhere, and the caller then reports it.
+// Waits until the cells [x0, x1) x [y0, y1) (a row or a column, at most 8) are
+// done.  They come earlier in z-order, so their warps are already running; the
+// bound (g_neighbor_wait_limit short sleeps after WAIT_POLLS polls) only guards
+// against a fault elsewhere, and the caller then reports it.
 __device__ __forceinline__ bool cells_done(const DecSmem &S, int x0, int x1, int y0, int y1, int lane) {
-    const int n = (x1 - x0) * (y1 - y0), w = x1 - x0;
-    for (int spins = 0; spins < (1 << 22); ++spins) {
-        bool ok = true;
-        if (lane < n) {
-            const int c = (y0 + lane / w) * 8 + x0 + lane % w;
-            ok = S.done[c] || S.leaf[c] == NO_LEAF;
-        }
-        if (__all_sync(0xffffffffu, ok)) return true;
+    const int k = lane & 7, n = x1 - x0 + y1 - y0 - 1;
+    const int c = (y0 + (y1 - y0 > 1 ? mini(k, n - 1) : 0)) * 8 + x0 + (x1 - x0 > 1 ? mini(k, n - 1) : 0);
+    auto done = [&] { return __all_sync(0xffffffffu, S.done[c] || S.leaf[c] == NO_LEAF); };
+    for (int i = 0; i < WAIT_POLLS; ++i)
+        if (done()) return true;
+    const long long limit = g_neighbor_wait_limit;
+    for (long long i = 0; i < limit; ++i) {
+        __nanosleep(128);
+        if (done()) return true;
     }
     return false;
 }
@@ -255,7 +257,7 @@ __device__ __forceinline__ void dec_area(DecSmem &S, const CtuOut *rec, int ctu_
     }
     __syncwarp();
     __threadfence_block();
-    if (lane == 0) S.done[cell] = 1;
+    if (lane == 0 && !(P.lose_area && cell == S.order[0])) S.done[cell] = 1;
 }
 
 __global__ void __launch_bounds__(NT, 1)

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/tcodec.h"
+#include "../../include/tcodec_b200.h"
 #include "tcb_encoder.h"
 #include "tcb_entropy.h"
 #include "tcb_launch.h"
@@ -117,6 +118,7 @@ struct DecImpl {
     int disp_active = 0, disp_next = 0;
     tc_frame_buf_t *disp_out = nullptr;
     int crc_valid = 1, entropy = 0, threads = 4, profile = 0;
+    int lose_area = 0;                // test hook, for the next v2 packet
     uint64_t prof[7] = {0, 0, 0, 0, 0, 0, 0};
 
     // All three planes or none: a partly allocated frame is freed again.
@@ -224,6 +226,16 @@ struct DecImpl {
         DevFrame f;
         if (!alloc_frame(f)) f = DevFrame();
         return f;
+    }
+    bool copy_frame(const DevFrame &dst, const DevFrame &src) {
+        return cudaMemcpyAsync(dst.y, src.y, (size_t)sy * fh, cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
+               cudaMemcpyAsync(dst.cb, src.cb, (size_t)sc * (fh / 2), cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
+               cudaMemcpyAsync(dst.cr, src.cr, (size_t)sc * (fh / 2), cudaMemcpyDeviceToDevice, st) == cudaSuccess;
+    }
+    void clear_frame(const DevFrame &f) {
+        cudaMemsetAsync(f.y, 0, (size_t)sy * fh, st);
+        cudaMemsetAsync(f.cb, 0, (size_t)sc * (fh / 2), st);
+        cudaMemsetAsync(f.cr, 0, (size_t)sc * (fh / 2), st);
     }
     bool d2h(tc_frame_buf_t *dst, const DevFrame &src) {
         return cudaMemcpy2DAsync(dst->y, dst->stride_y, src.y, sy, fw, fh, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
@@ -405,6 +417,8 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
     P.qp = hdr.qp;
     P.qp_c = clampi(hdr.qp + 1, 0, 63);
     P.fresh_skip = (hdr.tools & TC_TOOL_FRESH_SKIP) != 0;
+    P.lose_area = lose_area;
+    lose_area = 0;
     static const int qs[64] = TCB_QSCALE_INIT;
     static const int jw[4] = TCB_JND_INIT;
     for (int b = 0; b < 4; ++b) {
@@ -422,10 +436,20 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
     if (cudaMemcpyAsync(h_status, d_items + nctu, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return TC_ERR_INTERNAL;
     }   // v2 stream
+    // The picture is known to be good before it becomes a reference: a packet
+    // that fails here leaves the DPB, and the reconstruction that later packets
+    // build on, as they were.
+    if (!d2h(out, cur)) return TC_ERR_INTERNAL;
+    if (!legacy_stream && *h_status != 0) {   // an area gave up waiting
+        cudaMemsetAsync(d_items + rows * cols, 0, sizeof(int), st);
+        if (dpb_ok[0]) copy_frame(cur, dpb[0]);
+        else clear_frame(cur);
+        return TC_ERR_INTERNAL;
+    }
     // DPB: slot 3 falls out and its buffer takes a copy of the
     // reconstruction into slot 0 (another buffer when slot 3 is empty, taken
     // before anything moves, so a failed allocation leaves the DPB as it
-    // was).  The copy follows this frame's kernels on the stream.
+    // was).  The copy is ordered before the next packet's kernels on the stream.
     DevFrame nf;
     if (dpb_ok[TC_REF_FRAMES - 1]) {
         nf = dpb[TC_REF_FRAMES - 1];
@@ -433,17 +457,12 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
         nf = take_frame();
         if (!nf.y) return TC_ERR_MEMORY;
     }
-    for (int i = TC_REF_FRAMES - 1; i > 0; --i) { dpb[i] = dpb[i - 1]; dpb_ok[i] = dpb_ok[i - 1]; dpb_poc[i] = dpb_poc[i - 1]; }
-    if (cudaMemcpyAsync(nf.y, cur.y, (size_t)sy * fh, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(nf.cb, cur.cb, (size_t)sc * (fh / 2), cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(nf.cr, cur.cr, (size_t)sc * (fh / 2), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return TC_ERR_INTERNAL;
-    dpb[0] = nf; dpb_ok[0] = 1; dpb_poc[0] = hdr.frame_num;
-    if (!d2h(out, cur)) return TC_ERR_INTERNAL;
-    if (!legacy_stream && *h_status != 0) {   // an area gave up waiting
-        cudaMemset(d_items + rows * cols, 0, sizeof(int));
+    if (!copy_frame(nf, cur)) {
+        if (!dpb_ok[TC_REF_FRAMES - 1]) spare.push_back(nf);
         return TC_ERR_INTERNAL;
     }
+    for (int i = TC_REF_FRAMES - 1; i > 0; --i) { dpb[i] = dpb[i - 1]; dpb_ok[i] = dpb_ok[i - 1]; dpb_poc[i] = dpb_poc[i - 1]; }
+    dpb[0] = nf; dpb_ok[0] = 1; dpb_poc[0] = hdr.frame_num;
     const uint64_t t_rec = now_ns();
     if (profile) { prof[0] += t_parse1 - t_parse0; prof[2] += t_rec - t_parse1; }
     if (hdr.has_ext) {
@@ -594,6 +613,12 @@ void tc_decoder_get_profile(tc_decoder_t *dec, uint64_t *parse_ns, uint64_t *coe
 void tc_decoder_set_threads(tc_decoder_t *dec, int nthreads) {
     if (!dec || !dec->impl) return;
     dec->impl->threads = nthreads < 1 ? 1 : (nthreads > 16 ? 16 : nthreads);
+}
+
+tc_error_t tcb_debug_decoder_lose_area(tc_decoder_t *dec) {
+    if (!dec || !dec->impl) return TC_ERR_PARAM;
+    dec->impl->lose_area = 1;
+    return TC_OK;
 }
 
 }  // extern "C"

@@ -10,9 +10,11 @@
 // carries the vector of its own position.  Packets are raw Exp-Golomb key and
 // P frames without levels, written here.
 //
-// Usage: decoder_host_check <case> W0 H0 W H [W H ...]: a decoder created
-// for W0 x H0 (0 0: from the stream) is fed one packet per size.  Exit code 0
-// when every check holds.
+// Usage: decoder_host_check sizes|reorder W0 H0 W H [W H ...]: a decoder created
+// for W0 x H0 (0 0: from the stream) is fed two packets per size; or
+// decoder_host_check status|status_key W0 H0 W H n lost: n packets, of which
+// one (a key frame in status_key) fails in the kernel.  Exit code 0 when every
+// check holds.
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -114,6 +116,7 @@ void tcb_host_frame_free(tc_frame_buf_t *f) {
 static FrameParams g_last;            // parameters of the last launch
 static int g_fill = -1;               // luma value the fake reconstruction writes
 static bool g_give_up = false;        // it reports a wait that ran out
+static int g_before = -1, g_ref = -1; // luma of the reconstruction and of the first reference at the launch
 
 namespace tcb {
 std::atomic<long long> g_alloc_countdown{-1};
@@ -140,6 +143,10 @@ static void check_tree(const FrameParams &P, const CtuOut &o, int d, int ctu_x, 
 }
 cudaError_t launch_decode_items(const FrameParams *d_params, const int *d_items, int n, int *d_status, cudaStream_t) {
     const FrameParams &P = *d_params;
+    if (d_items[0] == 0) {            // the picture's first diagonal
+        g_before = P.rec_y[0];
+        g_ref = P.ref_valid[0] ? P.ref_y[0][0] : -1;
+    }
     g_last = P;
     for (int i = 0; i < n; ++i) {
         const int row = (d_items[i] >> 10) & 1023, col = d_items[i] & 1023, x = col * 64, y = row * 64;
@@ -244,6 +251,35 @@ static void sizes(tc_decoder_t *dec, const std::vector<int> &wh, bool reorder) {
         }
 }
 
+// Pictures 0 .. n-1, one of them (`lost`) with a wait that runs out: it is an
+// error, and the packets after it find references, picture order and base
+// picture as if it had not come.
+static void status(tc_decoder_t *dec, int W, int H, int n, int lost, bool key) {
+    const tc_pixel_t *y;
+    int ys, last = -1;
+    std::vector<int> pocs;
+    for (int t = 0; t < n; ++t) {
+        g_fill = 20 + t;
+        g_give_up = t == lost;
+        const bool k = t == 0 || (key && t == lost);
+        const tc_error_t e = feed(dec, packet(W, H, !k, t), &y, &ys);
+        if (e != (t == lost ? TC_ERR_INTERNAL : TC_OK)) bad("status not as expected");
+        if (k) pocs.clear();
+        const bool cleared = key && lost > 0 && t > lost && pocs.empty();
+        if (g_before != (last >= 0 && !cleared ? last : 0)) bad("the picture built on is not the last good one");
+        for (int i = 0; i < MAX_REFS; ++i) {
+            const bool have = i < (int)pocs.size();
+            if (g_last.ref_valid[i] != have) bad("references not those of the good pictures");
+            else if (have && g_last.ref_poc[i] != pocs[pocs.size() - 1 - i]) bad("picture order not that of the good pictures");
+        }
+        if (!pocs.empty() && g_ref != last) bad("the reference is not the last good picture");
+        if (t != lost) {
+            last = g_fill;
+            pocs.push_back(t);
+        }
+    }
+}
+
 int main(int argc, char **argv) {
     if (argc < 6) { fprintf(stderr, "usage\n"); return 2; }
     const std::string what = argv[1];
@@ -252,6 +288,7 @@ int main(int argc, char **argv) {
     tc_decoder_t *dec = tc_decoder_create(atoi(argv[2]), atoi(argv[3]));
     if (!dec) { printf("no decoder\n"); return 2; }
     if (what == "sizes" || what == "reorder") sizes(dec, wh, what == "reorder");
+    else if (what == "status" || what == "status_key") status(dec, wh[0], wh[1], wh[2], wh[3], what == "status_key");
     else bad("no such case");
     tc_decoder_destroy(dec);
     if (!g_mem.empty()) bad("memory left behind");

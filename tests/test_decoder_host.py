@@ -32,3 +32,9 @@ def run(exe, *args):
 @pytest.mark.parametrize("sizes", [(96, 80), (96, 80, 96, 16), (96, 16, 96, 80), (64, 64, 200, 136, 72, 8), (8, 8, 130, 70)])
 def test_the_kernel_gets_the_frames_size(exe, form, created, sizes):
     run(exe, form, *created, *sizes)
+
+
+@pytest.mark.parametrize("form", ["status", "status_key"])
+@pytest.mark.parametrize("lost", [0, 1, 2, 4, 5, 7])      # before, at and after the fourth reference
+def test_a_packet_that_fails_in_the_kernel_leaves_no_trace(exe, form, lost):
+    run(exe, form, 0, 0, 72, 40, 9, lost)
