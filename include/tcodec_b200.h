@@ -184,7 +184,11 @@ void tcb_server_get_timing(tcb_server_t *server, double *admit_ms, double *step_
  * tcb_mv_cell_bytes() each (prev may be NULL); ctu_records holds
  * ceil(W/64)*ceil(H/64) records of tcb_ctu_record_bytes() each: the
  * decision tree, quantised coefficients in syntax order and SAO
- * parameters of every CTU, ready for the v2 syntax writer. */
+ * parameters of every CTU, ready for the v2 syntax writer.  Where width or
+ * height is not a multiple of 8, rec_* must come in with the previous
+ * frame's reconstruction (zeros before the first) in the samples outside
+ * whole 8x8 blocks: they are not coded, SAO applies to them, and a decoder
+ * keeps them from picture to picture. */
 typedef struct tcb_frame_desc {
     int width, height, stride_y, stride_c;
     const tc_pixel_t *src_y, *src_cb, *src_cr;

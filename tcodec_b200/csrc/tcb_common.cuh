@@ -57,6 +57,7 @@ struct FrameParams {
     int grid_w, grid_h;                        // frame MV grid, 8x8 cells
     const uint8_t *cur_y, *cur_cb, *cur_cr;    // source picture
     uint8_t *rec_y, *rec_cb, *rec_cr;          // reconstruction (output)
+    const uint8_t *kept_y, *kept_cb, *kept_cr; // picture whose samples stand outside whole 8x8 blocks (encoder)
     const uint8_t *ref_y[MAX_REFS], *ref_cb[MAX_REFS], *ref_cr[MAX_REFS];
     int ref_valid[MAX_REFS];
     int ref_poc[MAX_REFS];

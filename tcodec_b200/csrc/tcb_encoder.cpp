@@ -371,6 +371,8 @@ tc_error_t EncImpl::stage_b() {
     P.ctu_cols = ctu_cols; P.ctu_rows = ctu_rows; P.grid_w = grid_w; P.grid_h = grid_h;
     P.cur_y = cur.y; P.cur_cb = cur.cb; P.cur_cr = cur.cr;
     P.rec_y = rec.y; P.rec_cb = rec.cb; P.rec_cr = rec.cr;
+    const DevFrame &kept = prev_rs >= 0 ? pool[prev_rs] : rec;     // (the pool starts cleared)
+    P.kept_y = kept.y; P.kept_cb = kept.cb; P.kept_cr = kept.cr;
     for (int i = 0; i < MAX_REFS; ++i) {
         const int s = dpb_slot[i];
         P.ref_valid[i] = s >= 0;
@@ -765,6 +767,7 @@ bool tcb::frame_params_from_desc(const tcb_frame_desc_t &d, FrameParams &P) {
     P.grid_w = (d.width + 7) / 8; P.grid_h = (d.height + 7) / 8;
     P.cur_y = d.src_y; P.cur_cb = d.src_cb; P.cur_cr = d.src_cr;
     P.rec_y = d.rec_y; P.rec_cb = d.rec_cb; P.rec_cr = d.rec_cr;
+    P.kept_y = d.rec_y; P.kept_cb = d.rec_cb; P.kept_cr = d.rec_cr;
     for (int i = 0; i < MAX_REFS; ++i) {
         const bool ok = d.ref_y[i] && d.ref_cb[i] && d.ref_cr[i];
         P.ref_valid[i] = ok;

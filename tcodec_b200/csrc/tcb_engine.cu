@@ -2061,6 +2061,21 @@ __device__ void encode_ctu(Smem &S, const FrameParams &P, int row, int col) {
             RC(S, c, -1, y) = __ldcg(src + (size_t)((ctu_y >> 1) + y) * P.stride_c + (ctu_x >> 1) - 1);
         }
     }
+    // Samples outside whole 8x8 blocks are never coded: they keep the picture
+    // before's, as in the decoder, whose reconstruction buffer persists.
+    if ((w | h) & 7) {
+        const int w8 = w & ~7, h8 = h & ~7;
+        for (int i = threadIdx.x; i < 64 * 64; i += NT) {
+            const int y = i >> 6, x = i & 63;
+            if (x < w && y < h && (x >= w8 || y >= h8))
+                RY(S, x, y) = P.kept_y[(size_t)(ctu_y + y) * P.stride_y + ctu_x + x];
+        }
+        for (int i = threadIdx.x; i < 2 * 32 * 32; i += NT) {
+            const int c = i >> 10, p = i & 1023, y = p >> 5, x = p & 31;
+            if (x < wc && y < hc && (x >= w8 >> 1 || y >= h8 >> 1))
+                RC(S, c, x, y) = (c ? P.kept_cr : P.kept_cb)[(size_t)((ctu_y >> 1) + y) * P.stride_c + (ctu_x >> 1) + x];
+        }
+    }
     for (int i = threadIdx.x; i < 64; i += NT) {
         S.grid[i].dx = 0; S.grid[i].dy = 0; S.grid[i].intra = 1; S.grid[i].pad = 0;
     }
