@@ -569,7 +569,9 @@ cudaError_t launch_group_vec(const DeblockFrame *frames, int m, cudaStream_t st,
     J.ctu_off[m] = total;
     if (total == 0) return cudaSuccess;
     const dim3 grid = ctu_grid(frames, m, total, frames[0].W >> 6, frames[0].H >> 6, J.grid3);
-    // Few CTUs: at most one per SM, so a CTU's latency is the launch's time.
+    // Few CTUs: at most one per SM (148 on the one device this is built for, and
+    // a matter of speed only), so a CTU's latency is the launch's time.  Asking the
+    // device took 0.1 to 0.2 of the 6.7 us of the smallest call.
     constexpr int SMS = 148;
     if (threads == 64) deblock_frames_kernel<64, false, N><<<grid, 64, 0, st>>>(J);
     else if (threads == 256) deblock_frames_kernel<256, false, N><<<grid, 256, 0, st>>>(J);
