@@ -1,18 +1,19 @@
-// tcb_legacy.cuh — the legacy (v0 / v1) block path: one CTU of fixed 8x8
-// blocks coded in raster order (reference src/encoder.c:1526-2269
-// encode_block, src/decoder.c:260-650 decode_block).
+// tcb_legacy.cuh — the legacy (v0 / v1) block path: reconstruction of fixed 8x8
+// blocks from parsed records (reference src/decoder.c:260-650 decode_block),
+// which the GPU decoder runs (tcb_legacy.cu), and for the CPU tests a
+// restatement of the encoder (src/encoder.c:1526-2269 encode_block), which
+// the GPU encoder (tcb_legacy_enc.cuh) is compared with.
 //
-// Each CTU is worked by one warp.  A block's 64 samples are spread over the
-// lanes (two each); decisions that depend on a whole block (SADs, SSEs,
-// non-zero counts) are warp reductions, and every lane then takes the same
-// branch, so the sequential order of the reference (search candidates
-// committed one at a time, blocks in raster order) is kept exactly.
+// A block is worked by one warp.  Its 64 samples are spread over the lanes (two
+// each); sums over a whole block are warp reductions, and every lane then
+// takes the same branch.
 //
 // The functions are written against a small "team" interface (lane index,
 // lane count, sum, sync) so that the same source also compiles as plain C++
-// with a team of one lane: the CPU tests run it that way against the
-// reference library (tests/legacy_emu.cpp).  The including translation unit
-// provides ldct4(k, n) / ldct8(k, n), the DCT-II matrices.
+// with a team of one lane: the CPU tests run both halves that way against the
+// reference library (tests/legacy_emu.cpp), and the encoder's beside the GPU's
+// (tests/legacy_restate.cpp).  The including translation unit provides
+// ldct4(k, n) / ldct8(k, n), the DCT-II matrices.
 #pragma once
 #include <stdint.h>
 #include "tcb_common.cuh"
@@ -58,16 +59,8 @@ struct LState {
     int32_t blk_mvx[64], blk_mvy[64];
 };
 
-// Normative tables (reference src/quantize.c:30-39, 72-77) and the search
-// patterns of tc_motion_est (src/motion.c:346-369), centre points dropped.
+// Normative tables (reference src/quantize.c:30-39, 72-77).
 LG_TABLE int lg_qscale[64] = TCB_QSCALE_INIT;
-LG_TABLE int8_t lg_hexl[6][2] = {{-2, -4}, {2, -4}, {-4, 0}, {4, 0}, {-2, 4}, {2, 4}};
-LG_TABLE int8_t lg_hexs[6][2] = {{-1, -2}, {1, -2}, {-2, 0}, {2, 0}, {-1, 2}, {1, 2}};
-LG_TABLE int8_t lg_dia[4][2] = {{0, -1}, {-1, 0}, {1, 0}, {0, 1}};
-LG_TABLE int8_t lg_qpel[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, 1}, {1, -1}, {-1, -1}};
-// Intra modes tried first (reference src/encoder.c:1563-1565).
-LG_TABLE int8_t lg_fast_modes[8] = {0, 1, 2, 5, 8, 9, 13, 17};
-
 LG_FN int qscale_of(int qp) { return lg_qscale[clampi(qp, 0, 63)]; }
 LG_FN int jnd_of(int band) {
     return band <= 0 ? 6 : band == 1 ? 7 : band == 2 ? 8 : 10;
@@ -176,88 +169,6 @@ LG_FN int intra_dc_value(const LState &S) {
     return (sum + 8) / 16;
 }
 
-// SAD of the block against intra mode m.
-LG_FN int intra_sad(const LState &S, int m, int dc) {
-    const int L = lane_id();
-    int s = 0;
-    for (int i = L; i < 64; i += NL) s += absi((int)S.orig[i] - intra_at(S.ra + 1, S.rl + 1, 8, m, dc, i & 7, i >> 3));
-    return team_sum(s);
-}
-
-// Integer SAD at (mx, my) with the reference's frame bounds check
-// (reference src/motion.c:371-380).
-LG_FN int sad_at(const LState &S, const uint8_t *ref, int s, int W, int H, int mx, int my) {
-    if (mx < 0 || my < 0 || mx + 8 > W || my + 8 > H) return SAD_MAX;
-    const int L = lane_id();
-    int a = 0;
-    for (int i = L; i < 64; i += NL) a += absi((int)S.orig[i] - (int)ref[(size_t)(my + (i >> 3)) * s + mx + (i & 7)]);
-    return team_sum(a);
-}
-
-// Quarter-sample SAD of the refinement stage: six-tap where the margins
-// allow, bilinear otherwise (reference src/motion.c:465-480, 308-341).
-LG_FN int qpel_sad(const LState &S, const uint8_t *ref, int s, int W, int H, int qx, int qy) {
-    const int fx = qx >> 2, fy = qy >> 2, dx = qx & 3, dy = qy & 3;
-    const int L = lane_id();
-    int a = 0;
-    if (fx >= 2 && fy >= 2 && fx + 8 + 2 < W && fy + 8 + 2 < H) {
-        for (int i = L; i < 64; i += NL) a += absi((int)S.orig[i] - luma_hv(ref, s, fx + (i & 7), fy + (i >> 3), dx, dy));
-    } else {
-        for (int i = L; i < 64; i += NL) {
-            const uint8_t *p = ref + (size_t)(fy + (i >> 3)) * s + fx + (i & 7);
-            const int top = interp_qpel(p[0], p[1], dx), bot = interp_qpel(p[s], p[s + 1], dx);
-            a += absi((int)S.orig[i] - interp_qpel(top, bot, dy));
-        }
-    }
-    return team_sum(a);
-}
-
-// Hexagonal search with sequential commit inside every pass, then the
-// quarter-sample refinement (reference src/motion.c:384-485 tc_motion_est).
-LG_FN void motion_est(const LState &S, const uint8_t *ref, int s, int W, int H, int cx, int cy, int range,
-                      int &mvx, int &mvy, int &sad_out) {
-    cx = clampi(cx, 0, W - 8);
-    cy = clampi(cy, 0, H - 8);
-    int bx = cx * 4, by = cy * 4;
-    int best = sad_at(S, ref, s, W, H, cx, cy);
-    const int step = maxi(1, range / 4);
-    for (int it = 0; it < 2; ++it) {
-        bool imp = false;
-        for (int p = 0; p < 6; ++p) {
-            const int mx = bx / 4 + lg_hexl[p][0] * step, my = by / 4 + lg_hexl[p][1] * step;
-            const int v = sad_at(S, ref, s, W, H, mx, my);
-            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
-        }
-        if (!imp) break;
-    }
-    for (int it = 0; it < 3; ++it) {
-        bool imp = false;
-        for (int p = 0; p < 6; ++p) {
-            const int mx = bx / 4 + lg_hexs[p][0], my = by / 4 + lg_hexs[p][1];
-            const int v = sad_at(S, ref, s, W, H, mx, my);
-            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
-        }
-        if (!imp) break;
-    }
-    for (int it = 0; it < 4; ++it) {
-        bool imp = false;
-        for (int p = 0; p < 4; ++p) {
-            const int mx = bx / 4 + lg_dia[p][0], my = by / 4 + lg_dia[p][1];
-            const int v = sad_at(S, ref, s, W, H, mx, my);
-            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
-        }
-        if (!imp) break;
-    }
-    for (int p = 0; p < 8; ++p) {
-        const int qx = bx + lg_qpel[p][0], qy = by + lg_qpel[p][1];
-        const int fx = qx >> 2, fy = qy >> 2;
-        if (fx < 0 || fy < 0 || fx + 9 > W || fy + 9 > H) continue;
-        const int v = qpel_sad(S, ref, s, W, H, qx, qy);
-        if (v < best) { best = v; bx = qx; by = qy; }
-    }
-    mvx = bx; mvy = by; sad_out = best;
-}
-
 // Luma motion compensation of the block into dst (reference
 // src/motion.c:493-584 tc_inter_predict).
 LG_FN void inter_pred(uint8_t *dst, const uint8_t *ref, int s, int W, int H, int mvx, int mvy) {
@@ -273,37 +184,6 @@ LG_FN void bi_pred(uint8_t *dst, const uint8_t *fwd, const uint8_t *bwd, int s, 
     a.init(fwd, s, W, H, mvx, mvy, 8);
     b.init(bwd, s, W, H, -mvx, -mvy, 8);
     for (int i = lane_id(); i < 64; i += NL) dst[i] = (uint8_t)((a.at(i & 7, i >> 3) + b.at(i & 7, i >> 3) + 1) >> 1);
-}
-
-LG_FN int sad_buf(const LState &S, const uint8_t *p) {
-    int a = 0;
-    for (int i = lane_id(); i < 64; i += NL) a += absi((int)S.orig[i] - (int)p[i]);
-    return team_sum(a);
-}
-
-// Median motion predictor of block `bi` from its left, above and
-// above-right neighbours inside the CTU (reference src/encoder.c:1619-1645,
-// src/decoder.c:346-372).  Returns whether one of them is inter.
-LG_FN bool median_mv(const LState &S, int bi, int &px, int &py) {
-    const int bx = bi & 7, by = bi >> 3;
-    int ax = 0, ay = 0, bxv = 0, byv = 0, cxv = 0, cyv = 0;
-    bool ha = false, hb = false, hc = false;
-    if (bx > 0 && S.blk_inter[bi - 1]) { ax = S.blk_mvx[bi - 1]; ay = S.blk_mvy[bi - 1]; ha = true; }
-    if (by > 0 && S.blk_inter[bi - 8]) { bxv = S.blk_mvx[bi - 8]; byv = S.blk_mvy[bi - 8]; hb = true; }
-    if (by > 0 && bx < 7 && S.blk_inter[bi - 7]) { cxv = S.blk_mvx[bi - 7]; cyv = S.blk_mvy[bi - 7]; hc = true; }
-    if (!(ha || hb || hc)) return false;
-    if (!ha) { ax = hb ? bxv : cxv; ay = hb ? byv : cyv; }
-    if (!hb) { bxv = ha ? ax : cxv; byv = ha ? ay : cyv; }
-    if (!hc) { cxv = ha ? ax : bxv; cyv = ha ? ay : byv; }
-    auto med = [](int a, int b, int c) {
-        if (a > b) { int t = a; a = b; b = t; }
-        if (b > c) { int t = b; b = c; c = t; }
-        if (a > b) { int t = a; a = b; b = t; }
-        return b;
-    };
-    px = med(ax, bxv, cxv);
-    py = med(ay, byv, cyv);
-    return true;
 }
 
 // Chroma of one block (reference src/encoder.c:2192-2268, decoder.c:553-638):
@@ -412,6 +292,182 @@ LG_FN void deblock_ctu(const LFrame &F, int ox, int oy, int t, int nt, Sync sync
         b[sc] = (uint8_t)clampi(qb - d, 0, 255);
     }
     sync();
+}
+
+// Luma of one 8x8 block from its parsed record (reference
+// src/decoder.c:260-650 decode_block, after parsing).
+LG_NOINL void decode_luma(LState &S, const LFrame &F, int fx, int fy, const LBlock &in) {
+    const int L = lane_id(), sy = F.sy, W = F.W, H = F.H, ftype = F.frame_type;
+    const bool intra = in.mode == 2, skip = in.mode == 0 || in.mode == 3;
+    if (intra) {
+        build_refs(S, F.rec_y, sy, fx, fy, W, H);
+        const int dc = intra_dc_value(S);
+        for (int i = L; i < 64; i += NL) S.pred[i] = (uint8_t)intra_at(S.ra + 1, S.rl + 1, 8, in.intra_mode, dc, i & 7, i >> 3);
+    } else {
+        const int mvx = in.mvd_x, mvy = in.mvd_y;
+        if (ftype == 2 && in.ref == 2) {
+            if (F.fwd_y && F.bwd_y) bi_pred(S.pred, F.fwd_y, F.bwd_y, sy, W, H, mvx, mvy);
+            else for (int i = L; i < 64; i += NL) S.pred[i] = 128;
+        } else {
+            const uint8_t *src = ftype == 2 ? (in.ref ? F.bwd_y : F.fwd_y) : F.dpb_y[in.ref & 3];
+            if (src) inter_pred(S.pred, src, sy, W, H, mvx, mvy);
+            else for (int i = L; i < 64; i += NL) S.pred[i] = 128;
+        }
+    }
+    team_sync();
+    if (skip) {
+        for (int i = L; i < 64; i += NL) F.rec_y[(size_t)(fy + (i >> 3)) * sy + fx + (i & 7)] = S.pred[i];
+    } else {
+        const int N = (in.tid & 2) ? 8 : 4, t = in.tid & 1;
+        const int scale = qscale_of(F.qp);
+        for (int e = L; e < 64; e += NL) {
+            int b, r, c, ras;
+            elem_pos(N, e, b, r, c, ras);
+            S.dq[ras] = (int16_t)lq_dequant(in.luma[e], eff_of(scale, freq_band(r * N + c, N * N)));
+        }
+        team_sync();
+        transform8(S, S.dq, S.inv, N, t, true);
+        for (int i = L; i < 64; i += NL)
+            F.rec_y[(size_t)(fy + (i >> 3)) * sy + fx + (i & 7)] = (uint8_t)clampi((int)S.pred[i] + S.inv[i], 0, 255);
+    }
+    team_sync();
+}
+// One component of its chroma, after its luma (intra blocks, never skip or
+// merge, predict from it; no component reads the other).
+LG_FN void decode_chroma(LState &S, const LFrame &F, int comp, int fx, int fy, const LBlock &in) {
+    int16_t lv[16];
+    for (int i = 0; i < 16; ++i) lv[i] = in.chroma[16 * comp + i];
+    chroma_block(S, F, false, nullptr, comp ? F.rec_cr : F.rec_cb, fx, fy, in.mode == 2, lv);
+}
+
+// --------------------------------------------------------------------
+// The encoder, restated for the CPU.  No kernel uses it: the GPU encodes with
+// tcb_legacy_enc.cuh, which the tests hold to this restatement packet by
+// packet, as they hold this to the reference.
+// --------------------------------------------------------------------
+#ifndef __CUDACC__
+
+// Search patterns of tc_motion_est (reference src/motion.c:346-369), centre
+// points dropped.
+LG_TABLE int8_t lg_hexl[6][2] = {{-2, -4}, {2, -4}, {-4, 0}, {4, 0}, {-2, 4}, {2, 4}};
+LG_TABLE int8_t lg_hexs[6][2] = {{-1, -2}, {1, -2}, {-2, 0}, {2, 0}, {-1, 2}, {1, 2}};
+LG_TABLE int8_t lg_dia[4][2] = {{0, -1}, {-1, 0}, {1, 0}, {0, 1}};
+LG_TABLE int8_t lg_qpel[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, 1}, {1, -1}, {-1, -1}};
+// Intra modes tried first (reference src/encoder.c:1563-1565).
+LG_TABLE int8_t lg_fast_modes[8] = {0, 1, 2, 5, 8, 9, 13, 17};
+
+
+// SAD of the block against intra mode m.
+LG_FN int intra_sad(const LState &S, int m, int dc) {
+    const int L = lane_id();
+    int s = 0;
+    for (int i = L; i < 64; i += NL) s += absi((int)S.orig[i] - intra_at(S.ra + 1, S.rl + 1, 8, m, dc, i & 7, i >> 3));
+    return team_sum(s);
+}
+
+// Integer SAD at (mx, my) with the reference's frame bounds check
+// (reference src/motion.c:371-380).
+LG_FN int sad_at(const LState &S, const uint8_t *ref, int s, int W, int H, int mx, int my) {
+    if (mx < 0 || my < 0 || mx + 8 > W || my + 8 > H) return SAD_MAX;
+    const int L = lane_id();
+    int a = 0;
+    for (int i = L; i < 64; i += NL) a += absi((int)S.orig[i] - (int)ref[(size_t)(my + (i >> 3)) * s + mx + (i & 7)]);
+    return team_sum(a);
+}
+
+// Quarter-sample SAD of the refinement stage: six-tap where the margins
+// allow, bilinear otherwise (reference src/motion.c:465-480, 308-341).
+LG_FN int qpel_sad(const LState &S, const uint8_t *ref, int s, int W, int H, int qx, int qy) {
+    const int fx = qx >> 2, fy = qy >> 2, dx = qx & 3, dy = qy & 3;
+    const int L = lane_id();
+    int a = 0;
+    if (fx >= 2 && fy >= 2 && fx + 8 + 2 < W && fy + 8 + 2 < H) {
+        for (int i = L; i < 64; i += NL) a += absi((int)S.orig[i] - luma_hv(ref, s, fx + (i & 7), fy + (i >> 3), dx, dy));
+    } else {
+        for (int i = L; i < 64; i += NL) {
+            const uint8_t *p = ref + (size_t)(fy + (i >> 3)) * s + fx + (i & 7);
+            const int top = interp_qpel(p[0], p[1], dx), bot = interp_qpel(p[s], p[s + 1], dx);
+            a += absi((int)S.orig[i] - interp_qpel(top, bot, dy));
+        }
+    }
+    return team_sum(a);
+}
+
+// Hexagonal search with sequential commit inside every pass, then the
+// quarter-sample refinement (reference src/motion.c:384-485 tc_motion_est).
+LG_FN void motion_est(const LState &S, const uint8_t *ref, int s, int W, int H, int cx, int cy, int range,
+                      int &mvx, int &mvy, int &sad_out) {
+    cx = clampi(cx, 0, W - 8);
+    cy = clampi(cy, 0, H - 8);
+    int bx = cx * 4, by = cy * 4;
+    int best = sad_at(S, ref, s, W, H, cx, cy);
+    const int step = maxi(1, range / 4);
+    for (int it = 0; it < 2; ++it) {
+        bool imp = false;
+        for (int p = 0; p < 6; ++p) {
+            const int mx = bx / 4 + lg_hexl[p][0] * step, my = by / 4 + lg_hexl[p][1] * step;
+            const int v = sad_at(S, ref, s, W, H, mx, my);
+            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
+        }
+        if (!imp) break;
+    }
+    for (int it = 0; it < 3; ++it) {
+        bool imp = false;
+        for (int p = 0; p < 6; ++p) {
+            const int mx = bx / 4 + lg_hexs[p][0], my = by / 4 + lg_hexs[p][1];
+            const int v = sad_at(S, ref, s, W, H, mx, my);
+            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
+        }
+        if (!imp) break;
+    }
+    for (int it = 0; it < 4; ++it) {
+        bool imp = false;
+        for (int p = 0; p < 4; ++p) {
+            const int mx = bx / 4 + lg_dia[p][0], my = by / 4 + lg_dia[p][1];
+            const int v = sad_at(S, ref, s, W, H, mx, my);
+            if (v < best) { best = v; bx = mx * 4; by = my * 4; imp = true; }
+        }
+        if (!imp) break;
+    }
+    for (int p = 0; p < 8; ++p) {
+        const int qx = bx + lg_qpel[p][0], qy = by + lg_qpel[p][1];
+        const int fx = qx >> 2, fy = qy >> 2;
+        if (fx < 0 || fy < 0 || fx + 9 > W || fy + 9 > H) continue;
+        const int v = qpel_sad(S, ref, s, W, H, qx, qy);
+        if (v < best) { best = v; bx = qx; by = qy; }
+    }
+    mvx = bx; mvy = by; sad_out = best;
+}
+
+LG_FN int sad_buf(const LState &S, const uint8_t *p) {
+    int a = 0;
+    for (int i = lane_id(); i < 64; i += NL) a += absi((int)S.orig[i] - (int)p[i]);
+    return team_sum(a);
+}
+
+// Median motion predictor of block `bi` from its left, above and
+// above-right neighbours inside the CTU (reference src/encoder.c:1619-1645,
+// src/decoder.c:346-372).  Returns whether one of them is inter.
+LG_FN bool median_mv(const LState &S, int bi, int &px, int &py) {
+    const int bx = bi & 7, by = bi >> 3;
+    int ax = 0, ay = 0, bxv = 0, byv = 0, cxv = 0, cyv = 0;
+    bool ha = false, hb = false, hc = false;
+    if (bx > 0 && S.blk_inter[bi - 1]) { ax = S.blk_mvx[bi - 1]; ay = S.blk_mvy[bi - 1]; ha = true; }
+    if (by > 0 && S.blk_inter[bi - 8]) { bxv = S.blk_mvx[bi - 8]; byv = S.blk_mvy[bi - 8]; hb = true; }
+    if (by > 0 && bx < 7 && S.blk_inter[bi - 7]) { cxv = S.blk_mvx[bi - 7]; cyv = S.blk_mvy[bi - 7]; hc = true; }
+    if (!(ha || hb || hc)) return false;
+    if (!ha) { ax = hb ? bxv : cxv; ay = hb ? byv : cyv; }
+    if (!hb) { bxv = ha ? ax : cxv; byv = ha ? ay : cyv; }
+    if (!hc) { cxv = ha ? ax : bxv; cyv = ha ? ay : byv; }
+    auto med = [](int a, int b, int c) {
+        if (a > b) { int t = a; a = b; b = t; }
+        if (b > c) { int t = b; b = c; c = t; }
+        if (a > b) { int t = a; a = b; b = t; }
+        return b;
+    };
+    px = med(ax, bxv, cxv);
+    py = med(ay, byv, cyv);
+    return true;
 }
 
 // Evaluate one transform type for the residual: forward transform,
@@ -583,52 +639,6 @@ LG_NOINL void encode_block(LState &S, const LFrame &F, int bi, int fx, int fy, L
     team_sync();
 }
 
-// Luma of one 8x8 block from its parsed record (reference
-// src/decoder.c:260-650 decode_block, after parsing).
-LG_NOINL void decode_luma(LState &S, const LFrame &F, int fx, int fy, const LBlock &in) {
-    const int L = lane_id(), sy = F.sy, W = F.W, H = F.H, ftype = F.frame_type;
-    const bool intra = in.mode == 2, skip = in.mode == 0 || in.mode == 3;
-    if (intra) {
-        build_refs(S, F.rec_y, sy, fx, fy, W, H);
-        const int dc = intra_dc_value(S);
-        for (int i = L; i < 64; i += NL) S.pred[i] = (uint8_t)intra_at(S.ra + 1, S.rl + 1, 8, in.intra_mode, dc, i & 7, i >> 3);
-    } else {
-        const int mvx = in.mvd_x, mvy = in.mvd_y;
-        if (ftype == 2 && in.ref == 2) {
-            if (F.fwd_y && F.bwd_y) bi_pred(S.pred, F.fwd_y, F.bwd_y, sy, W, H, mvx, mvy);
-            else for (int i = L; i < 64; i += NL) S.pred[i] = 128;
-        } else {
-            const uint8_t *src = ftype == 2 ? (in.ref ? F.bwd_y : F.fwd_y) : F.dpb_y[in.ref & 3];
-            if (src) inter_pred(S.pred, src, sy, W, H, mvx, mvy);
-            else for (int i = L; i < 64; i += NL) S.pred[i] = 128;
-        }
-    }
-    team_sync();
-    if (skip) {
-        for (int i = L; i < 64; i += NL) F.rec_y[(size_t)(fy + (i >> 3)) * sy + fx + (i & 7)] = S.pred[i];
-    } else {
-        const int N = (in.tid & 2) ? 8 : 4, t = in.tid & 1;
-        const int scale = qscale_of(F.qp);
-        for (int e = L; e < 64; e += NL) {
-            int b, r, c, ras;
-            elem_pos(N, e, b, r, c, ras);
-            S.dq[ras] = (int16_t)lq_dequant(in.luma[e], eff_of(scale, freq_band(r * N + c, N * N)));
-        }
-        team_sync();
-        transform8(S, S.dq, S.inv, N, t, true);
-        for (int i = L; i < 64; i += NL)
-            F.rec_y[(size_t)(fy + (i >> 3)) * sy + fx + (i & 7)] = (uint8_t)clampi((int)S.pred[i] + S.inv[i], 0, 255);
-    }
-    team_sync();
-}
-// One component of its chroma, after its luma (intra blocks, never skip or
-// merge, predict from it; no component reads the other).
-LG_FN void decode_chroma(LState &S, const LFrame &F, int comp, int fx, int fy, const LBlock &in) {
-    int16_t lv[16];
-    for (int i = 0; i < 16; ++i) lv[i] = in.chroma[16 * comp + i];
-    chroma_block(S, F, false, nullptr, comp ? F.rec_cr : F.rec_cb, fx, fy, in.mode == 2, lv);
-}
-
 // One CTU: its blocks in raster order, then deblocking when the CTU lies
 // wholly inside the frame (reference src/encoder.c:2323-2346,
 // src/decoder.c:656-683).
@@ -654,6 +664,8 @@ LG_FN void code_ctu(LState &S, const LFrame &F, int row, int col, bool enc) {
     }
     if (ox + 64 <= F.W && oy + 64 <= F.H) deblock_ctu(F, ox, oy, L, NL, [] { team_sync(); });
 }
+
+#endif  // __CUDACC__
 
 }  // namespace legacy
 }  // namespace tcb
