@@ -436,31 +436,27 @@ tc_error_t DecImpl::decode(const uint8_t *data, size_t size, const tc_pixel_t **
     if (cudaMemcpyAsync(h_status, d_items + nctu, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return TC_ERR_INTERNAL;
     }   // v2 stream
-    // The picture is known to be good before it becomes a reference: a packet
-    // that fails here leaves the DPB, and the reconstruction that later packets
-    // build on, as they were.
-    if (!d2h(out, cur)) return TC_ERR_INTERNAL;
-    if (!legacy_stream && *h_status != 0) {   // an area gave up waiting
-        cudaMemsetAsync(d_items + rows * cols, 0, sizeof(int), st);
+    // DPB: slot 3 falls out and its buffer takes a copy of the reconstruction
+    // into slot 0 (another buffer when slot 3 is empty, taken here, while the
+    // kernels run).  Nothing moves before the picture is known to be good: a
+    // packet that fails from here on leaves the DPB, and the reconstruction
+    // that later packets build on, as they were.
+    const bool reuse = dpb_ok[TC_REF_FRAMES - 1] != 0;
+    const DevFrame nf = reuse ? dpb[TC_REF_FRAMES - 1] : take_frame();
+    auto undo = [&](tc_error_t e) {
+        if (!reuse && nf.y) spare.push_back(nf);
         if (dpb_ok[0]) copy_frame(cur, dpb[0]);
         else clear_frame(cur);
-        return TC_ERR_INTERNAL;
+        return e;
+    };
+    if (!nf.y) return undo(TC_ERR_MEMORY);
+    if (!d2h(out, cur)) return undo(TC_ERR_INTERNAL);
+    if (!legacy_stream && *h_status != 0) {   // an area gave up waiting
+        cudaMemsetAsync(d_items + rows * cols, 0, sizeof(int), st);
+        return undo(TC_ERR_INTERNAL);
     }
-    // DPB: slot 3 falls out and its buffer takes a copy of the
-    // reconstruction into slot 0 (another buffer when slot 3 is empty, taken
-    // before anything moves, so a failed allocation leaves the DPB as it
-    // was).  The copy is ordered before the next packet's kernels on the stream.
-    DevFrame nf;
-    if (dpb_ok[TC_REF_FRAMES - 1]) {
-        nf = dpb[TC_REF_FRAMES - 1];
-    } else {
-        nf = take_frame();
-        if (!nf.y) return TC_ERR_MEMORY;
-    }
-    if (!copy_frame(nf, cur)) {
-        if (!dpb_ok[TC_REF_FRAMES - 1]) spare.push_back(nf);
-        return TC_ERR_INTERNAL;
-    }
+    // (ordered before the next packet's kernels on the stream)
+    if (!copy_frame(nf, cur)) return undo(TC_ERR_INTERNAL);
     for (int i = TC_REF_FRAMES - 1; i > 0; --i) { dpb[i] = dpb[i - 1]; dpb_ok[i] = dpb_ok[i - 1]; dpb_poc[i] = dpb_poc[i - 1]; }
     dpb[0] = nf; dpb_ok[0] = 1; dpb_poc[0] = hdr.frame_num;
     const uint64_t t_rec = now_ns();
