@@ -456,8 +456,9 @@ def run_standalone_kernels(lib, peak, iters=8, frames=64):
 
 
 # ---------------------------------------------------------------- engine phase profile
-PHASES = ["refs/mvp", "ME", "MC", "resid jobs", "skip chk", "scan", "CfL", "replay", "decide(total)",
-          "write pass", "deblock+sao", "me0:int", "me0:subpel"]
+PHASES = {0: "refs/mvp", 1: "search+intra", 3: "inter scoring", 4: "skip chk", 5: "scan", 7: "coding",
+          8: "decide(total)", 9: "close gaps", 10: "deblock+sao", 11: "me0:int", 12: "me0:subpel"}
+LEAF_PHASES = [k for k in PHASES if k < 8]
 
 
 def run_phase_profile(streams, steps, ops_out=None):
@@ -482,7 +483,7 @@ def run_phase_profile(streams, steps, ops_out=None):
     S = streams
     clip = synth.workload("rects_lines", frames=12)
     batch = api.BatchEncoder(lib, [make_cfg(lib) for _ in range(S)])
-    cyc, ops = (ctypes.c_ulonglong * 64)(), (ctypes.c_ulonglong * 4)()
+    cyc, ops = (ctypes.c_ulonglong * 60)(), (ctypes.c_ulonglong * 4)()
     tot, steady = [0, 0, 0, 0], 0
     for t in range(steps):
         t0 = time.time()
@@ -497,22 +498,19 @@ def run_phase_profile(streams, steps, ops_out=None):
               f"int SAD px {ops[0] / 1e9:.3f} G, qpel SAD px {ops[1] / 1e9:.3f} G, "
               f"TU8 {ops[2] / 1e6:.2f} M, TU4 {ops[3] / 1e6:.2f} M")
         if t == steps - 1:
-            for i, n in enumerate(PHASES):
+            for i, n in PHASES.items():
                 print(f"   {n:14s} {cyc[i] / 1e6:10.1f} Mcyc  {100 * cyc[i] / max(1, enc):5.1f} %")
             # per quadtree depth: leaf decisions, their phases (share of the
             # encode) and group 0's search split
-            print("   depth  leaves/CTU  kcyc/leaf  " + "  ".join(f"{n[:8]:>8s}" for n in PHASES[:8])
+            print("   depth  leaves/CTU  kcyc/leaf  " + "  ".join(f"{PHASES[k][:8]:>8s}" for k in LEAF_PHASES)
                   + "   me:int  me:qpel")
             nctu = S * ((1920 + 63) // 64) * ((1080 + 63) // 64)
             for d in range(4):
                 n = cyc[48 + d]
-                tot_d = sum(cyc[16 + 8 * d + k] for k in range(8))
-                row = "  ".join(f"{100 * cyc[16 + 8 * d + k] / max(1, enc):7.1f}%" for k in range(8))
+                tot_d = sum(cyc[16 + 8 * d + k] for k in LEAF_PHASES)
+                row = "  ".join(f"{100 * cyc[16 + 8 * d + k] / max(1, enc):7.1f}%" for k in LEAF_PHASES)
                 print(f"   {d:5d}  {n / nctu:10.1f}  {tot_d / max(1, n) / 1e3:9.1f}  {row}  "
                       f"{100 * cyc[52 + 2 * d] / max(1, enc):6.1f}%  {100 * cyc[53 + 2 * d] / max(1, enc):6.1f}%")
-            print("   inside residual jobs (thread 0, all leaves): " + ", ".join(
-                f"{n} {100 * cyc[k] / max(1, enc):.1f}%" for k, n in
-                ((60, "setup+residual"), (61, "8x8 transform chain"), (62, "recon+sums"), (63, "intra fill"))))
         if t >= 4 and coded == S:          # steady GOP4-B steps (after the first anchor)
             steady += 1
             for i in range(4):

@@ -43,14 +43,11 @@ namespace tcb {
 // Optional per-phase cycle counters (build with -DTCB_PHASE_PROFILE); thread
 // 0 of each CTA accumulates clock64() deltas into tcb_phase_cycles[].
 #ifdef TCB_PHASE_PROFILE
-// Slots 0..15 as listed by the profiling reader; 16 + 8 * depth + k: leaf
-// phase k (0..7) of leaves at that quadtree depth; 48 + depth: leaf
-// decisions at that depth; 52 + 2 * depth + {0, 1}: integer stages and
-// quarter-pel refinement of group 0's searches at that depth; 60..63:
-// thread 0's time inside one 8x8 residual job (setup and residual,
-// transform chain, reconstruction and sums) and the intra prediction fill
-// of build_refs.
-constexpr int PHASE_SLOTS = 64;
+// Slots 0..14 as listed by the profiling reader (2 and 6 are not used);
+// 16 + 8 * depth + k: leaf phase k (0..7) of leaves at that quadtree depth;
+// 48 + depth: leaf decisions at that depth; 52 + 2 * depth + {0, 1}: integer
+// stages and quarter-pel refinement of group 0's searches at that depth.
+constexpr int PHASE_SLOTS = 60;
 __device__ unsigned long long tcb_phase_cycles[PHASE_SLOTS];
 #define PHASE_T0() long long _ph_t = clock64()
 #define PHASE(k) do { if (threadIdx.x == 0) { const long long _n = clock64(); \
@@ -59,9 +56,6 @@ __device__ unsigned long long tcb_phase_cycles[PHASE_SLOTS];
     atomicAdd(&tcb_phase_cycles[k], (unsigned long long)(_n - _ph_t)); \
     atomicAdd(&tcb_phase_cycles[16 + 8 * (d) + (k)], (unsigned long long)(_n - _ph_t)); _ph_t = _n; } } while (0)
 #define COUNT_D(d) do { if (threadIdx.x == 0) atomicAdd(&tcb_phase_cycles[48 + (d)], 1ull); } while (0)
-#define PROBE_T0() long long _pb_t = clock64()
-#define PROBE(k) do { if (threadIdx.x == 0) { const long long _n = clock64(); \
-    atomicAdd(&tcb_phase_cycles[k], (unsigned long long)(_n - _pb_t)); _pb_t = _n; } } while (0)
 // Inside a motion search, thread 0 of group 0 splits its time into the
 // integer stages (slot 11) and the quarter-pel refinement (slot 12).
 #define ME_T0() long long _me_t = clock64()
@@ -79,8 +73,6 @@ __device__ unsigned long long tcb_op_counts[4];
 #define PHASE(k) do {} while (0)
 #define PHASE_D(k, d) do {} while (0)
 #define COUNT_D(d) do {} while (0)
-#define PROBE_T0() do {} while (0)
-#define PROBE(k) do {} while (0)
 #define ME_T0() do {} while (0)
 #define ME_MARK(k) do {} while (0)
 #define OPCOUNT(k, v) do {} while (0)
@@ -2515,9 +2507,9 @@ extern "C" __attribute__((visibility("default"))) int tcb_debug_op_counts(unsign
     unsigned long long z[4] = {0};
     return cudaMemcpyToSymbol(tcb::tcb_op_counts, z, sizeof(z)) == cudaSuccess ? 0 : -1;
 }
-extern "C" __attribute__((visibility("default"))) int tcb_debug_phase_cycles(unsigned long long *out64) {
+extern "C" __attribute__((visibility("default"))) int tcb_debug_phase_cycles(unsigned long long *out60) {
     cudaDeviceSynchronize();
-    if (cudaMemcpyFromSymbol(out64, tcb::tcb_phase_cycles, tcb::PHASE_SLOTS * sizeof(unsigned long long)) != cudaSuccess)
+    if (cudaMemcpyFromSymbol(out60, tcb::tcb_phase_cycles, tcb::PHASE_SLOTS * sizeof(unsigned long long)) != cudaSuccess)
         return -1;
     unsigned long long z[tcb::PHASE_SLOTS] = {0};
     return cudaMemcpyToSymbol(tcb::tcb_phase_cycles, z, sizeof(z)) == cudaSuccess ? 0 : -1;

@@ -12,8 +12,8 @@
 //    Ch and the 8 rows of Cl, so one MMA gives both partial sums Sh and Sl.
 //  * B operands are integers exact in f16 (|v| <= 2048): residuals
 //    (|r| <= 255), first-pass results (|t| <= 722), and dequantised levels
-//    and row-inverse results as f16(v) plus the remainder v - f16(v) (0 or
-//    +-1), against [C | C] with k = 16.
+//    and row-inverse results as f16(v) plus the remainder v - f16(v) (at most
+//    1 here, where |v| <= 3571), against [C | C] with k = 16.
 //  * Every product and sum is an integer below 2^24, so f32 holds it exactly:
 //    residuals of 8-bit pictures have norm <= 2040, a non-zero level
 //    dequantises to at most 1.75 |c| (q eff + eff / 6 with q eff <= |c| +
@@ -26,7 +26,7 @@
 // Everything up to the reconstruction stays in f32: the FMA pipe issues one
 // instruction a cycle where the integer ALU issues one every two, and the
 // integer form of the same steps was bound by the latter (142 cycles a
-// scheduler per area and TU size; now about half).
+// scheduler per area and TU size; now 125).
 //
 // Data layout: lane l owns row l >> 2, columns 2 (l & 3) and 2 (l & 3) + 1 of
 // the 8x8 area.  That is the C fragment of an m16n8 MMA (rows 0..7: the Ch
@@ -171,7 +171,9 @@ __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
     const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
-// B operands of two integers within +-4095: f16 values and remainders.
+// B operands of two integers below 2^14: f16 values and remainders, both exact
+// (remainders of at most 1 within +-4095, of at most 4 beyond: the decoder passes
+// up to 10,818, the block path up to 2^14).
 __device__ __forceinline__ void split_h2(float a, float b, uint32_t &hi, uint32_t &lo) {
     const __half2 h = __floats2half2_rn(a, b);
     hi = *reinterpret_cast<const uint32_t *>(&h);
