@@ -293,7 +293,7 @@ __device__ __forceinline__ void sao_count(int *col, int r, int o) {
     atomicAdd(&col[sao_row_of(r) * 32], 65536 + (int)SAO_BIAS + o - r);
 }
 
-// Bound: the integer ALU (about 2,300 instructions of a warp per CTU, a third
+// Bound: the integer ALU (2,210 instructions of a warp per CTU, a third
 // of them the adds and addresses of the statistics).  A column per thread
 // instead of per lane took four times the zeroing and row totals, and the
 // offset on 16-bit pairs twice the instructions of whole words: 3,060 per CTU.

@@ -43,7 +43,8 @@ struct McJobs {                      // passed by value as the kernel parameter
 // Threads per CTA are a template parameter (64, 128 or 256; the autotuner
 // times each per frame size, 256 without tuning); the register budget is
 // cut for 1,024 resident threads per SM (64 registers, a few spilled): the
-// six-tap path is bound by latency, and 16 frames of 1280x720 with random
+// six-tap path waits for instructions (the copies per phase and the edge path
+// outgrow the instruction cache) and for loads, and 16 frames of 1280x720 with random
 // vectors take 58.5 us so, 61.1 with 768 threads and 80 registers.
 constexpr int MC_DEFAULT_THREADS = 256;
 
